@@ -123,9 +123,10 @@ def tolerance(case):
     return {"rel": 1e-2, "max": 0.1}
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """The case's tensors, from the seed alone."""
     q, k = _lens(case)
-    H, Hkv, hid, form = case["heads"], case["kv_heads"], case["hidden"], case["form"]
+    H, Hkv, hid = case["heads"], case["kv_heads"], case["hidden"]
     dev = torch.device("cuda:0")
     g = torch.Generator(device=dev)
     g.manual_seed(int(seed))
@@ -133,13 +134,9 @@ def prepare(case, seed):
     def randn(*shape, std=1.0):
         return (torch.randn(*shape, generator=g, device=dev, dtype=torch.bfloat16) * std).contiguous()
 
-    meta = build_row_desc(q, seqlens_k=k)
     tq, tk = sum(q), sum(k)
-    cfg = choose_launch_config(meta, hid, 1)
-    W = randn(H * D, hid, std=(H * D) ** -0.5)
-    s = {"form": form, "meta": meta, "q": randn(tq, H, D)}
-    kw = {}
-    if form == "paged":
+    t = {"W_o": randn(H * D, hid, std=(H * D) ** -0.5), "q": randn(tq, H, D)}
+    if case["form"] == "paged":
         need = [-(-n // PAGE) for n in k]
         pages = sum(need) + 8
         perm = np.random.RandomState(int(seed) % (1 << 31)).permutation(pages).astype(np.int32)
@@ -148,27 +145,98 @@ def prepare(case, seed):
         for i, n in enumerate(need):
             table[i, :n] = perm[at:at + n]
             at += n
-        s["k"], s["v"] = randn(pages * PAGE, Hkv, D), randn(pages * PAGE, Hkv, D)
-        s["page_table"] = torch.from_numpy(table).to(dev)
-        s["cache_seqlens"] = torch.tensor(k, dtype=torch.int32, device=dev)
-        kw = dict(paged=True, max_num_pages=pages, max_num_pages_per_seq=table.shape[1])
+        t["k"], t["v"] = randn(pages * PAGE, Hkv, D), randn(pages * PAGE, Hkv, D)
+        t["pages"] = pages
+        t["page_table"] = torch.from_numpy(table).to(dev)
+        t["cache_seqlens"] = torch.tensor(k, dtype=torch.int32, device=dev)
     else:
-        s["k"], s["v"] = randn(tk, Hkv, D), randn(tk, Hkv, D)
+        t["k"], t["v"] = randn(tk, Hkv, D), randn(tk, Hkv, D)
+    if case["form"] == "step":
+        t["residual"] = randn(tq, hid)
+        t["weight"] = (1.0 + 0.1 * randn(hid)).contiguous()
+    return t
+
+
+def prepare(case, seed):
+    q, k = _lens(case)
+    H, Hkv, hid, form = case["heads"], case["kv_heads"], case["hidden"], case["form"]
+    dev = torch.device("cuda:0")
+    meta = build_row_desc(q, seqlens_k=k)
+    cfg = choose_launch_config(meta, hid, 1)
+    s = {"form": form, "meta": meta, **_inputs(case, seed)}
+    kw = {}
+    if form == "paged":
+        kw = dict(paged=True, max_num_pages=s["pages"],
+                  max_num_pages_per_seq=s["page_table"].shape[1])
     ws = FusedFaOprojArWorkspace.create(
         None, meta.num_row_tiles, hid, H, D, super_group_n_tiles=cfg.sg, q_per_kv=H // Hkv,
-        max_num_batch=meta.num_batch, max_tot_k=tk, device=dev, **kw)
+        max_num_batch=meta.num_batch, max_tot_k=sum(k), device=dev, **kw)
     ws.compile(w_fa=cfg.w_fa, w_oproj=cfg.w_oproj, w_ar=cfg.w_ar)
-    s["ws"], s["W_o"] = ws, W
+    s["ws"] = ws
     s["cu_q"] = torch.from_numpy(meta.cu_seqlens_q)
     s["cu_k"] = torch.from_numpy(meta.cu_seqlens_k)
     if form != "workspace":
-        s["layer"] = FusedPrefillLayer(ws, W)
+        s["layer"] = FusedPrefillLayer(ws, s["W_o"])
     if form == "step":
         s["rope"] = rope_meta(meta.cu_seqlens_q, meta.cu_seqlens_k, dev)
         s["inv_freq"] = default_inv_freq(10000.0, dev)
-        s["residual"] = randn(tq, hid)
-        s["weight"] = (1.0 + 0.1 * randn(hid)).contiguous()
     return s
+
+
+def _rotated(x, pos):
+    """Rotate-half RoPE of ``x [n, heads, 128]`` (float64) at positions ``pos [n]``."""
+    freq = 10000.0 ** (-torch.arange(0, D, 2, dtype=torch.float64, device=x.device) / D)
+    ang = pos.double()[:, None] * freq
+    c, s = ang.cos()[:, None], ang.sin()[:, None]
+    a, b = x[..., :D // 2], x[..., D // 2:]
+    return torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+
+
+def exact(case, seed):
+    """What ``run`` returns, in float64 from the definition."""
+    lens_q, lens_k = _lens(case)
+    H, Hkv, hid, form = case["heads"], case["kv_heads"], case["hidden"], case["form"]
+    if work(case)["flops"] > 1.5e12:          # minutes in float64
+        return None
+    t = _inputs(case, seed)
+    dev = t["q"].device
+    q, k, v = t["q"].double(), t["k"].double(), t["v"].double()
+    W = t["W_o"].double()
+    tiles = sum(-(-n // 128) for n in lens_q)
+    out = torch.zeros(tiles * 128, -(-hid // 128) * 128, dtype=torch.float64, device=dev)
+    packed = torch.empty(sum(lens_q), hid, dtype=torch.float64, device=dev)
+    q0 = k0 = row = 0
+    for i, (lq, lk) in enumerate(zip(lens_q, lens_k)):
+        if form == "paged":
+            idx = (t["page_table"][i].long()[:, None] * PAGE
+                   + torch.arange(PAGE, device=dev)).reshape(-1)[:lk]
+        else:
+            idx = torch.arange(k0, k0 + lk, device=dev)
+        if form == "step":
+            pos = torch.arange(lk - lq, lk, device=dev)
+            q[q0:q0 + lq] = _rotated(q[q0:q0 + lq], pos)
+            k[idx[lk - lq:]] = _rotated(k[idx[lk - lq:]], pos)
+        ks, vs = k[idx], v[idx]
+        attn = torch.empty(lq, H, D, dtype=torch.float64, device=dev)
+        for h in range(H):
+            for a in range(0, lq, 1024):
+                e = min(lq, a + 1024)
+                n = lk - lq + e                # keys the last of these rows may see
+                sc = q[q0 + a:q0 + e, h] @ ks[:n, h * Hkv // H].T * D ** -0.5
+                seen = torch.arange(lk - lq + a, n, device=dev)[:, None]
+                sc.masked_fill_(torch.arange(n, device=dev) > seen, -math.inf)
+                attn[a:e, h] = torch.softmax(sc, dim=-1) @ vs[:n, h * Hkv // H]
+        packed[q0:q0 + lq] = attn.view(lq, H * D) @ W
+        out[row:row + lq, :hid] = packed[q0:q0 + lq]
+        q0, k0, row = q0 + lq, k0 + lk, row + -(-lq // 128) * 128
+    if form == "workspace":
+        return packed
+    out = out.view(tiles, 128, -1, 128)
+    if form != "step":
+        return out
+    res = t["residual"].double() + packed
+    normed = res * torch.rsqrt(res.square().mean(-1, keepdim=True) + 1e-6) * t["weight"].double()
+    return {"attn": out, "normed": normed, "residual": res, "q": q, "k": k}
 
 
 def run(s):
