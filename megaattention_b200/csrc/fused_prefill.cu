@@ -17,11 +17,11 @@
 //
 // Warp roles (12 warps, 384 threads):
 //   warp 0 (lane 0)  TMA producer: Q tiles, the K/V ring, O_proj stages
-//   warp 1 (lane 0)  MMA issuer of attention tile 0 and of every O_proj task; warp 1 also
-//                    allocates and frees TMEM
+//   warp 1           MMA issuer of both attention tiles and of every O_proj task; allocates
+//                    and frees TMEM
 //   warp 2 (lane 0)  scheduler: claims tasks, fills one of two descriptor slots, publishes
 //                    completions (runs one task ahead of the workers)
-//   warp 3 (lane 0)  MMA issuer of attention tile 1
+//   warp 3 (lane 0)  stores the attention output tiles
 //   warps 4-7, 8-11  two compute warpgroups: online softmax (one thread per row), both
 //                    epilogues, AllReduce slots
 // An FA task is two q heads of one row tile whenever the rank has two: the two compute
@@ -62,17 +62,18 @@ struct Bars {
   uint64_t q_full[2];       // TMA: Q tile i landed
   uint64_t q_empty[2];      // MMA: last Q K^T of tile i done + epilogue: staging released (count 2)
   uint64_t kv_full[kKvSlots];
-  uint64_t kv_empty[kKvSlots];   // shared K/V stages: both MMA issuers release a slot (count 2);
-                                 // separate stages: the one issuer that reads it (count 1)
+  uint64_t kv_empty[kKvSlots];   // MMA: the last product that reads the slot completed (count 1)
   uint64_t s_full[2];       // MMA: S_i ready
+  uint64_t p_part[2];       // softmax warps: key columns 0-95 of P_i written (count 4)
   uint64_t p_full[2];       // softmax warps: P_i written (count 4, one arrival per warp)
+  uint64_t o_staged[2];     // epilogue warps: O_i staged in shared memory (count 4)
   uint64_t o_done[2];       // MMA: last P V of the task for tile i completed
   uint64_t o_free[2];       // epilogue warps: O_i read out (count 4)
   uint64_t op_full[4];
   uint64_t op_empty[4];
   uint64_t acc_full[2];     // MMA: O_proj accumulator half h complete
   uint64_t acc_free[2];     // epilogue warps: half h read out (count 8)
-  uint64_t drain[2];        // abort path only: an issuer's outstanding MMAs have retired
+  uint64_t drain;           // abort path only: the issuer's outstanding MMAs have retired
 };
 
 struct Env {
@@ -90,23 +91,23 @@ __device__ __noinline__ void report(const Env& e, uint32_t code, uint32_t site, 
   *e.abort_flag = 1;
 }
 
-// Bounded mbarrier wait.  Returns false once the wait limit passed or the CTA aborted.
+// Bounded mbarrier wait.  Returns false once the wait limit passed or the CTA aborted.  The
+// first look is a test_wait: on a phase that is complete it takes 45 cycles, a try_wait 120,
+// and these waits stand on the pipelines' chains.  What follows is short on purpose (a loop
+// of 32 quick tries before it cost the attention stage 3 %), and inline: as a call it made
+// every value that is live across a wait go through memory.
+constexpr uint32_t kWaitSleepNs = 20000;
 __device__ __forceinline__ bool wait_bar(const Env& e, uint32_t bar, uint32_t parity,
                                          uint32_t site) {
-  if (mbar_try_wait(bar, parity)) return true;
-  if (*e.abort_flag) return false;
-#pragma unroll 1
-  for (int i = 0; i < 32; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_test_wait(bar, parity)) return true;
+  if (mbar_try_wait_for(bar, parity, kWaitSleepNs)) return true;
   const uint64_t t0 = globaltimer_ns();
-  uint32_t it = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++it & 31u) == 0) {
-      if (*e.abort_flag) return false;
-      if (globaltimer_ns() - t0 > e.p->wait_limit_ns) {
-        report(e, ST_TIMEOUT_MBAR, site, parity);
-        return false;
-      }
+#pragma unroll 1
+  while (!mbar_try_wait_for(bar, parity, kWaitSleepNs)) {
+    if (*e.abort_flag) return false;
+    if (globaltimer_ns() - t0 > e.p->wait_limit_ns) {
+      report(e, ST_TIMEOUT_MBAR, site, parity);
+      return false;
     }
   }
   return true;
@@ -391,12 +392,14 @@ __device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t sm_q, uint32_
            kIdescQK, kk > 0);
   }
 }
-// O (+)= P V : P is bf16 in TMEM (8 columns per 16 kv), V tile is [kv][d] in two d panels.
+// O (+)= P V over the 16-key steps [k0, k1): P is bf16 in TMEM (8 columns per 16 kv), V tile
+// is [kv][d] in two d panels.
+template <int k0, int k1>
 __device__ __forceinline__ void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint32_t sm_v,
                                          bool acc) {
   const uint32_t v16 = sm_v >> 4;
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
+  for (int kk = k0; kk < k1; ++kk)
     mma_ts(tmem_o, tmem_p + kk * 8, smem_desc_at(kDescVmn, v16 + kk * 128), kIdescPV,
            (acc || kk > 0) ? 1u : 0u);
 }
@@ -510,9 +513,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
   __shared__ uint32_t s_tmem;
   __shared__ __align__(128) int s_abort_line[32];
   __shared__ __align__(128) int s_desc[2][T_WORDS];
-  __shared__ __align__(128) int s_pipe_line[32];
   int& s_abort = s_abort_line[0];
-  int& s_pipe_turn = s_pipe_line[0];   // serialises the two issuers' MMA batches (scheduling only)
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -522,7 +523,6 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 
   if (tid == 0) {
     s_abort = 0;
-    s_pipe_turn = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars.task_full[i]), 1);
       mbar_init(smem_u32(&bars.task_empty[i]), 11);
@@ -530,7 +530,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       mbar_init(smem_u32(&bars.q_full[i]), 1);
       mbar_init(smem_u32(&bars.q_empty[i]), 2);
       mbar_init(smem_u32(&bars.s_full[i]), 1);
+      mbar_init(smem_u32(&bars.p_part[i]), 4);
       mbar_init(smem_u32(&bars.p_full[i]), 4);
+      mbar_init(smem_u32(&bars.o_staged[i]), 4);
       mbar_init(smem_u32(&bars.o_done[i]), 1);
       mbar_init(smem_u32(&bars.o_free[i]), 4);
       mbar_init(smem_u32(&bars.acc_full[i]), 1);
@@ -538,14 +540,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     }
     for (int i = 0; i < kKvSlots; ++i) {
       mbar_init(smem_u32(&bars.kv_full[i]), 1);
-      mbar_init(smem_u32(&bars.kv_empty[i]), p.sep ? 1 : 2);   // issuers that consume a slot
+      mbar_init(smem_u32(&bars.kv_empty[i]), 1);
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(smem_u32(&bars.op_full[i]), 1);
       mbar_init(smem_u32(&bars.op_empty[i]), 1);
     }
-    mbar_init(smem_u32(&bars.drain[0]), 1);
-    mbar_init(smem_u32(&bars.drain[1]), 1);
+    mbar_init(smem_u32(&bars.drain), 1);
     fence_mbar_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
@@ -562,8 +563,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 
   // Every role walks the two descriptor slots in turn.  A role arrives on task_empty[k]
   // when its part of the task in slot k is finished; the scheduler publishes the task's
-  // completion and refills the slot once all eleven arrivals are in (producer, two MMA
-  // issuers, eight compute warps), so the scheduler runs
+  // completion and refills the slot once all eleven arrivals are in (producer, MMA issuer,
+  // attention store, eight compute warps), so the scheduler runs
   // one task ahead of the workers.  Attention tiles and O_proj tiles overlay the same
   // shared memory and TMEM: a role that goes from one kind to the other first waits for
   // the previous task to finish completely (same-kind neighbours overlap freely).
@@ -788,96 +789,112 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         mbar_arrive(smem_u32(&bars.loads_done[slot_k]));
         MA_TASK_DONE(mode)
       }
-    } else if ((warp == 1 || warp == 3) && lane == 0) {
-      // ============================================= MMA issuers: warp 1 -> attention tile 0
-      // and every O_proj task, warp 3 -> attention tile 1.  Both follow the K/V ring so a
-      // slot is released only when both tiles are done with it.
-      const int mi = (warp == 1) ? 0 : 1;
+    } else if (warp == 1) {
+      // ============================================= MMA issuer of both attention tiles and of
+      // every O_proj task.  The warp stays converged: every lane waits, one elected lane
+      // issues (see elect_one).
       uint32_t kv_slot = 0, kv_ph = 0, opc = 0;
-      uint32_t q_par = 0, p_par = 0, o_uses = 0, acc_uses[2] = {0, 0};
-      const uint32_t t_s = tmem + kTmemS + mi * 128, t_o = tmem + kTmemO + mi * 128;
-      const uint32_t sm_q = smem0 + kSmQ + mi * kTile;
-      // One tile's batch (P V, then the next Q K^T) is issued as a unit: when both tiles
-      // become ready together the second waits for the first, which staggers the two
-      // softmax warpgroups so that one tile's MMAs run under the other tile's softmax.
-      // The lock only shapes the schedule; giving up on it is harmless.
-      auto pipe_lock = [&]() {
-        for (int it = 0; it < (1 << 16); ++it)
-          if (atomicCAS(&s_pipe_turn, 0, 1) == 0) return;
-      };
-      auto pipe_unlock = [&]() { atomicExch(&s_pipe_turn, 0); };
+      uint32_t q_par[2] = {0, 0}, p_par[2] = {0, 0}, o_uses[2] = {0, 0}, acc_uses[2] = {0, 0};
       while (true) {
         MA_NEXT_TASK(d, mode)
         MA_DRAIN_IF_SWITCH(mode)
         if (mode == MODE_FA) {
+          // A tile's chain softmax -> P V -> next Q K^T is what bounds the loop: the V tile
+          // and the next K tile are looked at before P is waited for, and P V starts on the
+          // first three quarters of P.  The tiles take turns, which keeps them half a period
+          // apart: one tile's MMAs run under the other's softmax.  (Before: an issuing warp
+          // per tile and a lock between the two.  With issue at 56 cycles per MMA and 250 for
+          // the lock, a two-tile key block took 4000 cycles.  Attention stage, one box:
+          // 12 short turns on cached prompts 104.5 -> 95.6 us, six ragged prompts of 13400
+          // tokens 150 -> 137.6 us; with a 16384-token prompt the whole launch 631 -> 601 us.)
           const int nblk = d[TF_NBLK], nt = d[TF_NT];
-          const bool act = mi < nt;
-          // Shared K/V stages: both issuers follow every slot of the ring.  Separate stages
-          // (p.sep): a key block is nt K slots then nt V slots, issuer mi uses the mi-th of
-          // each group and leaves the others alone (an idle issuer only keeps count).
+          // Shared K/V stages: one slot per operand and key block.  Separate stages (p.sep):
+          // nt slots, the i-th for tile i.
           const bool sep = p.sep != 0;
-          const bool walk = act || !sep;
-          auto my_slot = [&](uint32_t& slot, uint32_t& ph) {
-            uint32_t s = kv_slot + (sep ? static_cast<uint32_t>(mi) : 0u), h = kv_ph;
-            if (s >= static_cast<uint32_t>(kKvSlots)) { s -= kKvSlots; h ^= 1u; }
-            slot = s; ph = h;
-            kv_slot += sep ? static_cast<uint32_t>(nt) : 1u;
+          const int per = sep ? nt : 1;
+          struct SlotAt { uint32_t slot, ph; };
+          auto take = [&]() {                       // the next `per` slots of the ring
+            const SlotAt r{kv_slot, kv_ph};
+            kv_slot += static_cast<uint32_t>(per);
             if (kv_slot >= static_cast<uint32_t>(kKvSlots)) { kv_slot -= kKvSlots; kv_ph ^= 1u; }
+            return r;
           };
-          if (act) {
-            wait_bar(env, smem_u32(&bars.q_full[mi]), q_par, 0x20 + mi);
-            q_par ^= 1u;
-          }
-          uint32_t slot_kk, ph_kk;
-          my_slot(slot_kk, ph_kk);
-          if (walk) wait_bar(env, smem_u32(&bars.kv_full[slot_kk]), ph_kk, 0x30 + slot_kk);
-          if (act) {
+          auto at = [&](SlotAt r, int i) {          // tile i's slot among them
+            if (sep && i) {
+              if (++r.slot == static_cast<uint32_t>(kKvSlots)) { r.slot = 0; r.ph ^= 1u; }
+            }
+            return r;
+          };
+          auto wait_slots = [&](SlotAt r, uint32_t site) {
+            for (int i = 0; i < per; ++i) {
+              const SlotAt x = at(r, i);
+              wait_bar(env, smem_u32(&bars.kv_full[x.slot]), x.ph, site + x.slot);
+            }
+          };
+          SlotAt k = take();
+          for (int i = 0; i < nt; ++i) {
+            wait_bar(env, smem_u32(&bars.q_full[i]), q_par[i], 0x20 + i);
+            q_par[i] ^= 1u;
+            if (i == 0) wait_slots(k, 0x30);
             tc_fence_after();
-            pipe_lock();
-            issue_qk(t_s, sm_q, smem0 + kSmKV + slot_kk * kTile);
-            tc_commit(smem_u32(&bars.s_full[mi]));
-            pipe_unlock();
-            if (nblk == 1) tc_commit(smem_u32(&bars.q_empty[mi]));
+            const uint32_t ks = at(k, i).slot;
+            if (elect_one()) {
+              issue_qk(tmem + kTmemS + i * 128, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+              tc_commit(smem_u32(&bars.s_full[i]));
+              if (sep || i == nt - 1) tc_commit(smem_u32(&bars.kv_empty[ks]));
+              if (nblk == 1) tc_commit(smem_u32(&bars.q_empty[i]));
+            }
+            __syncwarp();
           }
-          if (walk) tc_commit(smem_u32(&bars.kv_empty[slot_kk]));
           for (int jj = 0; jj < nblk; ++jj) {
-            uint32_t slot_v, ph_v;
-            my_slot(slot_v, ph_v);
-            if (walk) wait_bar(env, smem_u32(&bars.kv_full[slot_v]), ph_v, 0x40 + slot_v);
-            if (act) {
-              if (jj == 0) {   // the previous task's epilogue must have read O out
-                wait_bar(env, smem_u32(&bars.o_free[mi]), (o_uses & 1u) ^ 1u, 0x68 + mi);
-                ++o_uses;
-              }
-              wait_bar(env, smem_u32(&bars.p_full[mi]), p_par, 0x60 + mi);
-              p_par ^= 1u;
-              tc_fence_after();
-            }
             const bool has_next = (jj + 1 < nblk);
-            if (has_next) {          // K of the next block: prefetched long ago
-              my_slot(slot_kk, ph_kk);
-              if (walk) wait_bar(env, smem_u32(&bars.kv_full[slot_kk]), ph_kk, 0x50 + slot_kk);
-            }
-            if (act) {
-              pipe_lock();
-              issue_pv(t_o, t_s, smem0 + kSmKV + slot_v * kTile, jj > 0);
-              tc_commit(smem_u32(&bars.kv_empty[slot_v]));
-              if (has_next) {
-                issue_qk(t_s, sm_q, smem0 + kSmKV + slot_kk * kTile);
-                tc_commit(smem_u32(&bars.s_full[mi]));
-                pipe_unlock();
-                tc_commit(smem_u32(&bars.kv_empty[slot_kk]));
-                if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[mi]));
-              } else {
-                tc_commit(smem_u32(&bars.o_done[mi]));
-                pipe_unlock();
+            const SlotAt v = take();
+            if (has_next) k = take();
+            for (int i = 0; i < nt; ++i) {
+              const uint32_t t_s = tmem + kTmemS + i * 128, t_o = tmem + kTmemO + i * 128;
+              const uint32_t vs = at(v, i).slot, ks = at(k, i).slot;
+              const uint32_t sm_v = smem0 + kSmKV + vs * kTile;
+              const bool last_use = sep || i == nt - 1;
+              // The operands are nearly always there: one look at all their barriers, a lane
+              // each, and a wait one by one only if one of them is not.
+              if (sep || i == 0 || jj == 0) {
+                uint32_t bar = smem_u32(&bars.kv_full[vs]), par = at(v, i).ph;
+                if (lane == 1 && has_next) { bar = smem_u32(&bars.kv_full[ks]); par = at(k, i).ph; }
+                if (lane == 2 && jj == 0) { bar = smem_u32(&bars.o_free[i]); par = (o_uses[i] & 1u) ^ 1u; }
+                if (!__all_sync(0xffffffffu, mbar_test_wait(bar, par))) {
+                  wait_bar(env, smem_u32(&bars.kv_full[vs]), at(v, i).ph, 0x40 + vs);
+                  if (has_next) wait_bar(env, smem_u32(&bars.kv_full[ks]), at(k, i).ph, 0x50 + ks);
+                  // (the previous task's epilogue must have read O out)
+                  if (jj == 0) wait_bar(env, smem_u32(&bars.o_free[i]), (o_uses[i] & 1u) ^ 1u, 0x68 + i);
+                }
+                if (jj == 0) ++o_uses[i];
               }
-            } else if (walk) {
-              tc_commit(smem_u32(&bars.kv_empty[slot_v]));
-              if (has_next) tc_commit(smem_u32(&bars.kv_empty[slot_kk]));
+              wait_bar(env, smem_u32(&bars.p_part[i]), p_par[i], 0x58 + i);
+              tc_fence_after();
+              if (elect_one()) issue_pv<0, 6>(t_o, t_s, sm_v, jj > 0);
+              __syncwarp();
+              wait_bar(env, smem_u32(&bars.p_full[i]), p_par[i], 0x60 + i);
+              p_par[i] ^= 1u;
+              tc_fence_after();
+              if (elect_one()) {
+                issue_pv<6, 8>(t_o, t_s, sm_v, true);
+                if (has_next) {
+                  issue_qk(t_s, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+                  tc_commit(smem_u32(&bars.s_full[i]));
+                  if (last_use) {
+                    tc_commit(smem_u32(&bars.kv_empty[vs]));
+                    tc_commit(smem_u32(&bars.kv_empty[ks]));
+                  }
+                  if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[i]));
+                } else {
+                  tc_commit(smem_u32(&bars.o_done[i]));
+                  if (last_use) tc_commit(smem_u32(&bars.kv_empty[vs]));
+                }
+              }
+              __syncwarp();
             }
           }
-        } else if (mode == MODE_OPROJ && mi == 0) {
+        } else if (mode == MODE_OPROJ) {
           const int vnt = d[TO_VNT];
           const int nkc = p.K_local >> 6;
           for (int h = 0; h * 2 < vnt; ++h) {
@@ -892,15 +909,45 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
               tc_fence_after();
               const uint32_t a16 = (smem0 + st * kOpStage) >> 4;
               const uint32_t w16 = a16 + (kPanel >> 4);
+              if (elect_one()) {
 #pragma unroll
-              for (int kk = 0; kk < 4; ++kk)
-                mma_ss(tmem + h * 256, smem_desc_at(kDescK, a16 + kk * 2),
-                       smem_desc_at(kDescWmn, w16 + kk * 128), idesc,
-                       (kc > 0 || kk > 0) ? 1u : 0u);
-              tc_commit(smem_u32(&bars.op_empty[st]));
+                for (int kk = 0; kk < 4; ++kk)
+                  mma_ss(tmem + h * 256, smem_desc_at(kDescK, a16 + kk * 2),
+                         smem_desc_at(kDescWmn, w16 + kk * 128), idesc,
+                         (kc > 0 || kk > 0) ? 1u : 0u);
+                tc_commit(smem_u32(&bars.op_empty[st]));
+                if (kc + 1 == nkc) tc_commit(smem_u32(&bars.acc_full[h]));
+              }
+              __syncwarp();
             }
-            tc_commit(smem_u32(&bars.acc_full[h]));
           }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars.task_empty[slot_k]));
+        ++n_arrived[slot_k];
+        prev_mode = mode; prev_k = slot_k; slot_k ^= 1;
+      }
+    } else if (warp == 3 && lane == 0) {
+      // ==================================== attention output stores: O_scratch[ft, :, head, :]
+      // (a warp of their own, so that no softmax warp waits for a store to complete)
+      uint32_t st_par[2] = {0, 0};
+      while (true) {
+        MA_NEXT_TASK(d, mode)
+        if (mode == MODE_FA) {
+          const int ft = d[T_FT], head0 = d[TF_HEAD0], nt = d[TF_NT];
+          for (int i = 0; i < nt; ++i) {
+            if (!wait_bar(env, smem_u32(&bars.o_staged[i]), st_par[i], 0x88 + i)) break;
+            st_par[i] ^= 1u;
+            const uint32_t stg = smem0 + kSmQ + i * kTile;
+            tma_store_2d(&tmO, stg, (head0 + i) * 128, ft * 128);
+            tma_store_2d(&tmO, stg + kPanel, (head0 + i) * 128 + 64, ft * 128);
+            tma_store_commit();
+            tma_store_wait_read();
+            mbar_arrive(smem_u32(&bars.q_empty[i]));     // the producer may refill this Q buffer
+          }
+          tma_store_wait_all();
+          fence_proxy_async_all();     // O_scratch is read back by TMA loads of other CTAs
+          __threadfence();
         }
         MA_TASK_DONE(mode)
       }
@@ -917,12 +964,12 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       MA_NEXT_TASK(d, mode)
       if (mode == MODE_FA && wg < d[TF_NT]) {
         // -------------------------------------------- softmax + epilogue of tile `wg`
-        const int ft = d[T_FT], head = d[TF_HEAD0] + wg, valid_m = d[TF_VALID];
+        const int valid_m = d[TF_VALID];
         const int k_len = d[TF_KLEN], offset = d[TF_OFFSET], nblk = d[TF_NBLK], mb = d[TF_MB];
         const uint32_t t_s = tmem + kTmemS + wg * 128 + lane_base;
         const uint32_t t_o = tmem + kTmemO + wg * 128 + lane_base;
         const uint32_t bar_s = smem_u32(&bars.s_full[wg]);
-        const uint32_t bar_p = smem_u32(&bars.p_full[wg]);
+        const uint32_t bar_pp = smem_u32(&bars.p_part[wg]), bar_p = smem_u32(&bars.p_full[wg]);
         const float sl2 = p.scale_log2;
         // last kv position this row may see (bottom-right causal, clipped to k_len)
         const int lim_abs = min(mb * 128 + row + offset, k_len - 1);
@@ -946,119 +993,75 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
               for (int kx = 0; kx < 32; ++kx)
                 if (c * 32 + kx > lim) s[c][kx] = 0xff800000u;   // -inf
           }
-          // Fast path (every block after the first that needs no mask): the exponentials do
-          // not wait for this block's row maximum.  They are taken against the reference
-          // maximum as it stands while the block maximum is computed alongside; only if
-          // some row of the warp turns out to need a new reference (growth beyond 2^8,
-          // rare after the first block) the scores are read again from TMEM, where P has
-          // not been stored over them yet, and the block goes down the ordinary path.
-          // Scale-and-subtract and the row sums work on packed pairs (fma / add on two
-          // floats per instruction): the loop is short of issue slots, not of pipes.
-          bool done = false;
-          if (jj > 0 && !need_mask) {
-            const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref * sl2;
-            const uint64_t sl2x2 = pack_f32x2(sl2, sl2), negm2 = pack_f32x2(neg_m, neg_m);
-            uint64_t sum2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t pk[16];
+          for (int kx = 0; kx < 32; kx += 2)
 #pragma unroll
-              for (int kx = 0; kx < 16; ++kx) {
-                const float x0 = __uint_as_float(s[c][2 * kx]), x1 = __uint_as_float(s[c][2 * kx + 1]);
-                mx[kx & 3] = fmax3(mx[kx & 3], x0, x1);
-                const uint64_t a2 = fma_f32x2(pack_f32x2(x0, x1), sl2x2, negm2);
-                float a0, a1;
-                unpack_f32x2(a2, a0, a1);
-                const float e0 = ex2(a0), e1 = ex2(a1);
-                sum2[kx & 1] = add_f32x2(sum2[kx & 1], pack_f32x2(e0, e1));
-                pk[kx] = pack_bf16x2(e0, e1);
-              }
-              if ((c & 1) == 0) {
-#pragma unroll
-                for (int kx = 0; kx < 16; ++kx) s[c][kx] = pk[kx];
-              } else {
-#pragma unroll
-                for (int kx = 0; kx < 16; ++kx) s[c - 1][16 + kx] = pk[kx];
-              }
-            }
-            float s0, s1, s2, s3;
-            unpack_f32x2(sum2[0], s0, s1);
-            unpack_f32x2(sum2[1], s2, s3);
-            const float l_blk = (s0 + s1) + (s2 + s3);
-            const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const bool grow = (m_blk > -INFINITY) &&
-                              ((m_ref == -INFINITY) || ((m_blk - m_ref) * sl2 > kRescaleThreshold));
-            if (!__any_sync(0xffffffffu, grow)) {
-              tmem_st32(t_s, s[0]);
-              tmem_st32(t_s + 32, s[2]);
-              l_run += l_blk;
-              done = true;
-            } else {
-#pragma unroll
-              for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, s[c]);
-              tc_wait_ld();
-            }
-          }
-          if (!done) {
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int kx = 0; kx < 32; kx += 2)
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-                mx[c] = fmax3(mx[c], __uint_as_float(s[c][kx]), __uint_as_float(s[c][kx + 1]));
-            const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            // lazy rescale: move the reference max only when it would grow by > 2^8
-            const bool grow = (m_blk > -INFINITY) &&
-                              ((m_ref == -INFINITY) || ((m_blk - m_ref) * sl2 > kRescaleThreshold));
+            for (int c = 0; c < 4; ++c)
+              mx[c] = fmax3(mx[c], __uint_as_float(s[c][kx]), __uint_as_float(s[c][kx + 1]));
+          const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+          // lazy rescale: move the reference max only when it would grow by > 2^8
+          const bool grow = (m_blk > -INFINITY) &&
+                            ((m_ref == -INFINITY) || ((m_blk - m_ref) * sl2 > kRescaleThreshold));
+          if (__any_sync(0xffffffffu, grow)) {
             float o_scale = 1.f;
             if (grow) {
               o_scale = (m_ref == -INFINITY) ? 0.f : ex2((m_ref - m_blk) * sl2);
               m_ref = m_blk;
               l_run *= o_scale;
             }
-            if (jj > 0 && __any_sync(0xffffffffu, grow)) {
+            if (jj > 0) {
               // the P V MMA of the previous block completed before this block's S was
               // committed (in-order tensor pipe), so O is quiescent here
 #pragma unroll 1
-              for (int c = 0; c < 4; ++c) {
-                uint32_t o[32];
-                tmem_ld32(t_o + c * 32, o);
+              for (int c = 0; c < 8; ++c) {
+                uint32_t o[16];
+                tmem_ld16(t_o + c * 16, o);
                 tc_wait_ld();
 #pragma unroll
-                for (int kx = 0; kx < 32; ++kx)
+                for (int kx = 0; kx < 16; ++kx)
                   o[kx] = __float_as_uint(__uint_as_float(o[kx]) * o_scale);
-                tmem_st32(t_o + c * 32, o);
+                tmem_st16(t_o + c * 16, o);
               }
             }
-            const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref * sl2;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+          }
+          // Scale-and-subtract and the row sums work on packed pairs (fma / add on two
+          // floats per instruction).  P goes out chunk by chunk over the S columns already
+          // in registers; three quarters of it are handed to the issuer while the last
+          // quarter's exponentials run.
+          const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref * sl2;
+          const uint64_t sl2x2 = pack_f32x2(sl2, sl2), negm2 = pack_f32x2(neg_m, neg_m);
+          uint64_t sum2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t pk[16];
+          for (int c = 0; c < 4; ++c) {
+            uint32_t pk[16];
 #pragma unroll
-              for (int kx = 0; kx < 16; ++kx) {
-                const float e0 = ex2(fmaf(__uint_as_float(s[c][2 * kx]), sl2, neg_m));
-                const float e1 = ex2(fmaf(__uint_as_float(s[c][2 * kx + 1]), sl2, neg_m));
-                sum[(kx & 1) * 2] += e0; sum[(kx & 1) * 2 + 1] += e1;
-                pk[kx] = pack_bf16x2(e0, e1);
-              }
-              // 16 packed columns per 32 scores: two chunks fill one 32-column store
-              if ((c & 1) == 0) {
-#pragma unroll
-                for (int kx = 0; kx < 16; ++kx) s[c][kx] = pk[kx];
-              } else {
-#pragma unroll
-                for (int kx = 0; kx < 16; ++kx) s[c - 1][16 + kx] = pk[kx];
-                tmem_st32(t_s + (c >> 1) * 32, s[c - 1]);
-              }
+            for (int kx = 0; kx < 16; ++kx) {
+              const uint64_t a2 = fma_f32x2(
+                  pack_f32x2(__uint_as_float(s[c][2 * kx]), __uint_as_float(s[c][2 * kx + 1])),
+                  sl2x2, negm2);
+              float a0, a1;
+              unpack_f32x2(a2, a0, a1);
+              const float e0 = ex2(a0), e1 = ex2(a1);
+              sum2[kx & 1] = add_f32x2(sum2[kx & 1], pack_f32x2(e0, e1));
+              pk[kx] = pack_bf16x2(e0, e1);
             }
-            l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            if (c == 3) {              // (stores 0-2 were issued a quarter ago)
+              tc_wait_st();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar_pp);
+            }
+            tmem_st16(t_s + c * 16, pk);
           }
           tc_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar_p);   // 4 arrivals, not 128 serialised ones
+          float s0, s1, s2, s3;
+          unpack_f32x2(sum2[0], s0, s1);
+          unpack_f32x2(sum2[1], s2, s3);
+          l_run += (s0 + s1) + (s2 + s3);
         }
         // epilogue: O / l -> bf16 -> O_scratch[ft, row, head, :]; tail rows are zeros
         wait_bar(env, smem_u32(&bars.o_done[wg]), o_par, 0x80 + wg);
@@ -1083,17 +1086,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           stage_row32(stg + hh * kPanel, row, 32, o[1], inv);
         }
         fence_proxy_async_smem();
-        named_bar_sync(1 + wg, 128);
-        if ((warp & 3) == 0 && lane == 0) {
-          tma_store_2d(&tmO, stg, head * 128, ft * 128);
-          tma_store_2d(&tmO, stg + kPanel, head * 128 + 64, ft * 128);
-          tma_store_commit();
-          tma_store_wait_read();
-          mbar_arrive(smem_u32(&bars.q_empty[wg]));     // the producer may refill this Q buffer
-          tma_store_wait_all();
-          fence_proxy_async_all();     // O_scratch is read back by TMA loads of other CTAs
-          __threadfence();
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars.o_staged[wg]));   // warp 3 stores the tile
       } else if (mode == MODE_OPROJ) {
         const int ft = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT], valid_m = d[TO_VALID];
         const bool leader = ((warp & 3) == 0 && lane == 0);
@@ -1216,13 +1210,15 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     // them may outlive the CTA's shared memory and TMEM.  Each issuer waits (bounded) for
     // its own MMAs, the store leaders for their bulk stores, and everybody gives loads
     // already issued 100 us to land (nothing issues new ones any more).
-    if ((warp == 1 || warp == 3) && lane == 0) {
-      const uint32_t bar = smem_u32(&bars.drain[warp == 1 ? 0 : 1]);
-      tc_commit(bar);
+    if (warp == 1) {
+      const uint32_t bar = smem_u32(&bars.drain);
+      __syncwarp();
+      if (elect_one()) tc_commit(bar);      // (the lane that issued the MMAs)
+      __syncwarp();
       for (int it = 0; it < (1 << 20); ++it)
         if (mbar_try_wait(bar, 0)) break;
     }
-    if ((warp == 4 || warp == 8) && lane == 0) tma_store_wait_all();
+    if ((warp == 3 || warp == 4 || warp == 8) && lane == 0) tma_store_wait_all();
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 100000ull) {}
   }
