@@ -75,7 +75,7 @@ int cdiv(int a, int b) { return (a + b - 1) / b; }
 // instruction as two 64-wide swizzled panels: the tensor is described as
 // {64 d, tokens, 2 d-halves, heads} so the box {64, 128, 2, 1} lands panel after panel.
 // W_o [K_local, width] is described as {64 n, K_local, width/64 panels}: the box
-// {64, 64, 4} is a 64-k slab of 256 output columns, panel after panel.
+// {64, 64, 2} is a 64-k slab of 128 output columns, panel after panel.
 int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint64_t oscr,
                          uint64_t W, uint64_t H, uint64_t Hkv, uint64_t tot_q, uint64_t tot_k,
                          uint64_t row_tiles, uint64_t w_width, uint64_t csym, uint64_t hidden,
@@ -105,7 +105,7 @@ int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, 
   if (rc == MA_OK) {
     const uint64_t dims[3] = {64, KL, w_width / 64};
     const uint64_t str[2] = {w_width * 2, 128};
-    const uint32_t box[3] = {64, 64, 4};
+    const uint32_t box[3] = {64, 64, 2};
     rc = encode(&maps[4], W, 3, dims, str, box);
   }
   if (rc == MA_OK) {

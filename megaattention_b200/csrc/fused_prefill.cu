@@ -6,11 +6,11 @@
 //   FA task    (row_tile, q head[s])  : S = Q K^T and O += P V as tcgen05 MMAs with fp32
 //                                       accumulators in TMEM, online softmax by one thread
 //                                       per row, result to O_scratch (bf16) by TMA store
-//   O_proj task (row_tile, n super-group): C[128, <=512] = O_scratch tile @ W_o columns in
-//                                       two passes of 256 columns, each into one of two
-//                                       ping-pong TMEM accumulators, so a pass's epilogue
-//                                       runs under the next pass's MMAs (the A tile
-//                                       streams once per pass)
+//   O_proj task                       : one rank: up to two row tiles x 256 columns, C =
+//                                       O_scratch tiles @ W_o columns, a TMEM accumulator
+//                                       per row tile, W stages shared.  Several ranks:
+//                                       (row_tile, n super-group), C[128, <=512] in two
+//                                       passes of 256 columns into the two accumulators
 //   AR task    (owned slot)           : multimem.ld_reduce / multimem.st over the NVLS
 //                                       multicast view of the symmetric output (or plain
 //                                       peer loads / stores with two ranks)
@@ -48,6 +48,7 @@ constexpr uint32_t kSmKV = 2 * kTile;      // ring of five K/V tiles
 constexpr int kKvSlots = 5;
 constexpr uint32_t kSmOpStaging = 4 * (16384 + 32768);   // O_proj output staging, 2 x 16 KB
 constexpr uint32_t kOpStage = 16384 + 32768;   // O_proj stage: A 128x64 + W 64x256 (4 stages)
+constexpr uint32_t kOpStage2 = 2 * 16384 + 32768;   // two row tiles: A 256x64 + W 64x256 (3 stages)
 constexpr uint32_t kWPanel = 8192;         // 64 k-rows x 64 n bf16
 constexpr uint32_t kTmemS = 0;             // S0 at 0, S1 at 128 (P aliases the first 64 cols)
 constexpr uint32_t kTmemO = 256;           // O0 at 256, O1 at 384
@@ -140,8 +141,10 @@ __device__ __forceinline__ bool try_fa(const KParams& p, int num_fa, int* arg) {
 // with one atomicAdd (every attempt succeeds) after seeing head < tail.  A ticket that lost
 // the race to a not-yet-published entry stays pending in this CTA (at most one) and is
 // served as soon as the publish index passes it; meanwhile the CTA keeps taking other work.
-__device__ __forceinline__ bool try_pop_oproj(const KParams& p, int total_op, int* pending,
-                                              int* arg) {
+// The queue holds row-tile groups in the order they became ready; each stands for its
+// `per_group` tasks, so ticket t is task t % per_group of entry t / per_group.
+__device__ __forceinline__ bool try_pop_oproj(const KParams& p, int total_op, int per_group,
+                                              int* pending, int* arg) {
   if (*pending < 0) {
     const uint32_t head = ld_relaxed_gpu(p.ctrl + C_OP_CONSUME);
     const uint32_t tail = ld_acquire_gpu(p.ctrl + C_OP_PUBLISH);
@@ -154,7 +157,8 @@ __device__ __forceinline__ bool try_pop_oproj(const KParams& p, int total_op, in
   } else if (static_cast<uint32_t>(*pending) >= ld_acquire_gpu(p.ctrl + C_OP_PUBLISH)) {
     return false;
   }
-  *arg = static_cast<int>(ld_relaxed_gpu(p.oproj_queue + *pending));
+  *arg = static_cast<int>(ld_relaxed_gpu(p.oproj_queue + *pending / per_group)) * per_group +
+         *pending % per_group;
   *pending = -1;
   return true;
 }
@@ -231,7 +235,7 @@ __device__ __noinline__ int try_claim_ar(const KParams& p, int local_owned, uint
 }
 
 __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, int total_op,
-                                           int local_owned, uint32_t poll_no, bool busy,
+                                           int per_group, int local_owned, uint32_t poll_no, bool busy,
                                            int* pending, int* mode, int* arg) {
   const KParams& p = *e.p;
   *mode = MODE_IDLE;
@@ -267,7 +271,7 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   if (!fa_only) {
     const int op_d = static_cast<int>(ld_acquire_gpu(p.ctrl + C_OP_DONE));
     const int ar_d = static_cast<int>(ld_acquire_gpu(p.ctrl + C_AR_DONE));
-    done = done && op_d >= total_op && ((p.flags & 16u) || ar_d >= local_owned);
+    done = done && op_d >= total_op && (p.tp == 1 || (p.flags & 16u) || ar_d >= local_owned);
   }
   if (done) { *mode = MODE_DONE; return; }
   // probe order by role: 0: FA,OPROJ,AR  1: OPROJ,AR,FA  2: AR,FA,OPROJ (the reference's
@@ -285,7 +289,7 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
     bool ok = false;
     if (m == MODE_FA) ok = try_fa(p, num_fa, arg);
     else if (fa_only) ok = false;
-    else if (m == MODE_OPROJ) ok = try_pop_oproj(p, total_op, pending, arg);
+    else if (m == MODE_OPROJ) ok = try_pop_oproj(p, total_op, per_group, pending, arg);
     else if (p.tp > 1 && !(p.flags & 16u) &&
              !(busy && static_cast<int>(ld_relaxed_gpu(p.ctrl + C_OP_CONSUME)) >= total_op))
     {
@@ -299,12 +303,12 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   }
 }
 
-// Reserve, fill and publish (in reservation order) the O_proj slots of one row tile.
-__device__ __noinline__ void publish_oproj(const Env& e, int row_tile) {
+// Reserve, fill and publish (in reservation order) the O_proj tasks of one row-tile group.
+__device__ __noinline__ void publish_oproj(const Env& e, int group, int per_group) {
   const KParams& p = *e.p;
-  const uint32_t n = static_cast<uint32_t>(p.nsg);
+  const uint32_t n = static_cast<uint32_t>(per_group);
   const uint32_t start = atom_add_relaxed_gpu(p.ctrl + C_OP_RESERVE, n);
-  for (uint32_t i = 0; i < n; ++i) p.oproj_queue[start + i] = row_tile * n + i;
+  p.oproj_queue[start / n] = static_cast<uint32_t>(group);
   fence_acq_rel_gpu();
   const uint64_t t0 = globaltimer_ns();
   uint32_t it = 0;
@@ -312,7 +316,7 @@ __device__ __noinline__ void publish_oproj(const Env& e, int row_tile) {
     if ((++it & 63u) == 0) {
       if (ld_relaxed_gpu(p.status) != 0u) { *e.abort_flag = 1; return; }
       if (globaltimer_ns() - t0 > p.wait_limit_ns) {
-        report(e, ST_TIMEOUT_PUBLISH, start, row_tile);
+        report(e, ST_TIMEOUT_PUBLISH, start, group);
         return;
       }
     }
@@ -330,12 +334,9 @@ __device__ __forceinline__ void finish_ar_slot(const KParams& p, int slot) {
 
 // After an O_proj task: tell the slot's owner rank that this rank's partial is in place.
 __device__ __noinline__ void publish_ar_ready(const KParams& p, int slot) {
-  if (p.flags & 16u) {
-    // partial sums only (measurement aid): no AllReduce, no cross-rank traffic
-  } else if (p.tp == 1) {
-    // one rank: the partial is the result; account the (identity) AllReduce right here
-    fence_acq_rel_gpu();
-    finish_ar_slot(p, slot);
+  if ((p.flags & 16u) || p.tp == 1) {
+    // one rank (the partial is the result), or partial sums only (measurement aid): no
+    // AllReduce to account, no cross-rank traffic
   } else {
     const int owner_rank = slot % p.tp;
     const int owner_idx = slot / p.tp;
@@ -422,6 +423,15 @@ __device__ __forceinline__ void stage_row32(uint32_t panel, int row, int col0,
   }
 }
 
+// A whole panel row already in bf16.
+__device__ __forceinline__ void stage_panel_row(uint32_t panel, int row, const uint32_t (&pk)[32]) {
+  const uint32_t rbase = panel + static_cast<uint32_t>(row) * 128u;
+  const uint32_t sw = static_cast<uint32_t>(row & 7);
+#pragma unroll
+  for (uint32_t c = 0; c < 8; ++c)
+    st_shared_v4(rbase + ((c ^ sw) << 4), pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+}
+
 // ---------------------------------------------------------------- AllReduce of one slot
 // One AllReduce slot: 128 rows x (vnt x 128) bf16 columns, reduced in the switch and
 // written back to every rank.  `nthr` threads cooperate; each keeps U 16-byte reductions in
@@ -488,11 +498,29 @@ __device__ __forceinline__ void ar_slot(const KParams& p, int ft, int base_out, 
 
 }  // namespace
 
+// O_proj task of a single rank: nrt row tiles x nnt column tiles in one pass.  What bounds the
+// product is shared memory, which carries the loads and the MMAs' operands: for 64 k of two row
+// tiles x 256 columns 96 + 96 KB when each row tile loads W for itself, 64 + 96 KB when they
+// share it.  So 2 x 2 is the shape for large launches (O_proj stage
+// alone, 22600 tokens, hidden 16384: 1330 -> 1210 us; 13400 tokens, hidden 4096: 110 -> 103).
+// With few tasks what counts is how soon the last row tile's product is done: one column tile
+// per task up to 1.25 waves of 2 x 2 tasks, two up to 3 waves.  Whole launches, us, as 2 x 2 /
+// 1 x 2 / 1 x 1:  0.1 waves (520 tokens, hidden 1024) 53 / 48 / 46, 0.9 waves (four prompts of
+// 1024, K = 2048, hidden 2048) 109 / 97 / 94, 1.3 waves 83 / 81 / 88, 3.5 waves (16384 tokens)
+// 525 / 537 / 595, 5.8 waves 226 / 250 / 322.
+__device__ __forceinline__ void op_task_shape(int n_tiles, int num_out, int ctas, int* nrt,
+                                              int* nnt) {
+  const int t22 = (n_tiles + 1) / 2 * ((num_out + 1) / 2);
+  *nrt = t22 >= 3 * ctas ? 2 : 1;
+  *nnt = 4 * t22 >= 5 * ctas ? 2 : 1;
+}
+
 // Task descriptor words written by the scheduler (shared memory, two slots).
 enum : int { T_MODE = 0, T_FT = 1,
              TF_HEAD0 = 2, TF_NT = 3, TF_KVH = 4, TF_QROW0 = 5, TF_VALID = 6, TF_KSTART = 7,
              TF_KLEN = 8, TF_OFFSET = 9, TF_NBLK = 10, TF_MB = 11,
-             TO_BASE = 2, TO_VNT = 3, TO_VALID = 4, TO_SLOT = 5, T_WORDS = 12 };
+             TO_BASE = 2, TO_VNT = 3, TO_VALID = 4, TO_SLOT = 5, TO_NRT = 6, TO_VALID1 = 7,
+             T_WORDS = 12 };
 
 __device__ __forceinline__ bool is_tile_mode(int m) { return m == MODE_FA || m == MODE_OPROJ; }
 
@@ -592,8 +620,19 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     if (warp == 2 && lane == 0) {
       // ==================================================================== scheduler
       const int num_fa = p.actv[0];
-      const int total_op = p.actv[1];
       const int local_owned = p.actv[5];
+      // O_proj tasks.  With several ranks a task is an AllReduce slot: one row tile, up to
+      // `sg` column tiles in two passes (TO_NRT = 0).  One rank is free to choose: nrt row
+      // tiles x nnt column tiles (<= 2 x 2) in one pass, the row tiles sharing every W stage.
+      int nrt = 0, nnt = p.sg, per_group = p.nsg, total_op = p.actv[1];
+      const int n_tiles = p.actv[2];
+      if (p.tp == 1) {
+        op_task_shape(n_tiles, p.num_out, static_cast<int>(gridDim.x), &nrt, &nnt);
+        per_group = (p.num_out + nnt - 1) / nnt;
+        // (plus what the host's count of slots is off by: such a launch must not end well)
+        total_op = (n_tiles + nrt - 1) / nrt * per_group + (total_op - n_tiles * p.nsg);
+      }
+      const int grp = max(nrt, 1);              // row tiles whose attention a task group needs
       int role;
       {
         const int wsum = p.w_fa + p.w_oproj + p.w_ar;
@@ -617,8 +656,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         if (p.audit) {      // exactly-once audit (audit build only): one count per finished unit
           if (occ_mode[kk] == MODE_FA) {
             for (int i = 0; i < occ_b[kk]; ++i) atomicAdd(p.audit + occ_a[kk] * p.H + occ_h[kk] + i, 1u);
-          } else if (occ_mode[kk] == MODE_OPROJ) {
+          } else if (occ_mode[kk] == MODE_OPROJ && nrt == 0) {
             atomicAdd(p.audit + p.audit_op_base + occ_a[kk], 1u);
+          } else if (occ_mode[kk] == MODE_OPROJ) {     // a slot counts with its first column tile
+            const int r0 = occ_a[kk] / per_group * nrt, o0 = occ_a[kk] % per_group * nnt;
+            for (int r = r0; r < min(r0 + nrt, n_tiles); ++r)
+              for (int o = o0; o < min(o0 + nnt, p.num_out); ++o)
+                if (o % p.sg == 0) atomicAdd(p.audit + p.audit_op_base + r * p.nsg + o / p.sg, 1u);
           } else if (occ_mode[kk] == MODE_AR) {
             atomicAdd(p.audit + p.audit_ar_base + occ_a[kk] / p.tp, 1u);
           }
@@ -626,10 +670,12 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 #endif
         if (occ_mode[kk] == MODE_FA) {
           fence_acq_rel_gpu();
-          const uint32_t old = atom_add_acqrel_gpu(p.head_ready + occ_a[kk],
+          const int g = occ_a[kk] / grp;
+          const uint32_t old = atom_add_acqrel_gpu(p.head_ready + g,
                                                    static_cast<uint32_t>(occ_b[kk]));
-          if (!(p.flags & 1u) && static_cast<int>(old) + occ_b[kk] == p.H)
-            publish_oproj(env, occ_a[kk]);
+          if (!(p.flags & 1u) &&
+              static_cast<int>(old) + occ_b[kk] == p.H * min(grp, n_tiles - g * grp))
+            publish_oproj(env, g, per_group);
           atom_add_release_gpu(p.ctrl + C_FA_DONE, static_cast<uint32_t>(occ_b[kk]));
         } else if (occ_mode[kk] == MODE_OPROJ) {
           publish_ar_ready(p, occ_a[kk]);
@@ -659,7 +705,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         int mode, arg;
         uint64_t idle_t0 = 0;
         while (true) {
-          schedule_pick(env, role, num_fa, total_op, local_owned, poll_no++, occupied[k ^ 1],
+          schedule_pick(env, role, num_fa, total_op, per_group, local_owned, poll_no++, occupied[k ^ 1],
                         &pending_ticket, &mode, &arg);
           if (mode != MODE_IDLE) break;
           // nothing to do and not finished: bounded like every other wait (a rank that
@@ -706,12 +752,17 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           occ_h[k] = head0;
 #endif
         } else if (mode == MODE_OPROJ || mode == MODE_AR) {
-          const int ft = arg / p.nsg, g = arg % p.nsg;
-          const int base_out = g * p.sg;
-          const int b = p.fa_b[ft], mb = p.fa_mb[ft];
-          const int q_len = p.cu_q[b + 1] - p.cu_q[b];
-          d[T_FT] = ft; d[TO_BASE] = base_out; d[TO_VNT] = min(p.sg, p.num_out - base_out);
-          d[TO_VALID] = min(128, q_len - mb * 128); d[TO_SLOT] = arg;
+          const bool own = mode == MODE_OPROJ && nrt > 0;     // a shape of this rank's choice
+          const int ft = own ? arg / per_group * nrt : arg / p.nsg;
+          const int width = own ? nnt : p.sg;
+          const int base_out = (own ? arg % per_group : arg % p.nsg) * width;
+          const int rows = own ? min(nrt, n_tiles - ft) : 1;
+          d[T_FT] = ft; d[TO_BASE] = base_out; d[TO_VNT] = min(width, p.num_out - base_out);
+          for (int r = 0; r < rows; ++r) {
+            const int b = p.fa_b[ft + r], mb = p.fa_mb[ft + r];
+            d[r ? TO_VALID1 : TO_VALID] = min(128, p.cu_q[b + 1] - p.cu_q[b] - mb * 128);
+          }
+          d[TO_NRT] = own ? rows : 0; d[TO_SLOT] = arg;
           occ_a[k] = arg;
         }
         d[T_MODE] = mode;
@@ -727,7 +778,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       }
     } else if (warp == 0 && lane == 0) {
       // ==================================================================== TMA producer
-      uint32_t kv_slot = 0, kv_ph = 0, opc = 0, q_uses[2] = {0, 0};
+      uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0, q_uses[2] = {0, 0};
       while (true) {
         MA_NEXT_TASK(d, mode)
         MA_DRAIN_IF_SWITCH(mode)
@@ -766,23 +817,29 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
             }
           }
         } else if (mode == MODE_OPROJ) {
-          const int ft = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT];
+          const int ft = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT], nrt = d[TO_NRT];
           const int nkc = p.K_local >> 6;
+          const int rows = max(nrt, 1), passes = nrt ? 1 : (vnt + 1) >> 1;
+          const uint32_t stage = nrt ? kOpStage2 : kOpStage, w_off = nrt ? 2 * kPanel : kPanel;
+          const uint32_t stages = nrt ? 3 : 4;
           fence_proxy_async_global();   // O_scratch was written by other CTAs' TMA stores
           bool ok = true;
-          for (int h = 0; h * 2 < vnt && ok; ++h) {
+          for (int h = 0; h < passes && ok; ++h) {
+            const int nw = min(2, vnt - 2 * h);            // column tiles of this pass
             for (int kc = 0; kc < nkc; ++kc) {
-              const uint32_t st = opc & 3u;
-              ok = wait_bar(env, smem_u32(&bars.op_empty[st]), ((opc >> 2) & 1u) ^ 1u, 0x90 + st);
+              ok = wait_bar(env, smem_u32(&bars.op_empty[op_st]), op_ph ^ 1u, 0x90 + op_st);
               if (!ok) break;
-              const uint32_t bar = smem_u32(&bars.op_full[st]);
-              const uint32_t a_dst = smem0 + st * kOpStage;
-              // A chunk 128 x 64 and a W slab of 64 k x 256 n (4 panels; panels past the
-              // padded width are filled with zeros)
-              mbar_expect_tx(bar, kPanel + 4u * kWPanel);
-              tma_load_2d(a_dst, &tmO, bar, kc * 64, ft * 128);
-              tma_load_3d(a_dst + kPanel, &tmW, bar, 0, kc * 64, (base_out + 2 * h) * 2);
-              ++opc;
+              const uint32_t bar = smem_u32(&bars.op_full[op_st]);
+              const uint32_t dst = smem0 + op_st * stage;
+              // A chunks of 128 x 64 and W slabs of 64 k x 128 n (2 panels each; panels past
+              // the padded width are filled with zeros)
+              mbar_expect_tx(bar, rows * kPanel + nw * 2 * kWPanel);
+              for (int r = 0; r < rows; ++r)
+                tma_load_2d(dst + r * kPanel, &tmO, bar, kc * 64, (ft + r) * 128);
+              for (int j = 0; j < nw; ++j)
+                tma_load_3d(dst + w_off + j * 2 * kWPanel, &tmW, bar, 0, kc * 64,
+                            (base_out + 2 * h + j) * 2);
+              if (++op_st == stages) { op_st = 0; op_ph ^= 1u; }
             }
           }
         }
@@ -793,7 +850,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       // ============================================= MMA issuer of both attention tiles and of
       // every O_proj task.  The warp stays converged: every lane waits, one elected lane
       // issues (see elect_one).
-      uint32_t kv_slot = 0, kv_ph = 0, opc = 0;
+      uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0;
       uint32_t q_par[2] = {0, 0}, p_par[2] = {0, 0}, o_uses[2] = {0, 0}, acc_uses[2] = {0, 0};
       while (true) {
         MA_NEXT_TASK(d, mode)
@@ -895,30 +952,39 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
             }
           }
         } else if (mode == MODE_OPROJ) {
-          const int vnt = d[TO_VNT];
+          const int vnt = d[TO_VNT], nrt = d[TO_NRT];
           const int nkc = p.K_local >> 6;
-          for (int h = 0; h * 2 < vnt; ++h) {
+          const int rows = max(nrt, 1), passes = nrt ? 1 : (vnt + 1) >> 1;
+          const uint32_t stage = nrt ? kOpStage2 : kOpStage, w_off = nrt ? 2 * kPanel : kPanel;
+          const uint32_t stages = nrt ? 3 : 4;
+          for (int h = 0; h < passes; ++h) {
             const int ncols = min(2, vnt - 2 * h) * 128;
             const uint32_t idesc = make_idesc_bf16(128, ncols, 0, 1);
-            wait_bar(env, smem_u32(&bars.acc_free[h]), (acc_uses[h] & 1u) ^ 1u, 0xA8 + h);
-            ++acc_uses[h];
             for (int kc = 0; kc < nkc; ++kc) {
-              const uint32_t st = opc & 3u;
-              wait_bar(env, smem_u32(&bars.op_full[st]), (opc >> 2) & 1u, 0xA0 + st);
-              ++opc;
-              tc_fence_after();
-              const uint32_t a16 = (smem0 + st * kOpStage) >> 4;
-              const uint32_t w16 = a16 + (kPanel >> 4);
-              if (elect_one()) {
+              wait_bar(env, smem_u32(&bars.op_full[op_st]), op_ph, 0xA0 + op_st);
+              const uint32_t a16 = (smem0 + op_st * stage) >> 4;
+              const uint32_t w16 = a16 + (w_off >> 4);
+              // accumulator h + r: row tile r's (the passes of a slot have one row tile)
+              for (int r = 0; r < rows; ++r) {
+                if (kc == 0) {
+                  wait_bar(env, smem_u32(&bars.acc_free[h + r]), (acc_uses[h + r] & 1u) ^ 1u,
+                           0xA8 + h + r);
+                  ++acc_uses[h + r];
+                }
+                tc_fence_after();
+                if (elect_one()) {
+                  const uint32_t a16r = a16 + r * (kPanel >> 4);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                  mma_ss(tmem + h * 256, smem_desc_at(kDescK, a16 + kk * 2),
-                         smem_desc_at(kDescWmn, w16 + kk * 128), idesc,
-                         (kc > 0 || kk > 0) ? 1u : 0u);
-                tc_commit(smem_u32(&bars.op_empty[st]));
-                if (kc + 1 == nkc) tc_commit(smem_u32(&bars.acc_full[h]));
+                  for (int kk = 0; kk < 4; ++kk)
+                    mma_ss(tmem + (h + r) * 256, smem_desc_at(kDescK, a16r + kk * 2),
+                           smem_desc_at(kDescWmn, w16 + kk * 128), idesc,
+                           (kc > 0 || kk > 0) ? 1u : 0u);
+                  if (r + 1 == rows) tc_commit(smem_u32(&bars.op_empty[op_st]));
+                  if (kc + 1 == nkc) tc_commit(smem_u32(&bars.acc_full[h + r]));
+                }
+                __syncwarp();
               }
-              __syncwarp();
+              if (++op_st == stages) { op_st = 0; op_ph ^= 1u; }
             }
           }
         }
@@ -980,25 +1046,35 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           wait_bar(env, bar_s, s_par, 0x70 + wg);
           s_par ^= 1u;
           tc_fence_after();
-          uint32_t s[4][32];
+          // Four chunks of 32 scores.  The last is read for the maximum and read again for its
+          // exponentials: held all along it takes the registers that the rest of the kernel
+          // needs (spilled, the attention stage lost 3 %).
+          uint32_t s[3][32], last[32];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, s[c]);
+          for (int c = 0; c < 3; ++c) tmem_ld32(t_s + c * 32, s[c]);
+          tmem_ld32(t_s + 96, last);
           tc_wait_ld();
           const bool need_mask = ((j + 1) * 128 - 1 > mb * 128 + offset) || ((j + 1) * 128 > k_len);
+          const int lim = lim_abs - j * 128;      // columns > lim are masked
+          auto mask = [&](uint32_t (&x)[32], int c) {
+#pragma unroll
+            for (int kx = 0; kx < 32; ++kx)
+              if (c * 32 + kx > lim) x[kx] = 0xff800000u;   // -inf
+          };
           if (need_mask) {
-            const int lim = lim_abs - j * 128;    // columns > lim are masked
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int kx = 0; kx < 32; ++kx)
-                if (c * 32 + kx > lim) s[c][kx] = 0xff800000u;   // -inf
+            mask(s[0], 0);
+            mask(s[1], 1);
+            mask(s[2], 2);
+            mask(last, 3);
           }
           float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int kx = 0; kx < 32; kx += 2)
+          for (int kx = 0; kx < 32; kx += 2) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < 3; ++c)
               mx[c] = fmax3(mx[c], __uint_as_float(s[c][kx]), __uint_as_float(s[c][kx + 1]));
+            mx[3] = fmax3(mx[3], __uint_as_float(last[kx]), __uint_as_float(last[kx + 1]));
+          }
           const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
           // lazy rescale: move the reference max only when it would grow by > 2^8
           const bool grow = (m_blk > -INFINITY) &&
@@ -1032,27 +1108,42 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref * sl2;
           const uint64_t sl2x2 = pack_f32x2(sl2, sl2), negm2 = pack_f32x2(neg_m, neg_m);
           uint64_t sum2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t pk[16];
+          auto exps = [&](const uint32_t (&x)[32], uint32_t (&pk)[16]) {
 #pragma unroll
             for (int kx = 0; kx < 16; ++kx) {
               const uint64_t a2 = fma_f32x2(
-                  pack_f32x2(__uint_as_float(s[c][2 * kx]), __uint_as_float(s[c][2 * kx + 1])),
-                  sl2x2, negm2);
+                  pack_f32x2(__uint_as_float(x[2 * kx]), __uint_as_float(x[2 * kx + 1])), sl2x2,
+                  negm2);
               float a0, a1;
               unpack_f32x2(a2, a0, a1);
               const float e0 = ex2(a0), e1 = ex2(a1);
               sum2[kx & 1] = add_f32x2(sum2[kx & 1], pack_f32x2(e0, e1));
               pk[kx] = pack_bf16x2(e0, e1);
             }
-            if (c == 3) {              // (stores 0-2 were issued a quarter ago)
-              tc_wait_st();
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(bar_pp);
-            }
+          };
+          {
+            uint32_t pk[16];
+            exps(s[0], pk);
+            tmem_st16(t_s, pk);
+          }
+          uint32_t x3[32];
+          tmem_ld32(t_s + 96, x3);                // (P takes columns 0-63 only)
+#pragma unroll
+          for (int c = 1; c < 3; ++c) {
+            uint32_t pk[16];
+            exps(s[c], pk);
             tmem_st16(t_s + c * 16, pk);
+          }
+          {
+            uint32_t pk[16];
+            tc_wait_ld();
+            if (need_mask) mask(x3, 3);
+            exps(x3, pk);
+            tc_wait_st();                         // (stores 0-2 were issued a quarter ago)
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_pp);
+            tmem_st16(t_s + 48, pk);
           }
           tc_wait_st();
           tc_fence_before();
@@ -1089,70 +1180,87 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.o_staged[wg]));   // warp 3 stores the tile
       } else if (mode == MODE_OPROJ) {
-        const int ft = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT], valid_m = d[TO_VALID];
+        const int ft0 = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT], nrt = d[TO_NRT];
         const bool leader = ((warp & 3) == 0 && lane == 0);
         const uint32_t stg = smem0 + kSmOpStaging + wg * kPanel;   // [128 rows][64 cols] bf16
-        for (int h = 0; h * 2 < vnt; ++h) {
+        bool direct = false;
+        // Accumulator h holds row tile h of the task, or columns 2h and 2h + 1 of a slot; this
+        // warpgroup's 128 columns of it go out as two panels of 64, by way of bf16 words in
+        // registers.
+        auto wait_acc = [&](int h) {
           wait_bar(env, smem_u32(&bars.acc_full[h]), acc_par[h], 0xB0 + h);
           acc_par[h] ^= 1u;
           tc_fence_after();
-          const int o_t = 2 * h + wg;                   // column tile inside the super-group
-          if (o_t < vnt) {
-            const int out_n = base_out + o_t;
+        };
+        auto free_acc = [&](int h) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bars.acc_free[h]));
+        };
+        auto load_panel = [&](int h, int hh, uint32_t (&pk)[32]) {
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              uint32_t r[2][32];
-              tmem_ld32(tmem + lane_base + h * 256 + wg * 128 + hh * 64, r[0]);
-              tmem_ld32(tmem + lane_base + h * 256 + wg * 128 + hh * 64 + 32, r[1]);
-              tc_wait_ld();
-              if (hh == 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars.acc_free[h]));
-              }
-              if (valid_m == 128) {
-                // full row tile: stage 64 columns, one TMA store (clipped at `hidden`)
-                if (leader) tma_store_wait_read();
-                named_bar_sync(1 + wg, 128);
-                stage_row32(stg, row, 0, r[0], 1.f);
-                stage_row32(stg, row, 32, r[1], 1.f);
-                fence_proxy_async_smem();
-                named_bar_sync(1 + wg, 128);
-                if (leader) {
-                  tma_store_2d(&tmC, stg, out_n * 128 + hh * 64, ft * 128);
-                  tma_store_commit();
-                }
-              } else if (row < valid_m) {
-                // last tile of a sequence: rows past valid_m must stay untouched
-                uint16_t* dst = p.csym + ((static_cast<size_t>(ft * 128 + row) * p.num_out + out_n) * 128);
+          for (int c = 0; c < 2; ++c) {
+            uint32_t r[32];
+            tmem_ld32(tmem + lane_base + h * 256 + wg * 128 + hh * 64 + c * 32, r);
+            tc_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                  const int col0 = out_n * 128 + hh * 64 + c * 32;
-                  if (col0 + 32 <= p.hidden) {
-                    uint4* d4 = reinterpret_cast<uint4*>(dst + hh * 64 + c * 32);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                      uint4 v;
-                      v.x = pack_bf16x2(__uint_as_float(r[c][8 * q + 0]), __uint_as_float(r[c][8 * q + 1]));
-                      v.y = pack_bf16x2(__uint_as_float(r[c][8 * q + 2]), __uint_as_float(r[c][8 * q + 3]));
-                      v.z = pack_bf16x2(__uint_as_float(r[c][8 * q + 4]), __uint_as_float(r[c][8 * q + 5]));
-                      v.w = pack_bf16x2(__uint_as_float(r[c][8 * q + 6]), __uint_as_float(r[c][8 * q + 7]));
-                      d4[q] = v;
-                    }
-                  } else {
-#pragma unroll
-                    for (int kx = 0; kx < 32; ++kx)
-                      if (col0 + kx < p.hidden)
-                        dst[hh * 64 + c * 32 + kx] = static_cast<uint16_t>(
-                            pack_bf16x2(__uint_as_float(r[c][kx]), 0.f) & 0xFFFFu);
-                  }
-                }
-              }
+            for (int kx = 0; kx < 16; ++kx)
+              pk[c * 16 + kx] =
+                  pack_bf16x2(__uint_as_float(r[2 * kx]), __uint_as_float(r[2 * kx + 1]));
+          }
+        };
+        auto emit_panel = [&](int h, int hh, const uint32_t (&pk)[32]) {
+          const int ft = nrt ? ft0 + h : ft0;
+          const int out_n = base_out + (nrt ? 0 : 2 * h) + wg;
+          const int valid_m = d[(nrt && h) ? TO_VALID1 : TO_VALID];
+          if (valid_m == 128) {
+            // full row tile: stage 64 columns, one TMA store (clipped at `hidden`)
+            if (leader) tma_store_wait_read();
+            named_bar_sync(1 + wg, 128);
+            stage_panel_row(stg, row, pk);
+            fence_proxy_async_smem();
+            named_bar_sync(1 + wg, 128);
+            if (leader) {
+              tma_store_2d(&tmC, stg, out_n * 128 + hh * 64, ft * 128);
+              tma_store_commit();
             }
-          } else {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bars.acc_free[h]));
+            return;
+          }
+          // last tile of a sequence: rows past valid_m must stay untouched
+          direct = true;
+          if (row >= valid_m) return;
+          const int col0 = out_n * 128 + hh * 64;
+          uint16_t* dst = p.csym + static_cast<size_t>(ft * 128 + row) * p.num_out * 128 + col0;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            if (col0 + c * 8 + 8 <= p.hidden) {
+              reinterpret_cast<uint4*>(dst)[c] =
+                  make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+            } else {
+#pragma unroll
+              for (int kx = 0; kx < 8; ++kx)
+                if (col0 + c * 8 + kx < p.hidden)
+                  dst[c * 8 + kx] = static_cast<uint16_t>(pk[4 * c + (kx >> 1)] >> ((kx & 1) * 16));
+            }
+          }
+        };
+        // Both panels leave TMEM before the first is written out, so that the accumulator is
+        // soon free for the next task's MMAs.  (All of the second accumulator as well, before
+        // the first is written, takes more registers than there are: spilled, 129 us for 105.)
+        const int halves = nrt ? nrt : (vnt + 1) >> 1;
+#pragma unroll 1
+        for (int h = 0; h < halves; ++h) {
+          const bool mine = (nrt ? 0 : 2 * h) + wg < vnt;
+          uint32_t pa[32], pb[32];
+          wait_acc(h);
+          if (mine) {
+            load_panel(h, 0, pa);
+            load_panel(h, 1, pb);
+          }
+          free_acc(h);
+          if (mine) {
+            emit_panel(h, 0, pa);
+            emit_panel(h, 1, pb);
           }
         }
         // Ordering towards other CTAs / ranks: the leader waits for its TMA stores, rows
@@ -1163,7 +1271,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           tma_store_wait_all();
           fence_proxy_async_all();
         }
-        if (valid_m != 128) __threadfence();
+        if (direct) __threadfence();
       } else if (mode == MODE_AR) {
         ar_slot(p, d[T_FT], d[TO_BASE], d[TO_VNT], tid - 128, 256);
         if (lane == 0) __threadfence_system();   // one per warp; the scheduler fences again

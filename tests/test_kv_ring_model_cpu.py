@@ -90,3 +90,52 @@ def test_shared_and_separate_stage_rings_stay_consistent():
     check([(1, 1)], sep=True)
     check([(1, 3), (1, 2), (1, 7)], sep=False)        # a single head per rank: issuer 1 only keeps count
     check([(2, 1), (1, 1), (2, 3)], sep=True)
+
+
+def one_issuer_walk(tasks, sep):
+    """[(slot, pass, task, block, which, tile)] in the order in which the one issuing warp of
+    both tiles releases the slots: it takes a group of slots per operand (one, or one per head
+    with separate stages) and gives a slot back with the last product that reads it."""
+    slot, rpass, out = 0, 0, []
+
+    def take(per):
+        nonlocal slot, rpass
+        s, p = slot, rpass
+        slot += per
+        if slot >= KV_SLOTS:
+            slot, rpass = slot - KV_SLOTS, rpass + 1
+        return s, p
+
+    def at(r, i):
+        s, p = r
+        if sep and i:
+            s += 1
+            if s == KV_SLOTS:
+                s, p = 0, p + 1
+        return s, p
+
+    for t, (nt, nblk) in enumerate(tasks):
+        per = nt if sep else 1
+        k = take(per)
+        for i in range(nt):
+            if sep or i == nt - 1:
+                out.append((*at(k, i), t, 0, 0, i if sep else None))
+        for jj in range(nblk):
+            v = take(per)
+            if jj + 1 < nblk:
+                k = take(per)
+            for i in range(nt):
+                if sep or i == nt - 1:
+                    out.append((*at(v, i), t, jj, 1, i if sep else None))
+                    if jj + 1 < nblk:
+                        out.append((*at(k, i), t, jj + 1, 0, i if sep else None))
+    return out
+
+
+def test_one_issuer_releases_every_slot_once():
+    rng = random.Random(8)
+    for _ in range(200):
+        for sep in (False, True):
+            tasks = [(rng.choice((1, 2, 2)), rng.randint(1, 9)) for _ in range(rng.randint(1, 12))]
+            walk = one_issuer_walk(tasks, sep)
+            assert sorted(walk, key=str) == sorted(producer_sequence(tasks, sep), key=str)
