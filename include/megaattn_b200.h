@@ -281,6 +281,21 @@ typedef struct ma_rope_args {
 
 int ma_rope_qk(const ma_rope_args* args, void* stream);
 
+/*
+ * Packed copy of the fused launch's output: out[cu_q[b] + i, :] = row i of sequence b of the
+ * tile-padded C_sym, first `hidden` columns.  csym and out are device addresses, 16-byte
+ * aligned; cu_q is a HOST array (num_batch + 1, ascending from 0) that is read before the
+ * call returns.  row_pitch is C_sym's row length in elements.  Asynchronous on `stream`.
+ */
+typedef struct ma_detile_args {
+  uint64_t csym, out;               /* bf16                                             */
+  const int32_t* cu_q;              /* host, i32 [num_batch + 1]                        */
+  int32_t num_batch, hidden, row_pitch;
+  int32_t reserved0;
+} ma_detile_args;
+
+int ma_detile(const ma_detile_args* args, void* stream);
+
 const char* ma_strerror(int code);
 
 #ifdef __cplusplus

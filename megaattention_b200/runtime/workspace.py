@@ -448,14 +448,18 @@ class FusedFaOprojArWorkspace:
                 "the workspace control state is undefined — call debug_zero_all()")
 
     def output(self, meta=None):
-        """De-tiled ``[tot_q, hidden]`` copy of the valid region of ``csym``."""
+        """De-tiled ``[tot_q, hidden]`` copy of the valid region of ``csym``, queued on the
+        current stream."""
         meta = meta or self._meta
-        flat = self.csym.view(self.max_num_row_tiles, 128, self.hidden_pad)
-        tot = int(meta.cu_seqlens_q[-1])
-        out = torch.empty(tot, self.hidden, dtype=self.dtype, device=self.dev)
-        for t in range(meta.num_row_tiles):
-            s, vm = meta.q_tile_start(t), meta.valid_m(t)
-            out[s:s + vm] = flat[t, :vm, :self.hidden]
+        cu_q = np.ascontiguousarray(meta.cu_seqlens_q, dtype=np.int32)
+        assert meta.num_row_tiles <= self.max_num_row_tiles
+        out = torch.empty(int(cu_q[-1]), self.hidden, dtype=self.dtype, device=self.dev)
+        args = _cabi.DetileArgs(self.csym.data_ptr(), out.data_ptr(), cu_q.ctypes.data,
+                                cu_q.size - 1, self.hidden, self.hidden_pad, 0)
+        with torch.cuda.device(self.dev):
+            _cabi.check(self._lib.ma_detile(
+                C.byref(args), C.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)),
+                "ma_detile")
         return out
 
     # ------------------------------------------------------------------ debug
