@@ -296,6 +296,37 @@ typedef struct ma_detile_args {
 
 int ma_detile(const ma_detile_args* args, void* stream);
 
+/*
+ * Host side of one step's varlen metadata (no device work).  ma_row_desc builds the row-tile
+ * schedule from cumulative lengths and returns the number of row tiles (>= 1) or an error:
+ * MA_ERR_INVALID unless both start at 0 and 0 < q_len <= k_len for every sequence,
+ * MA_ERR_CAPACITY past max_row_tiles (the length of batch_idx and m_block) or 2^31 - 1 rows.
+ * The other outputs hold num_batch + 1 words.
+ */
+int ma_row_desc(const int64_t* cu_q, const int64_t* cu_k, int32_t num_batch,
+                int32_t max_row_tiles, int32_t* cu_q_out, int32_t* cu_k_out,
+                int32_t* cu_m_blocks, int32_t* batch_idx, int32_t* m_block);
+
+/*
+ * ma_stage_meta fills the staging copy of the six device arrays (offsets in words): the four
+ * given ones, the attention claim order and the active counts.  prime: 0 = longest row tile
+ * first, > 0 = that many of the shortest to the front, < 0 = long and short interleaved; with
+ * auto_prime it is chosen from the batch (interleaved below a KV-aware work ratio of 2).
+ */
+typedef struct ma_stage_meta_args {
+  const int32_t* cu_q;
+  const int32_t* cu_k;
+  const int32_t* batch_idx;
+  const int32_t* m_block;
+  int32_t* staging;
+  int32_t num_batch, num_row_tiles, hidden, H_local, num_super_groups, tp_size, rank;
+  int32_t auto_prime, prime;
+  int32_t off_cu_q, off_cu_k, off_batch_idx, off_m_block, off_order, off_actv;
+  int32_t reserved0;
+} ma_stage_meta_args;
+
+int ma_stage_meta(const ma_stage_meta_args* args);
+
 const char* ma_strerror(int code);
 
 #ifdef __cplusplus

@@ -28,7 +28,7 @@ MA_ERR_CAPACITY = -5
 
 EXPORTS = ("ma_query_device", "ma_plan_create", "ma_launch", "ma_plan_set_inputs", "ma_read_status",
            "ma_plan_destroy", "ma_strerror", "ma_fused_prefill_noalloc", "ma_residual_rmsnorm", "ma_rope_qk",
-           "ma_detile")
+           "ma_detile", "ma_row_desc", "ma_stage_meta")
 
 MA_NOALLOC_OSCRATCH_BYTES = 16 << 20
 MA_NOALLOC_MAX_BATCH = 512
@@ -104,6 +104,14 @@ class DetileArgs(C.Structure):
                 ("reserved0", C.c_int32)]
 
 
+class StageMetaArgs(C.Structure):
+    _fields_ = ([(n, C.c_void_p) for n in ("cu_q", "cu_k", "batch_idx", "m_block", "staging")]
+                + [(n, C.c_int32) for n in (
+                    "num_batch", "num_row_tiles", "hidden", "H_local", "num_super_groups", "tp_size",
+                    "rank", "auto_prime", "prime", "off_cu_q", "off_cu_k", "off_batch_idx",
+                    "off_m_block", "off_order", "off_actv", "reserved0")])
+
+
 def _load(path=None, audit=False):
     path = path or (_build.LIB_AUDIT if audit else _build.LIB)
     if not os.path.exists(path) or _build._stale(path):
@@ -135,6 +143,10 @@ def _load(path=None, audit=False):
     lib.ma_rope_qk.restype = C.c_int
     lib.ma_detile.argtypes = [C.POINTER(DetileArgs), C.c_void_p]
     lib.ma_detile.restype = C.c_int
+    lib.ma_row_desc.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32] + [C.c_void_p] * 5
+    lib.ma_row_desc.restype = C.c_int
+    lib.ma_stage_meta.argtypes = [C.POINTER(StageMetaArgs)]
+    lib.ma_stage_meta.restype = C.c_int
     lib.ma_strerror.argtypes = [C.c_int]
     lib.ma_strerror.restype = C.c_char_p
     return lib

@@ -30,13 +30,13 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from ..metadata.row_desc import build_row_desc
+from .workspace import native_row_desc
 
 
-def _seqlens(cu):
-    cu = np.asarray(cu.cpu() if torch.is_tensor(cu) else cu, dtype=np.int64)
+def _cumulative(cu):
+    cu = np.asarray(cu.cpu().numpy() if torch.is_tensor(cu) else cu, dtype=np.int64)
     assert cu.ndim == 1 and cu.size >= 2 and cu[0] == 0, "cu_seqlens must start at 0"
-    return np.diff(cu)
+    return cu
 
 
 class FusedPrefillLayer:
@@ -66,7 +66,8 @@ class FusedPrefillLayer:
         the token pool ``[num_slots, H_kv, D]`` with ``num_slots % 128 == 0``.
         """
         ws = self.ws
-        lens_q = _seqlens(cu_seqlens_q)
+        cu_q = _cumulative(cu_seqlens_q)
+        pages = None
         if ws.paged:
             assert page_table is not None and cache_seqlens is not None, \
                 "a paged workspace needs page_table and cache_seqlens"
@@ -78,16 +79,26 @@ class FusedPrefillLayer:
                 assert k.shape[0] % 128 == 0 and v.shape == k.shape
                 k = k.view(-1, 128, ws.H_kv, ws.D)
                 v = v.view(-1, 128, ws.H_kv, ws.D)
-            lens_k = cache_seqlens.cpu().numpy().astype(np.int64)
-            assert page_table.dim() == 2 and page_table.shape[0] == lens_q.size == lens_k.size
+            assert page_table.dim() == 2 and cache_seqlens.dim() == 1
+            assert page_table.shape[0] == cu_q.size - 1 == cache_seqlens.shape[0]
+            # the lengths and the page numbers reach the host in one copy, one wait
+            if page_table.device == cache_seqlens.device:
+                both = torch.cat((cache_seqlens, page_table.reshape(-1))).cpu().numpy()
+                lens_k, pages = both[:cu_q.size - 1].astype(np.int64), both[cu_q.size - 1:]
+            else:
+                lens_k = cache_seqlens.cpu().numpy().astype(np.int64)
             assert page_table.shape[1] >= int((-(-lens_k // 128)).max()), \
                 "page_table is narrower than the longest sequence needs"
         else:
             assert page_table is None and cache_seqlens is None, \
                 "page_table / cache_seqlens need a workspace created with paged=True"
-            lens_k = lens_q if cu_seqlens_k is None else _seqlens(cu_seqlens_k)
-        meta = build_row_desc(lens_q, seqlens_k=lens_k)      # asserts 0 < q_len <= k_len
-        ws.bind_inputs(meta, q, k, v, self.W_o, page_table=page_table, cache_seqlens=cache_seqlens)
+            cu_k = cu_q if cu_seqlens_k is None else _cumulative(cu_seqlens_k)
+        if ws.paged:
+            cu_k = np.zeros(cu_q.size, dtype=np.int64)
+            np.cumsum(lens_k, out=cu_k[1:])
+        meta = native_row_desc(cu_q, cu_k, ws.max_num_row_tiles)      # asserts 0 < q_len <= k_len
+        ws.bind_inputs(meta, q, k, v, self.W_o, page_table=page_table, cache_seqlens=cache_seqlens,
+                       page_table_host=pages)
         ws.launch(flags)
         self.meta = meta
         return ws.csym[:meta.num_row_tiles]

@@ -19,14 +19,15 @@ torch is used for device memory, streams and (tp > 1) symmetric-memory bootstrap
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 
 import numpy as np
 import torch
 
 from .. import _cabi
-from ..metadata.launch_heuristic import fa_prime_tiles_b200, launch_flags_b200
-from ..metadata.row_desc import active_counts, oproj_task_counts
+from ..metadata.launch_heuristic import launch_flags_b200
+from ..metadata.row_desc import RowDescMeta, oproj_task_counts
 
 NUM_CTRL = 8
 NUM_SYNC = 3
@@ -64,6 +65,28 @@ def claim_order(meta, prime: int = 0) -> np.ndarray:
     if prime:
         order = np.concatenate([order[order.size - prime:][::-1], order[:order.size - prime]])
     return order
+
+
+def native_row_desc(cu_q, cu_k, max_row_tiles: int) -> RowDescMeta:
+    """``build_row_desc`` from cumulative lengths (int64 arrays), natively: the same object
+    and the same refusals, a tenth of the host time.  ``max_row_tiles`` bounds the schedule."""
+    cu_q = np.ascontiguousarray(cu_q, dtype=np.int64)
+    cu_k = np.ascontiguousarray(cu_k, dtype=np.int64)
+    nb = cu_q.size - 1
+    assert nb > 0 and cu_k.size == nb + 1
+    cap = int(max(0, min(max_row_tiles, int(cu_q[nb]) // 128 + nb)))
+    buf = np.empty(3 * (nb + 1) + 2 * cap, dtype=np.int32)
+    o_q, o_k, o_m = buf[:nb + 1], buf[nb + 1:2 * nb + 2], buf[2 * nb + 2:3 * nb + 3]
+    base = buf.ctypes.data
+    at = base + 12 * (nb + 1)
+    n = _cabi.lib.ma_row_desc(cu_q.ctypes.data, cu_k.ctypes.data, nb, cap, base, base + 4 * (nb + 1),
+                              base + 8 * (nb + 1), at, at + 4 * cap)
+    assert n != _cabi.MA_ERR_INVALID, "0 < q_len <= k_len per sequence"
+    assert n > 0, "more row tiles than the workspace was created for"
+    at = 3 * (nb + 1)
+    return RowDescMeta(num_batch=nb, M_TILE=128, cu_seqlens_q=o_q, cu_seqlens_k=o_k,
+                       num_row_tiles=n, cu_m_blocks=o_m, batch_idx=buf[at:at + n],
+                       m_block=buf[at + cap:at + cap + n])
 
 
 class FusedFaOprojArWorkspace:
@@ -309,7 +332,8 @@ class FusedFaOprojArWorkspace:
                 self.V[:tk].copy_(V, non_blocking=True)
             self._set_meta(meta)
 
-    def bind_inputs(self, meta, Q, K, V, W_o, page_table=None, cache_seqlens=None):
+    def bind_inputs(self, meta, Q, K, V, W_o, page_table=None, cache_seqlens=None, *,
+                    page_table_host=None):
         """Zero-copy alternative to ``set_layer``: the kernel reads the caller's device
         tensors in place (only the varlen metadata is uploaded).  ``W_o`` may be the plain
         ``[K_local, hidden]`` weight when ``hidden % 64 == 0``, else a zero-padded
@@ -331,7 +355,10 @@ class FusedFaOprojArWorkspace:
             page_table = torch.as_tensor(page_table, dtype=torch.int32)
             cache_seqlens = torch.as_tensor(cache_seqlens, dtype=torch.int32)
             assert page_table.shape[1] <= self.max_num_pages_per_seq
-            assert int(page_table.max()) < K.shape[0] and int(page_table.min()) >= 0
+            # (the caller may have the page table's values on the host already: one copy of
+            # theirs instead of two reductions and two waits for the GPU here)
+            pages = page_table if page_table_host is None else page_table_host
+            assert int(pages.max()) < K.shape[0] and int(pages.min()) >= 0
         else:
             assert tuple(K.shape[1:]) == (self.H_kv, self.D) == tuple(V.shape[1:])
             tot_k = K.shape[0]
@@ -340,7 +367,7 @@ class FusedFaOprojArWorkspace:
             self._plan, Q.data_ptr(), K.data_ptr(), V.data_ptr(), W_o.data_ptr(),
             int(Q.shape[0]), int(tot_k), int(W_o.shape[1])), "ma_plan_set_inputs")
         self._bound = (Q, K, V, W_o)          # keep them alive
-        with torch.cuda.stream(self._stream()):
+        with self._on_stream():
             if self.paged:
                 self.page_table[:nb, :page_table.shape[1]].copy_(page_table.to(self.dev))
                 self.cache_seqlens[:nb].copy_(cache_seqlens.to(self.dev))
@@ -377,22 +404,32 @@ class FusedFaOprojArWorkspace:
         self._meta_i += 1
         if slot[1] is not None:
             slot[1].synchronize()
-        buf = slot[0].numpy()
         o = self._meta_offs
-        prime = self.fa_prime_tiles
-        if prime is None:
-            prime = fa_prime_tiles_b200(meta, self.hidden, self.tp_size, self.H_local)
         self._auto_flags = launch_flags_b200(meta, self.hidden, self.tp_size, self.H_local)
-        for i, arr in enumerate((meta.cu_seqlens_q, meta.cu_seqlens_k, meta.batch_idx, meta.m_block,
-                                 claim_order(meta, prime),
-                                 active_counts(R, self.H_local, self.num_super_groups,
-                                               self.tp_size, self.rank))):
-            arr = np.asarray(arr, dtype=np.int32)
-            buf[o[i]:o[i] + arr.size] = arr
+        cu_q, cu_k, b_idx, m_blk = (np.ascontiguousarray(x, dtype=np.int32) for x in (
+            meta.cu_seqlens_q, meta.cu_seqlens_k, meta.batch_idx, meta.m_block))
+        assert b_idx.size == m_blk.size == R and cu_q.size == cu_k.size == meta.num_batch + 1
+        prime = self.fa_prime_tiles
+        args = _cabi.StageMetaArgs(
+            cu_q.ctypes.data, cu_k.ctypes.data, b_idx.ctypes.data, m_blk.ctypes.data,
+            slot[0].data_ptr(), cu_q.size - 1, R, self.hidden, self.H_local, self.num_super_groups,
+            self.tp_size, self.rank, int(prime is None),
+            0 if prime is None else max(-1, min(int(prime), R)),
+            o[0], o[1], o[2], o[3], o[4], o[5], 0)
+        _cabi.check(_cabi.lib.ma_stage_meta(C.byref(args)), "ma_stage_meta")
         self.meta_dev.copy_(slot[0], non_blocking=True)
-        slot[1] = torch.cuda.Event()
+        if slot[1] is None:
+            slot[1] = torch.cuda.Event()
         slot[1].record(torch.cuda.current_stream(self.dev))
         self._meta = meta
+
+    def _on_stream(self):
+        """``torch.cuda.stream(self._stream())``, or nothing to do if that is current (device
+        included): the usual case, and a fifth of a small step's host time."""
+        st = self._stream()
+        if torch.cuda.current_stream() == st:
+            return contextlib.nullcontext()
+        return torch.cuda.stream(st)
 
     def _stream(self):
         return getattr(self, "_ts", None) or torch.cuda.current_stream(self.dev)
