@@ -115,22 +115,24 @@ __device__ __forceinline__ bool wait_bar(const Env& e, uint32_t bar, uint32_t pa
 }
 
 // ---------------------------------------------------------------- scheduler (thread 0)
+// Attention task ids: CTA c starts with id c, without asking anybody; the counter hands out
+// the ids from gridDim.x on.  (A first task by way of the counters cost five dependent trips to
+// L2 with every CTA at the same words: 1.5 to 4 us of a launch.)
+// An id stands for one head, two heads of a kv group (pair), or two heads that share no kv
+// head and the last head of an odd count alone (sep); arg is position * H + first head.
+__device__ __forceinline__ int fa_tasks_per_tile(const KParams& p) {
+  return (p.pair || p.sep) ? (p.H + 1) >> 1 : p.H;
+}
+__device__ __forceinline__ int fa_task_arg(const KParams& p, int id) {
+  const int n = fa_tasks_per_tile(p);
+  return (id / n) * p.H + (id % n) * ((p.pair || p.sep) ? 2 : 1);
+}
 __device__ __forceinline__ bool try_fa(const KParams& p, int num_fa, int* arg) {
-  if (p.sep) {
-    // two heads per task, the last head of an odd count alone: the counter numbers tasks,
-    // (H + 1) / 2 per row tile; arg stays position * H + first head
-    const int hp = (p.H + 1) >> 1;
-    const int n_tasks = (num_fa / p.H) * hp;
-    if (static_cast<int>(ld_relaxed_gpu(p.ctrl + C_FA_COUNTER)) < n_tasks) {
-      const int id = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
-      if (id < n_tasks) { *arg = (id / hp) * p.H + 2 * (id % hp); return true; }
-    }
-    return false;
-  }
-  const uint32_t step = p.pair ? 2u : 1u;
-  if (static_cast<int>(ld_relaxed_gpu(p.ctrl + C_FA_COUNTER)) < num_fa) {
-    const uint32_t id = atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, step);
-    if (static_cast<int>(id) < num_fa) { *arg = static_cast<int>(id); return true; }
+  const int n_tasks = (num_fa / p.H) * fa_tasks_per_tile(p);
+  const int base = static_cast<int>(gridDim.x);
+  if (base + static_cast<int>(ld_relaxed_gpu(p.ctrl + C_FA_COUNTER)) < n_tasks) {
+    const int id = base + static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+    if (id < n_tasks) { *arg = fa_task_arg(p, id); return true; }
   }
   return false;
 }
@@ -619,6 +621,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     reg_dec<80>();
     if (warp == 2 && lane == 0) {
       // ==================================================================== scheduler
+      // (a launch after one that gave up does nothing until the state has been cleared)
+      const uint32_t status0 = ld_relaxed_gpu(p.status);
       const int num_fa = p.actv[0];
       const int local_owned = p.actv[5];
       // O_proj tasks.  With several ranks a task is an AllReduce slot: one row tile, up to
@@ -646,6 +650,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       bool ld_pending[2] = {false, false}, ld_skip[2] = {false, false};
       int pending_ticket = -1;
       uint32_t poll_no = 0;
+      bool first = true;
       int occ_mode[2] = {0, 0}, occ_a[2] = {0, 0}, occ_b[2] = {0, 0};
 #ifdef MA_AUDIT
       int occ_h[2] = {0, 0};
@@ -702,9 +707,17 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           ld_par[k ^ 1] ^= 1u;        // that task's loads_done phase is never waited for
           ld_skip[k ^ 1] = false;
         }
-        int mode, arg;
+        int mode = MODE_IDLE, arg = -1;
+        if (first) {
+          first = false;
+          const int id = static_cast<int>(blockIdx.x);
+          if (status0 == 0u && !(p.flags & (8u | 32u)) && id < (num_fa / p.H) * fa_tasks_per_tile(p)) {
+            mode = MODE_FA;
+            arg = fa_task_arg(p, id);
+          }
+        }
         uint64_t idle_t0 = 0;
-        while (true) {
+        while (mode == MODE_IDLE) {
           schedule_pick(env, role, num_fa, total_op, per_group, local_owned, poll_no++, occupied[k ^ 1],
                         &pending_ticket, &mode, &arg);
           if (mode != MODE_IDLE) break;
