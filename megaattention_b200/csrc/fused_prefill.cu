@@ -535,10 +535,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ CUtensorMap tmC,
                      const __grid_constant__ KParams p) {
   extern __shared__ uint8_t dyn_smem[];
-  // The words that threads spin on (the abort flag is read in every wait loop, the issuers'
-  // lock is hammered with atomics) get 128-byte lines of their own, away from the mbarriers:
-  // where the compiler put them next to the barrier block by default depended on the
-  // block's size, and one such placement cost the attention stage 2.5 % (0.1597 vs 0.1560 ms).
+  // The abort flag, read in every wait loop, gets a 128-byte line of its own: where the
+  // compiler put it next to the barrier block by default depended on the block's size, and one
+  // such placement cost the attention stage 2.5 % (0.1597 vs 0.1560 ms).
   __shared__ __align__(128) Bars bars;
   __shared__ uint32_t s_tmem;
   __shared__ __align__(128) int s_abort_line[32];
@@ -603,12 +602,19 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
   uint32_t n_arrived[2] = {0, 0};
   int prev_mode = MODE_IDLE, prev_k = 0;
 
-#define MA_NEXT_TASK(desc_ptr, mode_var)                                                   \
-  if (!wait_bar(env, smem_u32(&bars.task_full[slot_k]), tf_par[slot_k], 0x100 + warp)) break; \
+#define MA_TASK_FULL                                                                       \
+  wait_bar(env, smem_u32(&bars.task_full[slot_k]), tf_par[slot_k], 0x100 + warp)
+#define MA_NEXT_TASK_IF(full, desc_ptr, mode_var)                                          \
+  if (!(full)) break;                                                                      \
   tf_par[slot_k] ^= 1u;                                                                    \
   const int* desc_ptr = s_desc[slot_k];                                                    \
   const int mode_var = desc_ptr[T_MODE];                                                   \
   if (mode_var == MODE_DONE) break;
+#define MA_NEXT_TASK(desc_ptr, mode_var) MA_NEXT_TASK_IF(MA_TASK_FULL, desc_ptr, mode_var)
+// A whole warp takes the task or leaves together: its lanes may see an abort at different
+// times, and what follows has instructions that wait for all of them.
+#define MA_NEXT_TASK_WARP(desc_ptr, mode_var) \
+  MA_NEXT_TASK_IF(__all_sync(0xffffffffu, MA_TASK_FULL), desc_ptr, mode_var)
 #define MA_DRAIN_IF_SWITCH(mode_var)                                                       \
   if (is_tile_mode(mode_var) && is_tile_mode(prev_mode) && mode_var != prev_mode)          \
     wait_bar(env, smem_u32(&bars.task_empty[prev_k]), (n_arrived[prev_k] - 1u) & 1u, 0x110 + warp);
@@ -630,7 +636,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       // tiles x nnt column tiles (<= 2 x 2) in one pass, the row tiles sharing every W stage.
       int nrt = 0, nnt = p.sg, per_group = p.nsg, total_op = p.actv[1];
       const int n_tiles = p.actv[2];
-      if (p.tp == 1) {
+      if (p.tp == 1 && !(p.flags & 16u)) {      // (without AllReduce: slots, as with several)
         op_task_shape(n_tiles, p.num_out, static_cast<int>(gridDim.x), &nrt, &nnt);
         per_group = (p.num_out + nnt - 1) / nnt;
         // (plus what the host's count of slots is off by: such a launch must not end well)
@@ -866,7 +872,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0;
       uint32_t q_par[2] = {0, 0}, p_par[2] = {0, 0}, o_uses[2] = {0, 0}, acc_uses[2] = {0, 0};
       while (true) {
-        MA_NEXT_TASK(d, mode)
+        MA_NEXT_TASK_WARP(d, mode)
         MA_DRAIN_IF_SWITCH(mode)
         if (mode == MODE_FA) {
           // A tile's chain softmax -> P V -> next Q K^T is what bounds the loop: the V tile
@@ -1040,7 +1046,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     uint32_t s_par = 0, o_par = 0, acc_par[2] = {0, 0};
     while (true) {
-      MA_NEXT_TASK(d, mode)
+      MA_NEXT_TASK_WARP(d, mode)
       if (mode == MODE_FA && wg < d[TF_NT]) {
         // -------------------------------------------- softmax + epilogue of tile `wg`
         const int valid_m = d[TF_VALID];
@@ -1295,7 +1301,10 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       prev_mode = mode; prev_k = slot_k; slot_k ^= 1;
     }
   }
+#undef MA_TASK_FULL
+#undef MA_NEXT_TASK_IF
 #undef MA_NEXT_TASK
+#undef MA_NEXT_TASK_WARP
 #undef MA_DRAIN_IF_SWITCH
 #undef MA_TASK_DONE
 
