@@ -81,9 +81,14 @@ class FusedPrefillLayer:
                 v = v.view(-1, 128, ws.H_kv, ws.D)
             assert page_table.dim() == 2 and cache_seqlens.dim() == 1
             assert page_table.shape[0] == cu_q.size - 1 == cache_seqlens.shape[0]
-            # the lengths and the page numbers reach the host in one copy, one wait
-            if page_table.device == cache_seqlens.device:
-                both = torch.cat((cache_seqlens, page_table.reshape(-1))).cpu().numpy()
+            # The lengths, and what the page numbers are checked by, reach the host in one copy
+            # and one wait: a small table as it is, a large one as its smallest and largest
+            # number (copy / reduce / three waits: 33 / 39 / 59 us at 8000 entries, 38 / 40 / 59
+            # at 16000, 67 / 39 / 78 at 65000).
+            if page_table.device == cache_seqlens.device and page_table.numel():
+                what = (page_table.reshape(1, -1) if page_table.numel() < 16384
+                        else torch.stack(torch.aminmax(page_table)).reshape(1, -1))
+                both = torch.cat((cache_seqlens, what[0])).cpu().numpy()
                 lens_k, pages = both[:cu_q.size - 1].astype(np.int64), both[cu_q.size - 1:]
             else:
                 lens_k = cache_seqlens.cpu().numpy().astype(np.int64)
