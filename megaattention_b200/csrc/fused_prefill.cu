@@ -943,6 +943,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
                   // (the previous task's epilogue must have read O out)
                   if (jj == 0) wait_bar(env, smem_u32(&bars.o_free[i]), (o_uses[i] & 1u) ^ 1u, 0x68 + i);
                 }
+                // The lane that issues has seen one of these barriers at most, and a vote orders
+                // no memory: this hands it what the other lanes acquired (K by TMA, O read out).
+                __syncwarp();
                 if (jj == 0) ++o_uses[i];
               }
               wait_bar(env, smem_u32(&bars.p_part[i]), p_par[i], 0x58 + i);
