@@ -115,9 +115,10 @@ __device__ __forceinline__ bool wait_bar(const Env& e, uint32_t bar, uint32_t pa
 }
 
 // ---------------------------------------------------------------- scheduler (thread 0)
-// Attention task ids: CTA c starts with id c, without asking anybody; the counter hands out
-// the ids from gridDim.x on.  (A first task by way of the counters cost five dependent trips to
-// L2 with every CTA at the same words: 1.5 to 4 us of a launch.)
+// Attention task ids come from the counter, the first of every CTA too: a task belongs to a CTA
+// only once that CTA runs.  (Ids by CTA number save that atomic, but then a CTA that gets its
+// SM late - another stream's kernel holds it - keeps its task from all the others, which wait
+// for it up to the wait limit.)
 // An id stands for one head, two heads of a kv group (pair), or two heads that share no kv
 // head and the last head of an odd count alone (sep); arg is position * H + first head.
 __device__ __forceinline__ int fa_tasks_per_tile(const KParams& p) {
@@ -129,9 +130,8 @@ __device__ __forceinline__ int fa_task_arg(const KParams& p, int id) {
 }
 __device__ __forceinline__ bool try_fa(const KParams& p, int num_fa, int* arg) {
   const int n_tasks = (num_fa / p.H) * fa_tasks_per_tile(p);
-  const int base = static_cast<int>(gridDim.x);
-  if (base + static_cast<int>(ld_relaxed_gpu(p.ctrl + C_FA_COUNTER)) < n_tasks) {
-    const int id = base + static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+  if (static_cast<int>(ld_relaxed_gpu(p.ctrl + C_FA_COUNTER)) < n_tasks) {
+    const int id = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
     if (id < n_tasks) { *arg = fa_task_arg(p, id); return true; }
   }
   return false;
@@ -715,11 +715,16 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         }
         int mode = MODE_IDLE, arg = -1;
         if (first) {
+          // the first attention task with one atomic: nothing else can be ready yet, so none
+          // of schedule_pick's dependent loads is needed (five trips to L2 with every CTA at
+          // the same words, 1.5 to 4 us of a launch)
           first = false;
-          const int id = static_cast<int>(blockIdx.x);
-          if (status0 == 0u && !(p.flags & (8u | 32u)) && id < (num_fa / p.H) * fa_tasks_per_tile(p)) {
-            mode = MODE_FA;
-            arg = fa_task_arg(p, id);
+          if (status0 == 0u && !(p.flags & (8u | 32u))) {
+            const int id = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+            if (id < (num_fa / p.H) * fa_tasks_per_tile(p)) {
+              mode = MODE_FA;
+              arg = fa_task_arg(p, id);
+            }
           }
         }
         uint64_t idle_t0 = 0;

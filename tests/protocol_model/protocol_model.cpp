@@ -19,6 +19,8 @@
 // Faults are injected on the host only:
 //   --drop-arrival R S   rank R never reports O_proj slot S to its owner (a lost message)
 //   --straggler R MS     rank R starts every launch MS milliseconds late
+//   --late K MS          CTA K of every rank starts every launch MS milliseconds late (its SM
+//                        was taken); the others must not need it
 //   --leave R L          rank R does not take part in launches >= L (a rank that left between
 //                        steps); the others must time out and return, not hang
 //
@@ -43,9 +45,10 @@ enum { MODE_IDLE, MODE_FA, MODE_OPROJ, MODE_AR, MODE_DONE };
 struct Config {
   int tp = 2, ctas = 6, R = 12, H = 4, nsg = 3, launches = 3, limit_ms = 300;
   int drop_rank = -1, drop_slot = -1, strag_rank = -1, strag_ms = 0, leave_rank = -1, leave_from = 0;
-  // attention-task numbering, as in the kernel: 0 = one head per task; 1 = two heads that
-  // share a kv head (H even, the counter steps by 2 over head ids); 2 = two heads without a
-  // shared kv head (the counter numbers tasks, (H + 1) / 2 per row tile, last odd head alone)
+  int late_cta = -1, late_ms = 0;
+  // attention tasks, as in the kernel: 0 = one head per task; 1 = two heads that share a kv
+  // head (H even); 2 = two heads without a shared kv head (last odd head alone).  A row tile
+  // has (H + 1) / 2 of the two-headed ones.
   int pairing = 0;
 };
 
@@ -81,26 +84,21 @@ void report(Rank& r, uint32_t code, uint32_t site) {
 }
 
 // ---- the scheduler's three sources (same order of operations as the kernel)
+// attention tasks are numbered; the counter hands the numbers out
+int fa_tasks_per_tile(const Config& c) { return c.pairing ? (c.H + 1) >> 1 : c.H; }
+bool fa_task(const Config& c, int id, int num_fa, int* arg, int* nt) {
+  const int n = fa_tasks_per_tile(c);
+  if (id >= (num_fa / c.H) * n) return false;
+  const int head0 = (id % n) * (c.pairing ? 2 : 1);
+  *arg = (id / n) * c.H + head0;
+  *nt = c.pairing ? std::min(2, c.H - head0) : 1;
+  return true;
+}
 bool try_fa(Rank& r, const Config& c, int num_fa, int* arg, int* nt) {
-  if (c.pairing == 2) {
-    const int hp = (c.H + 1) >> 1, n_tasks = (num_fa / c.H) * hp;
-    if (static_cast<int>(r.ctrl[C_FA_COUNTER].load(std::memory_order_relaxed)) < n_tasks) {
-      const int id = static_cast<int>(r.ctrl[C_FA_COUNTER].fetch_add(1, std::memory_order_relaxed));
-      if (id < n_tasks) {
-        const int head0 = 2 * (id % hp);
-        *arg = (id / hp) * c.H + head0;
-        *nt = std::min(2, c.H - head0);
-        return true;
-      }
-    }
-    return false;
-  }
-  const uint32_t step = c.pairing == 1 ? 2u : 1u;
-  if (static_cast<int>(r.ctrl[C_FA_COUNTER].load(std::memory_order_relaxed)) < num_fa) {
-    const uint32_t id = r.ctrl[C_FA_COUNTER].fetch_add(step, std::memory_order_relaxed);
-    if (static_cast<int>(id) < num_fa) { *arg = static_cast<int>(id); *nt = static_cast<int>(step); return true; }
-  }
-  return false;
+  const int n_tasks = (num_fa / c.H) * fa_tasks_per_tile(c);
+  if (static_cast<int>(r.ctrl[C_FA_COUNTER].load(std::memory_order_relaxed)) >= n_tasks) return false;
+  return fa_task(c, static_cast<int>(r.ctrl[C_FA_COUNTER].fetch_add(1, std::memory_order_relaxed)),
+                 num_fa, arg, nt);
 }
 
 bool try_pop_oproj(Rank& r, int total_op, int* pending, int* arg) {
@@ -177,20 +175,29 @@ void cta_main(World& w, int rank, int cta) {
   bool aborted = false;
   auto idle_t0 = clk::now();
   bool idle = false;
+  bool first = r.status.load(std::memory_order_relaxed) == 0;
   while (true) {
-    if (r.status.load(std::memory_order_relaxed) != 0) { aborted = true; break; }
-    const bool done = static_cast<int>(r.ctrl[C_FA_DONE].load(std::memory_order_acquire)) >= num_fa &&
-                      static_cast<int>(r.ctrl[C_OP_DONE].load(std::memory_order_acquire)) >= total_op &&
-                      static_cast<int>(r.ctrl[C_AR_DONE].load(std::memory_order_acquire)) >= local_owned;
-    if (done) break;
     int mode = MODE_IDLE, arg = -1, nt = 1;
-    for (int i = 0; i < 3 && mode == MODE_IDLE; ++i) {
-      const int m = 1 + (role + i) % 3;
-      bool ok = false;
-      if (m == MODE_FA) ok = try_fa(r, c, num_fa, &arg, &nt);
-      else if (m == MODE_OPROJ) ok = try_pop_oproj(r, total_op, &pending, &arg);
-      else ok = try_claim_ar(w, rank, &arg);
-      if (ok) mode = m;
+    if (first) {              // the first attention task: one atomic, nothing else looked at
+      first = false;
+      if (fa_task(c, static_cast<int>(r.ctrl[C_FA_COUNTER].fetch_add(1, std::memory_order_relaxed)),
+                  num_fa, &arg, &nt))
+        mode = MODE_FA;
+    }
+    if (mode == MODE_IDLE) {
+      if (r.status.load(std::memory_order_relaxed) != 0) { aborted = true; break; }
+      const bool done = static_cast<int>(r.ctrl[C_FA_DONE].load(std::memory_order_acquire)) >= num_fa &&
+                        static_cast<int>(r.ctrl[C_OP_DONE].load(std::memory_order_acquire)) >= total_op &&
+                        static_cast<int>(r.ctrl[C_AR_DONE].load(std::memory_order_acquire)) >= local_owned;
+      if (done) break;
+      for (int i = 0; i < 3 && mode == MODE_IDLE; ++i) {
+        const int m = 1 + (role + i) % 3;
+        bool ok = false;
+        if (m == MODE_FA) ok = try_fa(r, c, num_fa, &arg, &nt);
+        else if (m == MODE_OPROJ) ok = try_pop_oproj(r, total_op, &pending, &arg);
+        else ok = try_claim_ar(w, rank, &arg);
+        if (ok) mode = m;
+      }
     }
     if (mode == MODE_IDLE) {
       if (!idle) { idle = true; idle_t0 = clk::now(); }
@@ -244,6 +251,7 @@ int main(int argc, char** argv) {
     else if (!strcmp(argv[i], "--limit-ms")) { c.limit_ms = next(1); i += 1; }
     else if (!strcmp(argv[i], "--drop-arrival")) { c.drop_rank = next(1); c.drop_slot = next(2); i += 2; }
     else if (!strcmp(argv[i], "--straggler")) { c.strag_rank = next(1); c.strag_ms = next(2); i += 2; }
+    else if (!strcmp(argv[i], "--late")) { c.late_cta = next(1); c.late_ms = next(2); i += 2; }
     else if (!strcmp(argv[i], "--leave")) { c.leave_rank = next(1); c.leave_from = next(2); i += 2; }
     else { std::fprintf(stderr, "unknown argument %s\n", argv[i]); return 2; }
   }
@@ -264,6 +272,7 @@ int main(int argc, char** argv) {
       for (int k = 0; k < c.ctas; ++k)
         th.emplace_back([&w, r, k, &c]() {
           if (r == c.strag_rank) std::this_thread::sleep_for(std::chrono::milliseconds(c.strag_ms));
+          if (k == c.late_cta) std::this_thread::sleep_for(std::chrono::milliseconds(c.late_ms));
           cta_main(w, r, k);
         });
     }

@@ -39,14 +39,24 @@ def test_every_task_runs_exactly_once_and_the_exit_is_clean(model, tp, ctas, til
 
 @pytest.mark.parametrize("pairing,heads", [(1, 4), (1, 8), (2, 2), (2, 3), (2, 5), (2, 8)])
 def test_attention_tasks_of_two_heads_count_every_head_once(model, pairing, heads):
-    """The kernel's two-head attention tasks: heads sharing a kv head (the counter steps by
-    two over head ids) and heads that share none (the counter numbers tasks, the last head of
-    an odd count runs alone).  Every (row tile, head) once, the row tile's head count reaches
+    """The kernel's two-head attention tasks: heads sharing a kv head and heads that
+    share none (the last head of an odd count runs alone); the counter numbers tasks.  Every (row tile, head) once, the row tile's head count reaches
     H exactly once, six launches without a reset."""
     out = model("--tp", 2, "--ctas", 5, "--tiles", 9, "--heads", heads, "--nsg", 3,
                 "--pairing", pairing, "--launches", 6, "--limit-ms", 5000)
     assert out["launches_ok"] == 6 and out["exactly_once"] and out["clean_exit"], out
     assert all(s == [0, 0] for s in out["status"]), out
+
+
+@pytest.mark.parametrize("ctas,cta", [(5, 0), (5, 2), (5, 4), (2, 0)])
+def test_nobody_waits_for_a_cta_that_starts_late(model, ctas, cta):
+    """A CTA whose SM is held by another kernel starts when the wait limit of the others is
+    long past: they do its share (no task belongs to a CTA that does not run), and it finds
+    the launch done."""
+    out = model("--tp", 1, "--ctas", ctas, "--tiles", 9, "--heads", 4, "--nsg", 3, "--pairing", 1,
+                "--launches", 2, "--limit-ms", 250, "--late", cta, 1000)
+    assert out["launches_ok"] == 2 and out["exactly_once"] and out["clean_exit"], out
+    assert out["status"] == [[0, 0]] and out["worst_launch_ms"] >= 1000, out
 
 
 def test_a_straggler_rank_is_waited_for(model):
