@@ -300,8 +300,10 @@ int ma_detile(const ma_detile_args* args, void* stream);
  * Host side of one step's varlen metadata (no device work).  ma_row_desc builds the row-tile
  * schedule from cumulative lengths and returns the number of row tiles (>= 1) or an error:
  * MA_ERR_INVALID unless both start at 0 and 0 < q_len <= k_len for every sequence,
- * MA_ERR_CAPACITY past max_row_tiles (the length of batch_idx and m_block) or 2^31 - 1 rows.
- * The other outputs hold num_batch + 1 words.
+ * MA_ERR_CAPACITY past max_row_tiles (the length of batch_idx and m_block), 2^31 - 1 query
+ * rows or 2^31 - 1 keys of one sequence.  The other outputs hold num_batch + 1 words; cu_k_out
+ * is the sum modulo 2^32 (the sequences of a paged batch may share pages, so that their lengths
+ * sum past any cache), and ma_stage_meta takes its differences the same way.
  */
 int ma_row_desc(const int64_t* cu_q, const int64_t* cu_k, int32_t num_batch,
                 int32_t max_row_tiles, int32_t* cu_q_out, int32_t* cu_k_out,

@@ -23,7 +23,7 @@ extern "C" int ma_row_desc(const int64_t* cu_q, const int64_t* cu_k, int32_t num
   for (int b = 0; b < num_batch; ++b) {
     const int64_t lq = cu_q[b + 1] - cu_q[b], lk = cu_k[b + 1] - cu_k[b];
     if (lq <= 0 || lk < lq) return MA_ERR_INVALID;
-    if (cu_q[b + 1] > 0x7fffffff || cu_k[b + 1] > 0x7fffffff) return MA_ERR_CAPACITY;
+    if (cu_q[b + 1] > 0x7fffffff || lk > 0x7fffffff) return MA_ERR_CAPACITY;
     const int64_t n = (lq + 127) / 128;
     if (tiles + n > max_row_tiles) return MA_ERR_CAPACITY;
     for (int64_t j = 0; j < n; ++j) {
@@ -32,7 +32,9 @@ extern "C" int ma_row_desc(const int64_t* cu_q, const int64_t* cu_k, int32_t num
     }
     tiles += n;
     cu_q_out[b + 1] = static_cast<int32_t>(cu_q[b + 1]);
-    cu_k_out[b + 1] = static_cast<int32_t>(cu_k[b + 1]);
+    // (paged sequences share pages: their lengths may sum past 2^31, and only differences of
+    // this sum are used)
+    cu_k_out[b + 1] = static_cast<int32_t>(static_cast<uint32_t>(cu_k[b + 1]));
     cu_m_blocks[b + 1] = static_cast<int32_t>(tiles);
   }
   return static_cast<int>(tiles);
@@ -53,10 +55,12 @@ extern "C" int ma_stage_meta(const ma_stage_meta_args* a) {
     for (int t = 0; t < R; ++t) {
       const int b = a->batch_idx[t];
       if (b < 0 || b >= B) return MA_ERR_INVALID;
-      const int64_t lq = a->cu_q[b + 1] - a->cu_q[b], lk = a->cu_k[b + 1] - a->cu_k[b];
+      const int64_t lq = static_cast<int64_t>(a->cu_q[b + 1]) - a->cu_q[b];
+      const int64_t lk = static_cast<int32_t>(static_cast<uint32_t>(a->cu_k[b + 1]) -
+                                              static_cast<uint32_t>(a->cu_k[b]));
       const int64_t last = (static_cast<int64_t>(a->m_block[t]) + 1) * 128 + (lk - lq);
       const int64_t n = std::min((lk + 127) / 128, (last + 127) / 128);
-      if (n < 0 || n > 0x7fffffff / 128) return MA_ERR_INVALID;
+      if (n < 0) return MA_ERR_INVALID;
       nblk[t] = static_cast<int32_t>(n);
       sum += n;
       most = std::max(most, nblk[t]);

@@ -67,3 +67,26 @@ def test_more_tiles_than_the_bound_is_refused():
     assert native_row_desc([0, 257], [0, 257], 3).num_row_tiles == 3
     with pytest.raises(AssertionError):
         native_row_desc([0, 257], [0, 257], 2)
+
+
+def test_key_lengths_may_sum_past_int32():
+    """Paged sequences share pages, so a batch's key lengths may sum past 2^31 - 1; the numpy
+    statement narrows the sum and goes on, and so does the native one, with the true lengths in
+    the claim order."""
+    big = 1 << 30
+    q, k = [1, 300, 1, 200], [big, big + 256, big - 128, 250]
+    want, got = build_row_desc(q, seqlens_k=k), native_row_desc(_cu(q), _cu(k), 100)
+    for f in ("cu_seqlens_q", "cu_seqlens_k", "cu_m_blocks", "batch_idx", "m_block"):
+        assert np.array_equal(getattr(got, f), getattr(want, f)), f
+    R, nb = got.num_row_tiles, got.num_batch
+    offs = np.cumsum([0, nb + 1, nb + 1, R, R, R])
+    buf = np.zeros(int(offs[-1]) + 6, dtype=np.int32)
+    for meta in (got, want):
+        a = _cabi.StageMetaArgs(
+            meta.cu_seqlens_q.ctypes.data, meta.cu_seqlens_k.ctypes.data, meta.batch_idx.ctypes.data,
+            meta.m_block.ctypes.data, buf.ctypes.data, nb, R, 4096, 8, 8, 1, 0, 0, 0, *map(int, offs), 0)
+        assert _cabi.lib.ma_stage_meta(C.byref(a)) == _cabi.MA_OK
+        # key blocks beyond 2^23: 0 | 1, 2, 2 | -1; the last sequence has two a tile
+        assert buf[offs[4]:offs[5]].tolist() == [2, 3, 1, 0, 4, 5, 6]
+    with pytest.raises(AssertionError):
+        native_row_desc(_cu([1]), _cu([1 << 31]), 100)
