@@ -517,6 +517,8 @@ __device__ __forceinline__ void op_task_shape(int n_tiles, int num_out, int ctas
   *nnt = 4 * t22 >= 5 * ctas ? 2 : 1;
 }
 
+template <bool kSeparate> struct Layout { static constexpr bool value = kSeparate; };   // of K/V stages
+
 // Task descriptor words written by the scheduler (shared memory, two slots).
 enum : int { T_MODE = 0, T_FT = 1,
              TF_HEAD0 = 2, TF_NT = 3, TF_KVH = 4, TF_QROW0 = 5, TF_VALID = 6, TF_KSTART = 7,
@@ -890,94 +892,119 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           // tokens 150 -> 137.6 us; with a 16384-token prompt the whole launch 631 -> 601 us.)
           const int nblk = d[TF_NBLK], nt = d[TF_NT];
           // Shared K/V stages: one slot per operand and key block.  Separate stages (p.sep):
-          // nt slots, the i-th for tile i.
-          const bool sep = p.sep != 0;
-          const int per = sep ? nt : 1;
-          struct SlotAt { uint32_t slot, ph; };
-          auto take = [&]() {                       // the next `per` slots of the ring
-            const SlotAt r{kv_slot, kv_ph};
-            kv_slot += static_cast<uint32_t>(per);
-            if (kv_slot >= static_cast<uint32_t>(kKvSlots)) { kv_slot -= kKvSlots; kv_ph ^= 1u; }
-            return r;
-          };
-          auto at = [&](SlotAt r, int i) {          // tile i's slot among them
-            if (sep && i) {
-              if (++r.slot == static_cast<uint32_t>(kKvSlots)) { r.slot = 0; r.ph ^= 1u; }
-            }
-            return r;
-          };
-          auto wait_slots = [&](SlotAt r, uint32_t site) {
-            for (int i = 0; i < per; ++i) {
-              const SlotAt x = at(r, i);
-              wait_bar(env, smem_u32(&bars.kv_full[x.slot]), x.ph, site + x.slot);
-            }
-          };
-          SlotAt k = take();
-          for (int i = 0; i < nt; ++i) {
-            wait_bar(env, smem_u32(&bars.q_full[i]), q_par[i], 0x20 + i);
-            q_par[i] ^= 1u;
-            if (i == 0) wait_slots(k, 0x30);
-            tc_fence_after();
-            const uint32_t ks = at(k, i).slot;
-            if (elect_one()) {
-              issue_qk(tmem + kTmemS + i * 128, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
-              tc_commit(smem_u32(&bars.s_full[i]));
-              if (sep || i == nt - 1) tc_commit(smem_u32(&bars.kv_empty[ks]));
-              if (nblk == 1) tc_commit(smem_u32(&bars.q_empty[i]));
-            }
-            __syncwarp();
-          }
-          for (int jj = 0; jj < nblk; ++jj) {
-            const bool has_next = (jj + 1 < nblk);
-            const SlotAt v = take();
-            if (has_next) k = take();
+          // nt slots, the i-th for tile i.  Two instances of the loop: a test of the layout in it
+          // costs the shared one 2 %.
+          auto run = [&](auto layout) {
+            constexpr bool sep = decltype(layout)::value;
+            const int per = sep ? nt : 1;
+            struct SlotAt { uint32_t slot, ph; };
+            auto take = [&]() {                       // the next `per` slots of the ring
+              const SlotAt r{kv_slot, kv_ph};
+              kv_slot += static_cast<uint32_t>(per);
+              if (kv_slot >= static_cast<uint32_t>(kKvSlots)) { kv_slot -= kKvSlots; kv_ph ^= 1u; }
+              return r;
+            };
+            auto at = [&](SlotAt r, int i) {          // tile i's slot among them
+              if (sep && i) {
+                if (++r.slot == static_cast<uint32_t>(kKvSlots)) { r.slot = 0; r.ph ^= 1u; }
+              }
+              return r;
+            };
+            auto wait_slots = [&](SlotAt r, uint32_t site) {
+              for (int i = 0; i < per; ++i) {
+                const SlotAt x = at(r, i);
+                wait_bar(env, smem_u32(&bars.kv_full[x.slot]), x.ph, site + x.slot);
+              }
+            };
+            SlotAt k = take();
             for (int i = 0; i < nt; ++i) {
-              const uint32_t t_s = tmem + kTmemS + i * 128, t_o = tmem + kTmemO + i * 128;
-              const uint32_t vs = at(v, i).slot, ks = at(k, i).slot;
-              const uint32_t sm_v = smem0 + kSmKV + vs * kTile;
-              const bool last_use = sep || i == nt - 1;
-              // The operands are nearly always there: one look at all their barriers, a lane
-              // each, and a wait one by one only if one of them is not.
-              if (sep || i == 0 || jj == 0) {
-                uint32_t bar = smem_u32(&bars.kv_full[vs]), par = at(v, i).ph;
-                if (lane == 1 && has_next) { bar = smem_u32(&bars.kv_full[ks]); par = at(k, i).ph; }
-                if (lane == 2 && jj == 0) { bar = smem_u32(&bars.o_free[i]); par = (o_uses[i] & 1u) ^ 1u; }
-                if (!__all_sync(0xffffffffu, mbar_test_wait(bar, par))) {
-                  wait_bar(env, smem_u32(&bars.kv_full[vs]), at(v, i).ph, 0x40 + vs);
-                  if (has_next) wait_bar(env, smem_u32(&bars.kv_full[ks]), at(k, i).ph, 0x50 + ks);
-                  // (the previous task's epilogue must have read O out)
-                  if (jj == 0) wait_bar(env, smem_u32(&bars.o_free[i]), (o_uses[i] & 1u) ^ 1u, 0x68 + i);
-                }
-                // The lane that issues has seen one of these barriers at most, and a vote orders
-                // no memory: this hands it what the other lanes acquired (K by TMA, O read out).
-                __syncwarp();
-                if (jj == 0) ++o_uses[i];
-              }
-              wait_bar(env, smem_u32(&bars.p_part[i]), p_par[i], 0x58 + i);
+              wait_bar(env, smem_u32(&bars.q_full[i]), q_par[i], 0x20 + i);
+              q_par[i] ^= 1u;
+              if (i == 0) wait_slots(k, 0x30);
               tc_fence_after();
-              if (elect_one()) issue_pv<0, 6>(t_o, t_s, sm_v, jj > 0);
-              __syncwarp();
-              wait_bar(env, smem_u32(&bars.p_full[i]), p_par[i], 0x60 + i);
-              p_par[i] ^= 1u;
-              tc_fence_after();
+              const uint32_t ks = at(k, i).slot;
               if (elect_one()) {
-                issue_pv<6, 8>(t_o, t_s, sm_v, true);
-                if (has_next) {
-                  issue_qk(t_s, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
-                  tc_commit(smem_u32(&bars.s_full[i]));
-                  if (last_use) {
-                    tc_commit(smem_u32(&bars.kv_empty[vs]));
-                    tc_commit(smem_u32(&bars.kv_empty[ks]));
-                  }
-                  if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[i]));
-                } else {
-                  tc_commit(smem_u32(&bars.o_done[i]));
-                  if (last_use) tc_commit(smem_u32(&bars.kv_empty[vs]));
-                }
+                issue_qk(tmem + kTmemS + i * 128, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+                tc_commit(smem_u32(&bars.s_full[i]));
+                if (sep || i == nt - 1) tc_commit(smem_u32(&bars.kv_empty[ks]));
+                if (nblk == 1) tc_commit(smem_u32(&bars.q_empty[i]));
               }
               __syncwarp();
             }
-          }
+            for (int jj = 0; jj < nblk; ++jj) {
+              const bool has_next = (jj + 1 < nblk);
+              const SlotAt v = take();
+              if (has_next) k = take();
+              for (int i = 0; i < nt; ++i) {
+                const uint32_t t_s = tmem + kTmemS + i * 128, t_o = tmem + kTmemO + i * 128;
+                const uint32_t vs = at(v, i).slot, ks = at(k, i).slot;
+                const uint32_t sm_v = smem0 + kSmKV + vs * kTile;
+                const bool last_use = sep || i == nt - 1;
+                // The operands are nearly always there: one look at all their barriers, a lane
+                // each, and a wait one by one only if one of them is not.
+                if (sep || i == 0 || jj == 0) {
+                  uint32_t bar = smem_u32(&bars.kv_full[vs]), par = at(v, i).ph;
+                  if (!sep && lane == 1 && has_next) { bar = smem_u32(&bars.kv_full[ks]); par = at(k, i).ph; }
+                  if (lane == 2 && jj == 0) { bar = smem_u32(&bars.o_free[i]); par = (o_uses[i] & 1u) ^ 1u; }
+                  if (!__all_sync(0xffffffffu, mbar_test_wait(bar, par))) {
+                    wait_bar(env, smem_u32(&bars.kv_full[vs]), at(v, i).ph, 0x40 + vs);
+                    if (!sep && has_next) wait_bar(env, smem_u32(&bars.kv_full[ks]), at(k, i).ph, 0x50 + ks);
+                    // (the previous task's epilogue must have read O out)
+                    if (jj == 0) wait_bar(env, smem_u32(&bars.o_free[i]), (o_uses[i] & 1u) ^ 1u, 0x68 + i);
+                  }
+                  // The lane that issues has seen one of these barriers at most, and a vote orders
+                  // no memory: this hands it what the other lanes acquired (K by TMA, O read out).
+                  __syncwarp();
+                  if (jj == 0) ++o_uses[i];
+                }
+                wait_bar(env, smem_u32(&bars.p_part[i]), p_par[i], 0x58 + i);
+                tc_fence_after();
+                if (elect_one()) issue_pv<0, 6>(t_o, t_s, sm_v, jj > 0);
+                __syncwarp();
+                wait_bar(env, smem_u32(&bars.p_full[i]), p_par[i], 0x60 + i);
+                p_par[i] ^= 1u;
+                tc_fence_after();
+                if constexpr (sep) {
+                  // The ring holds 1.25 key blocks here: the next K tile comes late, and P V must not
+                  // wait for it (looked at before P as below, the stage lost up to 12 % on MHA).
+                  if (has_next) {
+                    if (elect_one()) {
+                      issue_pv<6, 8>(t_o, t_s, sm_v, true);
+                      tc_commit(smem_u32(&bars.kv_empty[vs]));
+                    }
+                    __syncwarp();
+                    wait_bar(env, smem_u32(&bars.kv_full[ks]), at(k, i).ph, 0x50 + ks);
+                    tc_fence_after();
+                    if (elect_one()) {
+                      issue_qk(t_s, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+                      tc_commit(smem_u32(&bars.s_full[i]));
+                      tc_commit(smem_u32(&bars.kv_empty[ks]));
+                      if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[i]));
+                    }
+                    __syncwarp();
+                    continue;
+                  }
+                }
+                if (elect_one()) {
+                  issue_pv<6, 8>(t_o, t_s, sm_v, true);
+                  if (!sep && has_next) {
+                    issue_qk(t_s, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+                    tc_commit(smem_u32(&bars.s_full[i]));
+                    if (last_use) {
+                      tc_commit(smem_u32(&bars.kv_empty[vs]));
+                      tc_commit(smem_u32(&bars.kv_empty[ks]));
+                    }
+                    if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[i]));
+                  } else {
+                    tc_commit(smem_u32(&bars.o_done[i]));
+                    if (last_use) tc_commit(smem_u32(&bars.kv_empty[vs]));
+                  }
+                }
+                __syncwarp();
+              }
+            }
+          };
+          if (p.sep) run(Layout<true>{}); else run(Layout<false>{});
         } else if (mode == MODE_OPROJ) {
           const int vnt = d[TO_VNT], nrt = d[TO_NRT];
           const int nkc = p.K_local >> 6;
