@@ -5,8 +5,9 @@
 // scheduler.  The state machines are the ones of csrc/fused_prefill.cu (which follow the
 // reference's src/mega_attention/kernels/sm90/fused_fa_oproj_ar.py:148-398, 1154-1177):
 //
-//   attention task counter -> per-row-tile head count -> ordered O_proj ready queue
-//   (reserve / fill / publish in reservation order) -> ticket pop -> owner rank's ready count
+//   attention task counter -> head count per group of row tiles -> ordered O_proj ready queue
+//   (reserve / fill / publish in reservation order; an entry is a group and stands for its
+//   tickets) -> ticket pop -> owner rank's ready count
 //   (one arrival per rank, one byte per slot) -> claim by atomic OR of the slot's flag -> done counters -> count-out exit with
 //   full-capacity clear by the last CTA -> phase/sign barrier across the ranks.
 //
@@ -50,6 +51,8 @@ struct Config {
   // head (H even); 2 = two heads without a shared kv head (last odd head alone).  A row tile
   // has (H + 1) / 2 of the two-headed ones.
   int pairing = 0;
+  int group = 1;         // row tiles of an O_proj task (2 on one rank only), nsg tasks per group
+  int groups() const { return (R + group - 1) / group; }
 };
 
 struct Rank {
@@ -60,8 +63,9 @@ struct Rank {
   std::atomic<uint32_t> nvl_counter{0};
   // audit (not part of the protocol)
   std::vector<std::atomic<uint32_t>> fa_runs, op_runs, ar_runs;
-  Rank(int R, int H, int total, int owned)
-      : head_ready(R), queue(total), ready_count(owned), fa_runs(R * H), op_runs(total), ar_runs(owned) {
+  std::atomic<uint32_t> early{0};      // O_proj tasks that ran before their attention
+  Rank(int R, int H, int groups, int total, int owned)
+      : head_ready(R), queue(groups), ready_count(owned), fa_runs(R * H), op_runs(total), ar_runs(owned) {
     for (auto& c : ctrl) c = 0;
     nvl_signal[0] = 0; nvl_signal[1] = 0;
   }
@@ -70,7 +74,7 @@ struct Rank {
 struct World {
   Config cfg;
   std::vector<Rank*> ranks;
-  int total_op() const { return cfg.R * cfg.nsg; }
+  int total_op() const { return cfg.groups() * cfg.nsg; }
   int owned(int rank) const { int t = total_op() - rank; return t <= 0 ? 0 : (t + cfg.tp - 1) / cfg.tp; }
 };
 
@@ -101,7 +105,7 @@ bool try_fa(Rank& r, const Config& c, int num_fa, int* arg, int* nt) {
                  num_fa, arg, nt);
 }
 
-bool try_pop_oproj(Rank& r, int total_op, int* pending, int* arg) {
+bool try_pop_oproj(Rank& r, int total_op, int per_group, int* pending, int* arg) {
   if (*pending < 0) {
     const uint32_t head = r.ctrl[C_OP_CONSUME].load(std::memory_order_relaxed);
     const uint32_t tail = r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire);
@@ -113,7 +117,8 @@ bool try_pop_oproj(Rank& r, int total_op, int* pending, int* arg) {
   } else if (static_cast<uint32_t>(*pending) >= r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire)) {
     return false;
   }
-  *arg = static_cast<int>(r.queue[*pending].load(std::memory_order_relaxed));
+  *arg = static_cast<int>(r.queue[*pending / per_group].load(std::memory_order_relaxed)) * per_group +
+         *pending % per_group;
   *pending = -1;
   return true;
 }
@@ -136,10 +141,10 @@ bool try_claim_ar(World& w, int rank, int* arg) {
   return false;
 }
 
-void publish_oproj(World& w, Rank& r, int row_tile) {
+void publish_oproj(World& w, Rank& r, int group) {
   const uint32_t n = static_cast<uint32_t>(w.cfg.nsg);
   const uint32_t start = r.ctrl[C_OP_RESERVE].fetch_add(n, std::memory_order_relaxed);
-  for (uint32_t i = 0; i < n; ++i) r.queue[start + i].store(row_tile * n + i, std::memory_order_relaxed);
+  r.queue[start / n].store(static_cast<uint32_t>(group), std::memory_order_relaxed);
   std::atomic_thread_fence(std::memory_order_acq_rel);
   const auto t0 = clk::now();
   while (r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire) != start) {
@@ -194,7 +199,7 @@ void cta_main(World& w, int rank, int cta) {
         const int m = 1 + (role + i) % 3;
         bool ok = false;
         if (m == MODE_FA) ok = try_fa(r, c, num_fa, &arg, &nt);
-        else if (m == MODE_OPROJ) ok = try_pop_oproj(r, total_op, &pending, &arg);
+        else if (m == MODE_OPROJ) ok = try_pop_oproj(r, total_op, c.nsg, &pending, &arg);
         else ok = try_claim_ar(w, rank, &arg);
         if (ok) mode = m;
       }
@@ -208,12 +213,15 @@ void cta_main(World& w, int rank, int cta) {
     idle = false;
     if (mode == MODE_FA) {
       for (int i = 0; i < nt; ++i) r.fa_runs[arg + i].fetch_add(1);
-      const int ft = arg / c.H;
-      const uint32_t old = r.head_ready[ft].fetch_add(static_cast<uint32_t>(nt), std::memory_order_acq_rel);
-      if (static_cast<int>(old) + nt == c.H) publish_oproj(w, r, ft);
+      const int g = arg / c.H / c.group;
+      const uint32_t old = r.head_ready[g].fetch_add(static_cast<uint32_t>(nt), std::memory_order_acq_rel);
+      if (static_cast<int>(old) + nt == c.H * std::min(c.group, c.R - g * c.group)) publish_oproj(w, r, g);
       r.ctrl[C_FA_DONE].fetch_add(static_cast<uint32_t>(nt), std::memory_order_release);
     } else if (mode == MODE_OPROJ) {
       r.op_runs[arg].fetch_add(1);
+      for (int t = arg / c.nsg * c.group; t < std::min(c.R, (arg / c.nsg + 1) * c.group); ++t)
+        for (int h = 0; h < c.H; ++h)      // its row tiles' attention has to be done
+          if (r.fa_runs[t * c.H + h].load() != 1) r.early.fetch_add(1);
       const int owner = arg % c.tp, idx = arg / c.tp;
       if (!(rank == c.drop_rank && arg == c.drop_slot))           // injected lost arrival
         w.ranks[owner]->ready_count[idx >> 2].fetch_add(1u << ((idx & 3) * 8), std::memory_order_release);
@@ -247,6 +255,7 @@ int main(int argc, char** argv) {
     else if (!strcmp(argv[i], "--heads")) { c.H = next(1); i += 1; }
     else if (!strcmp(argv[i], "--nsg")) { c.nsg = next(1); i += 1; }
     else if (!strcmp(argv[i], "--pairing")) { c.pairing = next(1); i += 1; }
+    else if (!strcmp(argv[i], "--group")) { c.group = next(1); i += 1; }
     else if (!strcmp(argv[i], "--launches")) { c.launches = next(1); i += 1; }
     else if (!strcmp(argv[i], "--limit-ms")) { c.limit_ms = next(1); i += 1; }
     else if (!strcmp(argv[i], "--drop-arrival")) { c.drop_rank = next(1); c.drop_slot = next(2); i += 2; }
@@ -257,8 +266,8 @@ int main(int argc, char** argv) {
   }
   World w;
   w.cfg = c;
-  const int total = c.R * c.nsg;
-  for (int r = 0; r < c.tp; ++r) w.ranks.push_back(new Rank(c.R, c.H, total, w.owned(r) + 1));
+  for (int r = 0; r < c.tp; ++r)
+    w.ranks.push_back(new Rank(c.R, c.H, c.groups(), w.total_op(), w.owned(r) + 1));
 
   bool exactly_once = true, clean_exit = true;
   int launches_ok = 0;
@@ -292,6 +301,7 @@ int main(int argc, char** argv) {
     for (int r = 0; r < c.tp; ++r) {
       Rank& k = *w.ranks[r];
       for (auto& x : k.fa_runs) { if (x.load() != 1) exactly_once = false; x = 0; }
+      if (k.early.load()) exactly_once = false;
       for (auto& x : k.op_runs) { if (x.load() != 1) exactly_once = false; x = 0; }
       for (int i = 0; i < w.owned(r); ++i) { if (k.ar_runs[i].load() != 1) exactly_once = false; k.ar_runs[i] = 0; }
       for (int i = 0; i < C_NUM; ++i) if (k.ctrl[i].load() != 0) clean_exit = false;

@@ -48,6 +48,17 @@ def test_attention_tasks_of_two_heads_count_every_head_once(model, pairing, head
     assert all(s == [0, 0] for s in out["status"]), out
 
 
+@pytest.mark.parametrize("tiles", [1, 2, 9, 10])
+@pytest.mark.parametrize("pairing", [0, 1, 2])
+def test_one_rank_groups_of_two_row_tiles(model, tiles, pairing):
+    """One rank's O_proj tasks of two row tiles: a queue entry stands for a group's tasks and is
+    published when the attention of all its row tiles is done (the last group may have one)."""
+    for nsg in (1, 3):
+        out = model("--tp", 1, "--ctas", 6, "--tiles", tiles, "--heads", 4, "--nsg", nsg, "--group", 2,
+                    "--pairing", pairing, "--launches", 6, "--limit-ms", 5000)
+        assert out["launches_ok"] == 6 and out["exactly_once"] and out["clean_exit"], out
+
+
 @pytest.mark.parametrize("ctas,cta", [(5, 0), (5, 2), (5, 4), (2, 0)])
 def test_nobody_waits_for_a_cta_that_starts_late(model, ctas, cta):
     """A CTA whose SM is held by another kernel starts when the wait limit of the others is
