@@ -39,6 +39,20 @@ def _cumulative(cu):
     return cu
 
 
+def _lengths_and_pages(cache_seqlens, page_table):
+    """The key lengths on the host (int64), and numbers whose smallest and largest are the page
+    table's (None: look at the table itself), both from one copy and one wait: a small table
+    comes as it is, a large one as its extremes (copy / reduce / three waits: 33 / 39 / 59 us at
+    8000 entries, 38 / 40 / 59 at 16000, 67 / 39 / 78 at 65000)."""
+    if page_table.device != cache_seqlens.device or not page_table.numel():
+        return cache_seqlens.cpu().numpy().astype(np.int64), None
+    what = (page_table.reshape(-1) if page_table.numel() < 16384
+            else torch.stack(torch.aminmax(page_table)))
+    both = torch.cat((cache_seqlens, what)).cpu().numpy()
+    n = cache_seqlens.shape[0]
+    return both[:n].astype(np.int64), both[n:]
+
+
 class FusedPrefillLayer:
     def __init__(self, workspace, W_o):
         """``W_o [K_local, hidden]`` (input-major, i.e. ``nn.Linear.weight.T``), host or
@@ -81,17 +95,7 @@ class FusedPrefillLayer:
                 v = v.view(-1, 128, ws.H_kv, ws.D)
             assert page_table.dim() == 2 and cache_seqlens.dim() == 1
             assert page_table.shape[0] == cu_q.size - 1 == cache_seqlens.shape[0]
-            # The lengths, and what the page numbers are checked by, reach the host in one copy
-            # and one wait: a small table as it is, a large one as its smallest and largest
-            # number (copy / reduce / three waits: 33 / 39 / 59 us at 8000 entries, 38 / 40 / 59
-            # at 16000, 67 / 39 / 78 at 65000).
-            if page_table.device == cache_seqlens.device and page_table.numel():
-                what = (page_table.reshape(1, -1) if page_table.numel() < 16384
-                        else torch.stack(torch.aminmax(page_table)).reshape(1, -1))
-                both = torch.cat((cache_seqlens, what[0])).cpu().numpy()
-                lens_k, pages = both[:cu_q.size - 1].astype(np.int64), both[cu_q.size - 1:]
-            else:
-                lens_k = cache_seqlens.cpu().numpy().astype(np.int64)
+            lens_k, pages = _lengths_and_pages(cache_seqlens, page_table)
             assert page_table.shape[1] >= int((-(-lens_k // 128)).max()), \
                 "page_table is narrower than the longest sequence needs"
         else:

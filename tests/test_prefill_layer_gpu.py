@@ -80,3 +80,41 @@ def test_paged_token_pool_cache():
     with pytest.raises(AssertionError):                  # page table too narrow
         layer(Q.cuda(), pool_k, pool_v, _cu(sq), page_table=table[:, :1].contiguous().cuda(),
               cache_seqlens=lens.cuda())
+
+
+@pytest.mark.parametrize("width", [0, 8192])
+def test_page_numbers_out_of_range_are_refused_before_the_launch(width):
+    """A narrow table and one of 16384 entries or more (checked by its extremes): a valid call,
+    then a page that does not exist at the first and the last entry, refused on the host."""
+    from megaattention_b200.runtime import FusedFaOprojArWorkspace, FusedPrefillLayer
+    name = "chunk_gqa_q4"
+    sq, H, hidden, qpk, sk, seed = CASES[name]
+    Q, K, V, W = make_inputs(name)
+    pages = sum((s + 127) // 128 for s in sk) + 3
+    Kc, Vc, table, lens = make_paged_kv(K, V, sk, num_pages=pages, shuffle=True, seed=6)
+    if width:
+        table = torch.cat((table, torch.full((len(sk), width), pages - 1, dtype=torch.int32)), 1)
+        assert table.numel() >= 16384
+    ws = FusedFaOprojArWorkspace.create(
+        None, sum((s + 127) // 128 for s in sq), hidden, H, 128, q_per_kv=qpk, paged=True,
+        max_num_pages=pages, max_num_pages_per_seq=table.shape[1], device="cuda:0")
+    ws.compile(w_fa=2, w_oproj=1, w_ar=0)
+    layer = FusedPrefillLayer(ws, W)
+    call = (Q.cuda(), Kc.cuda(), Vc.cuda(), _cu(sq))
+    layer(*call, page_table=table.cuda(), cache_seqlens=lens.cuda())
+    ws.check_status()
+    got = layer.output().clone()
+    _, Yp, _ = full_chain_oracle(Q, K, V, W, sq, sk)
+    assert err_beyond_rounding(got.cpu(), Yp) <= 8e-3
+    ws.csym.zero_()
+    for at in ((0, 0), (len(sk) - 1, table.shape[1] - 1)):
+        for page in (-1, pages):
+            bad = table.clone()
+            bad[at] = page
+            with pytest.raises(AssertionError):
+                layer(*call, page_table=bad.cuda(), cache_seqlens=lens.cuda())
+    torch.cuda.synchronize()
+    assert not bool(ws.csym.any())                       # nothing was launched
+    layer(*call, page_table=table.cuda(), cache_seqlens=lens.cuda())
+    ws.check_status()
+    assert torch.equal(layer.output(), got)
