@@ -47,7 +47,9 @@ constexpr uint32_t kSmQ = 0;               // two Q tiles
 constexpr uint32_t kSmKV = 2 * kTile;      // ring of five K/V tiles
 constexpr int kKvSlots = 5;
 constexpr uint32_t kSmOpStaging = 4 * (16384 + 32768);   // O_proj output staging, 2 x 16 KB
-constexpr uint32_t kOpStage = 16384 + 32768;   // O_proj stage: A 128x64 + W 64x256 (4 stages)
+// O_proj stages, by what the launch's tasks are.  (Three of the large ones for every task of one
+// rank: K_local 4096, hidden 8192, 1024 and 2048 tokens took 170 and 177 us for 144 and 154.)
+constexpr uint32_t kOpStage = 16384 + 32768;   // one row tile: A 128x64 + W 64x256 (4 stages)
 constexpr uint32_t kOpStage2 = 2 * 16384 + 32768;   // two row tiles: A 256x64 + W 64x256 (3 stages)
 constexpr uint32_t kWPanel = 8192;         // 64 k-rows x 64 n bf16
 constexpr uint32_t kTmemS = 0;             // S0 at 0, S1 at 128 (P aliases the first 64 cols)
@@ -523,7 +525,7 @@ template <bool kSeparate> struct Layout { static constexpr bool value = kSeparat
 enum : int { T_MODE = 0, T_FT = 1,
              TF_HEAD0 = 2, TF_NT = 3, TF_KVH = 4, TF_QROW0 = 5, TF_VALID = 6, TF_KSTART = 7,
              TF_KLEN = 8, TF_OFFSET = 9, TF_NBLK = 10, TF_MB = 11,
-             TO_BASE = 2, TO_VNT = 3, TO_VALID = 4, TO_SLOT = 5, TO_NRT = 6, TO_VALID1 = 7,
+             TO_BASE = 2, TO_VNT = 3, TO_VALID = 4, TO_SLOT = 5, TO_NRT = 6, TO_VALID1 = 7, TO_TWO = 8,
              T_WORDS = 12 };
 
 __device__ __forceinline__ bool is_tile_mode(int m) { return m == MODE_FA || m == MODE_OPROJ; }
@@ -788,7 +790,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
             const int b = p.fa_b[ft + r], mb = p.fa_mb[ft + r];
             d[r ? TO_VALID1 : TO_VALID] = min(128, p.cu_q[b + 1] - p.cu_q[b] - mb * 128);
           }
-          d[TO_NRT] = own ? rows : 0; d[TO_SLOT] = arg;
+          d[TO_NRT] = own ? rows : 0; d[TO_SLOT] = arg; d[TO_TWO] = nrt == 2;
           occ_a[k] = arg;
         }
         d[T_MODE] = mode;
@@ -846,8 +848,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           const int ft = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT], nrt = d[TO_NRT];
           const int nkc = p.K_local >> 6;
           const int rows = max(nrt, 1), passes = nrt ? 1 : (vnt + 1) >> 1;
-          const uint32_t stage = nrt ? kOpStage2 : kOpStage, w_off = nrt ? 2 * kPanel : kPanel;
-          const uint32_t stages = nrt ? 3 : 4;
+          const bool two = d[TO_TWO] != 0;      // (the launch's, also for a last row tile alone)
+          const uint32_t stage = two ? kOpStage2 : kOpStage, w_off = two ? 2 * kPanel : kPanel;
+          const uint32_t stages = two ? 3 : 4;
           fence_proxy_async_global();   // O_scratch was written by other CTAs' TMA stores
           bool ok = true;
           for (int h = 0; h < passes && ok; ++h) {
@@ -1009,8 +1012,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           const int vnt = d[TO_VNT], nrt = d[TO_NRT];
           const int nkc = p.K_local >> 6;
           const int rows = max(nrt, 1), passes = nrt ? 1 : (vnt + 1) >> 1;
-          const uint32_t stage = nrt ? kOpStage2 : kOpStage, w_off = nrt ? 2 * kPanel : kPanel;
-          const uint32_t stages = nrt ? 3 : 4;
+          const bool two = d[TO_TWO] != 0;      // (the launch's, also for a last row tile alone)
+          const uint32_t stage = two ? kOpStage2 : kOpStage, w_off = two ? 2 * kPanel : kPanel;
+          const uint32_t stages = two ? 3 : 4;
           for (int h = 0; h < passes; ++h) {
             const int ncols = min(2, vnt - 2 * h) * 128;
             const uint32_t idesc = make_idesc_bf16(128, ncols, 0, 1);
