@@ -278,6 +278,9 @@ int ma_launch(ma_plan* pl, const ma_launch_args* a, void* stream) {
     return MA_ERR_INVALID;
   if (kp.w_fa < 0 || kp.w_oproj < 0 || kp.w_ar < 0 || kp.w_fa + kp.w_oproj + kp.w_ar < 1)
     return MA_ERR_INVALID;
+  const bool alone = (kp.flags & MA_FLAG_OPROJ_ONLY) != 0;
+  kp.op_two_from = alone ? ma::kOpTwoFromAlone : ma::kOpTwoFrom;
+  kp.op_cols2_from = alone ? ma::kOpCols2FromAlone : ma::kOpCols2From;
   int n = a->num_ctas > 0 ? a->num_ctas : pl->num_sms;
   if (n > pl->num_sms) n = pl->num_sms;          // one CTA per SM: more could only start when others have left
   cudaError_t e = ma::launch_fused_prefill(pl->maps, kp, n, static_cast<cudaStream_t>(stream));

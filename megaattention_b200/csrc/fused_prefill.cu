@@ -502,21 +502,28 @@ __device__ __forceinline__ void ar_slot(const KParams& p, int ft, int base_out, 
 
 }  // namespace
 
-// O_proj task of a single rank: nrt row tiles x nnt column tiles in one pass.  What bounds the
-// product is shared memory, which carries the loads and the MMAs' operands: for 64 k of two row
-// tiles x 256 columns 96 + 96 KB when each row tile loads W for itself, 64 + 96 KB when they
-// share it.  So 2 x 2 is the shape for large launches (O_proj stage
-// alone, 22600 tokens, hidden 16384: 1330 -> 1210 us; 13400 tokens, hidden 4096: 110 -> 103).
-// With few tasks what counts is how soon the last row tile's product is done: one column tile
-// per task up to 1.25 waves of 2 x 2 tasks, two up to 3 waves.  Whole launches, us, as 2 x 2 /
-// 1 x 2 / 1 x 1:  0.1 waves (520 tokens, hidden 1024) 53 / 48 / 46, 0.9 waves (four prompts of
-// 1024, K = 2048, hidden 2048) 109 / 97 / 94, 1.3 waves 83 / 81 / 88, 3.5 waves (16384 tokens)
-// 525 / 537 / 595, 5.8 waves 226 / 250 / 322.
-__device__ __forceinline__ void op_task_shape(int n_tiles, int num_out, int ctas, int* nrt,
+// O_proj task of a single rank: nrt row tiles x nnt column tiles in one pass.  A task's time per
+// 64 k, from what a further round of tasks adds to the stage alone (K_local 2048): 0.35 us for
+// 1 x 1, 0.42 for 1 x 2, 0.75 for 2 x 2 - so 2 x 2 does the same work in nine tenths of the time of
+// 1 x 2, and a 1 x 1 task costs almost what a 1 x 2 one does.  (The tensor pipe needs 0.14, 0.28
+// and 0.56; what holds the small shapes up is not established.)
+// O_proj-only launches: every task is ready at the start, so 2 x 2 from half a wave of such tasks
+// and 1 x 1 only below a quarter.  The stage in us as 1 x 1 / 1 x 2 / 2 x 2 at K_local 2048: 0.2 waves
+// 30 / 32 / 42, 0.4 42 / 34 / 44, 0.65 53 / 45 / 44, 0.9 64 / 46 / 44, 1.3 86 / 59 / 67, 1.7 99 / 73 /
+// 68, 2.05 121 / 87 / 90, 2.8 155 / 106 / 92, 3.5 179 / 119 / 117.
+// Behind attention, with few tasks what counts is how soon the last row tile's product is done:
+// one column tile per task up to 1.25 waves, two up to 2.25.  Whole launches, us, as 1 x 1 / 1 x 2 /
+// 2 x 2: 0.1 waves (520 tokens, hidden 1024) 44 / 46 / 51, 0.9 waves (four prompts of 1024, hidden
+// 2048, K_local 2048) 90 / 93 / 103, 1.3 waves (3072 tokens, hidden 4096, K_local 512, 1024, 2048,
+// 4096) 70 / 70 / 62, 78 / 70 / 72, 107 / 87 / 101, 178 / 138 / 162.  As 1 x 2 / 2 x 2, hidden 4096 and
+// the same K_local: 1.95 waves 78 / 67, 85 / 82, 110 / 117, 197 / 190; 2.05 81 / 68, 88 / 84, 113 / 119,
+// 218 / 209; 2.3 86 / 70, 92 / 85, 122 / 124, 225 / 228; 2.8 101 / 76, 106 / 95, 147 / 137, 283 / 267.
+// (K_local 512 would take 2 x 2 from one wave on, a longer product has the longer last task.)
+__device__ __forceinline__ void op_task_shape(const KParams& p, int n_tiles, int ctas, int* nrt,
                                               int* nnt) {
-  const int t22 = (n_tiles + 1) / 2 * ((num_out + 1) / 2);
-  *nrt = t22 >= 3 * ctas ? 2 : 1;
-  *nnt = 4 * t22 >= 5 * ctas ? 2 : 1;
+  const int t22 = (n_tiles + 1) / 2 * ((p.num_out + 1) / 2);
+  *nrt = 4 * t22 >= p.op_two_from * ctas ? 2 : 1;
+  *nnt = 4 * t22 >= p.op_cols2_from * ctas ? 2 : 1;
 }
 
 template <bool kSeparate> struct Layout { static constexpr bool value = kSeparate; };   // of K/V stages
@@ -641,12 +648,15 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       int nrt = 0, nnt = p.sg, per_group = p.nsg, total_op = p.actv[1];
       const int n_tiles = p.actv[2];
       if (p.tp == 1 && !(p.flags & 16u)) {      // (without AllReduce: slots, as with several)
-        op_task_shape(n_tiles, p.num_out, static_cast<int>(gridDim.x), &nrt, &nnt);
+        op_task_shape(p, n_tiles, static_cast<int>(gridDim.x), &nrt, &nnt);
         per_group = (p.num_out + nnt - 1) / nnt;
         // (plus what the host's count of slots is off by: such a launch must not end well)
         total_op = (n_tiles + nrt - 1) / nrt * per_group + (total_op - n_tiles * p.nsg);
       }
       const int grp = max(nrt, 1);              // row tiles whose attention a task group needs
+#ifdef MA_AUDIT
+      if (p.audit && blockIdx.x == 0) { p.status[6] = nrt; p.status[7] = nnt; }   // for tests
+#endif
       int role;
       {
         const int wsum = p.w_fa + p.w_oproj + p.w_ar;

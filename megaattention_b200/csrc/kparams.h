@@ -27,6 +27,8 @@ struct KParams {
   int w_fa, w_oproj, w_ar;
   uint32_t flags;
   float scale_log2;
+  int op_two_from, op_cols2_from; // O_proj task shape of one rank, see op_task_shape: two row /
+                                  // column tiles from that many quarter waves of 2 x 2 tasks
   int pair;                       // 1: an FA task is two q heads sharing a kv head (q_per_kv even)
   int sep;                        // 1: an FA task is two q heads, each with K/V stages of its own
                                   //    (q_per_kv odd, MHA included; the last head of an odd count alone)
@@ -61,6 +63,9 @@ struct KParams {
   unsigned long long peer_nvl[kMaxTp];
   unsigned long long peer_csym[kMaxTp];   // every rank's C_sym (peer-load AllReduce, tp 2)
 };
+
+constexpr int kOpTwoFrom = 9, kOpCols2From = 5;             // behind attention
+constexpr int kOpTwoFromAlone = 2, kOpCols2FromAlone = 1;   // O_proj-only launches
 
 constexpr int kThreads = 384;
 constexpr int kSmemDynamic = 65536 + 5 * 32768 + 1024;   // Q x2, K/V ring x5, align slack

@@ -138,6 +138,7 @@ extern "C" int ma_fused_prefill_noalloc(const ma_noalloc_args* a, void* stream_)
   k.tp = 1; k.rank = 0;
   k.w_fa = a->w_fa > 0 ? a->w_fa : 2; k.w_oproj = a->w_oproj > 0 ? a->w_oproj : 1; k.w_ar = 0;
   k.flags = 0;
+  k.op_two_from = ma::kOpTwoFrom; k.op_cols2_from = ma::kOpCols2From;
   const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 0.08838834764831845f;
   k.scale_log2 = scale * 1.4426950408889634f;
   k.pair = (k.q_per_kv % 2 == 0) ? 1 : 0;

@@ -72,6 +72,7 @@ def run_case(name, w=(4, 1, 1), num_ctas=None, launches=1, audit=False):
         assert bool((fa == launches).all()) and bool((op == launches).all()), (fa, op)
         assert bool((ar == 0).all())        # one rank: the O_proj finisher accounts the slot
         assert int(ws.audit.sum()) == launches * (fa.numel() + op.numel())
+    shape = tuple(ws.status.cpu().tolist()[6:8]) if audit else None      # O_proj task shape
     O, Yp, Yf = full_chain_oracle(Q, K, V, W, sq, sk)
     oscr_ref = o_scratch_oracle(O, sq)
     oscr = ws.Oscr.float().cpu()
@@ -104,6 +105,7 @@ def run_case(name, w=(4, 1, 1), num_ctas=None, launches=1, audit=False):
     res["err_rel_fixture"] = err_rel(out, ref_yf)
     res["err_comp_fixture"] = err_beyond_rounding(out, ref_yf, extra_half_ulps=1.0)
     res["q_lt_k"] = sk is not None
+    res["op_shape"] = shape
     res["out"], res["oscr"], res["Yp"] = out, oscr, Yp
     return res
 
