@@ -66,7 +66,7 @@ extern "C" int ma_stage_meta(const ma_stage_meta_args* a) {
       most = std::max(most, nblk[t]);
     }
     int prime = a->prime;
-    if (a->auto_prime) {          // interleaved below the table's switch point of the ratio
+    if (a->auto_prime) {          // interleaved below 2.0, fa_prime_tiles_b200's switch point
       const int64_t tiles = static_cast<int64_t>(R) * ((a->hidden + 127) / 128);
       prime = static_cast<double>(2 * sum) / static_cast<double>(tiles) < 2.0 ? -1 : 0;
     }

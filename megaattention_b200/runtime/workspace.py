@@ -43,7 +43,10 @@ def claim_order(meta, prime: int = 0) -> np.ndarray:
     finishes within microseconds, so O_proj and AllReduce work exists almost from the start
     of the launch instead of only after the first long attention task (tens of
     microseconds) — worth it when the launch is bound by the AllReduce.  ``prime`` < 0
-    interleaves long and short row tiles instead (see below)."""
+    interleaves long and short row tiles instead (see below).
+
+    A launch's order is computed natively (``csrc/meta.cpp``); this is the statement of it that
+    the tests hold that to."""
     M = meta.M_TILE
     b = meta.batch_idx.astype(np.int64)
     lq = np.diff(meta.cu_seqlens_q.astype(np.int64))[b]

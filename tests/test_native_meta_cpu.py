@@ -90,3 +90,22 @@ def test_key_lengths_may_sum_past_int32():
         assert buf[offs[4]:offs[5]].tolist() == [2, 3, 1, 0, 4, 5, 6]
     with pytest.raises(AssertionError):
         native_row_desc(_cu([1]), _cu([1 << 31]), 100)
+
+
+@pytest.mark.parametrize("hidden,interleaved", [(257, True), (256, False), (384, True), (1, False)])
+def test_the_claim_order_switches_where_the_rule_does(hidden, interleaved):
+    """fa_prime_tiles_b200 and ma_stage_meta each have the switch point; a batch whose work ratio
+    is exactly 2 (one sequence of three row tiles, two column tiles: 2 * 6 / 6) and its
+    neighbours take the same side in both."""
+    meta = build_row_desc([384])
+    p = fa_prime_tiles_b200(meta, hidden, 1, 8)
+    assert (p < 0) == interleaved
+    R, nb = 3, 1
+    offs = np.cumsum([0, nb + 1, nb + 1, R, R, R])
+    buf = np.zeros(int(offs[-1]) + 6, dtype=np.int32)
+    a = _cabi.StageMetaArgs(
+        meta.cu_seqlens_q.ctypes.data, meta.cu_seqlens_k.ctypes.data, meta.batch_idx.ctypes.data,
+        meta.m_block.ctypes.data, buf.ctypes.data, nb, R, hidden, 8, 1, 1, 0, 1, 0, *map(int, offs), 0)
+    assert _cabi.lib.ma_stage_meta(C.byref(a)) == _cabi.MA_OK
+    assert buf[offs[4]:offs[5]].tolist() == claim_order(meta, p).tolist()
+    assert claim_order(meta, p).tolist() == ([2, 0, 1] if interleaved else [2, 1, 0])
