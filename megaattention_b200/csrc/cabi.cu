@@ -22,7 +22,7 @@ int encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint
 
 struct ma_plan {
   ma::KParams kp;
-  CUtensorMap maps[6];   // Q, K, V, O_scratch (2-D), W_o, C_sym (store)
+  CUtensorMap maps[7];   // Q, K, V, O_scratch (2-D), W_o (128 columns), C_sym (store), W_o (256)
   int device;
   int num_sms;
   ma_plan_desc desc;     // as given at creation (shapes for re-encoding)
@@ -71,11 +71,12 @@ int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 }  // namespace
 
-// The five TMA descriptors of the path.  A 128 x 128 tile of Q, K or V is fetched by ONE
+// The TMA descriptors of the path.  A 128 x 128 tile of Q, K or V is fetched by ONE
 // instruction as two 64-wide swizzled panels: the tensor is described as
 // {64 d, tokens, 2 d-halves, heads} so the box {64, 128, 2, 1} lands panel after panel.
 // W_o [K_local, width] is described as {64 n, K_local, width/64 panels}: the box
-// {64, 64, 2} is a 64-k slab of 128 output columns, panel after panel.
+// {64, 64, 2} is a 64-k slab of 128 output columns, panel after panel; {64, 64, 4} (the last
+// map) one of 256.
 int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint64_t oscr,
                          uint64_t W, uint64_t H, uint64_t Hkv, uint64_t tot_q, uint64_t tot_k,
                          uint64_t row_tiles, uint64_t w_width, uint64_t csym, uint64_t hidden,
@@ -106,7 +107,9 @@ int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, 
     const uint64_t dims[3] = {64, KL, w_width / 64};
     const uint64_t str[2] = {w_width * 2, 128};
     const uint32_t box[3] = {64, 64, 2};
+    const uint32_t box2[3] = {64, 64, 4};
     rc = encode(&maps[4], W, 3, dims, str, box);
+    if (rc == MA_OK) rc = encode(&maps[6], W, 3, dims, str, box2);
   }
   if (rc == MA_OK) {
     // output tiles are stored through TMA: [rows, hidden] with the padded row pitch, so a
@@ -293,7 +296,7 @@ int ma_plan_set_inputs(ma_plan* pl, uint64_t Q, uint64_t K, uint64_t V, uint64_t
   const ma_plan_desc& d = pl->desc;
   if (tot_q < 1 || tot_k < 1 || w_width < d.hidden || w_width % 64) return MA_ERR_INVALID;
   if (d.page_table && tot_k % 128) return MA_ERR_INVALID;
-  CUtensorMap fresh[6];
+  CUtensorMap fresh[7];
   const int rc = ma::encode_path_maps(fresh, Q, K, V, d.o_scratch, W_o,
                                       static_cast<uint64_t>(d.H_local),
                                       static_cast<uint64_t>(d.H_kv),
@@ -304,6 +307,7 @@ int ma_plan_set_inputs(ma_plan* pl, uint64_t Q, uint64_t K, uint64_t V, uint64_t
                                       static_cast<uint64_t>(pl->kp.num_out) * 128);
   if (rc != MA_OK) return rc;
   pl->maps[0] = fresh[0]; pl->maps[1] = fresh[1]; pl->maps[2] = fresh[2]; pl->maps[4] = fresh[4];
+  pl->maps[6] = fresh[6];
   return MA_OK;
 }
 

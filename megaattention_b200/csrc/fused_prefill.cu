@@ -544,6 +544,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ CUtensorMap tmO,
                      const __grid_constant__ CUtensorMap tmW,
                      const __grid_constant__ CUtensorMap tmC,
+                     const __grid_constant__ CUtensorMap tmW2,
                      const __grid_constant__ KParams p) {
   extern __shared__ uint8_t dyn_smem[];
   // The abort flag, read in every wait loop, gets a 128-byte line of its own: where the
@@ -591,6 +592,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmO); tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmC);
+    tma_prefetch_desc(&tmW2);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&s_tmem), 512);
@@ -870,14 +872,14 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
               if (!ok) break;
               const uint32_t bar = smem_u32(&bars.op_full[op_st]);
               const uint32_t dst = smem0 + op_st * stage;
-              // A chunks of 128 x 64 and W slabs of 64 k x 128 n (2 panels each; panels past
-              // the padded width are filled with zeros)
+              // A chunks of 128 x 64, and a W slab of 64 k x 128 or 256 columns in one load (2 or 4
+              // panels; panels past the padded width are filled with zeros).  256 columns as two
+              // loads: launches of slots 1 to 8 % slower (K_local 4096, hidden 1024, 2048 tokens
+              // 123 us for 112).
               mbar_expect_tx(bar, rows * kPanel + nw * 2 * kWPanel);
               for (int r = 0; r < rows; ++r)
                 tma_load_2d(dst + r * kPanel, &tmO, bar, kc * 64, (ft + r) * 128);
-              for (int j = 0; j < nw; ++j)
-                tma_load_3d(dst + w_off + j * 2 * kWPanel, &tmW, bar, 0, kc * 64,
-                            (base_out + 2 * h + j) * 2);
+              tma_load_3d(dst + w_off, nw == 2 ? &tmW2 : &tmW, bar, 0, kc * 64, (base_out + 2 * h) * 2);
               if (++op_st == stages) { op_st = 0; op_ph ^= 1u; }
             }
           }
@@ -1426,7 +1428,7 @@ cudaError_t launch_fused_prefill(const CUtensorMap* maps, const KParams& kp, int
     attr_set[dev] = true;
   }
   fused_prefill_kernel<<<num_ctas, kThreads, kSmemDynamic, stream>>>(maps[0], maps[1], maps[2],
-                                                                     maps[3], maps[4], maps[5], kp);
+                                                                     maps[3], maps[4], maps[5], maps[6], kp);
   return cudaGetLastError();
 }
 

@@ -164,7 +164,7 @@ extern "C" int ma_fused_prefill_noalloc(const ma_noalloc_args* a, void* stream_)
   k.oproj_queue = reinterpret_cast<uint32_t*>(scr + kOffQueue);
 
   // ---- TMA descriptors over the caller's tensors and the scratch (host-side encoding)
-  CUtensorMap maps[6];
+  CUtensorMap maps[7];
   // W_o is read in 64-column panels straight from the caller's tensor: hidden % 64 == 0
   rc = ma::encode_path_maps(maps, a->Q, a->K, a->V, reinterpret_cast<uint64_t>(k.o_scratch), a->W_o,
                             static_cast<uint64_t>(a->H_local), static_cast<uint64_t>(a->H_kv),
