@@ -519,6 +519,9 @@ __device__ __forceinline__ void ar_slot(const KParams& p, int ft, int base_out, 
 // the same K_local: 1.95 waves 78 / 67, 85 / 82, 110 / 117, 197 / 190; 2.05 81 / 68, 88 / 84, 113 / 119,
 // 218 / 209; 2.3 86 / 70, 92 / 85, 122 / 124, 225 / 228; 2.8 101 / 76, 106 / 95, 147 / 137, 283 / 267.
 // (K_local 512 would take 2 x 2 from one wave on, a longer product has the longer last task.)
+// These figures compare the shapes under an issuer that was converged per stage and with W in two
+// loads; since then every shape is faster (2 x 2 alone at 0.9 waves 44 -> 42 us, 2.6 91 -> 86, 3.5 117
+// -> 110; 0.9 waves as a whole launch 90 -> 86), and the lines were not moved.
 __device__ __forceinline__ void op_task_shape(const KParams& p, int n_tiles, int ctas, int* nrt,
                                               int* nnt) {
   const int t22 = (n_tiles + 1) / 2 * ((p.num_out + 1) / 2);
