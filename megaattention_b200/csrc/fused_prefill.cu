@@ -892,8 +892,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       }
     } else if (warp == 1) {
       // ============================================= MMA issuer of both attention tiles and of
-      // every O_proj task.  The warp stays converged: every lane waits, one elected lane
-      // issues (see elect_one).
+      // every O_proj task.  In attention the warp stays converged: every lane waits, one elected
+      // lane issues (see elect_one); an O_proj task is one elected lane's from start to end.
       uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0;
       uint32_t q_par[2] = {0, 0}, p_par[2] = {0, 0}, o_uses[2] = {0, 0}, acc_uses[2] = {0, 0};
       while (true) {
