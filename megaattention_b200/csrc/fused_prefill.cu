@@ -614,15 +614,14 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
   // shared memory and TMEM: a role that goes from one kind to the other first waits for
   // the previous task to finish completely (same-kind neighbours overlap freely).
   int slot_k = 0;
-  uint32_t tf_par[2] = {0, 0};
-  uint32_t n_arrived[2] = {0, 0};
+  uint32_t tf_par = 0, arrived = 0;        // a bit per slot: phase to wait for, arrivals made (mod 2)
   int prev_mode = MODE_IDLE, prev_k = 0;
 
 #define MA_TASK_FULL                                                                       \
-  wait_bar(env, smem_u32(&bars.task_full[slot_k]), tf_par[slot_k], 0x100 + warp)
+  wait_bar(env, smem_u32(&bars.task_full[slot_k]), (tf_par >> slot_k) & 1u, 0x100 + warp)
 #define MA_NEXT_TASK_IF(full, desc_ptr, mode_var)                                          \
   if (!(full)) break;                                                                      \
-  tf_par[slot_k] ^= 1u;                                                                    \
+  tf_par ^= 1u << slot_k;                                                                  \
   const int* desc_ptr = s_desc[slot_k];                                                    \
   const int mode_var = desc_ptr[T_MODE];                                                   \
   if (mode_var == MODE_DONE) break;
@@ -633,14 +632,14 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
   MA_NEXT_TASK_IF(__all_sync(0xffffffffu, MA_TASK_FULL), desc_ptr, mode_var)
 #define MA_DRAIN_IF_SWITCH(mode_var)                                                       \
   if (is_tile_mode(mode_var) && is_tile_mode(prev_mode) && mode_var != prev_mode)          \
-    wait_bar(env, smem_u32(&bars.task_empty[prev_k]), (n_arrived[prev_k] - 1u) & 1u, 0x110 + warp);
+    wait_bar(env, smem_u32(&bars.task_empty[prev_k]), ((arrived >> prev_k) & 1u) ^ 1u, 0x110 + warp);
 #define MA_TASK_DONE(mode_var)                                                             \
   mbar_arrive(smem_u32(&bars.task_empty[slot_k]));                                         \
-  ++n_arrived[slot_k];                                                                     \
+  arrived ^= 1u << slot_k;                                                                     \
   prev_mode = mode_var; prev_k = slot_k; slot_k ^= 1;
 
   if (warp < 4) {
-    reg_dec<80>();
+    reg_dec<88>();
     if (warp == 2 && lane == 0) {
       // ==================================================================== scheduler
       // (a launch after one that gave up does nothing until the state has been cleared)
@@ -821,7 +820,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       }
     } else if (warp == 0 && lane == 0) {
       // ==================================================================== TMA producer
-      uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0, q_uses[2] = {0, 0};
+      uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0, q_uses = 0;
       while (true) {
         MA_NEXT_TASK(d, mode)
         MA_DRAIN_IF_SWITCH(mode)
@@ -831,9 +830,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           // buffer that was not waited for
           bool ok = true;
           for (int i = 0; i < nt && ok; ++i) {
-            ok = wait_bar(env, smem_u32(&bars.q_empty[i]), (q_uses[i] & 1u) ^ 1u, 0x18 + i);
+            ok = wait_bar(env, smem_u32(&bars.q_empty[i]), ((q_uses >> i) & 1u) ^ 1u, 0x18 + i);
             if (!ok) break;
-            ++q_uses[i];
+            q_uses ^= 1u << i;
             const uint32_t bar = smem_u32(&bars.q_full[i]);
             mbar_expect_tx(bar, kTile);
             tma_load_4d(smem0 + kSmQ + i * kTile, &tmQ, bar, 0, d[TF_QROW0], 0, d[TF_HEAD0] + i);
@@ -892,10 +891,9 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       }
     } else if (warp == 1) {
       // ============================================= MMA issuer of both attention tiles and of
-      // every O_proj task.  In attention the warp stays converged: every lane waits, one elected
-      // lane issues (see elect_one); an O_proj task is one elected lane's from start to end.
+      // every O_proj task.  A task is one elected lane's from start to end (see elect_one).
       uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0;
-      uint32_t q_par[2] = {0, 0}, p_par[2] = {0, 0}, o_uses[2] = {0, 0}, acc_uses[2] = {0, 0};
+      uint32_t q_par = 0, p_par = 0, o_uses = 0, acc_uses = 0;     // a bit per tile / accumulator
       while (true) {
         MA_NEXT_TASK_WARP(d, mode)
         MA_DRAIN_IF_SWITCH(mode)
@@ -903,23 +901,32 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           // A tile's chain softmax -> P V -> next Q K^T is what bounds the loop: the V tile
           // and the next K tile are looked at before P is waited for, and P V starts on the
           // first three quarters of P.  The tiles take turns, which keeps them half a period
-          // apart: one tile's MMAs run under the other's softmax.  (Before: an issuing warp
-          // per tile and a lock between the two.  With issue at 56 cycles per MMA and 250 for
-          // the lock, a two-tile key block took 4000 cycles.  Attention stage, one box:
-          // 12 short turns on cached prompts 104.5 -> 95.6 us, six ragged prompts of 13400
-          // tokens 150 -> 137.6 us; with a 16384-token prompt the whole launch 631 -> 601 us.)
+          // apart: one tile's MMAs run under the other's softmax.
           const int nblk = d[TF_NBLK], nt = d[TF_NT];
+          // The task's first operands are nearly always there: one look at all their barriers, a
+          // lane each.  The lane that issues has seen one of them at most, and a vote orders no
+          // memory: the __syncwarp hands it what the other lanes acquired.
+          const uint32_t bar0 = smem_u32(lane == 0 ? &bars.q_full[0] : lane == 1 && nt == 2 ? &bars.q_full[1]
+                                                                     : &bars.kv_full[kv_slot]);
+          const uint32_t par0 = lane == 0 ? q_par & 1u : lane == 1 && nt == 2 ? q_par >> 1 : kv_ph;
+          const bool there = __all_sync(0xffffffffu, mbar_test_wait(bar0, par0));
+          __syncwarp();
           // Shared K/V stages: one slot per operand and key block.  Separate stages (p.sep):
           // nt slots, the i-th for tile i.  Two instances of the loop: a test of the layout in it
-          // costs the shared one 2 %.
+          // costs the shared one 2 %.  One elected lane runs the whole task, what every lane keeps
+          // is advanced after it, and the parities are bits (arrays indexed by the tile lived in
+          // local memory).  With a converged warp that waited and elected per batch the issuer
+          // itself was late where the K tiles are: MHA, six ragged prompts of 13400 tokens,
+          // attention stage 147 -> 137 us; shared stages the same time.
           auto run = [&](auto layout) {
             constexpr bool sep = decltype(layout)::value;
-            const int per = sep ? nt : 1;
+            const uint32_t per = sep ? nt : 1;
+            uint32_t slot = kv_slot, ph = kv_ph;
             struct SlotAt { uint32_t slot, ph; };
             auto take = [&]() {                       // the next `per` slots of the ring
-              const SlotAt r{kv_slot, kv_ph};
-              kv_slot += static_cast<uint32_t>(per);
-              if (kv_slot >= static_cast<uint32_t>(kKvSlots)) { kv_slot -= kKvSlots; kv_ph ^= 1u; }
+              const SlotAt r{slot, ph};
+              slot += per;
+              if (slot >= static_cast<uint32_t>(kKvSlots)) { slot -= kKvSlots; ph ^= 1u; }
               return r;
             };
             auto at = [&](SlotAt r, int i) {          // tile i's slot among them
@@ -928,101 +935,82 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
               }
               return r;
             };
-            auto wait_slots = [&](SlotAt r, uint32_t site) {
-              for (int i = 0; i < per; ++i) {
-                const SlotAt x = at(r, i);
-                wait_bar(env, smem_u32(&bars.kv_full[x.slot]), x.ph, site + x.slot);
-              }
+            auto wait_kv = [&](SlotAt r, uint32_t site) {
+              wait_bar(env, smem_u32(&bars.kv_full[0]) + r.slot * 8, r.ph, site + r.slot);
             };
+            auto kv_at = [&](SlotAt r) { return smem0 + kSmKV + r.slot * kTile; };
+            auto free_kv = [&](SlotAt r) { tc_commit(smem_u32(&bars.kv_empty[0]) + r.slot * 8); };
             SlotAt k = take();
-            for (int i = 0; i < nt; ++i) {
-              wait_bar(env, smem_u32(&bars.q_full[i]), q_par[i], 0x20 + i);
-              q_par[i] ^= 1u;
-              if (i == 0) wait_slots(k, 0x30);
-              tc_fence_after();
-              const uint32_t ks = at(k, i).slot;
-              if (elect_one()) {
-                issue_qk(tmem + kTmemS + i * 128, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (i < nt) {
+                if (!there) wait_bar(env, smem_u32(&bars.q_full[i]), (q_par >> i) & 1u, 0x20 + i);
+                if (sep ? i == 1 || !there : i == 0 && !there) wait_kv(at(k, i), 0x30);
+                tc_fence_after();
+                issue_qk(tmem + kTmemS + i * 128, smem0 + kSmQ + i * kTile, kv_at(at(k, i)));
                 tc_commit(smem_u32(&bars.s_full[i]));
-                if (sep || i == nt - 1) tc_commit(smem_u32(&bars.kv_empty[ks]));
+                if (sep || i == nt - 1) free_kv(at(k, i));
                 if (nblk == 1) tc_commit(smem_u32(&bars.q_empty[i]));
               }
-              __syncwarp();
             }
+            uint32_t par = p_par;
             for (int jj = 0; jj < nblk; ++jj) {
               const bool has_next = (jj + 1 < nblk);
               const SlotAt v = take();
               if (has_next) k = take();
-              for (int i = 0; i < nt; ++i) {
-                const uint32_t t_s = tmem + kTmemS + i * 128, t_o = tmem + kTmemO + i * 128;
-                const uint32_t vs = at(v, i).slot, ks = at(k, i).slot;
-                const uint32_t sm_v = smem0 + kSmKV + vs * kTile;
-                const bool last_use = sep || i == nt - 1;
-                // The operands are nearly always there: one look at all their barriers, a lane
-                // each, and a wait one by one only if one of them is not.
-                if (sep || i == 0 || jj == 0) {
-                  uint32_t bar = smem_u32(&bars.kv_full[vs]), par = at(v, i).ph;
-                  if (!sep && lane == 1 && has_next) { bar = smem_u32(&bars.kv_full[ks]); par = at(k, i).ph; }
-                  if (lane == 2 && jj == 0) { bar = smem_u32(&bars.o_free[i]); par = (o_uses[i] & 1u) ^ 1u; }
-                  if (!__all_sync(0xffffffffu, mbar_test_wait(bar, par))) {
-                    wait_bar(env, smem_u32(&bars.kv_full[vs]), at(v, i).ph, 0x40 + vs);
-                    if (!sep && has_next) wait_bar(env, smem_u32(&bars.kv_full[ks]), at(k, i).ph, 0x50 + ks);
-                    // (the previous task's epilogue must have read O out)
-                    if (jj == 0) wait_bar(env, smem_u32(&bars.o_free[i]), (o_uses[i] & 1u) ^ 1u, 0x68 + i);
-                  }
-                  // The lane that issues has seen one of these barriers at most, and a vote orders
-                  // no memory: this hands it what the other lanes acquired (K by TMA, O read out).
-                  __syncwarp();
-                  if (jj == 0) ++o_uses[i];
-                }
-                wait_bar(env, smem_u32(&bars.p_part[i]), p_par[i], 0x58 + i);
-                tc_fence_after();
-                if (elect_one()) issue_pv<0, 6>(t_o, t_s, sm_v, jj > 0);
-                __syncwarp();
-                wait_bar(env, smem_u32(&bars.p_full[i]), p_par[i], 0x60 + i);
-                p_par[i] ^= 1u;
-                tc_fence_after();
-                if constexpr (sep) {
-                  // The ring holds 1.25 key blocks here: the next K tile comes late, and P V must not
-                  // wait for it (looked at before P as below, the stage lost up to 12 % on MHA).
+              if (!sep) {
+                wait_kv(v, 0x40);
+                if (has_next) wait_kv(k, 0x50);
+              }
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                if (i < nt) {
+                  const uint32_t t_s = tmem + kTmemS + i * 128, t_o = tmem + kTmemO + i * 128;
+                  const bool last_use = sep || i == nt - 1;
+                  if (sep) wait_kv(at(v, i), 0x40);
+                  // (the previous task's epilogue must have read O out)
+                  if (jj == 0) wait_bar(env, smem_u32(&bars.o_free[i]), ((o_uses >> i) & 1u) ^ 1u, 0x68 + i);
+                  wait_bar(env, smem_u32(&bars.p_part[i]), (par >> i) & 1u, 0x58 + i);
+                  tc_fence_after();
+                  issue_pv<0, 6>(t_o, t_s, kv_at(at(v, i)), jj > 0);
+                  wait_bar(env, smem_u32(&bars.p_full[i]), (par >> i) & 1u, 0x60 + i);
+                  tc_fence_after();
+                  issue_pv<6, 8>(t_o, t_s, kv_at(at(v, i)), true);
                   if (has_next) {
-                    if (elect_one()) {
-                      issue_pv<6, 8>(t_o, t_s, sm_v, true);
-                      tc_commit(smem_u32(&bars.kv_empty[vs]));
+                    if (sep) {
+                      // The ring holds 1.25 key blocks here: the next K tile comes late, and P V must
+                      // not wait for it (looked at before P, the stage lost up to 12 % on MHA).
+                      free_kv(at(v, i));
+                      wait_kv(at(k, i), 0x50);
+                      tc_fence_after();
                     }
-                    __syncwarp();
-                    wait_bar(env, smem_u32(&bars.kv_full[ks]), at(k, i).ph, 0x50 + ks);
-                    tc_fence_after();
-                    if (elect_one()) {
-                      issue_qk(t_s, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
-                      tc_commit(smem_u32(&bars.s_full[i]));
-                      tc_commit(smem_u32(&bars.kv_empty[ks]));
-                      if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[i]));
-                    }
-                    __syncwarp();
-                    continue;
-                  }
-                }
-                if (elect_one()) {
-                  issue_pv<6, 8>(t_o, t_s, sm_v, true);
-                  if (!sep && has_next) {
-                    issue_qk(t_s, smem0 + kSmQ + i * kTile, smem0 + kSmKV + ks * kTile);
+                    issue_qk(t_s, smem0 + kSmQ + i * kTile, kv_at(at(k, i)));
                     tc_commit(smem_u32(&bars.s_full[i]));
                     if (last_use) {
-                      tc_commit(smem_u32(&bars.kv_empty[vs]));
-                      tc_commit(smem_u32(&bars.kv_empty[ks]));
+                      if (!sep) free_kv(at(v, i));
+                      free_kv(at(k, i));
                     }
                     if (jj + 2 == nblk) tc_commit(smem_u32(&bars.q_empty[i]));
                   } else {
                     tc_commit(smem_u32(&bars.o_done[i]));
-                    if (last_use) tc_commit(smem_u32(&bars.kv_empty[vs]));
+                    if (last_use) free_kv(at(v, i));
                   }
                 }
-                __syncwarp();
               }
+              par ^= 3u;
             }
           };
-          if (p.sep) run(Layout<true>{}); else run(Layout<false>{});
+          if (elect_one()) {
+            if (p.sep) run(Layout<true>{}); else run(Layout<false>{});
+          }
+          __syncwarp();
+          const uint32_t used = static_cast<uint32_t>(2 * nblk) * (p.sep ? nt : 1) + kv_slot;
+          kv_ph ^= (used / kKvSlots) & 1u;
+          kv_slot = used % kKvSlots;
+          const uint32_t tiles = nt == 2 ? 3u : 1u;
+          q_par ^= tiles;
+          o_uses ^= tiles;
+          if (nblk & 1) p_par ^= tiles;
         } else if (mode == MODE_OPROJ) {
           const int vnt = d[TO_VNT], nrt = d[TO_NRT];
           const int nkc = p.K_local >> 6;
@@ -1044,7 +1032,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
                 // accumulator h + r: row tile r's (the passes of a slot have one row tile)
                 for (int r = 0; r < rows; ++r) {
                   if (kc == 0)
-                    wait_bar(env, smem_u32(&bars.acc_free[h + r]), (acc_uses[h + r] & 1u) ^ 1u,
+                    wait_bar(env, smem_u32(&bars.acc_free[h + r]), ((acc_uses >> (h + r)) & 1u) ^ 1u,
                              0xA8 + h + r);
                   tc_fence_after();
                   const uint32_t a16r = a16 + r * (kPanel >> 4);
@@ -1064,25 +1052,24 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           const uint32_t end = op_st + static_cast<uint32_t>(passes * nkc);
           op_ph ^= (end / stages) & 1u;
           op_st = end % stages;
-          ++acc_uses[0];
-          if (rows == 2 || passes == 2) ++acc_uses[1];
+          acc_uses ^= (rows == 2 || passes == 2) ? 3u : 1u;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.task_empty[slot_k]));
-        ++n_arrived[slot_k];
+        arrived ^= 1u << slot_k;
         prev_mode = mode; prev_k = slot_k; slot_k ^= 1;
       }
     } else if (warp == 3 && lane == 0) {
       // ==================================== attention output stores: O_scratch[ft, :, head, :]
       // (a warp of their own, so that no softmax warp waits for a store to complete)
-      uint32_t st_par[2] = {0, 0};
+      uint32_t st_par = 0;
       while (true) {
         MA_NEXT_TASK(d, mode)
         if (mode == MODE_FA) {
           const int ft = d[T_FT], head0 = d[TF_HEAD0], nt = d[TF_NT];
           for (int i = 0; i < nt; ++i) {
-            if (!wait_bar(env, smem_u32(&bars.o_staged[i]), st_par[i], 0x88 + i)) break;
-            st_par[i] ^= 1u;
+            if (!wait_bar(env, smem_u32(&bars.o_staged[i]), (st_par >> i) & 1u, 0x88 + i)) break;
+            st_par ^= 1u << i;
             const uint32_t stg = smem0 + kSmQ + i * kTile;
             tma_store_2d(&tmO, stg, (head0 + i) * 128, ft * 128);
             tma_store_2d(&tmO, stg + kPanel, (head0 + i) * 128 + 64, ft * 128);
@@ -1104,7 +1091,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     const int wg = (warp - 4) >> 2;                            // compute warpgroup 0 / 1
     const int row = (warp & 3) * 32 + lane;                    // TMEM lane == tile row
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    uint32_t s_par = 0, o_par = 0, acc_par[2] = {0, 0};
+    uint32_t s_par = 0, o_par = 0, acc_par = 0;
     while (true) {
       MA_NEXT_TASK_WARP(d, mode)
       if (mode == MODE_FA && wg < d[TF_NT]) {
@@ -1267,8 +1254,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         // warpgroup's 128 columns of it go out as two panels of 64, by way of bf16 words in
         // registers.
         auto wait_acc = [&](int h) {
-          wait_bar(env, smem_u32(&bars.acc_full[h]), acc_par[h], 0xB0 + h);
-          acc_par[h] ^= 1u;
+          wait_bar(env, smem_u32(&bars.acc_full[h]), (acc_par >> h) & 1u, 0xB0 + h);
+          acc_par ^= 1u << h;
           tc_fence_after();
         };
         auto free_acc = [&](int h) {
@@ -1357,7 +1344,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bars.task_empty[slot_k]));
-      ++n_arrived[slot_k];
+      arrived ^= 1u << slot_k;
       prev_mode = mode; prev_k = slot_k; slot_k ^= 1;
     }
   }
