@@ -166,6 +166,13 @@ int ma_launch(ma_plan* plan, const ma_launch_args* args, void* stream);
 int ma_plan_set_inputs(ma_plan* plan, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
                        int64_t tot_q, int64_t tot_k, int64_t w_width);
 
+/* Gives the plan a table of its attention tasks in claim order, as ma_stage_tasks lays it out
+ * (device address, 16-byte aligned, int32[4 + 8 * max_row_tiles]; 0: none).  The kernel then
+ * finds a task's row tile, sequence and lengths with one read of memory instead of three that
+ * wait for one another.  The table has to agree with the plan's other arrays; a count of 0 in
+ * it, or MA_FLAG_TILE_ORDER, means that they are read as without a table. */
+int ma_plan_set_tasks(ma_plan* plan, uint64_t tasks);
+
 /* Reads the device status block (synchronises `stream` first).  No reference
  * counterpart: the reference's device waits are unbounded. */
 int ma_read_status(ma_plan* plan, void* stream, ma_status* out);
@@ -328,6 +335,19 @@ typedef struct ma_stage_meta_args {
 } ma_stage_meta_args;
 
 int ma_stage_meta(const ma_stage_meta_args* args);
+
+/*
+ * ma_stage_tasks does what ma_stage_meta does and writes the task table (ma_plan_set_tasks) as
+ * well, off_tasks words into the staging copy (a multiple of 4): the number of tasks, three
+ * zeros, then for every position of the claim order {row tile, sequence, block in the sequence,
+ * cu_q, q_len, cu_k, k_len, 0}.  MA_ERR_CAPACITY past max_tasks positions.
+ */
+typedef struct ma_stage_tasks_args {
+  ma_stage_meta_args meta;
+  int32_t off_tasks, max_tasks;
+} ma_stage_tasks_args;
+
+int ma_stage_tasks(const ma_stage_tasks_args* args);
 
 const char* ma_strerror(int code);
 

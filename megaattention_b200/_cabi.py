@@ -28,7 +28,7 @@ MA_ERR_CAPACITY = -5
 
 EXPORTS = ("ma_query_device", "ma_plan_create", "ma_launch", "ma_plan_set_inputs", "ma_read_status",
            "ma_plan_destroy", "ma_strerror", "ma_fused_prefill_noalloc", "ma_residual_rmsnorm", "ma_rope_qk",
-           "ma_detile", "ma_row_desc", "ma_stage_meta")
+           "ma_detile", "ma_row_desc", "ma_stage_meta", "ma_plan_set_tasks", "ma_stage_tasks")
 
 MA_NOALLOC_OSCRATCH_BYTES = 16 << 20
 MA_NOALLOC_MAX_BATCH = 512
@@ -112,6 +112,13 @@ class StageMetaArgs(C.Structure):
                     "off_m_block", "off_order", "off_actv", "reserved0")])
 
 
+class StageTasksArgs(C.Structure):
+    _fields_ = [("meta", StageMetaArgs), ("off_tasks", C.c_int32), ("max_tasks", C.c_int32)]
+
+
+TASK_WORDS = 8           # of one position of the task table, behind a header of 4
+
+
 def _load(path=None, audit=False):
     path = path or (_build.LIB_AUDIT if audit else _build.LIB)
     if not os.path.exists(path) or _build._stale(path):
@@ -147,6 +154,10 @@ def _load(path=None, audit=False):
     lib.ma_row_desc.restype = C.c_int
     lib.ma_stage_meta.argtypes = [C.POINTER(StageMetaArgs)]
     lib.ma_stage_meta.restype = C.c_int
+    lib.ma_plan_set_tasks.argtypes = [C.c_void_p, C.c_uint64]
+    lib.ma_plan_set_tasks.restype = C.c_int
+    lib.ma_stage_tasks.argtypes = [C.POINTER(StageTasksArgs)]
+    lib.ma_stage_tasks.restype = C.c_int
     lib.ma_strerror.argtypes = [C.c_int]
     lib.ma_strerror.restype = C.c_char_p
     return lib

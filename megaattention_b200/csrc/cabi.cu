@@ -311,6 +311,12 @@ int ma_plan_set_inputs(ma_plan* pl, uint64_t Q, uint64_t K, uint64_t V, uint64_t
   return MA_OK;
 }
 
+int ma_plan_set_tasks(ma_plan* pl, uint64_t tasks) {
+  if (!pl || (tasks & 15u)) return MA_ERR_INVALID;
+  pl->kp.tasks = reinterpret_cast<const int*>(tasks);
+  return MA_OK;
+}
+
 int ma_read_status(ma_plan* pl, void* stream, ma_status* out) {
   if (!pl || !out) return MA_ERR_INVALID;
   uint32_t h[4] = {0, 0, 0, 0};

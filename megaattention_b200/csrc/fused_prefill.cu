@@ -122,21 +122,9 @@ __device__ __forceinline__ bool wait_bar(const Env& e, uint32_t bar, uint32_t pa
 // SM late - another stream's kernel holds it - keeps its task from all the others, which wait
 // for it up to the wait limit.)
 // An id stands for one head, two heads of a kv group (pair), or two heads that share no kv
-// head and the last head of an odd count alone (sep); arg is position * H + first head.
+// head and the last head of an odd count alone (sep), of one position of the claim order.
 __device__ __forceinline__ int fa_tasks_per_tile(const KParams& p) {
   return (p.pair || p.sep) ? (p.H + 1) >> 1 : p.H;
-}
-__device__ __forceinline__ int fa_task_arg(const KParams& p, int id) {
-  const int n = fa_tasks_per_tile(p);
-  return (id / n) * p.H + (id % n) * ((p.pair || p.sep) ? 2 : 1);
-}
-__device__ __forceinline__ bool try_fa(const KParams& p, int num_fa, int* arg) {
-  const int n_tasks = (num_fa / p.H) * fa_tasks_per_tile(p);
-  if (static_cast<int>(ld_relaxed_gpu(p.ctrl + C_FA_COUNTER)) < n_tasks) {
-    const int id = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
-    if (id < n_tasks) { *arg = fa_task_arg(p, id); return true; }
-  }
-  return false;
 }
 
 // Pop from the published O_proj ready queue.  The reference pops with a CAS on the consume
@@ -147,18 +135,17 @@ __device__ __forceinline__ bool try_fa(const KParams& p, int num_fa, int* arg) {
 // served as soon as the publish index passes it; meanwhile the CTA keeps taking other work.
 // The queue holds row-tile groups in the order they became ready; each stands for its
 // `per_group` tasks, so ticket t is task t % per_group of entry t / per_group.
+// `head` and `tail` (acquired) are the consume and publish counts as the caller read them.
 __device__ __forceinline__ bool try_pop_oproj(const KParams& p, int total_op, int per_group,
-                                              int* pending, int* arg) {
+                                              uint32_t head, uint32_t tail, int* pending, int* arg) {
   if (*pending < 0) {
-    const uint32_t head = ld_relaxed_gpu(p.ctrl + C_OP_CONSUME);
-    const uint32_t tail = ld_acquire_gpu(p.ctrl + C_OP_PUBLISH);
     if (head >= tail) return false;
     const uint32_t t = atom_add_relaxed_gpu(p.ctrl + C_OP_CONSUME, 1u);
     if (static_cast<int>(t) >= total_op) return false;    // past the end: nothing there
     *pending = static_cast<int>(t);
     if (t >= tail && static_cast<uint32_t>(*pending) >= ld_acquire_gpu(p.ctrl + C_OP_PUBLISH))
       return false;
-  } else if (static_cast<uint32_t>(*pending) >= ld_acquire_gpu(p.ctrl + C_OP_PUBLISH)) {
+  } else if (static_cast<uint32_t>(*pending) >= tail) {
     return false;
   }
   *arg = static_cast<int>(ld_relaxed_gpu(p.oproj_queue + *pending / per_group)) * per_group +
@@ -238,13 +225,24 @@ __device__ __noinline__ int try_claim_ar(const KParams& p, int local_owned, uint
   return -1;
 }
 
-__device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, int total_op,
+// What limits a claim is the number of trips to L2 that wait for one another, 600-700 cycles
+// each: the words that decide it are read together.  (One after the other, with the tile's
+// descriptor behind them, a claim took 6500 cycles - most of what lies between two attention
+// tasks, and several times in the chain of a small launch.  In-kernel cycles of a whole launch:
+// three short prompts 77400 -> 71700, six ragged prompts of 13400 tokens 371200 -> 363600, 12
+// short turns on cached prompts 199300 -> 193100, a wide layer 2191000 -> 2193000.)
+__device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, int n_fa_tasks, int total_op,
                                            int per_group, int local_owned, uint32_t poll_no, bool busy,
-                                           int* pending, int* mode, int* arg) {
+                                           bool* fa_left, int* pending, int* mode, int* arg) {
   const KParams& p = *e.p;
   *mode = MODE_IDLE;
   *arg = -1;
-  if (ld_relaxed_gpu(p.status) != 0u) {       // some CTA (or rank) gave up: leave
+  const uint32_t status = ld_relaxed_gpu(p.status);
+  const uint32_t fa_next = ld_relaxed_gpu(p.ctrl + C_FA_COUNTER), fa_d = ld_relaxed_gpu(p.ctrl + C_FA_DONE);
+  const uint32_t op_next = ld_relaxed_gpu(p.ctrl + C_OP_CONSUME), op_d = ld_relaxed_gpu(p.ctrl + C_OP_DONE);
+  const uint32_t ar_next = ld_relaxed_gpu(p.ctrl + C_AR_CURSOR), ar_d = ld_relaxed_gpu(p.ctrl + C_AR_DONE);
+  const uint32_t tail = ld_acquire_gpu(p.ctrl + C_OP_PUBLISH);
+  if (status != 0u) {       // some CTA (or rank) gave up: leave
     *e.abort_flag = 1;
     *mode = MODE_DONE;
     return;
@@ -252,8 +250,8 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   if (p.flags & 8u) {
     // AllReduce-only launch: every owned slot is taken as ready (the caller made sure all
     // ranks' partials are in place); slots are handed out by a counter
-    if (static_cast<int>(ld_acquire_gpu(p.ctrl + C_AR_DONE)) >= local_owned) { *mode = MODE_DONE; return; }
-    if (static_cast<int>(ld_relaxed_gpu(p.ctrl + C_AR_CURSOR)) < local_owned) {
+    if (static_cast<int>(ar_d) >= local_owned) { *mode = MODE_DONE; return; }
+    if (static_cast<int>(ar_next) < local_owned) {
       const int idx = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_AR_CURSOR, 1u));
       if (idx < local_owned) { *mode = MODE_AR; *arg = idx * p.tp + p.rank; }
     }
@@ -262,21 +260,19 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   if (p.flags & 32u) {
     // O_proj-only launch (single rank): O_scratch is taken as complete, slots are handed
     // out in order by the consume counter
-    if (static_cast<int>(ld_acquire_gpu(p.ctrl + C_OP_DONE)) >= total_op) { *mode = MODE_DONE; return; }
-    if (static_cast<int>(ld_relaxed_gpu(p.ctrl + C_OP_CONSUME)) < total_op) {
+    if (static_cast<int>(op_d) >= total_op) { *mode = MODE_DONE; return; }
+    if (static_cast<int>(op_next) < total_op) {
       const int t = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_OP_CONSUME, 1u));
       if (t < total_op) { *mode = MODE_OPROJ; *arg = t; }
     }
     return;
   }
   const bool fa_only = (p.flags & 1u) != 0;
-  const int fa_d = static_cast<int>(ld_acquire_gpu(p.ctrl + C_FA_DONE));
-  bool done = fa_d >= num_fa;
-  if (!fa_only) {
-    const int op_d = static_cast<int>(ld_acquire_gpu(p.ctrl + C_OP_DONE));
-    const int ar_d = static_cast<int>(ld_acquire_gpu(p.ctrl + C_AR_DONE));
-    done = done && op_d >= total_op && (p.tp == 1 || (p.flags & 16u) || ar_d >= local_owned);
-  }
+  // (each count is final once it is at its target; what they stand for is read by nobody before
+  // the exit protocol's fence)
+  const bool done = static_cast<int>(fa_d) >= num_fa &&
+                    (fa_only || (static_cast<int>(op_d) >= total_op &&
+                                 (p.tp == 1 || (p.flags & 16u) || static_cast<int>(ar_d) >= local_owned)));
   if (done) { *mode = MODE_DONE; return; }
   // probe order by role: 0: FA,OPROJ,AR  1: OPROJ,AR,FA  2: AR,FA,OPROJ (the reference's
   // three orders).  With the "drain first" launch flag downstream work goes first so that
@@ -291,11 +287,16 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
       m = (src > MODE_AR) ? src - 3 : src;
     }
     bool ok = false;
-    if (m == MODE_FA) ok = try_fa(p, num_fa, arg);
-    else if (fa_only) ok = false;
-    else if (m == MODE_OPROJ) ok = try_pop_oproj(p, total_op, per_group, pending, arg);
+    if (m == MODE_FA) {
+      if (*fa_left && static_cast<int>(fa_next) < n_fa_tasks) {
+        *arg = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+        ok = *arg < n_fa_tasks;
+      }
+      if (!ok) *fa_left = false;
+    } else if (fa_only) ok = false;
+    else if (m == MODE_OPROJ) ok = try_pop_oproj(p, total_op, per_group, op_next, tail, pending, arg);
     else if (p.tp > 1 && !(p.flags & 16u) &&
-             !(busy && static_cast<int>(ld_relaxed_gpu(p.ctrl + C_OP_CONSUME)) >= total_op))
+             !(busy && static_cast<int>(op_next) >= total_op))
     {
       // (once every O_proj task has been handed out only reductions are left and CTAs go
       // idle: a CTA that still has a task running leaves ready slots to them instead of
@@ -651,6 +652,12 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       // tiles x nnt column tiles (<= 2 x 2) in one pass, the row tiles sharing every W stage.
       int nrt = 0, nnt = p.sg, per_group = p.nsg, total_op = p.actv[1];
       const int n_tiles = p.actv[2];
+      // the table of attention tasks, in claim order (none: the claim order's arrays)
+      const int* tasks = (p.flags & 4u) ? nullptr : p.tasks;
+      int n_pos = tasks ? tasks[0] : 0;
+      if (n_pos == 0) { tasks = nullptr; n_pos = num_fa / p.H; }
+      const int n_fa_tasks = n_pos * fa_tasks_per_tile(p);
+      bool fa_left = !(p.flags & (8u | 32u));
       if (p.tp == 1 && !(p.flags & 16u)) {      // (without AllReduce: slots, as with several)
         op_task_shape(p, n_tiles, static_cast<int>(gridDim.x), &nrt, &nnt);
         per_group = (p.num_out + nnt - 1) / nnt;
@@ -732,23 +739,21 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           ld_skip[k ^ 1] = false;
         }
         int mode = MODE_IDLE, arg = -1;
-        if (first) {
-          // the first attention task with one atomic: nothing else can be ready yet, so none
-          // of schedule_pick's dependent loads is needed (five trips to L2 with every CTA at
-          // the same words, 1.5 to 4 us of a launch)
-          first = false;
-          if (status0 == 0u && !(p.flags & (8u | 32u))) {
-            const int id = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
-            if (id < (num_fa / p.H) * fa_tasks_per_tile(p)) {
-              mode = MODE_FA;
-              arg = fa_task_arg(p, id);
-            }
+        if (fa_left && (first || role == 0)) {
+          // An attention task where that is what the CTA asks for first: one atomic, and whether
+          // somebody gave up comes with it.  (The first task of every CTA: nothing else can be
+          // ready yet.)
+          const uint32_t status = first ? status0 : ld_relaxed_gpu(p.status);
+          if (status == 0u) {
+            arg = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+            if (arg < n_fa_tasks) mode = MODE_FA; else fa_left = false;
           }
+          first = false;
         }
         uint64_t idle_t0 = 0;
         while (mode == MODE_IDLE) {
-          schedule_pick(env, role, num_fa, total_op, per_group, local_owned, poll_no++, occupied[k ^ 1],
-                        &pending_ticket, &mode, &arg);
+          schedule_pick(env, role, num_fa, n_fa_tasks, total_op, per_group, local_owned, poll_no++,
+                        occupied[k ^ 1], &fa_left, &pending_ticket, &mode, &arg);
           if (mode != MODE_IDLE) break;
           // nothing to do and not finished: bounded like every other wait (a rank that
           // never shows up, or counts that can never be reached, must not hang the GPU)
@@ -772,15 +777,24 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         }
         int* d = s_desc[k];
         if (mode == MODE_FA) {
-          const int pos = arg / p.H, head0 = arg % p.H;
+          const int per_tile = fa_tasks_per_tile(p);
+          const int pos = arg / per_tile, head0 = (arg % per_tile) * ((p.pair || p.sep) ? 2 : 1);
           const int nt = p.pair ? 2 : (p.sep ? min(2, p.H - head0) : 1);
-          const int ft = (p.fa_order && !(p.flags & 4u)) ? p.fa_order[pos] : pos;
-          const int b = p.fa_b[ft], mb = p.fa_mb[ft];
-          const int q0 = p.cu_q[b], q_len = p.cu_q[b + 1] - q0;
+          int ft, b, mb, q0, q_len, k0, k_len;
+          if (tasks) {          // one trip to L2; by the arrays below it is three
+            const int4* r = reinterpret_cast<const int4*>(tasks + 4 + pos * kTaskWords);
+            const int4 r0 = r[0], r1 = r[1];
+            ft = r0.x; b = r0.y; mb = r0.z; q0 = r0.w;
+            q_len = r1.x; k0 = r1.y; k_len = r1.z;
+          } else {
+            ft = (p.fa_order && !(p.flags & 4u)) ? p.fa_order[pos] : pos;
+            b = p.fa_b[ft]; mb = p.fa_mb[ft];
+            q0 = p.cu_q[b]; q_len = p.cu_q[b + 1] - q0;
+            k0 = p.cu_k[b]; k_len = p.cu_k[b + 1] - k0;
+          }
           // contiguous KV: rows [k0, k0 + k_len) of K/V; paged KV: k0 is the sequence's row
           // in the page table and the length comes from cache_seqlens
-          const int k0 = p.page_table ? b * p.pps : p.cu_k[b];
-          const int k_len = p.page_table ? p.cache_seqlens[b] : p.cu_k[b + 1] - k0;
+          if (p.page_table) { k0 = b * p.pps; k_len = p.cache_seqlens[b]; }
           const int offset = k_len - q_len;
           int nblk = (k_len + 127) >> 7;
           const int nb2 = ((mb + 1) * 128 + offset + 127) >> 7;

@@ -50,6 +50,8 @@ struct KParams {
   const int* fa_b;
   const int* fa_mb;
   const int* fa_order;            // row tiles in claim order (longest first), or null
+  const int* tasks;               // attention tasks in claim order: {count, 0, 0, 0}, then kTaskWords each
+                                  // (see kTaskWords), or null: from the arrays above
   const int* page_table;          // paged KV: [batch][pps] page of each 128-key block, or null
   const int* cache_seqlens;       // paged KV: KV length per sequence
   int pps;                        // page-table row pitch
@@ -66,6 +68,10 @@ struct KParams {
 
 constexpr int kOpTwoFrom = 9, kOpCols2From = 5;             // behind attention
 constexpr int kOpTwoFromAlone = 2, kOpCols2FromAlone = 1;   // O_proj-only launches
+
+// A position of the task table: {row tile, sequence, block in the sequence, cu_q of the sequence,
+// q_len, cu_k of the sequence, k_len, 0}; written by ma_stage_tasks.
+constexpr int kTaskWords = 8;
 
 constexpr int kThreads = 384;
 constexpr int kSmemDynamic = 65536 + 5 * 32768 + 1024;   // Q x2, K/V ring x5, align slack

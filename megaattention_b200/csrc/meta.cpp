@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/megaattn_b200.h"
+#include "kparams.h"
 
 extern "C" int ma_row_desc(const int64_t* cu_q, const int64_t* cu_k, int32_t num_batch,
                            int32_t max_row_tiles, int32_t* cu_q_out, int32_t* cu_k_out,
@@ -101,5 +102,30 @@ extern "C" int ma_stage_meta(const ma_stage_meta_args* a) {
   actv[3] = static_cast<int32_t>(slots);
   actv[4] = static_cast<int32_t>((slots + 63) / 64);
   actv[5] = static_cast<int32_t>((owned + tp - 1) / tp);
+  return MA_OK;
+}
+
+extern "C" int ma_stage_tasks(const ma_stage_tasks_args* a) {
+  if (!a || a->off_tasks < 0 || (a->off_tasks & 3)) return MA_ERR_INVALID;
+  const ma_stage_meta_args& m = a->meta;
+  const int rc = ma_stage_meta(&m);
+  if (rc != MA_OK) return rc;
+  if (m.num_row_tiles > a->max_tasks) return MA_ERR_CAPACITY;
+  const int32_t* order = m.staging + m.off_order;
+  int32_t* head = m.staging + a->off_tasks;
+  head[0] = m.num_row_tiles;
+  head[1] = head[2] = head[3] = 0;
+  for (int i = 0; i < m.num_row_tiles; ++i) {
+    int32_t* r = head + 4 + i * ma::kTaskWords;
+    const int t = order[i], b = m.batch_idx[t];
+    r[0] = t;
+    r[1] = b;
+    r[2] = m.m_block[t];
+    r[3] = m.cu_q[b];
+    r[4] = m.cu_q[b + 1] - m.cu_q[b];
+    r[5] = m.cu_k[b];
+    r[6] = static_cast<int32_t>(static_cast<uint32_t>(m.cu_k[b + 1]) - static_cast<uint32_t>(m.cu_k[b]));
+    r[7] = 0;
+  }
   return MA_OK;
 }

@@ -173,17 +173,17 @@ class FusedFaOprojArWorkspace:
             rc_ptrs, rb_ptrs, nvl_peer_ptrs, csym_peer_ptrs = [], [], [], []
 
         # varlen metadata: one device buffer, so a layer's descriptors arrive in one copy;
-        # cu_q | cu_k | fa_b | fa_mb | fa_order | actv are views at fixed (capacity) offsets,
-        # each 16-byte aligned
+        # cu_q | cu_k | fa_b | fa_mb | fa_order | actv | task table are views at fixed (capacity)
+        # offsets, each 16-byte aligned
         def up4(n):
             return (n + 3) // 4 * 4
         sizes = (max_num_batch + 1, max_num_batch + 1, max_num_row_tiles, max_num_row_tiles,
-                 max_num_row_tiles, 8)
+                 max_num_row_tiles, 8, 4 + _cabi.TASK_WORDS * max_num_row_tiles)
         offs = [0]
         for n in sizes:
             offs.append(offs[-1] + up4(n))
         meta_dev = zeros(offs[-1], torch.int32)
-        mviews = [meta_dev[offs[i]:offs[i] + sizes[i]] for i in range(6)]
+        mviews = [meta_dev[offs[i]:offs[i] + sizes[i]] for i in range(7)]
         ws = cls(
             dev=dev, dtype=dtype, meta_dev=meta_dev, _meta_offs=offs, tp_size=tp_size, rank=rank, group_name=group_name,
             H_local=H_local, H_kv=H_kv, D=D, K_local=K_local, hidden=hidden,
@@ -198,6 +198,7 @@ class FusedFaOprojArWorkspace:
             head_ready=zeros(max_num_row_tiles, torch.uint32),
             oproj_queue=zeros(max_total, torch.uint32),
             ar_done_bits=zeros(max_owner_words, torch.int64),
+            tasks=mviews[6],
             cu_q=mviews[0], cu_k=mviews[1], fa_b=mviews[2], fa_mb=mviews[3], fa_order=mviews[4],
             Q=zeros((tot_cap, H_local, D), dtype),
             K=(None if paged else zeros((max_tot_k, H_kv, D), dtype)),
@@ -278,6 +279,7 @@ class FusedFaOprojArWorkspace:
         plan = C.c_void_p()
         _cabi.check(self._lib.ma_plan_create(C.byref(d), C.byref(plan)), "ma_plan_create")
         self._plan = plan
+        _cabi.check(self._lib.ma_plan_set_tasks(plan, self.tasks.data_ptr()), "ma_plan_set_tasks")
         self._args = _cabi.LaunchArgs(int(w_fa), int(w_oproj), int(w_ar),
                                       int(num_ctas) if num_ctas else 0, 0)
         self._ts = torch.cuda.current_stream(self.dev)
@@ -413,13 +415,13 @@ class FusedFaOprojArWorkspace:
             meta.cu_seqlens_q, meta.cu_seqlens_k, meta.batch_idx, meta.m_block))
         assert b_idx.size == m_blk.size == R and cu_q.size == cu_k.size == meta.num_batch + 1
         prime = self.fa_prime_tiles
-        args = _cabi.StageMetaArgs(
+        args = _cabi.StageTasksArgs(_cabi.StageMetaArgs(
             cu_q.ctypes.data, cu_k.ctypes.data, b_idx.ctypes.data, m_blk.ctypes.data,
             slot[0].data_ptr(), cu_q.size - 1, R, self.hidden, self.H_local, self.num_super_groups,
             self.tp_size, self.rank, int(prime is None),
             0 if prime is None else max(-1, min(int(prime), R)),
-            o[0], o[1], o[2], o[3], o[4], o[5], 0)
-        _cabi.check(_cabi.lib.ma_stage_meta(C.byref(args)), "ma_stage_meta")
+            o[0], o[1], o[2], o[3], o[4], o[5], 0), o[6], self.max_num_row_tiles)
+        _cabi.check(_cabi.lib.ma_stage_tasks(C.byref(args)), "ma_stage_tasks")
         self.meta_dev.copy_(slot[0], non_blocking=True)
         if slot[1] is None:
             slot[1] = torch.cuda.Event()
@@ -507,7 +509,7 @@ class FusedFaOprojArWorkspace:
         """Fault localisation only; never on the production / bench / test default path.
         With tp > 1 every rank must call it, followed by a host barrier."""
         for t in (self.ctrl, self.sync_ctrl, self.actv, self.head_ready, self.oproj_queue,
-                  self.fa_order, self.rco, self.rbits, self.ar_done_bits, self.nvl, self.csym, self.Oscr,
+                  self.fa_order, self.tasks, self.rco, self.rbits, self.ar_done_bits, self.nvl, self.csym, self.Oscr,
                   self.status):
             t.zero_()
 
