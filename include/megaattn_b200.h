@@ -349,6 +349,15 @@ typedef struct ma_stage_tasks_args {
 
 int ma_stage_tasks(const ma_stage_tasks_args* args);
 
+/*
+ * ma_upload_meta does what ma_stage_tasks does and queues the active parts of the staging copy
+ * for the device's copy of it (device address, 16-byte aligned, same offsets) on `stream`.  The
+ * words travel in kernel parameters: the staging copy may be reused once the call has returned,
+ * and a captured call keeps the words it was captured with.  Returns what ma_stage_tasks does, or
+ * MA_ERR_CUDA.
+ */
+int ma_upload_meta(const ma_stage_tasks_args* args, uint64_t meta_dev, void* stream);
+
 const char* ma_strerror(int code);
 
 #ifdef __cplusplus

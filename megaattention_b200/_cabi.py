@@ -28,7 +28,8 @@ MA_ERR_CAPACITY = -5
 
 EXPORTS = ("ma_query_device", "ma_plan_create", "ma_launch", "ma_plan_set_inputs", "ma_read_status",
            "ma_plan_destroy", "ma_strerror", "ma_fused_prefill_noalloc", "ma_residual_rmsnorm", "ma_rope_qk",
-           "ma_detile", "ma_row_desc", "ma_stage_meta", "ma_plan_set_tasks", "ma_stage_tasks")
+           "ma_detile", "ma_row_desc", "ma_stage_meta", "ma_plan_set_tasks", "ma_stage_tasks",
+           "ma_upload_meta")
 
 MA_NOALLOC_OSCRATCH_BYTES = 16 << 20
 MA_NOALLOC_MAX_BATCH = 512
@@ -158,6 +159,8 @@ def _load(path=None, audit=False):
     lib.ma_plan_set_tasks.restype = C.c_int
     lib.ma_stage_tasks.argtypes = [C.POINTER(StageTasksArgs)]
     lib.ma_stage_tasks.restype = C.c_int
+    lib.ma_upload_meta.argtypes = [C.POINTER(StageTasksArgs), C.c_uint64, C.c_void_p]
+    lib.ma_upload_meta.restype = C.c_int
     lib.ma_strerror.argtypes = [C.c_int]
     lib.ma_strerror.restype = C.c_char_p
     return lib

@@ -398,17 +398,10 @@ class FusedFaOprojArWorkspace:
 
     def _set_meta(self, meta):
         R = meta.num_row_tiles
-        # ONE asynchronous H2D copy: the six arrays are packed at their capacity offsets into
-        # a pinned staging buffer (a ring of four, so the host never rewrites a buffer whose
-        # copy may still be in flight)
-        if getattr(self, "_meta_ring", None) is None:
-            self._meta_ring = [[torch.zeros(self._meta_offs[-1], dtype=torch.int32).pin_memory(), None]
-                               for _ in range(4)]
-            self._meta_i = 0
-        slot = self._meta_ring[self._meta_i % 4]
-        self._meta_i += 1
-        if slot[1] is not None:
-            slot[1].synchronize()
+        # (the words travel in a kernel's parameters, so the staging copy is free again on return)
+        if getattr(self, "_meta_host", None) is None:
+            self._meta_host = np.zeros(self._meta_offs[-1], dtype=np.int32)
+            self._meta_at = self._meta_host.ctypes.data
         o = self._meta_offs
         self._auto_flags = launch_flags_b200(meta, self.hidden, self.tp_size, self.H_local)
         cu_q, cu_k, b_idx, m_blk = (np.ascontiguousarray(x, dtype=np.int32) for x in (
@@ -417,15 +410,13 @@ class FusedFaOprojArWorkspace:
         prime = self.fa_prime_tiles
         args = _cabi.StageTasksArgs(_cabi.StageMetaArgs(
             cu_q.ctypes.data, cu_k.ctypes.data, b_idx.ctypes.data, m_blk.ctypes.data,
-            slot[0].data_ptr(), cu_q.size - 1, R, self.hidden, self.H_local, self.num_super_groups,
+            self._meta_at, cu_q.size - 1, R, self.hidden, self.H_local, self.num_super_groups,
             self.tp_size, self.rank, int(prime is None),
             0 if prime is None else max(-1, min(int(prime), R)),
             o[0], o[1], o[2], o[3], o[4], o[5], 0), o[6], self.max_num_row_tiles)
-        _cabi.check(_cabi.lib.ma_stage_tasks(C.byref(args)), "ma_stage_tasks")
-        self.meta_dev.copy_(slot[0], non_blocking=True)
-        if slot[1] is None:
-            slot[1] = torch.cuda.Event()
-        slot[1].record(torch.cuda.current_stream(self.dev))
+        rc = _cabi.lib.ma_upload_meta(C.byref(args), self.meta_dev.data_ptr(),
+                                      torch.cuda.current_stream(self.dev).cuda_stream)
+        _cabi.check(min(rc, 0), "ma_upload_meta")
         self._meta = meta
 
     def _on_stream(self):
