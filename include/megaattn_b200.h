@@ -167,11 +167,18 @@ int ma_plan_set_inputs(ma_plan* plan, uint64_t Q, uint64_t K, uint64_t V, uint64
                        int64_t tot_q, int64_t tot_k, int64_t w_width);
 
 /* Gives the plan a table of its attention tasks in claim order, as ma_stage_tasks lays it out
- * (device address, 16-byte aligned, int32[4 + 8 * max_row_tiles]; 0: none).  The kernel then
+ * (device address, 16-byte aligned, int32[4 + 8 * max_tasks]; 0: none).  The kernel then
  * finds a task's row tile, sequence and lengths with one read of memory instead of three that
  * wait for one another.  The table has to agree with the plan's other arrays; a count of 0 in
  * it, or MA_FLAG_TILE_ORDER, means that they are read as without a table. */
 int ma_plan_set_tasks(ma_plan* plan, uint64_t tasks);
+
+/* Gives the plan room for parts of an attention task's keys (device addresses; 0, 0: none, and a
+ * row tile that the task table splits is then one task all the same): parts, 16-byte aligned,
+ * float[slots * H_local * MA_PART_FLOATS], and counts u32[slots * H_local], zero at first.  slots as
+ * in ma_stage_tasks_args; the plan's launches must not overlap with others that use the same room. */
+#define MA_PART_FLOATS (128 * 128 + 2 * 128)
+int ma_plan_set_split(ma_plan* plan, uint64_t parts, uint64_t counts);
 
 /* Reads the device status block (synchronises `stream` first).  No reference
  * counterpart: the reference's device waits are unbounded. */
@@ -340,11 +347,16 @@ int ma_stage_meta(const ma_stage_meta_args* args);
  * ma_stage_tasks does what ma_stage_meta does and writes the task table (ma_plan_set_tasks) as
  * well, off_tasks words into the staging copy (a multiple of 4): the number of tasks, three
  * zeros, then for every position of the claim order {row tile, sequence, block in the sequence,
- * cu_q, q_len, cu_k, k_len, 0}.  MA_ERR_CAPACITY past max_tasks positions.
+ * cu_q, q_len, cu_k, k_len, split}.  MA_ERR_CAPACITY if the row tiles are more than max_tasks.
+ * Where a few long tasks would keep the launch waiting, a row tile's keys are split: it has a
+ * position per part then, split = parts | part << 8 | first slot << 16 (0: not split), as far as
+ * max_tasks positions and split_slots slots (ma_plan_set_split; 0: no splitting) go round.  num_ctas
+ * is the launch's.
  */
 typedef struct ma_stage_tasks_args {
   ma_stage_meta_args meta;
   int32_t off_tasks, max_tasks;
+  int32_t split_slots, num_ctas;
 } ma_stage_tasks_args;
 
 int ma_stage_tasks(const ma_stage_tasks_args* args);

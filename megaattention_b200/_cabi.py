@@ -29,7 +29,7 @@ MA_ERR_CAPACITY = -5
 EXPORTS = ("ma_query_device", "ma_plan_create", "ma_launch", "ma_plan_set_inputs", "ma_read_status",
            "ma_plan_destroy", "ma_strerror", "ma_fused_prefill_noalloc", "ma_residual_rmsnorm", "ma_rope_qk",
            "ma_detile", "ma_row_desc", "ma_stage_meta", "ma_plan_set_tasks", "ma_stage_tasks",
-           "ma_upload_meta")
+           "ma_upload_meta", "ma_plan_set_split")
 
 MA_NOALLOC_OSCRATCH_BYTES = 16 << 20
 MA_NOALLOC_MAX_BATCH = 512
@@ -114,10 +114,12 @@ class StageMetaArgs(C.Structure):
 
 
 class StageTasksArgs(C.Structure):
-    _fields_ = [("meta", StageMetaArgs), ("off_tasks", C.c_int32), ("max_tasks", C.c_int32)]
+    _fields_ = [("meta", StageMetaArgs), ("off_tasks", C.c_int32), ("max_tasks", C.c_int32),
+                ("split_slots", C.c_int32), ("num_ctas", C.c_int32)]
 
 
 TASK_WORDS = 8           # of one position of the task table, behind a header of 4
+PART_FLOATS = 128 * 128 + 2 * 128     # of one head of a slot (ma_plan_set_split)
 
 
 def _load(path=None, audit=False):
@@ -157,6 +159,8 @@ def _load(path=None, audit=False):
     lib.ma_stage_meta.restype = C.c_int
     lib.ma_plan_set_tasks.argtypes = [C.c_void_p, C.c_uint64]
     lib.ma_plan_set_tasks.restype = C.c_int
+    lib.ma_plan_set_split.argtypes = [C.c_void_p, C.c_uint64, C.c_uint64]
+    lib.ma_plan_set_split.restype = C.c_int
     lib.ma_stage_tasks.argtypes = [C.POINTER(StageTasksArgs)]
     lib.ma_stage_tasks.restype = C.c_int
     lib.ma_upload_meta.argtypes = [C.POINTER(StageTasksArgs), C.c_uint64, C.c_void_p]

@@ -317,6 +317,13 @@ int ma_plan_set_tasks(ma_plan* pl, uint64_t tasks) {
   return MA_OK;
 }
 
+int ma_plan_set_split(ma_plan* pl, uint64_t parts, uint64_t counts) {
+  if (!pl || (parts & 15u) || (counts & 3u) || !parts != !counts) return MA_ERR_INVALID;
+  pl->kp.part_o = reinterpret_cast<float*>(parts);
+  pl->kp.part_count = reinterpret_cast<uint32_t*>(counts);
+  return MA_OK;
+}
+
 int ma_read_status(ma_plan* pl, void* stream, ma_status* out) {
   if (!pl || !out) return MA_ERR_INVALID;
   uint32_t h[4] = {0, 0, 0, 0};

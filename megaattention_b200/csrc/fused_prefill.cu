@@ -410,15 +410,16 @@ __device__ __forceinline__ void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint3
            (acc || kk > 0) ? 1u : 0u);
 }
 
-// Convert 32 fp32 values (columns col0..col0+31 of this thread's row, col0 in {0, 32}) to
+// Convert N fp32 values (columns col0..col0+N-1 of this thread's row, N and col0 multiples of 8) to
 // bf16 and put them into a [128 rows][64 columns] staging panel laid out as TMA expects
 // for a 128-byte-swizzled box: 16-byte chunk c of row r lives at chunk c ^ (r & 7).
-__device__ __forceinline__ void stage_row32(uint32_t panel, int row, int col0,
-                                            const uint32_t (&v)[32], float scale) {
+template <int N>
+__device__ __forceinline__ void stage_row(uint32_t panel, int row, int col0,
+                                          const uint32_t (&v)[N], float scale) {
   const uint32_t rbase = panel + static_cast<uint32_t>(row) * 128u;
   const uint32_t sw = static_cast<uint32_t>(row & 7);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < N / 8; ++q) {
     const uint32_t c = static_cast<uint32_t>((col0 >> 3) + q);
     st_shared_v4(rbase + ((c ^ sw) << 4),
                  pack_bf16x2(__uint_as_float(v[8 * q + 0]) * scale, __uint_as_float(v[8 * q + 1]) * scale),
@@ -536,8 +537,97 @@ template <bool kSeparate> struct Layout { static constexpr bool value = kSeparat
 enum : int { T_MODE = 0, T_FT = 1,
              TF_HEAD0 = 2, TF_NT = 3, TF_KVH = 4, TF_QROW0 = 5, TF_VALID = 6, TF_KSTART = 7,
              TF_KLEN = 8, TF_OFFSET = 9, TF_NBLK = 10, TF_MB = 11,
+             TF_PARTS = 12,     // parts its keys are split into (1: none); TF_PART: which of them
+             TF_PART = 13, TF_SLOT = 14,
+             TF_FIN0 = 15, TF_FIN1 = 16,   // head 0 / 1 of the task is finished when the task is
              TO_BASE = 2, TO_VNT = 3, TO_VALID = 4, TO_SLOT = 5, TO_NRT = 6, TO_VALID1 = 7, TO_TWO = 8,
-             T_WORDS = 12 };
+             T_WORDS = 17 };
+
+// End of a head's attention over a part of its keys.  The part's O (not divided), reference maximum
+// and row sum go to memory in fp32; whichever part of the head is there last adds them all up and
+// stages the head's output - nobody waits for anybody.  Its own O it has in TMEM, but it adds in the
+// parts' order, so that the result does not depend on who was last.
+// What it costs is trips to L2: 4.5 us to put a part of 64 KB there and look, 2.5 us for each part
+// that is read.  A thread's row of it lies strided ([column / 4][row] of float4: a warp's accesses are
+// 512 bytes in a row).  More than 32 columns of one part in flight would take the registers that the
+// attention loop lives on (two parts': the kernel's spills 240 -> 1000 bytes, every task slower).
+__device__ __noinline__ void finish_part(const KParams& p, int* d, int wg, int row, uint32_t t_o,
+                                         uint32_t stg, uint32_t bar_o_free, float m, float l) {
+  const int n = d[TF_PARTS], own = d[TF_PART], head = d[TF_HEAD0] + wg, first = d[TF_SLOT];
+  const size_t pitch = static_cast<size_t>(p.H) * kPartFloats;      // from one part to the next
+  float* base = p.part_o + static_cast<size_t>(first) * pitch + static_cast<size_t>(head) * kPartFloats;
+  float* mine = base + own * pitch;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t o[32];
+    tmem_ld32(t_o + c * 32, o);
+    tc_wait_ld();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      __stcg(reinterpret_cast<uint4*>(mine) + (c * 8 + q) * 128 + row,
+             make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]));
+  }
+  __stcg(mine + kPartMax + row, m);
+  __stcg(mine + kPartSum + row, l);
+  named_bar_sync(1 + wg, 128);
+  if (row == 0) {
+    uint32_t* count = p.part_count + first * p.H + head;
+    fence_acq_rel_gpu();                        // (the warpgroup's stores: ordered by the barrier)
+    const bool last = atom_add_relaxed_gpu(count, 1u) == static_cast<uint32_t>(n - 1);
+    fence_acq_rel_gpu();
+    if (last) *count = 0u;                      // (the next launch's parts count from zero)
+    d[TF_FIN0 + wg] = last ? 1 : 0;
+  }
+  named_bar_sync(1 + wg, 128);
+  if (d[TF_FIN0 + wg] != 0) {
+    float top = -INFINITY, sum = 0.f;
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) top = fmaxf(top, __ldcg(base + i * pitch + kPartMax + row));
+    auto weight = [&](float mi) { return mi == -INFINITY ? 0.f : ex2((mi - top) * p.scale_log2); };
+#pragma unroll 4
+    for (int i = 0; i < n; ++i)
+      sum += weight(__ldcg(base + i * pitch + kPartMax + row)) * __ldcg(base + i * pitch + kPartSum + row);
+    const float inv = (row < d[TF_VALID] && sum > 0.f) ? (1.f / sum) : 0.f;
+    const float w_own = weight(m);
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      float acc[32];
+#pragma unroll
+      for (int q = 0; q < 32; ++q) acc[q] = 0.f;
+      auto add_own = [&]() {
+        uint32_t o[32];
+        tmem_ld32(t_o + c * 32, o);
+        tc_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 32; ++q) acc[q] += w_own * __uint_as_float(o[q]);
+      };
+#pragma unroll 1
+      for (int j = 0; j < n - 1; ++j) {
+        const float* part = base + (j + (j >= own ? 1 : 0)) * pitch;
+        const float4* src = reinterpret_cast<const float4*>(part) + c * 8 * 128 + row;
+        float4 x[8];
+        const float mi = __ldcg(part + kPartMax + row);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = __ldcg(src + q * 128);
+        if (j == own) add_own();
+        const float w = weight(mi);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          acc[4 * q] += w * x[q].x; acc[4 * q + 1] += w * x[q].y;
+          acc[4 * q + 2] += w * x[q].z; acc[4 * q + 3] += w * x[q].w;
+        }
+      }
+      if (own == n - 1) add_own();
+      uint32_t bits[32];
+#pragma unroll
+      for (int q = 0; q < 32; ++q) bits[q] = __float_as_uint(acc[q]);
+      stage_row(stg + (c >> 1) * kPanel, row, (c & 1) * 32, bits, inv);
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  if ((row & 31) == 0) mbar_arrive(bar_o_free);
+}
 
 __device__ __forceinline__ bool is_tile_mode(int m) { return m == MODE_FA || m == MODE_OPROJ; }
 
@@ -682,7 +772,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       int pending_ticket = -1;
       uint32_t poll_no = 0;
       bool first = true;
-      int occ_mode[2] = {0, 0}, occ_a[2] = {0, 0}, occ_b[2] = {0, 0};
+      int occ_mode[2] = {0, 0}, occ_a[2] = {0, 0};
 #ifdef MA_AUDIT
       int occ_h[2] = {0, 0};
 #endif
@@ -691,7 +781,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 #ifdef MA_AUDIT
         if (p.audit) {      // exactly-once audit (audit build only): one count per finished unit
           if (occ_mode[kk] == MODE_FA) {
-            for (int i = 0; i < occ_b[kk]; ++i) atomicAdd(p.audit + occ_a[kk] * p.H + occ_h[kk] + i, 1u);
+            for (int i = 0; i < 2; ++i)
+              if (s_desc[kk][TF_FIN0 + i]) atomicAdd(p.audit + occ_a[kk] * p.H + occ_h[kk] + i, 1u);
           } else if (occ_mode[kk] == MODE_OPROJ && nrt == 0) {
             atomicAdd(p.audit + p.audit_op_base + occ_a[kk], 1u);
           } else if (occ_mode[kk] == MODE_OPROJ) {     // a slot counts with its first column tile
@@ -705,14 +796,16 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         }
 #endif
         if (occ_mode[kk] == MODE_FA) {
+          // heads that are finished (one of which another part is still running counts with that)
+          const int heads = s_desc[kk][TF_FIN0] + s_desc[kk][TF_FIN1];
+          if (heads == 0) return;
           fence_acq_rel_gpu();
           const int g = occ_a[kk] / grp;
-          const uint32_t old = atom_add_acqrel_gpu(p.head_ready + g,
-                                                   static_cast<uint32_t>(occ_b[kk]));
+          const uint32_t old = atom_add_acqrel_gpu(p.head_ready + g, static_cast<uint32_t>(heads));
           if (!(p.flags & 1u) &&
-              static_cast<int>(old) + occ_b[kk] == p.H * min(grp, n_tiles - g * grp))
+              static_cast<int>(old) + heads == p.H * min(grp, n_tiles - g * grp))
             publish_oproj(env, g, per_group);
-          atom_add_release_gpu(p.ctrl + C_FA_DONE, static_cast<uint32_t>(occ_b[kk]));
+          atom_add_release_gpu(p.ctrl + C_FA_DONE, static_cast<uint32_t>(heads));
         } else if (occ_mode[kk] == MODE_OPROJ) {
           publish_ar_ready(p, occ_a[kk]);
         } else if (occ_mode[kk] == MODE_AR) {
@@ -738,76 +831,97 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           ld_par[k ^ 1] ^= 1u;        // that task's loads_done phase is never waited for
           ld_skip[k ^ 1] = false;
         }
-        int mode = MODE_IDLE, arg = -1;
-        if (fa_left && (first || role == 0)) {
-          // An attention task where that is what the CTA asks for first: one atomic, and whether
-          // somebody gave up comes with it.  (The first task of every CTA: nothing else can be
-          // ready yet.)
-          const uint32_t status = first ? status0 : ld_relaxed_gpu(p.status);
-          if (status == 0u) {
-            arg = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
-            if (arg < n_fa_tasks) mode = MODE_FA; else fa_left = false;
+        int mode, arg;
+        int* d = s_desc[k];
+        do {
+          mode = MODE_IDLE;
+          arg = -1;
+          if (fa_left && (first || role == 0)) {
+            // An attention task where that is what the CTA asks for first: one atomic, and whether
+            // somebody gave up comes with it.  (The first task of every CTA: nothing else can be
+            // ready yet.)
+            const uint32_t status = first ? status0 : ld_relaxed_gpu(p.status);
+            if (status == 0u) {
+              arg = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+              if (arg < n_fa_tasks) mode = MODE_FA; else fa_left = false;
+            }
+            first = false;
           }
-          first = false;
-        }
-        uint64_t idle_t0 = 0;
-        while (mode == MODE_IDLE) {
-          schedule_pick(env, role, num_fa, n_fa_tasks, total_op, per_group, local_owned, poll_no++,
-                        occupied[k ^ 1], &fa_left, &pending_ticket, &mode, &arg);
-          if (mode != MODE_IDLE) break;
-          // nothing to do and not finished: bounded like every other wait (a rank that
-          // never shows up, or counts that can never be reached, must not hang the GPU)
-          if ((poll_no & 15u) == 0) {
-            const uint64_t now = globaltimer_ns();
-            if (idle_t0 == 0) idle_t0 = now;
-            else if (now - idle_t0 > p.wait_limit_ns) {
-              report(env, ST_TIMEOUT_IDLE, poll_no, static_cast<uint32_t>(pending_ticket));
-              mode = MODE_DONE;
-              break;
+          uint64_t idle_t0 = 0;
+          while (mode == MODE_IDLE) {
+            schedule_pick(env, role, num_fa, n_fa_tasks, total_op, per_group, local_owned, poll_no++,
+                          occupied[k ^ 1], &fa_left, &pending_ticket, &mode, &arg);
+            if (mode != MODE_IDLE) break;
+            // nothing to do and not finished: bounded like every other wait (a rank that
+            // never shows up, or counts that can never be reached, must not hang the GPU)
+            if ((poll_no & 15u) == 0) {
+              const uint64_t now = globaltimer_ns();
+              if (idle_t0 == 0) idle_t0 = now;
+              else if (now - idle_t0 > p.wait_limit_ns) {
+                report(env, ST_TIMEOUT_IDLE, poll_no, static_cast<uint32_t>(pending_ticket));
+                mode = MODE_DONE;
+                break;
+              }
+            }
+            const int o = k ^ 1;
+            if (occupied[o] && mbar_try_wait(smem_u32(&bars.task_empty[o]), te_par[o])) {
+              te_par[o] ^= 1u;
+              occupied[o] = false;
+              publish(o);
+            } else {
+              __nanosleep(100);
             }
           }
-          const int o = k ^ 1;
-          if (occupied[o] && mbar_try_wait(smem_u32(&bars.task_empty[o]), te_par[o])) {
-            te_par[o] ^= 1u;
-            occupied[o] = false;
-            publish(o);
-          } else {
-            __nanosleep(100);
-          }
-        }
-        int* d = s_desc[k];
-        if (mode == MODE_FA) {
-          const int per_tile = fa_tasks_per_tile(p);
-          const int pos = arg / per_tile, head0 = (arg % per_tile) * ((p.pair || p.sep) ? 2 : 1);
-          const int nt = p.pair ? 2 : (p.sep ? min(2, p.H - head0) : 1);
-          int ft, b, mb, q0, q_len, k0, k_len;
-          if (tasks) {          // one trip to L2; by the arrays below it is three
-            const int4* r = reinterpret_cast<const int4*>(tasks + 4 + pos * kTaskWords);
-            const int4 r0 = r[0], r1 = r[1];
-            ft = r0.x; b = r0.y; mb = r0.z; q0 = r0.w;
-            q_len = r1.x; k0 = r1.y; k_len = r1.z;
-          } else {
-            ft = (p.fa_order && !(p.flags & 4u)) ? p.fa_order[pos] : pos;
-            b = p.fa_b[ft]; mb = p.fa_mb[ft];
-            q0 = p.cu_q[b]; q_len = p.cu_q[b + 1] - q0;
-            k0 = p.cu_k[b]; k_len = p.cu_k[b + 1] - k0;
-          }
-          // contiguous KV: rows [k0, k0 + k_len) of K/V; paged KV: k0 is the sequence's row
-          // in the page table and the length comes from cache_seqlens
-          if (p.page_table) { k0 = b * p.pps; k_len = p.cache_seqlens[b]; }
-          const int offset = k_len - q_len;
-          int nblk = (k_len + 127) >> 7;
-          const int nb2 = ((mb + 1) * 128 + offset + 127) >> 7;
-          if (nb2 < nblk) nblk = nb2;
-          d[T_FT] = ft; d[TF_HEAD0] = head0; d[TF_NT] = nt; d[TF_KVH] = head0 / p.q_per_kv;
-          d[TF_QROW0] = q0 + mb * 128; d[TF_VALID] = min(128, q_len - mb * 128);
-          d[TF_KSTART] = k0; d[TF_KLEN] = k_len; d[TF_OFFSET] = offset; d[TF_NBLK] = nblk;
-          d[TF_MB] = mb;
-          occ_a[k] = ft; occ_b[k] = nt;
+          if (mode == MODE_FA) {
+            const int per_tile = fa_tasks_per_tile(p);
+            const int pos = arg / per_tile, head0 = (arg % per_tile) * ((p.pair || p.sep) ? 2 : 1);
+            const int nt = p.pair ? 2 : (p.sep ? min(2, p.H - head0) : 1);
+            int ft, b, mb, q0, q_len, k0, k_len;
+            uint32_t split = 1u;           // parts | which << 8 | first slot of the row tile's << 16
+            if (tasks) {          // one trip to L2; by the arrays below it is three
+              const int4* r = reinterpret_cast<const int4*>(tasks + 4 + pos * kTaskWords);
+              const int4 r0 = r[0], r1 = r[1];
+              ft = r0.x; b = r0.y; mb = r0.z; q0 = r0.w;
+              q_len = r1.x; k0 = r1.y; k_len = r1.z; split = static_cast<uint32_t>(r1.w);
+            } else {
+              ft = (p.fa_order && !(p.flags & 4u)) ? p.fa_order[pos] : pos;
+              b = p.fa_b[ft]; mb = p.fa_mb[ft];
+              q0 = p.cu_q[b]; q_len = p.cu_q[b + 1] - q0;
+              k0 = p.cu_k[b]; k_len = p.cu_k[b + 1] - k0;
+            }
+            // contiguous KV: rows [k0, k0 + k_len) of K/V; paged KV: k0 is the sequence's row
+            // in the page table and the length comes from cache_seqlens
+            if (p.page_table) { k0 = b * p.pps; k_len = p.cache_seqlens[b]; }
+            int offset = k_len - q_len;
+            int nblk = (k_len + 127) >> 7;
+            const int nb2 = ((mb + 1) * 128 + offset + 127) >> 7;
+            if (nb2 < nblk) nblk = nb2;
+            // A part of the keys: its blocks are counted from its first one, for which the start moves
+            // up and the lengths shrink.  (The host split by its own lengths; with fewer blocks than
+            // parts, or nowhere to put parts, the last of them are empty.)
+            const int parts = max(1, min(static_cast<int>(split & 255u), p.part_o ? nblk : 1));
+            const int part = static_cast<int>(split >> 8 & 255u);
+            if (part >= parts) { mode = MODE_IDLE; continue; }
+            if (parts > 1) {
+              const int lo = nblk * part / parts;
+              nblk = nblk * (part + 1) / parts - lo;
+              k0 += p.page_table ? lo : lo * 128;
+              offset -= lo * 128;
+              k_len -= lo * 128;
+            }
+            d[T_FT] = ft; d[TF_HEAD0] = head0; d[TF_NT] = nt; d[TF_KVH] = head0 / p.q_per_kv;
+            d[TF_QROW0] = q0 + mb * 128; d[TF_VALID] = min(128, q_len - mb * 128);
+            d[TF_KSTART] = k0; d[TF_KLEN] = k_len; d[TF_OFFSET] = offset; d[TF_NBLK] = nblk;
+            d[TF_MB] = mb;
+            d[TF_PARTS] = parts; d[TF_PART] = part; d[TF_SLOT] = static_cast<int>(split >> 16);
+            d[TF_FIN0] = 1; d[TF_FIN1] = nt - 1;
+            occ_a[k] = ft;
 #ifdef MA_AUDIT
-          occ_h[k] = head0;
+            occ_h[k] = head0;
 #endif
-        } else if (mode == MODE_OPROJ || mode == MODE_AR) {
+          }
+        } while (mode == MODE_IDLE);
+        if (mode == MODE_OPROJ || mode == MODE_AR) {
           const bool own = mode == MODE_OPROJ && nrt > 0;     // a shape of this rank's choice
           const int ft = own ? arg / per_group * nrt : arg / p.nsg;
           const int width = own ? nnt : p.sg;
@@ -1084,11 +1198,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           for (int i = 0; i < nt; ++i) {
             if (!wait_bar(env, smem_u32(&bars.o_staged[i]), (st_par >> i) & 1u, 0x88 + i)) break;
             st_par ^= 1u << i;
-            const uint32_t stg = smem0 + kSmQ + i * kTile;
-            tma_store_2d(&tmO, stg, (head0 + i) * 128, ft * 128);
-            tma_store_2d(&tmO, stg + kPanel, (head0 + i) * 128 + 64, ft * 128);
-            tma_store_commit();
-            tma_store_wait_read();
+            if (d[TF_FIN0 + i]) {       // (else a part of the keys, and not the last)
+              const uint32_t stg = smem0 + kSmQ + i * kTile;
+              tma_store_2d(&tmO, stg, (head0 + i) * 128, ft * 128);
+              tma_store_2d(&tmO, stg + kPanel, (head0 + i) * 128 + 64, ft * 128);
+              tma_store_commit();
+              tma_store_wait_read();
+            }
             mbar_arrive(smem_u32(&bars.q_empty[i]));     // the producer may refill this Q buffer
           }
           tma_store_wait_all();
@@ -1238,23 +1354,27 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         wait_bar(env, smem_u32(&bars.o_done[wg]), o_par, 0x80 + wg);
         o_par ^= 1u;
         tc_fence_after();
-        const float inv = (row < valid_m && l_run > 0.f) ? (1.f / l_run) : 0.f;
-        // O / l -> bf16 -> this tile's Q buffer (free: every Q K^T of the task is done),
-        // then two TMA stores of 128 rows x 64 columns into O_scratch[ft, :, head, :].
         const uint32_t stg = smem0 + kSmQ + wg * kTile;
+        if (d[TF_PARTS] > 1) {
+          finish_part(p, s_desc[slot_k], wg, row, t_o, stg, smem_u32(&bars.o_free[wg]), m_ref, l_run);
+        } else {
+          const float inv = (row < valid_m && l_run > 0.f) ? (1.f / l_run) : 0.f;
+          // O / l -> bf16 -> this tile's Q buffer (free: every Q K^T of the task is done),
+          // then two TMA stores of 128 rows x 64 columns into O_scratch[ft, :, head, :].
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          uint32_t o[2][32];
-          tmem_ld32(t_o + hh * 64, o[0]);
-          tmem_ld32(t_o + hh * 64 + 32, o[1]);
-          tc_wait_ld();
-          if (hh == 1) {            // all of O is in registers: the next task may overwrite it
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bars.o_free[wg]));
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t o[2][32];
+            tmem_ld32(t_o + hh * 64, o[0]);
+            tmem_ld32(t_o + hh * 64 + 32, o[1]);
+            tc_wait_ld();
+            if (hh == 1) {            // all of O is in registers: the next task may overwrite it
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&bars.o_free[wg]));
+            }
+            stage_row(stg + hh * kPanel, row, 0, o[0], inv);
+            stage_row(stg + hh * kPanel, row, 32, o[1], inv);
           }
-          stage_row32(stg + hh * kPanel, row, 0, o[0], inv);
-          stage_row32(stg + hh * kPanel, row, 32, o[1], inv);
         }
         fence_proxy_async_smem();
         __syncwarp();

@@ -52,6 +52,9 @@ struct KParams {
   const int* fa_order;            // row tiles in claim order (longest first), or null
   const int* tasks;               // attention tasks in claim order: {count, 0, 0, 0}, then kTaskWords each
                                   // (see kTaskWords), or null: from the arrays above
+  float* part_o;                  // parts of a head's attention: [slot][H][kPartFloats], or null: no
+                                  // row tile's keys are split
+  uint32_t* part_count;           // [slot][H], at a row tile's first slot: parts of the head that are there
   const int* page_table;          // paged KV: [batch][pps] page of each 128-key block, or null
   const int* cache_seqlens;       // paged KV: KV length per sequence
   int pps;                        // page-table row pitch
@@ -70,8 +73,12 @@ constexpr int kOpTwoFrom = 9, kOpCols2From = 5;             // behind attention
 constexpr int kOpTwoFromAlone = 2, kOpCols2FromAlone = 1;   // O_proj-only launches
 
 // A position of the task table: {row tile, sequence, block in the sequence, cu_q of the sequence,
-// q_len, cu_k of the sequence, k_len, 0}; written by ma_stage_tasks.
+// q_len, cu_k of the sequence, k_len, split}; written by ma_stage_tasks.  split: parts the keys are
+// split into | which of them << 8 | the row tile's first slot of part_o << 16.
 constexpr int kTaskWords = 8;
+constexpr int kPartMax = 128 * 128, kPartSum = kPartMax + 128;   // a part's O, then its rows'
+constexpr int kPartFloats = kPartSum + 128;                      // reference maxima and sums
+constexpr int kMaxParts = 16;
 
 constexpr int kThreads = 384;
 constexpr int kSmemDynamic = 65536 + 5 * 32768 + 1024;   // Q x2, K/V ring x5, align slack

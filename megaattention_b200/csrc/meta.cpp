@@ -6,11 +6,115 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
 #include <new>
 #include <vector>
 
 #include "../../include/megaattn_b200.h"
 #include "kparams.h"
+
+namespace {
+
+// Key blocks that row tile t's attention visits, of the host's lengths (< 0: bad lengths).
+int64_t key_blocks(const ma_stage_meta_args& a, int t) {
+  const int b = a.batch_idx[t];
+  const int64_t lq = static_cast<int64_t>(a.cu_q[b + 1]) - a.cu_q[b];
+  const int64_t lk = static_cast<int32_t>(static_cast<uint32_t>(a.cu_k[b + 1]) -
+                                          static_cast<uint32_t>(a.cu_k[b]));
+  const int64_t last = (static_cast<int64_t>(a.m_block[t]) + 1) * 128 + (lk - lq);
+  return std::min((lk + 127) / 128, (last + 127) / 128);
+}
+
+// The claim order asked for (ma_stage_meta), by default interleaved below a work ratio of 2.0,
+// fa_prime_tiles_b200's switch point.
+int claim_prime(const ma_stage_meta_args& a, int64_t blocks) {
+  if (!a.auto_prime) return a.prime;
+  const int64_t tiles = static_cast<int64_t>(a.num_row_tiles) * ((a.hidden + 127) / 128);
+  return static_cast<double>(2 * blocks) / static_cast<double>(tiles) < 2.0 ? -1 : 0;
+}
+
+// Claim order of things sorted longest first.
+void arrange(const int32_t* sorted, int n, int prime, int32_t* order) {
+  if (prime < 0) {              // longest, shortest, second longest, second shortest, ...
+    const int half = (n + 1) / 2;
+    for (int i = 0; i < half; ++i) order[2 * i] = sorted[i];
+    for (int i = half; i < n; ++i) order[2 * (n - 1 - i) + 1] = sorted[i];
+  } else {                      // the `prime` shortest to the front
+    const int p = std::min(prime, n);
+    for (int i = 0; i < p; ++i) order[i] = sorted[n - 1 - i];
+    for (int i = p; i < n; ++i) order[i] = sorted[i - p];
+  }
+}
+
+// Splitting of row tiles' keys.  A task's key blocks are a serial chain, 2 us each, and with few or
+// uneven tasks the longest one is the launch while other CTAs have nothing to do.  Lengths here are
+// in key blocks: a task costs two more than it has (its first loads, the epilogue), a part another
+// one for putting its sums down, reading a head's parts back half a one per part, and the O_proj of
+// a row tile's 128 columns a fifth of one per head.  Launches in us as 1 / 2 / 3 / 4 / 6 / 8 parts of the
+// longest: 64 tokens behind 4000 keys, 8 heads 103 / 85 / 79 / 75 / 75 / 77; one token behind 15000, 4
+// heads 243 / 152 / 122 / 106 / 93 / 89; 100 and 300 behind 1500 and 2500 81 / 77 / 75 / 69 / 73 / 75;
+// 2000 behind 15871 270 / 179 / 212 / 185; 12 short turns on up to 5217 keys 122 / 95 / 89 / 89 / 97 / 101.
+constexpr int kMinPart = 5;
+constexpr double kTaskCost = 2.0, kPartCost = 1.0, kJoinCost = 0.5, kOprojCost = 0.2, kWorthIt = 0.9;
+
+struct Unit { int32_t tile, split, len; };    // split: as in the task table
+
+// What the launch's attention takes, claimed longest first by `lanes` groups of CTAs (one CTA of
+// a group per task of a row tile).
+double makespan(std::vector<double>& costs, int lanes, std::vector<double>& busy) {
+  std::sort(costs.begin(), costs.end(), std::greater<double>());
+  busy.assign(static_cast<size_t>(lanes), 0.0);     // a heap, the first free lane at its top
+  double most = 0.0;
+  for (double c : costs) {
+    std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+    busy.back() += c;
+    most = std::max(most, busy.back());
+    std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+  }
+  return most;
+}
+
+// Parts of every row tile, from splits of the longest into 2, 3, ... parts and of the others into
+// parts of that length; false: none is worth it.  A launch ends with its attention, or once all of
+// its work is done, O_proj's too (CTAs without attention have that to do: 4500 tokens of one prompt,
+// 4096 columns, attention alone would be shorter in two parts, the launch is 118 us and 119).
+bool choose_parts(const std::vector<int32_t>& nblk, int H, int num_out, int ctas, int slots,
+                  std::vector<int32_t>& parts) {
+  const int R = static_cast<int>(nblk.size()), per_tile = (H + 1) / 2;
+  const int lanes = std::max(1, ctas / per_tile);
+  const int32_t most = *std::max_element(nblk.begin(), nblk.end());
+  // (three tasks per CTA fill each other's gaps)
+  if (slots < 2 || most < 2 * kMinPart || static_cast<int64_t>(R) * per_tile > 3 * ctas) return false;
+  const double oproj = kOprojCost * R * num_out * H / ctas;
+  std::vector<double> costs(R), busy;
+  double sum = 0.0;
+  for (int t = 0; t < R; ++t) sum += costs[t] = nblk[t] + kTaskCost;
+  if (most + kTaskCost <= sum / lanes + oproj) return false;
+  double best = kWorthIt * std::max(makespan(costs, lanes, busy), sum / lanes + oproj);
+  int32_t best_len = 0;
+  for (int k = 2; k <= ma::kMaxParts && most >= k * kMinPart; ++k) {
+    const int32_t len = (most + k - 1) / k;
+    costs.clear();
+    int used = 0;
+    sum = 0.0;
+    for (int32_t n : nblk) {
+      const int m = (n + len - 1) / len;
+      if (m > 1) used += m;
+      for (int i = 0; i < m; ++i) {
+        costs.push_back(n * (i + 1) / m - n * i / m + kTaskCost + (m > 1 ? kPartCost : 0.0));
+        sum += costs.back();
+      }
+    }
+    if (used > slots) break;
+    const double t = std::max(makespan(costs, lanes, busy), sum / lanes + oproj) + k * kJoinCost;
+    if (t < best) { best = t; best_len = len; }
+  }
+  if (best_len == 0) return false;
+  for (int t = 0; t < R; ++t) parts[t] = std::max(1, (nblk[t] + best_len - 1) / best_len);
+  return true;
+}
+
+}  // namespace
 
 extern "C" int ma_row_desc(const int64_t* cu_q, const int64_t* cu_k, int32_t num_batch,
                            int32_t max_row_tiles, int32_t* cu_q_out, int32_t* cu_k_out,
@@ -56,35 +160,18 @@ extern "C" int ma_stage_meta(const ma_stage_meta_args* a) {
     for (int t = 0; t < R; ++t) {
       const int b = a->batch_idx[t];
       if (b < 0 || b >= B) return MA_ERR_INVALID;
-      const int64_t lq = static_cast<int64_t>(a->cu_q[b + 1]) - a->cu_q[b];
-      const int64_t lk = static_cast<int32_t>(static_cast<uint32_t>(a->cu_k[b + 1]) -
-                                              static_cast<uint32_t>(a->cu_k[b]));
-      const int64_t last = (static_cast<int64_t>(a->m_block[t]) + 1) * 128 + (lk - lq);
-      const int64_t n = std::min((lk + 127) / 128, (last + 127) / 128);
+      const int64_t n = key_blocks(*a, t);
       if (n < 0) return MA_ERR_INVALID;
       nblk[t] = static_cast<int32_t>(n);
       sum += n;
       most = std::max(most, nblk[t]);
-    }
-    int prime = a->prime;
-    if (a->auto_prime) {          // interleaved below 2.0, fa_prime_tiles_b200's switch point
-      const int64_t tiles = static_cast<int64_t>(R) * ((a->hidden + 127) / 128);
-      prime = static_cast<double>(2 * sum) / static_cast<double>(tiles) < 2.0 ? -1 : 0;
     }
     // longest first, stable: counting sort on the number of blocks
     std::vector<int32_t> at(static_cast<size_t>(most) + 2, 0), sorted(R);
     for (int t = 0; t < R; ++t) ++at[most - nblk[t] + 1];
     for (int i = 1; i <= most + 1; ++i) at[i] += at[i - 1];
     for (int t = 0; t < R; ++t) sorted[at[most - nblk[t]]++] = t;
-    if (prime < 0) {              // longest, shortest, second longest, second shortest, ...
-      const int half = (R + 1) / 2;
-      for (int i = 0; i < half; ++i) order[2 * i] = sorted[i];
-      for (int i = half; i < R; ++i) order[2 * (R - 1 - i) + 1] = sorted[i];
-    } else {                      // the `prime` shortest to the front
-      const int p = std::min(prime, R);
-      for (int i = 0; i < p; ++i) order[i] = sorted[R - 1 - i];
-      for (int i = p; i < R; ++i) order[i] = sorted[i - p];
-    }
+    arrange(sorted.data(), R, claim_prime(*a, sum), order);
   } catch (const std::bad_alloc&) {
     return MA_ERR_CAPACITY;
   }
@@ -111,13 +198,44 @@ extern "C" int ma_stage_tasks(const ma_stage_tasks_args* a) {
   const int rc = ma_stage_meta(&m);
   if (rc != MA_OK) return rc;
   if (m.num_row_tiles > a->max_tasks) return MA_ERR_CAPACITY;
+  const int R = m.num_row_tiles;
   const int32_t* order = m.staging + m.off_order;
   int32_t* head = m.staging + a->off_tasks;
-  head[0] = m.num_row_tiles;
+  // positions of the table: {row tile, split}
+  std::vector<Unit> units;
+  try {
+    std::vector<int32_t> nblk(R), parts(R, 1);
+    for (int t = 0; t < R; ++t) nblk[t] = static_cast<int32_t>(key_blocks(m, t));
+    const int slots = std::min({a->split_slots, a->max_tasks - R, 0xffff});
+    if (m.H_local >= 1 && a->num_ctas >= 1 && choose_parts(nblk, m.H_local, (m.hidden + 127) / 128, a->num_ctas, slots, parts)) {
+      int64_t sum = 0;
+      std::vector<Unit> all;
+      int slot = 0;
+      for (int t = 0; t < R; ++t) {
+        const int32_t n = nblk[t], k = parts[t];
+        sum += n;
+        for (int i = 0; i < k; ++i)
+          all.push_back({t, k > 1 ? k | i << 8 | static_cast<int32_t>(static_cast<uint32_t>(slot) << 16) : 0,
+                         static_cast<int32_t>(static_cast<int64_t>(n) * (i + 1) / k - static_cast<int64_t>(n) * i / k)});
+        if (k > 1) slot += k;
+      }
+      std::stable_sort(all.begin(), all.end(), [](const Unit& x, const Unit& y) { return x.len > y.len; });
+      const int N = static_cast<int>(all.size());
+      std::vector<int32_t> sorted(N), at(N);
+      for (int i = 0; i < N; ++i) sorted[i] = i;
+      arrange(sorted.data(), N, claim_prime(m, sum), at.data());
+      for (int i = 0; i < N; ++i) units.push_back(all[at[i]]);
+    } else {
+      for (int i = 0; i < R; ++i) units.push_back({order[i], 0, 0});
+    }
+  } catch (const std::bad_alloc&) {
+    return MA_ERR_CAPACITY;
+  }
+  head[0] = static_cast<int32_t>(units.size());
   head[1] = head[2] = head[3] = 0;
-  for (int i = 0; i < m.num_row_tiles; ++i) {
+  for (int i = 0; i < head[0]; ++i) {
     int32_t* r = head + 4 + i * ma::kTaskWords;
-    const int t = order[i], b = m.batch_idx[t];
+    const int t = units[i].tile, b = m.batch_idx[t];
     r[0] = t;
     r[1] = b;
     r[2] = m.m_block[t];
@@ -125,7 +243,7 @@ extern "C" int ma_stage_tasks(const ma_stage_tasks_args* a) {
     r[4] = m.cu_q[b + 1] - m.cu_q[b];
     r[5] = m.cu_k[b];
     r[6] = static_cast<int32_t>(static_cast<uint32_t>(m.cu_k[b + 1]) - static_cast<uint32_t>(m.cu_k[b]));
-    r[7] = 0;
+    r[7] = units[i].split;
   }
   return MA_OK;
 }

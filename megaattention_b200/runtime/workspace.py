@@ -32,6 +32,8 @@ from ..metadata.row_desc import RowDescMeta, oproj_task_counts
 NUM_CTRL = 8
 NUM_SYNC = 3
 NUM_STATUS = 8
+SPLIT_HEADS = 640        # (two waves of tasks of two heads, and a little)
+MAX_PARTS = 16           # of one row tile, as in csrc/kparams.h
 
 
 def claim_order(meta, prime: int = 0) -> np.ndarray:
@@ -97,6 +99,7 @@ class FusedFaOprojArWorkspace:
         self.__dict__.update(kw)
         self._plan = None
         self._lib = _cabi.lib
+        self._split_ctas = 0           # (set by compile: before it nothing is split)
         self._args = None
         self._meta = None
         # Launch flags applied by launch() (OR of _cabi.MA_FLAG_*) and attention claim order
@@ -177,8 +180,13 @@ class FusedFaOprojArWorkspace:
         # offsets, each 16-byte aligned
         def up4(n):
             return (n + 3) // 4 * 4
+        # Slots for parts of row tiles' keys: up to SPLIT_HEADS heads' parts (fp32, 65 KB each),
+        # and no more than a row tile can have
+        slots = min(SPLIT_HEADS // H_local, MAX_PARTS * max_num_row_tiles)
+        slots = slots if slots >= 2 else 0
+        max_tasks = max_num_row_tiles + slots
         sizes = (max_num_batch + 1, max_num_batch + 1, max_num_row_tiles, max_num_row_tiles,
-                 max_num_row_tiles, 8, 4 + _cabi.TASK_WORDS * max_num_row_tiles)
+                 max_num_row_tiles, 8, 4 + _cabi.TASK_WORDS * max_tasks)
         offs = [0]
         for n in sizes:
             offs.append(offs[-1] + up4(n))
@@ -198,7 +206,9 @@ class FusedFaOprojArWorkspace:
             head_ready=zeros(max_num_row_tiles, torch.uint32),
             oproj_queue=zeros(max_total, torch.uint32),
             ar_done_bits=zeros(max_owner_words, torch.int64),
-            tasks=mviews[6],
+            tasks=mviews[6], max_tasks=max_tasks, split_slots=slots,
+            parts=torch.empty(slots * H_local * _cabi.PART_FLOATS, dtype=torch.float32, device=dev),
+            part_count=zeros(max(slots, 1) * H_local, torch.int32),
             cu_q=mviews[0], cu_k=mviews[1], fa_b=mviews[2], fa_mb=mviews[3], fa_order=mviews[4],
             Q=zeros((tot_cap, H_local, D), dtype),
             K=(None if paged else zeros((max_tot_k, H_kv, D), dtype)),
@@ -280,6 +290,11 @@ class FusedFaOprojArWorkspace:
         _cabi.check(self._lib.ma_plan_create(C.byref(d), C.byref(plan)), "ma_plan_create")
         self._plan = plan
         _cabi.check(self._lib.ma_plan_set_tasks(plan, self.tasks.data_ptr()), "ma_plan_set_tasks")
+        if self.split_slots:
+            _cabi.check(self._lib.ma_plan_set_split(plan, self.parts.data_ptr(), self.part_count.data_ptr()),
+                        "ma_plan_set_split")
+        self._split_ctas = int(num_ctas) if num_ctas else torch.cuda.get_device_properties(
+            self.dev).multi_processor_count
         self._args = _cabi.LaunchArgs(int(w_fa), int(w_oproj), int(w_ar),
                                       int(num_ctas) if num_ctas else 0, 0)
         self._ts = torch.cuda.current_stream(self.dev)
@@ -413,7 +428,8 @@ class FusedFaOprojArWorkspace:
             self._meta_at, cu_q.size - 1, R, self.hidden, self.H_local, self.num_super_groups,
             self.tp_size, self.rank, int(prime is None),
             0 if prime is None else max(-1, min(int(prime), R)),
-            o[0], o[1], o[2], o[3], o[4], o[5], 0), o[6], self.max_num_row_tiles)
+            o[0], o[1], o[2], o[3], o[4], o[5], 0), o[6], self.max_tasks, self.split_slots,
+            self._split_ctas)
         rc = _cabi.lib.ma_upload_meta(C.byref(args), self.meta_dev.data_ptr(),
                                       torch.cuda.current_stream(self.dev).cuda_stream)
         _cabi.check(min(rc, 0), "ma_upload_meta")
@@ -500,7 +516,7 @@ class FusedFaOprojArWorkspace:
         """Fault localisation only; never on the production / bench / test default path.
         With tp > 1 every rank must call it, followed by a host barrier."""
         for t in (self.ctrl, self.sync_ctrl, self.actv, self.head_ready, self.oproj_queue,
-                  self.fa_order, self.tasks, self.rco, self.rbits, self.ar_done_bits, self.nvl, self.csym, self.Oscr,
+                  self.fa_order, self.tasks, self.part_count, self.rco, self.rbits, self.ar_done_bits, self.nvl, self.csym, self.Oscr,
                   self.status):
             t.zero_()
 
