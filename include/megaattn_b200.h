@@ -75,7 +75,7 @@ typedef struct ma_devinfo {
  *   ar_done_bits u64[max_owner_words]
  *   nvl_signal i32[2] (symmetric)  cu_q, cu_k i32[max_batch+1]  fa_b, fa_mb, fa_order i32[max_row_tiles]
  *   status u32[8]
- * All control buffers must be zero when the plan is first launched.
+ * All control buffers, oproj_queue among them, must be zero when the plan is first launched.
  */
 typedef struct ma_plan_desc {
   int32_t device;

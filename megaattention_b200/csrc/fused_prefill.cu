@@ -117,6 +117,9 @@ __device__ __forceinline__ bool wait_bar(const Env& e, uint32_t bar, uint32_t pa
 }
 
 // ---------------------------------------------------------------- scheduler (thread 0)
+// One rank, or partial sums only: what a task leaves is read by nobody in this launch.
+__device__ __forceinline__ bool without_ar(const KParams& p) { return p.tp == 1 || (p.flags & 16u); }
+
 // Attention task ids come from the counter, the first of every CTA too: a task belongs to a CTA
 // only once that CTA runs.  (Ids by CTA number save that atomic, but then a CTA that gets its
 // SM late - another stream's kernel holds it - keeps its task from all the others, which wait
@@ -134,8 +137,12 @@ __device__ __forceinline__ int fa_tasks_per_tile(const KParams& p) {
 // the race to a not-yet-published entry stays pending in this CTA (at most one) and is
 // served as soon as the publish index passes it; meanwhile the CTA keeps taking other work.
 // The queue holds row-tile groups in the order they became ready; each stands for its
-// `per_group` tasks, so ticket t is task t % per_group of entry t / per_group.
-// `head` and `tail` (acquired) are the consume and publish counts as the caller read them.
+// `per_group` tasks, so ticket t is task t % per_group of entry t / per_group.  An entry is the
+// group's number plus one, written with release behind its reservation and zero before: who holds a
+// ticket waits for the entry itself.  (With a publish count that the publishers advanced in their
+// turn, a row tile's last head and its first O_proj task were two trips to L2 and two fences
+// further apart, 2 us.)
+// `head` and `tail` are the consume and reserve counts as the caller read them.
 __device__ __forceinline__ bool try_pop_oproj(const KParams& p, int total_op, int per_group,
                                               uint32_t head, uint32_t tail, int* pending, int* arg) {
   if (*pending < 0) {
@@ -143,13 +150,10 @@ __device__ __forceinline__ bool try_pop_oproj(const KParams& p, int total_op, in
     const uint32_t t = atom_add_relaxed_gpu(p.ctrl + C_OP_CONSUME, 1u);
     if (static_cast<int>(t) >= total_op) return false;    // past the end: nothing there
     *pending = static_cast<int>(t);
-    if (t >= tail && static_cast<uint32_t>(*pending) >= ld_acquire_gpu(p.ctrl + C_OP_PUBLISH))
-      return false;
-  } else if (static_cast<uint32_t>(*pending) >= tail) {
-    return false;
   }
-  *arg = static_cast<int>(ld_relaxed_gpu(p.oproj_queue + *pending / per_group)) * per_group +
-         *pending % per_group;
+  const uint32_t entry = ld_acquire_gpu(p.oproj_queue + *pending / per_group);
+  if (entry == 0u) return false;
+  *arg = static_cast<int>(entry - 1u) * per_group + *pending % per_group;
   *pending = -1;
   return true;
 }
@@ -241,7 +245,7 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   const uint32_t fa_next = ld_relaxed_gpu(p.ctrl + C_FA_COUNTER), fa_d = ld_relaxed_gpu(p.ctrl + C_FA_DONE);
   const uint32_t op_next = ld_relaxed_gpu(p.ctrl + C_OP_CONSUME), op_d = ld_relaxed_gpu(p.ctrl + C_OP_DONE);
   const uint32_t ar_next = ld_relaxed_gpu(p.ctrl + C_AR_CURSOR), ar_d = ld_relaxed_gpu(p.ctrl + C_AR_DONE);
-  const uint32_t tail = ld_acquire_gpu(p.ctrl + C_OP_PUBLISH);
+  const uint32_t tail = ld_relaxed_gpu(p.ctrl + C_OP_RESERVE);
   if (status != 0u) {       // some CTA (or rank) gave up: leave
     *e.abort_flag = 1;
     *mode = MODE_DONE;
@@ -260,7 +264,7 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   if (p.flags & 32u) {
     // O_proj-only launch (single rank): O_scratch is taken as complete, slots are handed
     // out in order by the consume counter
-    if (static_cast<int>(op_d) >= total_op) { *mode = MODE_DONE; return; }
+    *mode = MODE_DONE;
     if (static_cast<int>(op_next) < total_op) {
       const int t = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_OP_CONSUME, 1u));
       if (t < total_op) { *mode = MODE_OPROJ; *arg = t; }
@@ -268,11 +272,16 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
     return;
   }
   const bool fa_only = (p.flags & 1u) != 0;
-  // (each count is final once it is at its target; what they stand for is read by nobody before
-  // the exit protocol's fence)
-  const bool done = static_cast<int>(fa_d) >= num_fa &&
-                    (fa_only || (static_cast<int>(op_d) >= total_op &&
-                                 (p.tp == 1 || (p.flags & 16u) || static_cast<int>(ar_d) >= local_owned)));
+  // With an AllReduce to come everybody stays until all of it is done: slots become ready by other
+  // ranks' work.  (Each count is final once it is at its target; what they stand for is read by
+  // nobody before the exit protocol's fence.)  Without one a CTA leaves once every task is handed
+  // out and it holds no ticket: what is left is running, and the last CTA out ends the launch.  (To
+  // wait for the counts instead was a poll or two, 2 us, at the end of every launch.)
+  const bool done = without_ar(p)
+                        ? static_cast<int>(fa_next) >= n_fa_tasks && *pending < 0 &&
+                              (fa_only || static_cast<int>(op_next) >= total_op)
+                        : static_cast<int>(fa_d) >= num_fa &&
+                              (fa_only || (static_cast<int>(op_d) >= total_op && static_cast<int>(ar_d) >= local_owned));
   if (done) { *mode = MODE_DONE; return; }
   // probe order by role: 0: FA,OPROJ,AR  1: OPROJ,AR,FA  2: AR,FA,OPROJ (the reference's
   // three orders).  With the "drain first" launch flag downstream work goes first so that
@@ -295,9 +304,7 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
       if (!ok) *fa_left = false;
     } else if (fa_only) ok = false;
     else if (m == MODE_OPROJ) ok = try_pop_oproj(p, total_op, per_group, op_next, tail, pending, arg);
-    else if (p.tp > 1 && !(p.flags & 16u) &&
-             !(busy && static_cast<int>(op_next) >= total_op))
-    {
+    else if (!without_ar(p) && !(busy && static_cast<int>(op_next) >= total_op)) {
       // (once every O_proj task has been handed out only reductions are left and CTAs go
       // idle: a CTA that still has a task running leaves ready slots to them instead of
       // queueing one behind its own)
@@ -308,25 +315,11 @@ __device__ __noinline__ void schedule_pick(const Env& e, int role, int num_fa, i
   }
 }
 
-// Reserve, fill and publish (in reservation order) the O_proj tasks of one row-tile group.
-__device__ __noinline__ void publish_oproj(const Env& e, int group, int per_group) {
-  const KParams& p = *e.p;
+// Publish the O_proj tasks of one row-tile group (the caller has acquired what made it ready).
+__device__ __forceinline__ void publish_oproj(const KParams& p, int group, int per_group) {
   const uint32_t n = static_cast<uint32_t>(per_group);
   const uint32_t start = atom_add_relaxed_gpu(p.ctrl + C_OP_RESERVE, n);
-  p.oproj_queue[start / n] = static_cast<uint32_t>(group);
-  fence_acq_rel_gpu();
-  const uint64_t t0 = globaltimer_ns();
-  uint32_t it = 0;
-  while (ld_acquire_gpu(p.ctrl + C_OP_PUBLISH) != start) {
-    if ((++it & 63u) == 0) {
-      if (ld_relaxed_gpu(p.status) != 0u) { *e.abort_flag = 1; return; }
-      if (globaltimer_ns() - t0 > p.wait_limit_ns) {
-        report(e, ST_TIMEOUT_PUBLISH, start, group);
-        return;
-      }
-    }
-  }
-  atom_add_release_gpu(p.ctrl + C_OP_PUBLISH, n);
+  st_release_gpu(p.oproj_queue + start / n, static_cast<uint32_t>(group) + 1u);
 }
 
 __device__ __forceinline__ void finish_ar_slot(const KParams& p, int slot) {
@@ -339,15 +332,16 @@ __device__ __forceinline__ void finish_ar_slot(const KParams& p, int slot) {
 
 // After an O_proj task: tell the slot's owner rank that this rank's partial is in place.
 __device__ __noinline__ void publish_ar_ready(const KParams& p, int slot) {
-  if ((p.flags & 16u) || p.tp == 1) {
-    // one rank (the partial is the result), or partial sums only (measurement aid): no
-    // AllReduce to account, no cross-rank traffic
-  } else {
-    const int owner_rank = slot % p.tp;
-    const int owner_idx = slot / p.tp;
-    red_add_release_sys(reinterpret_cast<uint32_t*>(p.peer_rc[owner_rank]) + (owner_idx >> 2),
-                        1u << ((owner_idx & 3) * 8));      // one byte per slot
+  if (without_ar(p)) {
+    // the partial is the result, or partial sums only (measurement aid): no AllReduce to
+    // account, no cross-rank traffic
+    red_add_relaxed_gpu(p.ctrl + C_OP_DONE, 1u);
+    return;
   }
+  const int owner_rank = slot % p.tp;
+  const int owner_idx = slot / p.tp;
+  red_add_release_sys(reinterpret_cast<uint32_t*>(p.peer_rc[owner_rank]) + (owner_idx >> 2),
+                      1u << ((owner_idx & 3) * 8));      // one byte per slot
   atom_add_release_gpu(p.ctrl + C_OP_DONE, 1u);
 }
 
@@ -540,7 +534,7 @@ enum : int { T_MODE = 0, T_FT = 1,
              TF_PARTS = 12,     // parts its keys are split into (1: none); TF_PART: which of them
              TF_PART = 13, TF_SLOT = 14,
              TF_FIN0 = 15, TF_FIN1 = 16,   // head 0 / 1 of the task is finished when the task is
-             TO_BASE = 2, TO_VNT = 3, TO_VALID = 4, TO_SLOT = 5, TO_NRT = 6, TO_VALID1 = 7, TO_TWO = 8,
+             TO_BASE = 2, TO_VNT = 3, TO_SLOT = 5, TO_NRT = 6, TO_TWO = 8,
              T_WORDS = 17 };
 
 // End of a head's attention over a part of its keys.  The part's O (not divided), reference maximum
@@ -688,6 +682,18 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     tma_prefetch_desc(&tmO); tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmC);
     tma_prefetch_desc(&tmW2);
   }
+  // The scheduler's first trip to L2 runs under the set-up: whether an earlier launch gave up, the
+  // counts, and its first attention task, which is there for the taking (nothing else can be ready).
+  const bool has_fa = !(p.flags & (8u | 32u));
+  const int* tasks = (p.flags & 4u) ? nullptr : p.tasks;
+  uint32_t status0 = 0, first_fa = 0;
+  int num_fa = 0, total_op = 0, n_tiles = 0, local_owned = 0, n_pos = 0;
+  if (tid == 64) {
+    status0 = ld_relaxed_gpu(p.status);
+    num_fa = p.actv[0]; total_op = p.actv[1]; n_tiles = p.actv[2]; local_owned = p.actv[5];
+    if (tasks) n_pos = tasks[0];
+    if (has_fa) first_fa = atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u);
+  }
   if (warp == 1) {
     tmem_alloc(smem_u32(&s_tmem), 512);
     tmem_relinquish();
@@ -733,21 +739,14 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     reg_dec<88>();
     if (warp == 2 && lane == 0) {
       // ==================================================================== scheduler
-      // (a launch after one that gave up does nothing until the state has been cleared)
-      const uint32_t status0 = ld_relaxed_gpu(p.status);
-      const int num_fa = p.actv[0];
-      const int local_owned = p.actv[5];
       // O_proj tasks.  With several ranks a task is an AllReduce slot: one row tile, up to
       // `sg` column tiles in two passes (TO_NRT = 0).  One rank is free to choose: nrt row
       // tiles x nnt column tiles (<= 2 x 2) in one pass, the row tiles sharing every W stage.
-      int nrt = 0, nnt = p.sg, per_group = p.nsg, total_op = p.actv[1];
-      const int n_tiles = p.actv[2];
+      int nrt = 0, nnt = p.sg, per_group = p.nsg;
       // the table of attention tasks, in claim order (none: the claim order's arrays)
-      const int* tasks = (p.flags & 4u) ? nullptr : p.tasks;
-      int n_pos = tasks ? tasks[0] : 0;
       if (n_pos == 0) { tasks = nullptr; n_pos = num_fa / p.H; }
       const int n_fa_tasks = n_pos * fa_tasks_per_tile(p);
-      bool fa_left = !(p.flags & (8u | 32u));
+      bool fa_left = has_fa;
       if (p.tp == 1 && !(p.flags & 16u)) {      // (without AllReduce: slots, as with several)
         op_task_shape(p, n_tiles, static_cast<int>(gridDim.x), &nrt, &nnt);
         per_group = (p.num_out + nnt - 1) / nnt;
@@ -799,13 +798,17 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           // heads that are finished (one of which another part is still running counts with that)
           const int heads = s_desc[kk][TF_FIN0] + s_desc[kk][TF_FIN1];
           if (heads == 0) return;
-          fence_acq_rel_gpu();
-          const int g = occ_a[kk] / grp;
-          const uint32_t old = atom_add_acqrel_gpu(p.head_ready + g, static_cast<uint32_t>(heads));
-          if (!(p.flags & 1u) &&
-              static_cast<int>(old) + heads == p.H * min(grp, n_tiles - g * grp))
-            publish_oproj(env, g, per_group);
-          atom_add_release_gpu(p.ctrl + C_FA_DONE, static_cast<uint32_t>(heads));
+          if (!(p.flags & 1u)) {
+            fence_acq_rel_gpu();
+            const int g = occ_a[kk] / grp;
+            const uint32_t old = atom_add_relaxed_gpu(p.head_ready + g, static_cast<uint32_t>(heads));
+            if (static_cast<int>(old) + heads == p.H * min(grp, n_tiles - g * grp)) {
+              fence_acq_rel_gpu();
+              publish_oproj(p, g, per_group);
+            }
+          }
+          if (without_ar(p)) red_add_relaxed_gpu(p.ctrl + C_FA_DONE, static_cast<uint32_t>(heads));
+          else atom_add_release_gpu(p.ctrl + C_FA_DONE, static_cast<uint32_t>(heads));
         } else if (occ_mode[kk] == MODE_OPROJ) {
           publish_ar_ready(p, occ_a[kk]);
         } else if (occ_mode[kk] == MODE_AR) {
@@ -838,11 +841,11 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           arg = -1;
           if (fa_left && (first || role == 0)) {
             // An attention task where that is what the CTA asks for first: one atomic, and whether
-            // somebody gave up comes with it.  (The first task of every CTA: nothing else can be
-            // ready yet.)
+            // somebody gave up comes with it.  (The first was taken under the set-up.  A launch after
+            // one that gave up does nothing until the state has been cleared.)
             const uint32_t status = first ? status0 : ld_relaxed_gpu(p.status);
             if (status == 0u) {
-              arg = static_cast<int>(atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
+              arg = static_cast<int>(first ? first_fa : atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u));
               if (arg < n_fa_tasks) mode = MODE_FA; else fa_left = false;
             }
             first = false;
@@ -928,17 +931,20 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           const int base_out = (own ? arg % per_group : arg % p.nsg) * width;
           const int rows = own ? min(nrt, n_tiles - ft) : 1;
           d[T_FT] = ft; d[TO_BASE] = base_out; d[TO_VNT] = min(width, p.num_out - base_out);
-          for (int r = 0; r < rows; ++r) {
-            const int b = p.fa_b[ft + r], mb = p.fa_mb[ft + r];
-            d[r ? TO_VALID1 : TO_VALID] = min(128, p.cu_q[b + 1] - p.cu_q[b] - mb * 128);
-          }
           d[TO_NRT] = own ? rows : 0; d[TO_SLOT] = arg; d[TO_TWO] = nrt == 2;
           occ_a[k] = arg;
         }
         d[T_MODE] = mode;
         occ_mode[k] = mode;
         mbar_arrive(smem_u32(&bars.task_full[k]));
-        if (mode == MODE_DONE) break;
+        if (mode == MODE_DONE) {
+          // (without an AllReduce a CTA is done when nothing is left to claim, with a task running)
+          if (occupied[k ^ 1]) {
+            wait_bar(env, smem_u32(&bars.task_empty[k ^ 1]), te_par[k ^ 1], 0x122 + k);
+            publish(k ^ 1);
+          }
+          break;
+        }
         occupied[k] = true;
         // claim-ahead is only held back behind long attention tasks; short tasks (O_proj,
         // AllReduce, a few key blocks) want their successor posted before they end
@@ -1208,8 +1214,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
             mbar_arrive(smem_u32(&bars.q_empty[i]));     // the producer may refill this Q buffer
           }
           tma_store_wait_all();
-          fence_proxy_async_all();     // O_scratch is read back by TMA loads of other CTAs
-          __threadfence();
+          fence_proxy_async_all();     // O_scratch is read back by TMA loads of other CTAs (the
+                                       // scheduler's fence covers them)
         }
         MA_TASK_DONE(mode)
       }
@@ -1384,6 +1390,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         const bool leader = ((warp & 3) == 0 && lane == 0);
         const uint32_t stg = smem0 + kSmOpStaging + wg * kPanel;   // [128 rows][64 cols] bf16
         bool direct = false;
+        // rows of the task's row tiles, looked up while the product runs (by the scheduler they were
+        // two trips to L2 of every claim)
+        auto rows_of = [&](int ft) {
+          const int b = p.fa_b[ft];
+          return min(128, p.cu_q[b + 1] - p.cu_q[b] - p.fa_mb[ft] * 128);
+        };
+        const int rows0 = rows_of(ft0), rows1 = nrt == 2 ? rows_of(ft0 + 1) : 0;
         // Accumulator h holds row tile h of the task, or columns 2h and 2h + 1 of a slot; this
         // warpgroup's 128 columns of it go out as two panels of 64, by way of bf16 words in
         // registers.
@@ -1412,7 +1425,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         auto emit_panel = [&](int h, int hh, const uint32_t (&pk)[32]) {
           const int ft = nrt ? ft0 + h : ft0;
           const int out_n = base_out + (nrt ? 0 : 2 * h) + wg;
-          const int valid_m = d[(nrt && h) ? TO_VALID1 : TO_VALID];
+          const int valid_m = (nrt && h) ? rows1 : rows0;
           if (valid_m == 128) {
             // full row tile: stage 64 columns, one TMA store (clipped at `hidden`)
             if (leader) tma_store_wait_read();
@@ -1467,11 +1480,17 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         // written directly get a gpu-scope fence; the one system-scope fence per task is
         // the scheduler's, after it has seen every warp arrive.  (A system fence by each of
         // the 256 threads costs tens of microseconds per task while NVLink is busy.)
-        if (leader) {
-          tma_store_wait_all();
-          fence_proxy_async_all();
+        // Without an AllReduce nobody looks before the launch has ended: the leader waits only until
+        // its staging has been read.
+        if (without_ar(p)) {
+          if (leader) tma_store_wait_read();
+        } else {
+          if (leader) {
+            tma_store_wait_all();
+            fence_proxy_async_all();
+          }
+          if (direct) __threadfence();
         }
-        if (direct) __threadfence();
       } else if (mode == MODE_AR) {
         ar_slot(p, d[T_FT], d[TO_BASE], d[TO_VNT], tid - 128, 256);
         if (lane == 0) __threadfence_system();   // one per warp; the scheduler fences again
@@ -1501,16 +1520,20 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     __shared__ int s_last;
     if (tid == 0) {
       fence_acq_rel_gpu();
-      s_last = (atom_add_acqrel_gpu(p.sync_ctrl + S_GS_QUIESCE, 1u) == gridDim.x - 1) ? 1 : 0;
+      s_last = (atom_add_relaxed_gpu(p.sync_ctrl + S_GS_QUIESCE, 1u) == gridDim.x - 1) ? 1 : 0;
+      if (s_last) fence_acq_rel_gpu();
     }
     __syncthreads();
     if (s_last) {
-      for (int i = tid; i < p.max_row_tiles; i += kThreads) p.head_ready[i] = 0u;
+      for (int i = tid; i < p.max_row_tiles; i += kThreads) {
+        p.head_ready[i] = 0u;
+        p.oproj_queue[i] = 0u;      // (an entry per row-tile group at most)
+      }
       for (int i = tid; i < p.max_owner_slots; i += kThreads) p.ready_count[i] = 0u;
       for (int i = tid; i < p.max_owner_words; i += kThreads) p.ar_done_bits[i] = 0ull;
       if (tid < 8) p.ctrl[tid] = 0u;
       if (tid == 8) p.sync_ctrl[S_GS_QUIESCE] = 0u;
-      __threadfence_system();
+      if (p.tp > 1) __threadfence_system();
       if (p.tp > 1 && !(p.flags & (1u | 16u))) rank_barrier(env);
     }
   }

@@ -5,7 +5,8 @@
 namespace ma {
 
 // Control-word indices: same numbering as the reference kernel
-// (src/mega_attention/kernels/sm90/fused_fa_oproj_ar.py:47-67), which host code reads.
+// (src/mega_attention/kernels/sm90/fused_fa_oproj_ar.py:47-67), which host code reads.  (The ready
+// queue's entries are published one by one here, so C_OP_PUBLISH stays 0 and its wait is gone.)
 enum : int {
   C_FA_COUNTER = 0, C_FA_DONE = 1, C_OP_RESERVE = 2, C_OP_PUBLISH = 3,
   C_OP_CONSUME = 4, C_OP_DONE = 5, C_AR_DONE = 6, C_AR_CURSOR = 7

@@ -329,6 +329,12 @@ __device__ __forceinline__ uint32_t atom_add_relaxed_gpu(uint32_t* p, uint32_t v
                : "memory");
   return o;
 }
+__device__ __forceinline__ void red_add_relaxed_gpu(uint32_t* p, uint32_t v) {
+  asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ uint32_t atom_add_release_gpu(uint32_t* p, uint32_t v) {
   uint32_t o;
   asm volatile("atom.release.gpu.global.add.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v)

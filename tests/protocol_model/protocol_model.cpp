@@ -5,11 +5,13 @@
 // scheduler.  The state machines are the ones of csrc/fused_prefill.cu (which follow the
 // reference's src/mega_attention/kernels/sm90/fused_fa_oproj_ar.py:148-398, 1154-1177):
 //
-//   attention task counter -> head count per group of row tiles -> ordered O_proj ready queue
-//   (reserve / fill / publish in reservation order; an entry is a group and stands for its
-//   tickets) -> ticket pop -> owner rank's ready count
+//   attention task counter -> head count per group of row tiles -> O_proj ready queue
+//   (reserve / write the entry: a group's number plus one, which stands for its tickets) -> ticket
+//   pop, by who waits for the ticket's entry -> owner rank's ready count
 //   (one arrival per rank, one byte per slot) -> claim by atomic OR of the slot's flag -> done counters -> count-out exit with
 //   full-capacity clear by the last CTA -> phase/sign barrier across the ranks.
+//
+// One rank has no AllReduce: a CTA leaves once every task is handed out and it holds no ticket.
 //
 // Every wait is bounded as in the kernel: when the limit passes, the waiter writes a status
 // {code, site, cta} once, everybody who sees a non-zero status leaves, and the launch
@@ -39,8 +41,8 @@
 namespace {
 
 using clk = std::chrono::steady_clock;
-enum { C_FA_COUNTER, C_FA_DONE, C_OP_RESERVE, C_OP_PUBLISH, C_OP_CONSUME, C_OP_DONE, C_AR_DONE, C_QUIESCE, C_NUM };
-enum { ST_OK = 0, ST_TIMEOUT_PUBLISH = 2, ST_TIMEOUT_NVL = 4, ST_TIMEOUT_IDLE = 6 };
+enum { C_FA_COUNTER, C_FA_DONE, C_OP_RESERVE, C_OP_CONSUME, C_OP_DONE, C_AR_DONE, C_QUIESCE, C_NUM };
+enum { ST_OK = 0, ST_TIMEOUT_NVL = 4, ST_TIMEOUT_IDLE = 6 };
 enum { MODE_IDLE, MODE_FA, MODE_OPROJ, MODE_AR, MODE_DONE };
 
 struct Config {
@@ -75,7 +77,7 @@ struct World {
   Config cfg;
   std::vector<Rank*> ranks;
   int total_op() const { return cfg.groups() * cfg.nsg; }
-  int owned(int rank) const { int t = total_op() - rank; return t <= 0 ? 0 : (t + cfg.tp - 1) / cfg.tp; }
+  int owned(int rank) const { if (cfg.tp == 1) return 0; int t = total_op() - rank; return t <= 0 ? 0 : (t + cfg.tp - 1) / cfg.tp; }
 };
 
 bool expired(clk::time_point t0, int limit_ms) {
@@ -108,17 +110,15 @@ bool try_fa(Rank& r, const Config& c, int num_fa, int* arg, int* nt) {
 bool try_pop_oproj(Rank& r, int total_op, int per_group, int* pending, int* arg) {
   if (*pending < 0) {
     const uint32_t head = r.ctrl[C_OP_CONSUME].load(std::memory_order_relaxed);
-    const uint32_t tail = r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire);
+    const uint32_t tail = r.ctrl[C_OP_RESERVE].load(std::memory_order_relaxed);
     if (head >= tail) return false;
     const uint32_t t = r.ctrl[C_OP_CONSUME].fetch_add(1, std::memory_order_relaxed);
     if (static_cast<int>(t) >= total_op) return false;
     *pending = static_cast<int>(t);
-    if (t >= tail && t >= r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire)) return false;
-  } else if (static_cast<uint32_t>(*pending) >= r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire)) {
-    return false;
   }
-  *arg = static_cast<int>(r.queue[*pending / per_group].load(std::memory_order_relaxed)) * per_group +
-         *pending % per_group;
+  const uint32_t entry = r.queue[*pending / per_group].load(std::memory_order_acquire);
+  if (entry == 0) return false;
+  *arg = static_cast<int>(entry - 1) * per_group + *pending % per_group;
   *pending = -1;
   return true;
 }
@@ -144,15 +144,7 @@ bool try_claim_ar(World& w, int rank, int* arg) {
 void publish_oproj(World& w, Rank& r, int group) {
   const uint32_t n = static_cast<uint32_t>(w.cfg.nsg);
   const uint32_t start = r.ctrl[C_OP_RESERVE].fetch_add(n, std::memory_order_relaxed);
-  r.queue[start / n].store(static_cast<uint32_t>(group), std::memory_order_relaxed);
-  std::atomic_thread_fence(std::memory_order_acq_rel);
-  const auto t0 = clk::now();
-  while (r.ctrl[C_OP_PUBLISH].load(std::memory_order_acquire) != start) {
-    if (r.status.load() != 0) return;
-    if (expired(t0, w.cfg.limit_ms)) { report(r, ST_TIMEOUT_PUBLISH, start); return; }
-    std::this_thread::yield();
-  }
-  r.ctrl[C_OP_PUBLISH].fetch_add(n, std::memory_order_release);
+  r.queue[start / n].store(static_cast<uint32_t>(group) + 1u, std::memory_order_release);
 }
 
 void rank_barrier(World& w, int rank) {
@@ -191,7 +183,11 @@ void cta_main(World& w, int rank, int cta) {
     }
     if (mode == MODE_IDLE) {
       if (r.status.load(std::memory_order_relaxed) != 0) { aborted = true; break; }
-      const bool done = static_cast<int>(r.ctrl[C_FA_DONE].load(std::memory_order_acquire)) >= num_fa &&
+      const bool done =
+          c.tp == 1 ? static_cast<int>(r.ctrl[C_FA_COUNTER].load(std::memory_order_relaxed)) >=
+                              c.R * fa_tasks_per_tile(c) && pending < 0 &&
+                          static_cast<int>(r.ctrl[C_OP_CONSUME].load(std::memory_order_relaxed)) >= total_op
+                    : static_cast<int>(r.ctrl[C_FA_DONE].load(std::memory_order_acquire)) >= num_fa &&
                         static_cast<int>(r.ctrl[C_OP_DONE].load(std::memory_order_acquire)) >= total_op &&
                         static_cast<int>(r.ctrl[C_AR_DONE].load(std::memory_order_acquire)) >= local_owned;
       if (done) break;
@@ -223,7 +219,7 @@ void cta_main(World& w, int rank, int cta) {
         for (int h = 0; h < c.H; ++h)      // its row tiles' attention has to be done
           if (r.fa_runs[t * c.H + h].load() != 1) r.early.fetch_add(1);
       const int owner = arg % c.tp, idx = arg / c.tp;
-      if (!(rank == c.drop_rank && arg == c.drop_slot))           // injected lost arrival
+      if (c.tp > 1 && !(rank == c.drop_rank && arg == c.drop_slot))   // injected lost arrival
         w.ranks[owner]->ready_count[idx >> 2].fetch_add(1u << ((idx & 3) * 8), std::memory_order_release);
       r.ctrl[C_OP_DONE].fetch_add(1, std::memory_order_release);
     } else {
@@ -236,6 +232,7 @@ void cta_main(World& w, int rank, int cta) {
   // cross-rank barrier alone
   if (r.ctrl[C_QUIESCE].fetch_add(1, std::memory_order_acq_rel) == static_cast<uint32_t>(c.ctas - 1)) {
     for (auto& x : r.head_ready) x = 0;
+    for (auto& x : r.queue) x = 0;
     for (auto& x : r.ready_count) x = 0;
     for (int i = 0; i < C_NUM; ++i) r.ctrl[i] = 0;
     std::atomic_thread_fence(std::memory_order_seq_cst);
@@ -306,6 +303,7 @@ int main(int argc, char** argv) {
       for (int i = 0; i < w.owned(r); ++i) { if (k.ar_runs[i].load() != 1) exactly_once = false; k.ar_runs[i] = 0; }
       for (int i = 0; i < C_NUM; ++i) if (k.ctrl[i].load() != 0) clean_exit = false;
       for (auto& x : k.head_ready) if (x.load() != 0) clean_exit = false;
+      for (auto& x : k.queue) if (x.load() != 0) clean_exit = false;
       for (auto& x : k.ready_count) if (x.load() != 0) clean_exit = false;
     }
   }
