@@ -370,6 +370,44 @@ int ma_stage_tasks(const ma_stage_tasks_args* args);
  */
 int ma_upload_meta(const ma_stage_tasks_args* args, uint64_t meta_dev, void* stream);
 
+/*
+ * ma_step queues one layer of a single-rank plan: it encodes the inputs' descriptors (as
+ * ma_plan_set_inputs), builds and uploads the batch's metadata (ma_row_desc, ma_upload_meta) and
+ * launches (ma_launch), all on `stream`, and returns the number of row tiles.  Of `stage` the four
+ * arrays, num_batch and num_row_tiles are filled in by the call.  cu_q, cu_k: host, num_batch + 1
+ * words from 0 (cu_k NULL: the same as cu_q).
+ * With page_table set (device, i32 [num_batch][table_pitch], table_width columns of it) the key
+ * lengths are cache_seqlens's (device, i32 [num_batch]): a kernel copies both to the plan's own
+ * (page_table_out with a pitch of table_pitch_out, cache_seqlens_out) and brings the lengths and the
+ * range of the page numbers to host_words (pinned, i32 [num_batch + 2 * MA_STEP_BLOCKS]), and the
+ * call waits for that - the only wait in it.  tot_k is 128 times the number of pages.
+ * A batch that does not fit is refused after the wait, with nothing else queued and the plan's
+ * inputs as they were: MA_STEP_NARROW (a sequence needs more than table_width pages), MA_STEP_PAGES
+ * (a page number outside the cache), MA_STEP_LENGTHS (not 0 < q_len <= k_len), MA_STEP_TILES (more
+ * than max_row_tiles).  Otherwise an ma_error code.
+ */
+#define MA_STEP_BLOCKS 32
+#define MA_STEP_NARROW (-101)
+#define MA_STEP_PAGES (-102)
+#define MA_STEP_LENGTHS (-103)
+#define MA_STEP_TILES (-104)
+typedef struct ma_step_args {
+  ma_stage_tasks_args stage;
+  const int64_t* cu_q;
+  const int64_t* cu_k;
+  uint64_t Q, K, V, W_o, meta_dev;
+  int64_t tot_q, tot_k, w_width;
+  uint64_t page_table, cache_seqlens, page_table_out, cache_seqlens_out;
+  int32_t* host_words;
+  int64_t table_pitch;
+  int32_t table_width, table_pitch_out;
+  int32_t num_batch, max_row_tiles;
+  ma_launch_args launch;
+  int32_t reserved0;
+} ma_step_args;
+
+int ma_step(ma_plan* plan, const ma_step_args* args, void* stream);
+
 const char* ma_strerror(int code);
 
 #ifdef __cplusplus

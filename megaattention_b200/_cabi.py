@@ -29,7 +29,7 @@ MA_ERR_CAPACITY = -5
 EXPORTS = ("ma_query_device", "ma_plan_create", "ma_launch", "ma_plan_set_inputs", "ma_read_status",
            "ma_plan_destroy", "ma_strerror", "ma_fused_prefill_noalloc", "ma_residual_rmsnorm", "ma_rope_qk",
            "ma_detile", "ma_row_desc", "ma_stage_meta", "ma_plan_set_tasks", "ma_stage_tasks",
-           "ma_upload_meta", "ma_plan_set_split")
+           "ma_upload_meta", "ma_plan_set_split", "ma_step")
 
 MA_NOALLOC_OSCRATCH_BYTES = 16 << 20
 MA_NOALLOC_MAX_BATCH = 512
@@ -118,6 +118,23 @@ class StageTasksArgs(C.Structure):
                 ("split_slots", C.c_int32), ("num_ctas", C.c_int32)]
 
 
+STEP_BLOCKS = 32
+STEP_REFUSED = {-101: "page_table is narrower than the longest sequence needs",
+                -102: "page_table has a page that is not in the cache",
+                -103: "0 < q_len <= k_len per sequence",
+                -104: "more row tiles than the workspace was created for"}
+
+
+class StepArgs(C.Structure):
+    _fields_ = ([("stage", StageTasksArgs)] + [(n, C.c_void_p) for n in ("cu_q", "cu_k")]
+                + [(n, C.c_uint64) for n in ("Q", "K", "V", "W_o", "meta_dev")]
+                + [(n, C.c_int64) for n in ("tot_q", "tot_k", "w_width")]
+                + [(n, C.c_uint64) for n in ("page_table", "cache_seqlens", "page_table_out", "cache_seqlens_out")]
+                + [("host_words", C.c_void_p), ("table_pitch", C.c_int64)]
+                + [(n, C.c_int32) for n in ("table_width", "table_pitch_out", "num_batch", "max_row_tiles")]
+                + [("launch", LaunchArgs), ("reserved0", C.c_int32)])
+
+
 TASK_WORDS = 8           # of one position of the task table, behind a header of 4
 PART_FLOATS = 128 * 128 + 2 * 128     # of one head of a slot (ma_plan_set_split)
 
@@ -165,6 +182,8 @@ def _load(path=None, audit=False):
     lib.ma_stage_tasks.restype = C.c_int
     lib.ma_upload_meta.argtypes = [C.POINTER(StageTasksArgs), C.c_uint64, C.c_void_p]
     lib.ma_upload_meta.restype = C.c_int
+    lib.ma_step.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.ma_step.restype = C.c_int
     lib.ma_strerror.argtypes = [C.c_int]
     lib.ma_strerror.restype = C.c_char_p
     return lib

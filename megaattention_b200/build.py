@@ -14,7 +14,7 @@ LIB = os.path.join(HERE, "libmegaattn_b200.so")
 # (measured: +1.2 % on the attention stage).
 LIB_AUDIT = os.path.join(HERE, "libmegaattn_b200_audit.so")
 SOURCES = ["fused_prefill.cu", "cabi.cu", "noalloc.cu", "residual_rmsnorm.cu", "rope.cu",
-           "detile.cu", "meta_upload.cu", "meta.cpp"]
+           "detile.cu", "meta_upload.cu", "step.cu", "meta.cpp"]
 HEADERS = ["ptx.cuh", "kparams.h", os.path.join("..", "..", "include", "megaattn_b200.h")]
 
 

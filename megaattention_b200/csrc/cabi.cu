@@ -18,6 +18,9 @@ int encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint
                      uint64_t W, uint64_t H, uint64_t Hkv, uint64_t tot_q, uint64_t tot_k,
                      uint64_t row_tiles, uint64_t w_width, uint64_t csym, uint64_t hidden,
                      uint64_t csym_pitch);
+int plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
+                       int64_t tot_q, int64_t tot_k, int64_t w_width);
+void plan_take_inputs(ma_plan* pl, const CUtensorMap* fresh);
 }  // namespace ma
 
 struct ma_plan {
@@ -77,39 +80,43 @@ int cdiv(int a, int b) { return (a + b - 1) / b; }
 // W_o [K_local, width] is described as {64 n, K_local, width/64 panels}: the box
 // {64, 64, 2} is a 64-k slab of 128 output columns, panel after panel; {64, 64, 4} (the last
 // map) one of 256.
-int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint64_t oscr,
-                         uint64_t W, uint64_t H, uint64_t Hkv, uint64_t tot_q, uint64_t tot_k,
-                         uint64_t row_tiles, uint64_t w_width, uint64_t csym, uint64_t hidden,
-                         uint64_t csym_pitch) {
+static int encode_input_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint64_t W, uint64_t H,
+                      uint64_t Hkv, uint64_t tot_q, uint64_t tot_k, uint64_t w_width) {
   if (w_width % 64) return MA_ERR_INVALID;
-  const uint64_t KL = H * 128;
+  const uint32_t box[4] = {64, 128, 2, 1};
   int rc;
   {
     const uint64_t dims[4] = {64, tot_q, 2, H};
     const uint64_t str[3] = {H * 256, 128, 256};
-    const uint32_t box[4] = {64, 128, 2, 1};
     rc = encode(&maps[0], Q, 4, dims, str, box);
   }
   if (rc == MA_OK) {
     const uint64_t dims[4] = {64, tot_k, 2, Hkv};
     const uint64_t str[3] = {Hkv * 256, 128, 256};
-    const uint32_t box[4] = {64, 128, 2, 1};
     rc = encode(&maps[1], K, 4, dims, str, box);
     if (rc == MA_OK) rc = encode(&maps[2], V, 4, dims, str, box);
   }
+  if (rc == MA_OK) {
+    const uint64_t dims[3] = {64, H * 128, w_width / 64};
+    const uint64_t str[2] = {w_width * 2, 128};
+    const uint32_t box1[3] = {64, 64, 2}, box2[3] = {64, 64, 4};
+    rc = encode(&maps[4], W, 3, dims, str, box1);
+    if (rc == MA_OK) rc = encode(&maps[6], W, 3, dims, str, box2);
+  }
+  return rc;
+}
+
+int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint64_t oscr,
+                         uint64_t W, uint64_t H, uint64_t Hkv, uint64_t tot_q, uint64_t tot_k,
+                         uint64_t row_tiles, uint64_t w_width, uint64_t csym, uint64_t hidden,
+                         uint64_t csym_pitch) {
+  const uint64_t KL = H * 128;
+  int rc = encode_input_maps(maps, Q, K, V, W, H, Hkv, tot_q, tot_k, w_width);
   if (rc == MA_OK) {
     const uint64_t dims[2] = {KL, row_tiles * 128};
     const uint64_t str[1] = {KL * 2};
     const uint32_t box[2] = {64, 128};
     rc = encode(&maps[3], oscr, 2, dims, str, box);
-  }
-  if (rc == MA_OK) {
-    const uint64_t dims[3] = {64, KL, w_width / 64};
-    const uint64_t str[2] = {w_width * 2, 128};
-    const uint32_t box[3] = {64, 64, 2};
-    const uint32_t box2[3] = {64, 64, 4};
-    rc = encode(&maps[4], W, 3, dims, str, box);
-    if (rc == MA_OK) rc = encode(&maps[6], W, 3, dims, str, box2);
   }
   if (rc == MA_OK) {
     // output tiles are stored through TMA: [rows, hidden] with the padded row pitch, so a
@@ -120,6 +127,23 @@ int ma::encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, 
     rc = encode(&maps[5], csym, 2, dims, str, box);
   }
   return rc;
+}
+
+// A plan's input descriptors, encoded and then taken over (the output's stay as they are).
+int ma::plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
+                           int64_t tot_q, int64_t tot_k, int64_t w_width) {
+  if (!Q || !K || !V || !W_o) return MA_ERR_INVALID;
+  const ma_plan_desc& d = pl->desc;
+  if (tot_q < 1 || tot_k < 1 || w_width < d.hidden || w_width % 64) return MA_ERR_INVALID;
+  if (d.page_table && tot_k % 128) return MA_ERR_INVALID;
+  return encode_input_maps(fresh, Q, K, V, W_o, static_cast<uint64_t>(d.H_local), static_cast<uint64_t>(d.H_kv),
+                           static_cast<uint64_t>(tot_q), static_cast<uint64_t>(tot_k),
+                           static_cast<uint64_t>(w_width));
+}
+
+void ma::plan_take_inputs(ma_plan* pl, const CUtensorMap* fresh) {
+  pl->maps[0] = fresh[0]; pl->maps[1] = fresh[1]; pl->maps[2] = fresh[2]; pl->maps[4] = fresh[4];
+  pl->maps[6] = fresh[6];
 }
 
 extern "C" {
@@ -292,23 +316,11 @@ int ma_launch(ma_plan* pl, const ma_launch_args* a, void* stream) {
 
 int ma_plan_set_inputs(ma_plan* pl, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
                        int64_t tot_q, int64_t tot_k, int64_t w_width) {
-  if (!pl || !Q || !K || !V || !W_o) return MA_ERR_INVALID;
-  const ma_plan_desc& d = pl->desc;
-  if (tot_q < 1 || tot_k < 1 || w_width < d.hidden || w_width % 64) return MA_ERR_INVALID;
-  if (d.page_table && tot_k % 128) return MA_ERR_INVALID;
+  if (!pl) return MA_ERR_INVALID;
   CUtensorMap fresh[7];
-  const int rc = ma::encode_path_maps(fresh, Q, K, V, d.o_scratch, W_o,
-                                      static_cast<uint64_t>(d.H_local),
-                                      static_cast<uint64_t>(d.H_kv),
-                                      static_cast<uint64_t>(tot_q), static_cast<uint64_t>(tot_k),
-                                      static_cast<uint64_t>(d.max_row_tiles),
-                                      static_cast<uint64_t>(w_width), d.csym,
-                                      static_cast<uint64_t>(d.hidden),
-                                      static_cast<uint64_t>(pl->kp.num_out) * 128);
-  if (rc != MA_OK) return rc;
-  pl->maps[0] = fresh[0]; pl->maps[1] = fresh[1]; pl->maps[2] = fresh[2]; pl->maps[4] = fresh[4];
-  pl->maps[6] = fresh[6];
-  return MA_OK;
+  const int rc = ma::plan_encode_inputs(pl, fresh, Q, K, V, W_o, tot_q, tot_k, w_width);
+  if (rc == MA_OK) ma::plan_take_inputs(pl, fresh);
+  return rc;
 }
 
 int ma_plan_set_tasks(ma_plan* pl, uint64_t tasks) {

@@ -34,7 +34,7 @@ from .workspace import native_row_desc
 
 
 def _cumulative(cu):
-    cu = np.asarray(cu.cpu().numpy() if torch.is_tensor(cu) else cu, dtype=np.int64)
+    cu = np.ascontiguousarray(cu.cpu().numpy() if torch.is_tensor(cu) else cu, dtype=np.int64)
     assert cu.ndim == 1 and cu.size >= 2 and cu[0] == 0, "cu_seqlens must start at 0"
     return cu
 
@@ -95,6 +95,9 @@ class FusedPrefillLayer:
                 v = v.view(-1, 128, ws.H_kv, ws.D)
             assert page_table.dim() == 2 and cache_seqlens.dim() == 1
             assert page_table.shape[0] == cu_q.size - 1 == cache_seqlens.shape[0]
+            if ws.can_step(page_table, cache_seqlens):
+                self.meta = ws.step(q, k, v, self.W_o, cu_q, None, page_table, cache_seqlens, flags)
+                return ws.csym[:self.meta.num_row_tiles]
             lens_k, pages = _lengths_and_pages(cache_seqlens, page_table)
             assert page_table.shape[1] >= int((-(-lens_k // 128)).max()), \
                 "page_table is narrower than the longest sequence needs"
@@ -102,6 +105,9 @@ class FusedPrefillLayer:
             assert page_table is None and cache_seqlens is None, \
                 "page_table / cache_seqlens need a workspace created with paged=True"
             cu_k = cu_q if cu_seqlens_k is None else _cumulative(cu_seqlens_k)
+            if ws.can_step():
+                self.meta = ws.step(q, k, v, self.W_o, cu_q, cu_k, flags=flags)
+                return ws.csym[:self.meta.num_row_tiles]
         if ws.paged:
             cu_k = np.zeros(cu_q.size, dtype=np.int64)
             np.cumsum(lens_k, out=cu_k[1:])

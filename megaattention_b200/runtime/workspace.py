@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import functools
 
 import numpy as np
 import torch
@@ -94,12 +95,41 @@ def native_row_desc(cu_q, cu_k, max_row_tiles: int) -> RowDescMeta:
                        m_block=buf[at + cap:at + cap + n])
 
 
+class StepMeta(RowDescMeta):
+    """The schedule of a step that was queued natively: its arrays are made when somebody looks."""
+
+    def __init__(self, cu_q, lens_k, cu_k, num_row_tiles):
+        self.num_batch, self.M_TILE, self.num_row_tiles = cu_q.size - 1, 128, num_row_tiles
+        # (copies: the caller's arrays and the lengths' staging are their owners' again)
+        self._cu_q = cu_q.copy()
+        self._lens_k = None if lens_k is None else lens_k.copy()
+        self._cu_k = self._cu_q if cu_k is cu_q else (None if cu_k is None else cu_k.copy())
+
+    @functools.cached_property
+    def _all(self):
+        cu_k = self._cu_k
+        if cu_k is None:
+            cu_k = np.zeros(self.num_batch + 1, dtype=np.int64)
+            np.cumsum(self._lens_k, out=cu_k[1:])
+        return native_row_desc(self._cu_q, cu_k, self.num_row_tiles)
+
+    @functools.cached_property
+    def cu_seqlens_q(self):
+        return self._cu_q.astype(np.int32)
+
+    cu_seqlens_k = functools.cached_property(lambda self: self._all.cu_seqlens_k)
+    cu_m_blocks = functools.cached_property(lambda self: self._all.cu_m_blocks)
+    batch_idx = functools.cached_property(lambda self: self._all.batch_idx)
+    m_block = functools.cached_property(lambda self: self._all.m_block)
+
+
 class FusedFaOprojArWorkspace:
     def __init__(self, **kw):
         self.__dict__.update(kw)
         self._plan = None
         self._lib = _cabi.lib
         self._split_ctas = 0           # (set by compile: before it nothing is split)
+        self._step_args = None
         self._args = None
         self._meta = None
         # Launch flags applied by launch() (OR of _cabi.MA_FLAG_*) and attention claim order
@@ -218,6 +248,8 @@ class FusedFaOprojArWorkspace:
             page_table=(zeros((max_num_batch, max_num_pages_per_seq), torch.int32)
                         if paged else None),
             cache_seqlens=(zeros(max_num_batch, torch.int32) if paged else None),
+            _host_words=(torch.empty(max_num_batch + 2 * _cabi.STEP_BLOCKS, dtype=torch.int32, pin_memory=True).numpy()
+                         if paged else None),
             W_o=zeros((K_local, hidden_pad), dtype),
             Oscr=zeros((max_num_row_tiles, 128, H_local, D), dtype),
             csym=csym, rco=rco, rbits=rbits, nvl=nvl,
@@ -298,6 +330,7 @@ class FusedFaOprojArWorkspace:
         self._args = _cabi.LaunchArgs(int(w_fa), int(w_oproj), int(w_ar),
                                       int(num_ctas) if num_ctas else 0, 0)
         self._ts = torch.cuda.current_stream(self.dev)
+        self._step_args = None
         return self
 
     # ------------------------------------------------------------------ per layer
@@ -360,17 +393,11 @@ class FusedFaOprojArWorkspace:
         ``[K_local, hidden_pad]`` one.  The tensors must stay alive and unchanged until the
         launch has finished; a later ``set_layer`` goes back to the workspace's own buffers.
         """
-        for t in (Q, K, V, W_o):
-            assert t.is_cuda and t.device == self.dev and t.dtype == self.dtype
-            assert t.is_contiguous() and t.data_ptr() % 16 == 0
         R, nb = meta.num_row_tiles, meta.num_batch
-        assert R <= self.max_num_row_tiles and nb <= self.max_num_batch
-        assert tuple(Q.shape[1:]) == (self.H_local, self.D) and Q.shape[0] <= self.tot_cap
-        assert int(meta.cu_seqlens_q[-1]) == Q.shape[0]
-        assert W_o.shape[0] == self.K_local and W_o.shape[1] >= self.hidden and W_o.shape[1] % 64 == 0
+        assert R <= self.max_num_row_tiles
+        self._check_inputs(nb, int(meta.cu_seqlens_q[-1]), Q, K, V, W_o)
         if self.paged:
             assert page_table is not None and cache_seqlens is not None
-            assert tuple(K.shape[1:]) == (128, self.H_kv, self.D) == tuple(V.shape[1:])
             tot_k = K.shape[0] * 128
             page_table = torch.as_tensor(page_table, dtype=torch.int32)
             cache_seqlens = torch.as_tensor(cache_seqlens, dtype=torch.int32)
@@ -380,7 +407,6 @@ class FusedFaOprojArWorkspace:
             pages = page_table if page_table_host is None else page_table_host
             assert int(pages.max()) < K.shape[0] and int(pages.min()) >= 0
         else:
-            assert tuple(K.shape[1:]) == (self.H_kv, self.D) == tuple(V.shape[1:])
             tot_k = K.shape[0]
             assert int(meta.cu_seqlens_k[-1]) == tot_k
         _cabi.check(self._lib.ma_plan_set_inputs(
@@ -392,6 +418,80 @@ class FusedFaOprojArWorkspace:
                 self.page_table[:nb, :page_table.shape[1]].copy_(page_table.to(self.dev))
                 self.cache_seqlens[:nb].copy_(cache_seqlens.to(self.dev))
             self._set_meta(meta)
+
+    def _check_inputs(self, nb, tot_q, Q, K, V, W_o):
+        """What the kernel can read in place (bind_inputs, step)."""
+        for t in (Q, K, V, W_o):
+            assert t.is_cuda and t.device == self.dev and t.dtype == self.dtype
+            assert t.is_contiguous() and t.data_ptr() % 16 == 0
+        assert nb <= self.max_num_batch
+        assert Q.shape[1:] == (self.H_local, self.D) and Q.shape[0] <= self.tot_cap
+        assert tot_q == Q.shape[0]
+        assert W_o.shape[0] == self.K_local and W_o.shape[1] >= self.hidden and W_o.shape[1] % 64 == 0
+        want = (128, self.H_kv, self.D) if self.paged else (self.H_kv, self.D)
+        assert K.shape[1:] == want == V.shape[1:]
+
+    def can_step(self, *tables):
+        """Whether ``step`` takes a call made here and now: one rank, on the stream and device that
+        compile() was called on, ``tables`` on that device with columns next to each other."""
+        return (self.tp_size == 1 and self._plan is not None
+                and torch._C._cuda_getDevice() == self.dev.index == self._ts.device_index
+                and torch._C._cuda_getCurrentRawStream(self.dev.index) == self._ts.cuda_stream
+                and all(t.device == self.dev and t.stride(-1) == 1 and t.numel() for t in tables))
+
+    def step(self, Q, K, V, W_o, cu_q, cu_k=None, page_table=None, cache_seqlens=None, flags=None):
+        """``bind_inputs`` and ``launch`` in one native call (ma_step), for callers whose lengths are
+        host arrays (int64 ``cu_q``, ``cu_k``) or, paged, int32 device tensors.  Same refusals.
+        Returns the batch's schedule.  Only where ``can_step`` says so."""
+        nb = cu_q.size - 1
+        self._check_inputs(nb, int(cu_q[-1]), Q, K, V, W_o)
+        a = self._step_args
+        if a is None:
+            a = self._step_args = self._new_step_args()
+        if self.paged:
+            width = page_table.shape[1]
+            assert width <= self.max_num_pages_per_seq
+            a.page_table, a.cache_seqlens = page_table.data_ptr(), cache_seqlens.data_ptr()
+            a.table_pitch, a.table_width = page_table.stride(0), width
+            a.tot_k = K.shape[0] * 128
+        else:
+            assert cu_k.size == nb + 1 and int(cu_k[-1]) == K.shape[0]
+            a.cu_k = cu_k.ctypes.data
+            a.tot_k = K.shape[0]
+        a.cu_q, a.num_batch = cu_q.ctypes.data, nb
+        a.Q, a.K, a.V, a.W_o = Q.data_ptr(), K.data_ptr(), V.data_ptr(), W_o.data_ptr()
+        a.tot_q, a.w_width = Q.shape[0], W_o.shape[1]
+        prime = self.fa_prime_tiles
+        a.stage.meta.auto_prime, a.stage.meta.prime = int(prime is None), 0 if prime is None else max(-1, int(prime))
+        if flags is None:
+            flags = self.default_flags or 0      # (launch_flags_b200 is 0 on one rank)
+        a.launch.flags = int(flags)
+        rc = self._lib.ma_step(self._plan, self._step_at, self._ts.cuda_stream)
+        if rc < 0:
+            assert rc not in _cabi.STEP_REFUSED, _cabi.STEP_REFUSED[rc]
+            _cabi.check(rc, "ma_step")
+        self._bound = (Q, K, V, W_o)          # keep them alive
+        self._auto_flags = 0
+        self._meta = StepMeta(cu_q, self._host_words[:nb] if self.paged else None, cu_k, rc)
+        return self._meta
+
+    def _new_step_args(self):
+        """The part of ma_step's arguments that is the workspace's."""
+        if getattr(self, "_meta_host", None) is None:
+            self._meta_host = np.zeros(self._meta_offs[-1], dtype=np.int32)
+            self._meta_at = self._meta_host.ctypes.data
+        o = self._meta_offs
+        a = _cabi.StepArgs()
+        a.stage = _cabi.StageTasksArgs(_cabi.StageMetaArgs(
+            None, None, None, None, self._meta_at, 0, 0, self.hidden, self.H_local, self.num_super_groups,
+            self.tp_size, self.rank, 1, 0, o[0], o[1], o[2], o[3], o[4], o[5], 0), o[6], self.max_tasks,
+            self.split_slots, self._split_ctas)
+        a.meta_dev, a.max_row_tiles, a.launch = self.meta_dev.data_ptr(), self.max_num_row_tiles, self._args
+        if self.paged:
+            a.page_table_out, a.cache_seqlens_out = self.page_table.data_ptr(), self.cache_seqlens.data_ptr()
+            a.table_pitch_out, a.host_words = self.max_num_pages_per_seq, self._host_words.ctypes.data
+        self._step_at = C.addressof(a)
+        return a
 
     def _unbind(self):
         if getattr(self, "_bound", None) is not None:

@@ -1,0 +1,175 @@
+"""A layer's call in one native step (ma_step): the same results, schedule and refusals as the calls
+it stands for, for packed and paged keys; calls it does not take go the general way."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+import torch
+
+from cases import CASES, make_inputs
+from megaattention_b200 import _cabi
+from megaattention_b200.metadata import build_row_desc
+from megaattention_b200.runtime import FusedFaOprojArWorkspace, FusedPrefillLayer
+from megaattention_b200.runtime.workspace import StepMeta
+from oracle.chain_oracle import make_paged_kv
+
+HEADER = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include", "megaattn_b200.h")
+FIELDS = ("cu_seqlens_q", "cu_seqlens_k", "cu_m_blocks", "batch_idx", "m_block")
+
+
+def _cu(lens):
+    return np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+
+
+def _same_schedule(got, want):
+    assert (got.num_batch, got.num_row_tiles, got.M_TILE) == (want.num_batch, want.num_row_tiles, 128)
+    for f in FIELDS:
+        a, b = getattr(got, f), getattr(want, f)
+        assert a.dtype == b.dtype and np.array_equal(a, b), f
+
+
+def test_the_struct_is_the_headers(tmp_path):
+    names = [(s, f) for s, t in (("ma_step_args", _cabi.StepArgs), ("ma_stage_tasks_args", _cabi.StageTasksArgs))
+             for f, *_ in t._fields_]
+    src = tmp_path / "l.c"
+    src.write_text('#include <stdio.h>\n#include <stddef.h>\n#include "%s"\nint main(void) {\n' % HEADER
+                   + "".join('printf("%%zu\\n", offsetof(%s, %s));\n' % n for n in names)
+                   + 'printf("%zu %d\\n", sizeof(ma_step_args), MA_STEP_BLOCKS);return 0;}\n')
+    subprocess.run(["gcc", "-std=c99", "-o", str(tmp_path / "l"), str(src)], check=True)
+    out = subprocess.run([str(tmp_path / "l")], check=True, capture_output=True, text=True).stdout.split()
+    types = {"ma_step_args": _cabi.StepArgs, "ma_stage_tasks_args": _cabi.StageTasksArgs}
+    assert [int(x) for x in out] == ([getattr(types[s], f).offset for s, f in names]
+                                     + [C.sizeof(_cabi.StepArgs), _cabi.STEP_BLOCKS])
+
+
+@pytest.mark.parametrize("q,k", [([3, 200, 128], [3, 900, 128]), ([1], [1])])
+def test_the_schedule_is_made_when_looked_at(q, k):
+    want = build_row_desc(q, seqlens_k=k)
+    cu_q, lens = _cu(q), np.array(k, dtype=np.int32)
+    for meta in (StepMeta(cu_q, lens, None, want.num_row_tiles), StepMeta(cu_q, None, _cu(k), want.num_row_tiles)):
+        keep, keep_k = cu_q.copy(), lens.copy()
+        cu_q[:], lens[:] = -5, -5                    # (the caller's again)
+        _same_schedule(meta, want)
+        cu_q[:], lens[:] = keep, keep_k
+
+
+def _layer(name, paged):
+    sq, H, hidden, qpk, sk, _ = CASES[name]
+    sk = sq if sk is None else sk
+    Q, K, V, W = make_inputs(name)
+    kw, kv, pages = {}, (K, V), None
+    if paged:
+        pages = sum((s + 127) // 128 for s in sk) + 3
+        Kc, Vc, table, lens = make_paged_kv(K, V, sk, num_pages=pages, shuffle=True, seed=5)
+        kw = dict(paged=True, max_num_pages=pages, max_num_pages_per_seq=table.shape[1] + 2)
+        kv = (Kc, Vc, table.cuda(), lens.cuda())
+    R = sum((s + 127) // 128 for s in sq)
+    ws = FusedFaOprojArWorkspace.create(None, R + 2, hidden, H, 128, q_per_kv=qpk, max_num_batch=len(sq) + 1,
+                                        max_tot_k=sum(sk) + 64, device="cuda:0", **kw)
+    ws.compile(w_fa=2, w_oproj=1, w_ar=0)
+    layer = FusedPrefillLayer(ws, W)
+    args = [Q.cuda(), kv[0].cuda(), kv[1].cuda(), torch.from_numpy(_cu(sq))]
+    kwargs = dict(page_table=kv[2], cache_seqlens=kv[3]) if paged else dict(cu_seqlens_k=torch.from_numpy(_cu(sk)))
+    return ws, layer, args, kwargs, build_row_desc(sq, seqlens_k=sk), pages
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("paged", [False, True])
+def test_a_step_is_what_the_calls_it_stands_for_are(paged):
+    ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", paged)
+    outs, metas, tables = [], [], []
+    for native in (True, False, True):
+        ws.can_step, saved = (ws.can_step if native else lambda *t: False), ws.can_step
+        ws.csym.zero_()
+        ws.meta_dev.zero_()
+        out = layer(*args, **kwargs)
+        ws.check_status()
+        assert out.shape[0] == want.num_row_tiles and isinstance(layer.meta, StepMeta) == native
+        outs.append((layer.output().clone(), ws.csym.clone()))
+        tables.append(ws.meta_dev.clone())
+        metas.append(layer.meta)
+        ws.can_step = saved
+    for o, m, t in zip(outs, metas, tables):
+        assert torch.equal(o[0], outs[0][0]) and torch.equal(o[1], outs[0][1]) and torch.equal(t, tables[0])
+        _same_schedule(m, want)
+    # calls that are not for it: another current stream, a page table with columns apart
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        assert not ws.can_step()
+        layer(*args, **kwargs)
+    s.synchronize()
+    ws.check_status()
+    assert torch.equal(layer.output(), outs[0][0])
+    if paged:
+        t = kwargs["page_table"]
+        apart = t.t().contiguous().t()
+        wide = torch.full((t.shape[0], t.shape[1] + 5), -9, dtype=torch.int32, device="cuda")
+        wide[:, 3:3 + t.shape[1]] = t
+        for table, native in ((apart, t.shape[0] == 1 or t.shape[1] == 1), (wide[:, 3:3 + t.shape[1]], True)):
+            layer(*args, page_table=table, cache_seqlens=kwargs["cache_seqlens"])
+            ws.check_status()
+            assert isinstance(layer.meta, StepMeta) == native and torch.equal(layer.output(), outs[0][0])
+
+
+@pytest.mark.gpu
+def test_refusals_leave_the_last_step_in_place():
+    ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", True)
+    layer(*args, **kwargs)
+    ws.check_status()
+    ref = layer.output().clone()
+    table, lens = kwargs["page_table"], kwargs["cache_seqlens"]
+    ws.csym.zero_()
+    bad = []
+    for page in (-1, pages):
+        for at in ((0, 0), (-1, -1)):
+            t = table.clone()
+            t[at] = page
+            bad.append((t, lens))
+    for n in (0, -4, int(args[3][1]) - 1, table.shape[1] * 128 + 1):
+        x = lens.clone()
+        x[0] = n
+        bad.append((table, x))
+    for t, x in bad:
+        with pytest.raises(AssertionError):
+            layer(*args, page_table=t, cache_seqlens=x)
+    q = args[0]
+    for other in ([q[:-1], *args[1:]], [q.float(), *args[1:]], [q, args[1].cpu(), *args[2:]],
+                  [q, args[1][:, :, :, :64], *args[2:]]):
+        with pytest.raises(AssertionError):
+            layer(*other, **kwargs)
+    torch.cuda.synchronize()
+    assert not bool(ws.csym.any())                       # nothing was launched
+    ws.page_table[:table.shape[0], :table.shape[1]].copy_(table)
+    ws.cache_seqlens[:lens.shape[0]].copy_(lens)
+    ws.launch()                                          # the plan still has the first step's inputs
+    ws.check_status()
+    assert torch.equal(ws.output(), ref)
+    layer(*args, **kwargs)
+    ws.check_status()
+    assert torch.equal(layer.output(), ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [1, 300, 2000, 40000])       # one block, a few, all of them
+def test_a_table_of_any_width_is_copied_and_looked_through(width):
+    ws, layer, args, kwargs, want, pages = _layer("chunk_gqa_q4", True)
+    table, lens = kwargs["page_table"], kwargs["cache_seqlens"]
+    more = torch.randint(0, pages, (table.shape[0], width), dtype=torch.int32, device="cuda")
+    table = torch.cat((table, more), 1)
+    _, H, hidden, qpk, _, _ = CASES["chunk_gqa_q4"]
+    ws = FusedFaOprojArWorkspace.create(None, want.num_row_tiles, hidden, H, 128, q_per_kv=qpk, paged=True,
+                                        max_num_pages=pages, max_num_pages_per_seq=table.shape[1] + 1,
+                                        max_num_batch=want.num_batch, device="cuda:0").compile()
+    big = FusedPrefillLayer(ws, layer.W_o)
+    layer(*args, **kwargs)
+    big(*args, page_table=table, cache_seqlens=lens)
+    ws.check_status()
+    assert isinstance(big.meta, StepMeta) and torch.equal(big.output(), layer.output())
+    assert torch.equal(ws.page_table[:, :table.shape[1]], table) and not ws.page_table[:, table.shape[1]:].any()
+    for at in ((0, 0), (table.shape[0] - 1, table.shape[1] - 1), (0, table.shape[1] // 2)):
+        t = table.clone()
+        t[at] = pages
+        with pytest.raises(AssertionError):
+            big(*args, page_table=t, cache_seqlens=lens)
