@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "../../include/megaattn_b200.h"
+#include "launch.cuh"
 
 namespace ma {
 namespace {
@@ -25,8 +26,11 @@ struct DetileSeqs {
 
 template <typename T>
 __global__ void __launch_bounds__(kDtThreads)
-detile_kernel(const char* __restrict__ csym, char* __restrict__ out, size_t src_pitch,
+detile_kernel(const char* csym_, char* out_, size_t src_pitch,
               size_t dst_pitch, int n_vec, const __grid_constant__ DetileSeqs s) {
+  wait_for_previous();
+  const char* __restrict__ csym = from_here(csym_);
+  char* __restrict__ out = from_here(out_);
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (kDtThreads / 32);
   for (int row = s.row0[0] + blockIdx.x * (kDtThreads / 32) + (threadIdx.x >> 5);
@@ -74,8 +78,9 @@ extern "C" int ma_detile(const ma_detile_args* a, void* stream) {
   const char* src = reinterpret_cast<const char*>(a->csym);
   char* dst = reinterpret_cast<char*>(a->out);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaSuccess;
   long long tiles = 0;
-  for (int b0 = 0; b0 < a->num_batch; b0 += ma::kDtSeqs) {
+  for (int b0 = 0; b0 < a->num_batch && e == cudaSuccess; b0 += ma::kDtSeqs) {
     ma::DetileSeqs s;
     s.n = a->num_batch - b0 < ma::kDtSeqs ? a->num_batch - b0 : ma::kDtSeqs;
     for (int i = 0; i < s.n; ++i) {
@@ -90,11 +95,14 @@ extern "C" int ma_detile(const ma_detile_args* a, void* stream) {
     const int need = (rows + 7) / 8;
     const int grid = need < sms * 8 ? need : sms * 8;
     if (width == 16)
-      ma::detile_kernel<uint4><<<grid, ma::kDtThreads, 0, st>>>(src, dst, src_pitch, dst_pitch, n_vec, s);
+      e = ma::launch_behind(ma::detile_kernel<uint4>, grid, ma::kDtThreads, 0, st, src, dst, src_pitch, dst_pitch,
+                            n_vec, s);
     else if (width == 4)
-      ma::detile_kernel<uint32_t><<<grid, ma::kDtThreads, 0, st>>>(src, dst, src_pitch, dst_pitch, n_vec, s);
+      e = ma::launch_behind(ma::detile_kernel<uint32_t>, grid, ma::kDtThreads, 0, st, src, dst, src_pitch, dst_pitch,
+                            n_vec, s);
     else
-      ma::detile_kernel<uint16_t><<<grid, ma::kDtThreads, 0, st>>>(src, dst, src_pitch, dst_pitch, n_vec, s);
+      e = ma::launch_behind(ma::detile_kernel<uint16_t>, grid, ma::kDtThreads, 0, st, src, dst, src_pitch, dst_pitch,
+                            n_vec, s);
   }
-  return cudaGetLastError() == cudaSuccess ? MA_OK : MA_ERR_CUDA;
+  return e == cudaSuccess ? MA_OK : MA_ERR_CUDA;
 }

@@ -35,6 +35,7 @@
 #include <stdint.h>
 
 #include "kparams.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace ma {
@@ -682,8 +683,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     tma_prefetch_desc(&tmO); tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmC);
     tma_prefetch_desc(&tmW2);
   }
-  // The scheduler's first trip to L2 runs under the set-up: whether an earlier launch gave up, the
-  // counts, and its first attention task, which is there for the taking (nothing else can be ready).
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&s_tmem), 512);
+    tmem_relinquish();
+  }
+  wait_for_previous();        // (what is above touches nothing of the kernels before this one)
+  // The scheduler's first trip to L2: whether an earlier launch gave up, the counts, and its first
+  // attention task, which is there for the taking (nothing else can be ready).
   const bool has_fa = !(p.flags & (8u | 32u));
   const int* tasks = (p.flags & 4u) ? nullptr : p.tasks;
   uint32_t status0 = 0, first_fa = 0;
@@ -693,10 +699,6 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     num_fa = p.actv[0]; total_op = p.actv[1]; n_tiles = p.actv[2]; local_owned = p.actv[5];
     if (tasks) n_pos = tasks[0];
     if (has_fa) first_fa = atom_add_relaxed_gpu(p.ctrl + C_FA_COUNTER, 1u);
-  }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(&s_tmem), 512);
-    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
@@ -841,7 +843,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
           arg = -1;
           if (fa_left && (first || role == 0)) {
             // An attention task where that is what the CTA asks for first: one atomic, and whether
-            // somebody gave up comes with it.  (The first was taken under the set-up.  A launch after
+            // somebody gave up comes with it.  (The first was taken before the set-up's barrier.  A launch after
             // one that gave up does nothing until the state has been cleared.)
             const uint32_t status = first ? status0 : ld_relaxed_gpu(p.status);
             if (status == 0u) {
@@ -1574,9 +1576,8 @@ cudaError_t launch_fused_prefill(const CUtensorMap* maps, const KParams& kp, int
     if (err != cudaSuccess) return err;
     attr_set[dev] = true;
   }
-  fused_prefill_kernel<<<num_ctas, kThreads, kSmemDynamic, stream>>>(maps[0], maps[1], maps[2],
-                                                                     maps[3], maps[4], maps[5], maps[6], kp);
-  return cudaGetLastError();
+  return launch_behind(fused_prefill_kernel, num_ctas, kThreads, kSmemDynamic, stream, maps[0], maps[1], maps[2],
+                       maps[3], maps[4], maps[5], maps[6], kp);
 }
 
 cudaError_t fused_prefill_attributes(cudaFuncAttributes* out) {

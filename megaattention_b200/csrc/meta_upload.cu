@@ -15,6 +15,7 @@
 
 #include "../../include/megaattn_b200.h"
 #include "kparams.h"
+#include "launch.cuh"
 
 namespace ma {
 namespace {
@@ -31,6 +32,8 @@ struct Words {
 
 template <int N>
 __global__ void __launch_bounds__(kUpThreads) upload_kernel(int32_t* dst, const __grid_constant__ Words<N> s) {
+  let_next_start();
+  wait_for_previous();       // (it may be reading the arrays)
   for (int i = threadIdx.x; i < s.part_end[kParts - 1]; i += kUpThreads) {
     int k = 0;
 #pragma unroll
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(kUpThreads) upload_kernel(int32_t* dst, const 
 }
 
 template <int N>
-void upload(int32_t* dst, const int32_t* src, const int (&off)[kParts], const int (&len)[kParts], int from, int to,
+cudaError_t upload(int32_t* dst, const int32_t* src, const int (&off)[kParts], const int (&len)[kParts], int from, int to,
             cudaStream_t stream) {
   Words<N> s;
   int at = 0, seen = 0;
@@ -52,7 +55,7 @@ void upload(int32_t* dst, const int32_t* src, const int (&off)[kParts], const in
     s.part_end[k] = at;
     seen += len[k];
   }
-  upload_kernel<N><<<1, kUpThreads, 0, stream>>>(dst, s);
+  return launch_behind(upload_kernel<N>, 1, kUpThreads, 0, stream, dst, s);
 }
 
 }  // namespace
@@ -73,11 +76,12 @@ extern "C" int ma_upload_meta(const ma_stage_tasks_args* a, uint64_t meta_dev, v
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // (a launch copies all of its parameter block, so there is one for small steps)
   constexpr int kSmall = 960, kLarge = 7680;
+  cudaError_t e = cudaSuccess;
   if (total <= kSmall) {
-    ma::upload<kSmall>(dst, m.staging, off, len, 0, total, st);
+    e = ma::upload<kSmall>(dst, m.staging, off, len, 0, total, st);
   } else {
-    for (int from = 0; from < total; from += kLarge)
-      ma::upload<kLarge>(dst, m.staging, off, len, from, std::min(total, from + kLarge), st);
+    for (int from = 0; from < total && e == cudaSuccess; from += kLarge)
+      e = ma::upload<kLarge>(dst, m.staging, off, len, from, std::min(total, from + kLarge), st);
   }
-  return cudaGetLastError() == cudaSuccess ? rc : MA_ERR_CUDA;
+  return e == cudaSuccess ? rc : MA_ERR_CUDA;
 }

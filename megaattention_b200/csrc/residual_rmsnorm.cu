@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "../../include/megaattn_b200.h"
+#include "launch.cuh"
 
 namespace ma {
 namespace {
@@ -41,12 +42,17 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
 // 256 threads with eight: the latter needs 126 registers for the row and weight values.
 template <int NCH, int T>
 __global__ void __launch_bounds__(T, 1024 / T)
-residual_rmsnorm_kernel(const uint16_t* __restrict__ csym, const uint16_t* res_in,
-                        const uint16_t* __restrict__ weight, uint16_t* res_out,
-                        uint16_t* __restrict__ normed, const int* __restrict__ cu_q,
-                        const int* __restrict__ fa_b, const int* __restrict__ fa_mb,
-                        int num_row_tiles, int hidden, int row_pitch, float eps) {
+residual_rmsnorm_kernel(const uint16_t* csym_, const uint16_t* res_in, const uint16_t* weight_,
+                        uint16_t* res_out, uint16_t* normed_, const int* cu_q_, const int* fa_b_,
+                        const int* fa_mb_, int num_row_tiles, int hidden, int row_pitch, float eps) {
   __shared__ float s_part[2][T / 32];
+  wait_for_previous();
+  const uint16_t* __restrict__ csym = from_here(csym_);
+  const uint16_t* __restrict__ weight = from_here(weight_);
+  uint16_t* __restrict__ normed = from_here(normed_);
+  const int* __restrict__ cu_q = from_here(cu_q_);
+  const int* __restrict__ fa_b = from_here(fa_b_);
+  const int* __restrict__ fa_mb = from_here(fa_mb_);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nchunk = hidden >> 3;
   uint4 w[NCH];
@@ -139,8 +145,9 @@ extern "C" int ma_residual_rmsnorm(const ma_rmsnorm_args* a, void* stream) {
   const int per_sm = 1024 / threads;
   const int grid = rows < sms * per_sm ? rows : sms * per_sm;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e;
 #define MA_RN_LAUNCH(N, T)                                                                       \
-  ma::residual_rmsnorm_kernel<N, T><<<grid, T, 0, st>>>(                                        \
+  e = ma::launch_behind(ma::residual_rmsnorm_kernel<N, T>, grid, T, 0, st,                       \
       reinterpret_cast<const uint16_t*>(a->csym), reinterpret_cast<const uint16_t*>(a->residual_in), \
       reinterpret_cast<const uint16_t*>(a->weight), reinterpret_cast<uint16_t*>(a->residual_out),   \
       reinterpret_cast<uint16_t*>(a->normed_out), reinterpret_cast<const int*>(a->cu_q),           \
@@ -151,5 +158,5 @@ extern "C" int ma_residual_rmsnorm(const ma_rmsnorm_args* a, void* stream) {
   else if (nch <= 2) MA_RN_LAUNCH(2, 256);
   else MA_RN_LAUNCH(4, 256);
 #undef MA_RN_LAUNCH
-  return cudaGetLastError() == cudaSuccess ? MA_OK : MA_ERR_CUDA;
+  return e == cudaSuccess ? MA_OK : MA_ERR_CUDA;
 }

@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "../../include/megaattn_b200.h"
+#include "launch.cuh"
 
 namespace ma {
 namespace {
@@ -34,10 +35,14 @@ __device__ __forceinline__ uint32_t rb_pack(float lo, float hi) {
 }
 
 __global__ void __launch_bounds__(kRopeThreads)
-rope_kernel(uint16_t* q, uint16_t* k, const int* __restrict__ cu_q, const int* __restrict__ cu_k,
-            const int* __restrict__ tok_b, const float* __restrict__ inv_freq, int tot_q, int H,
-            int Hkv) {
+rope_kernel(uint16_t* q, uint16_t* k, const int* cu_q_, const int* cu_k_, const int* tok_b_,
+            const float* inv_freq_, int tot_q, int H, int Hkv) {
   __shared__ float s_cos[64], s_sin[64];
+  wait_for_previous();
+  const int* __restrict__ cu_q = from_here(cu_q_);
+  const int* __restrict__ cu_k = from_here(cu_k_);
+  const int* __restrict__ tok_b = from_here(tok_b_);
+  const float* __restrict__ inv_freq = from_here(inv_freq_);
   const int tid = threadIdx.x;
   for (int tok = blockIdx.x; tok < tot_q; tok += gridDim.x) {
     const int b = tok_b[tok];
@@ -94,10 +99,11 @@ extern "C" int ma_rope_qk(const ma_rope_args* a, void* stream) {
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return MA_ERR_CUDA;
   const int grid = a->tot_q < sms * 8 ? a->tot_q : sms * 8;
-  ma::rope_kernel<<<grid, ma::kRopeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  const cudaError_t e = ma::launch_behind(
+      ma::rope_kernel, grid, ma::kRopeThreads, 0, static_cast<cudaStream_t>(stream),
       reinterpret_cast<uint16_t*>(a->q), reinterpret_cast<uint16_t*>(a->k),
       reinterpret_cast<const int*>(a->cu_q), reinterpret_cast<const int*>(a->cu_k),
       reinterpret_cast<const int*>(a->token_batch), reinterpret_cast<const float*>(a->inv_freq),
       a->tot_q, a->H_local, a->H_kv);
-  return cudaGetLastError() == cudaSuccess ? MA_OK : MA_ERR_CUDA;
+  return e == cudaSuccess ? MA_OK : MA_ERR_CUDA;
 }

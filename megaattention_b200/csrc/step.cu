@@ -16,6 +16,7 @@
 
 #include "../../include/megaattn_b200.h"
 #include "kparams.h"
+#include "launch.cuh"
 
 namespace ma {
 int plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
@@ -31,6 +32,7 @@ __global__ void __launch_bounds__(kCollectThreads) collect_kernel(
     const int32_t* lens, const int32_t* table, int32_t num_batch, int32_t width, int64_t pitch, int32_t* lens_out,
     int32_t* table_out, int32_t pitch_out, int32_t* host) {
   __shared__ int32_t lo_s[kCollectThreads / 32], hi_s[kCollectThreads / 32];
+  wait_for_previous();
   const int first = blockIdx.x * kCollectThreads + threadIdx.x, step = gridDim.x * kCollectThreads;
   for (int b = first; b < num_batch; b += step) {
     const int32_t n = lens[b];
@@ -72,11 +74,13 @@ extern "C" int ma_step(ma_plan* plan, const ma_step_args* a, void* stream_) {
   if (paged) {
     const int64_t total = static_cast<int64_t>(B) * a->table_width;
     blocks = static_cast<int>(std::min<int64_t>((total + 2047) / 2048, MA_STEP_BLOCKS));
-    ma::collect_kernel<<<blocks, ma::kCollectThreads, 0, stream>>>(
-        reinterpret_cast<const int32_t*>(a->cache_seqlens), reinterpret_cast<const int32_t*>(a->page_table), B,
-        a->table_width, a->table_pitch, reinterpret_cast<int32_t*>(a->cache_seqlens_out),
-        reinterpret_cast<int32_t*>(a->page_table_out), a->table_pitch_out, a->host_words);
-    if (cudaGetLastError() != cudaSuccess) return MA_ERR_CUDA;
+    if (ma::launch_behind(ma::collect_kernel, blocks, ma::kCollectThreads, 0, stream,
+                          reinterpret_cast<const int32_t*>(a->cache_seqlens),
+                          reinterpret_cast<const int32_t*>(a->page_table), B, a->table_width, a->table_pitch,
+                          reinterpret_cast<int32_t*>(a->cache_seqlens_out),
+                          reinterpret_cast<int32_t*>(a->page_table_out), a->table_pitch_out,
+                          a->host_words) != cudaSuccess)
+      return MA_ERR_CUDA;
   }
   CUtensorMap fresh[7];
   int rc = ma::plan_encode_inputs(plan, fresh, a->Q, a->K, a->V, a->W_o, a->tot_q, a->tot_k, a->w_width);
