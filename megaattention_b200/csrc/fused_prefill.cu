@@ -21,7 +21,7 @@
 //                    and frees TMEM
 //   warp 2 (lane 0)  scheduler: claims tasks, fills one of two descriptor slots, publishes
 //                    completions (runs one task ahead of the workers)
-//   warp 3           nothing (the warpgroup's share of the registers goes with its four warps)
+//   warp 3 (lane 0)  stores the attention output tiles
 //   warps 4-7, 8-11  two compute warpgroups: online softmax (one thread per row), both
 //                    epilogues, AllReduce slots
 // An FA task is two q heads of one row tile whenever the rank has two: the two compute
@@ -61,15 +61,16 @@ constexpr float kRescaleThreshold = 8.0f;  // in log2 units
 
 struct Bars {
   uint64_t task_full[2];    // scheduler -> roles: descriptor k is valid        (count 1)
-  uint64_t task_empty[2];   // roles -> scheduler: task in slot k is finished   (count 10)
+  uint64_t task_empty[2];   // roles -> scheduler: task in slot k is finished   (count 11)
   uint64_t loads_done[2];   // producer: every load of the task in slot k is issued (count 1)
   uint64_t q_full[2];       // TMA: Q tile i landed
-  uint64_t q_empty[2];      // MMA: last Q K^T of tile i done (count 1)
+  uint64_t q_empty[2];      // MMA: last Q K^T of tile i done + epilogue: staging released (count 2)
   uint64_t kv_full[kKvSlots];
   uint64_t kv_empty[kKvSlots];   // MMA: the last product that reads the slot completed (count 1)
   uint64_t s_full[2];       // MMA: S_i ready
   uint64_t p_part[2];       // softmax warps: key columns 0-95 of P_i written (count 4)
   uint64_t p_full[2];       // softmax warps: P_i written (count 4, one arrival per warp)
+  uint64_t o_staged[2];     // epilogue warps: O_i staged in shared memory (count 4)
   uint64_t o_done[2];       // MMA: last P V of the task for tile i completed
   uint64_t o_free[2];       // epilogue warps: O_i read out (count 4)
   uint64_t op_full[4];
@@ -404,21 +405,23 @@ __device__ __forceinline__ void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint3
            (acc || kk > 0) ? 1u : 0u);
 }
 
-// 32 fp32 values times `scale`, as bf16, to columns col0.. of this thread's row of an attention output
-// tile in O_scratch.  Straight from registers, in stores of 32 bytes - a row is 256 bytes, a sector 32 -
-// so that the tile needs no staging: staged in its Q buffer and stored from there, the next task's Q
-// could be loaded only then, and between two tasks of a CTA its tensor pipe stood for 4 us (13400
-// tokens behind three times as many cached keys 924 us, 900 so; one prompt of 16384 tokens 575 and
-// 560; six ragged prompts the same 239).
-__device__ __forceinline__ void store_o32(uint16_t* o_row, int col0, const uint32_t (&v)[32], float scale) {
-  uint32_t w[16];
+// Convert N fp32 values (columns col0..col0+N-1 of this thread's row, N and col0 multiples of 8) to
+// bf16 and put them into a [128 rows][64 columns] staging panel laid out as TMA expects
+// for a 128-byte-swizzled box: 16-byte chunk c of row r lives at chunk c ^ (r & 7).
+template <int N>
+__device__ __forceinline__ void stage_row(uint32_t panel, int row, int col0,
+                                          const uint32_t (&v)[N], float scale) {
+  const uint32_t rbase = panel + static_cast<uint32_t>(row) * 128u;
+  const uint32_t sw = static_cast<uint32_t>(row & 7);
 #pragma unroll
-  for (int q = 0; q < 16; ++q)
-    w[q] = pack_bf16x2(__uint_as_float(v[2 * q]) * scale, __uint_as_float(v[2 * q + 1]) * scale);
-  st_global_row64(o_row + col0, w);
-}
-__device__ __forceinline__ uint16_t* o_row_of(const KParams& p, int ft, int head, int row) {
-  return p.o_scratch + (static_cast<size_t>(ft * 128 + row) * p.H + head) * 128;
+  for (int q = 0; q < N / 8; ++q) {
+    const uint32_t c = static_cast<uint32_t>((col0 >> 3) + q);
+    st_shared_v4(rbase + ((c ^ sw) << 4),
+                 pack_bf16x2(__uint_as_float(v[8 * q + 0]) * scale, __uint_as_float(v[8 * q + 1]) * scale),
+                 pack_bf16x2(__uint_as_float(v[8 * q + 2]) * scale, __uint_as_float(v[8 * q + 3]) * scale),
+                 pack_bf16x2(__uint_as_float(v[8 * q + 4]) * scale, __uint_as_float(v[8 * q + 5]) * scale),
+                 pack_bf16x2(__uint_as_float(v[8 * q + 6]) * scale, __uint_as_float(v[8 * q + 7]) * scale));
+  }
 }
 
 // A whole panel row already in bf16.
@@ -537,14 +540,14 @@ enum : int { T_MODE = 0, T_FT = 1,
 
 // End of a head's attention over a part of its keys.  The part's O (not divided), reference maximum
 // and row sum go to memory in fp32; whichever part of the head is there last adds them all up and
-// stores the head's output - nobody waits for anybody.  Its own O it has in TMEM, but it adds in the
+// stages the head's output - nobody waits for anybody.  Its own O it has in TMEM, but it adds in the
 // parts' order, so that the result does not depend on who was last.
 // What it costs is trips to L2: 4.5 us to put a part of 64 KB there and look, 2.5 us for each part
 // that is read.  A thread's row of it lies strided ([column / 4][row] of float4: a warp's accesses are
 // 512 bytes in a row).  More than 32 columns of one part in flight would take the registers that the
 // attention loop lives on (two parts': the kernel's spills 240 -> 1000 bytes, every task slower).
 __device__ __noinline__ void finish_part(const KParams& p, int* d, int wg, int row, uint32_t t_o,
-                                         uint32_t bar_o_free, float m, float l) {
+                                         uint32_t stg, uint32_t bar_o_free, float m, float l) {
   const int n = d[TF_PARTS], own = d[TF_PART], head = d[TF_HEAD0] + wg, first = d[TF_SLOT];
   const size_t pitch = static_cast<size_t>(p.H) * kPartFloats;      // from one part to the next
   float* base = p.part_o + static_cast<size_t>(first) * pitch + static_cast<size_t>(head) * kPartFloats;
@@ -581,7 +584,6 @@ __device__ __noinline__ void finish_part(const KParams& p, int* d, int wg, int r
       sum += weight(__ldcg(base + i * pitch + kPartMax + row)) * __ldcg(base + i * pitch + kPartSum + row);
     const float inv = (row < d[TF_VALID] && sum > 0.f) ? (1.f / sum) : 0.f;
     const float w_own = weight(m);
-    uint16_t* o_row = o_row_of(p, d[T_FT], head, row);
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
       float acc[32];
@@ -614,7 +616,7 @@ __device__ __noinline__ void finish_part(const KParams& p, int* d, int wg, int r
       uint32_t bits[32];
 #pragma unroll
       for (int q = 0; q < 32; ++q) bits[q] = __float_as_uint(acc[q]);
-      store_o32(o_row, c * 32, bits, inv);
+      stage_row(stg + (c >> 1) * kPanel, row, (c & 1) * 32, bits, inv);
     }
   }
   tc_fence_before();
@@ -653,13 +655,14 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     s_abort = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars.task_full[i]), 1);
-      mbar_init(smem_u32(&bars.task_empty[i]), 10);
+      mbar_init(smem_u32(&bars.task_empty[i]), 11);
       mbar_init(smem_u32(&bars.loads_done[i]), 1);
       mbar_init(smem_u32(&bars.q_full[i]), 1);
-      mbar_init(smem_u32(&bars.q_empty[i]), 1);
+      mbar_init(smem_u32(&bars.q_empty[i]), 2);
       mbar_init(smem_u32(&bars.s_full[i]), 1);
       mbar_init(smem_u32(&bars.p_part[i]), 4);
       mbar_init(smem_u32(&bars.p_full[i]), 4);
+      mbar_init(smem_u32(&bars.o_staged[i]), 4);
       mbar_init(smem_u32(&bars.o_done[i]), 1);
       mbar_init(smem_u32(&bars.o_free[i]), 4);
       mbar_init(smem_u32(&bars.acc_full[i]), 1);
@@ -704,8 +707,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 
   // Every role walks the two descriptor slots in turn.  A role arrives on task_empty[k]
   // when its part of the task in slot k is finished; the scheduler publishes the task's
-  // completion and refills the slot once all ten arrivals are in (producer, MMA issuer,
-  // eight compute warps), so the scheduler runs
+  // completion and refills the slot once all eleven arrivals are in (producer, MMA issuer,
+  // attention store, eight compute warps), so the scheduler runs
   // one task ahead of the workers.  Attention tiles and O_proj tiles overlay the same
   // shared memory and TMEM: a role that goes from one kind to the other first waits for
   // the previous task to finish completely (same-kind neighbours overlap freely).
@@ -1192,6 +1195,32 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         arrived ^= 1u << slot_k;
         prev_mode = mode; prev_k = slot_k; slot_k ^= 1;
       }
+    } else if (warp == 3 && lane == 0) {
+      // ==================================== attention output stores: O_scratch[ft, :, head, :]
+      // (a warp of their own, so that no softmax warp waits for a store to complete)
+      uint32_t st_par = 0;
+      while (true) {
+        MA_NEXT_TASK(d, mode)
+        if (mode == MODE_FA) {
+          const int ft = d[T_FT], head0 = d[TF_HEAD0], nt = d[TF_NT];
+          for (int i = 0; i < nt; ++i) {
+            if (!wait_bar(env, smem_u32(&bars.o_staged[i]), (st_par >> i) & 1u, 0x88 + i)) break;
+            st_par ^= 1u << i;
+            if (d[TF_FIN0 + i]) {       // (else a part of the keys, and not the last)
+              const uint32_t stg = smem0 + kSmQ + i * kTile;
+              tma_store_2d(&tmO, stg, (head0 + i) * 128, ft * 128);
+              tma_store_2d(&tmO, stg + kPanel, (head0 + i) * 128 + 64, ft * 128);
+              tma_store_commit();
+              tma_store_wait_read();
+            }
+            mbar_arrive(smem_u32(&bars.q_empty[i]));     // the producer may refill this Q buffer
+          }
+          tma_store_wait_all();
+          fence_proxy_async_all();     // O_scratch is read back by TMA loads of other CTAs (the
+                                       // scheduler's fence covers them)
+        }
+        MA_TASK_DONE(mode)
+      }
     }
     __syncwarp();
   } else {
@@ -1333,11 +1362,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         wait_bar(env, smem_u32(&bars.o_done[wg]), o_par, 0x80 + wg);
         o_par ^= 1u;
         tc_fence_after();
+        const uint32_t stg = smem0 + kSmQ + wg * kTile;
         if (d[TF_PARTS] > 1) {
-          finish_part(p, s_desc[slot_k], wg, row, t_o, smem_u32(&bars.o_free[wg]), m_ref, l_run);
+          finish_part(p, s_desc[slot_k], wg, row, t_o, stg, smem_u32(&bars.o_free[wg]), m_ref, l_run);
         } else {
           const float inv = (row < valid_m && l_run > 0.f) ? (1.f / l_run) : 0.f;
-          uint16_t* o_row = o_row_of(p, d[T_FT], d[TF_HEAD0] + wg, row);
+          // O / l -> bf16 -> this tile's Q buffer (free: every Q K^T of the task is done),
+          // then two TMA stores of 128 rows x 64 columns into O_scratch[ft, :, head, :].
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
             uint32_t o[2][32];
@@ -1349,13 +1380,13 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
               __syncwarp();
               if (lane == 0) mbar_arrive(smem_u32(&bars.o_free[wg]));
             }
-            store_o32(o_row, hh * 64, o[0], inv);
-            store_o32(o_row, hh * 64 + 32, o[1], inv);
+            stage_row(stg + hh * kPanel, row, 0, o[0], inv);
+            stage_row(stg + hh * kPanel, row, 32, o[1], inv);
           }
         }
-        // (read back by TMA loads of other CTAs: the scheduler's fence and the producer's proxy fence
-        // there lie between)
-        fence_proxy_async_global();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars.o_staged[wg]));   // warp 3 stores the tile
       } else if (mode == MODE_OPROJ) {
         const int ft0 = d[T_FT], base_out = d[TO_BASE], vnt = d[TO_VNT], nrt = d[TO_NRT];
         const bool leader = ((warp & 3) == 0 && lane == 0);
@@ -1523,7 +1554,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       for (int it = 0; it < (1 << 20); ++it)
         if (mbar_try_wait(bar, 0)) break;
     }
-    if ((warp == 4 || warp == 8) && lane == 0) tma_store_wait_all();
+    if ((warp == 3 || warp == 4 || warp == 8) && lane == 0) tma_store_wait_all();
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 100000ull) {}
   }

@@ -308,21 +308,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 
 // ------------------------------------------------------------------ scoped atomics / loads
-// 64 contiguous bytes, in 32-byte stores where the address allows (16-byte aligned otherwise)
-__device__ __forceinline__ void st_global_row64(void* dst, const uint32_t (&v)[16]) {
-  if ((reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                   ::"l"(static_cast<char*>(dst) + 32 * q), "r"(v[8 * q]), "r"(v[8 * q + 1]), "r"(v[8 * q + 2]),
-                     "r"(v[8 * q + 3]), "r"(v[8 * q + 4]), "r"(v[8 * q + 5]), "r"(v[8 * q + 6]), "r"(v[8 * q + 7])
-                   : "memory");
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      reinterpret_cast<uint4*>(dst)[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-  }
-}
 __device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

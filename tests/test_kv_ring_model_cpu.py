@@ -1,6 +1,6 @@
 """Host model of the attention pipeline's bookkeeping (megaattention_b200/csrc/fused_prefill.cu):
-the TMA producer, the one MMA issuer of both tiles and the two softmax warpgroups, which store
-their outputs themselves, on mbarriers with phases and parities as the hardware has them, in both stage layouts of
+the TMA producer, the one MMA issuer of both tiles, the two softmax warpgroups and the store
+warp, on mbarriers with phases and parities as the hardware has them, in both stage layouts of
 the K/V ring: shared stages (the heads of a task share a kv head: one K and one V tile per key
 block) and separate stages (per key block the K tiles of the task's heads, then their V tiles).
 
@@ -37,11 +37,11 @@ class Model:
         self.tasks, self.sep, self.n, self.rng, self.late_k = tasks, sep, kv_slots, rng, late_k
         n = kv_slots
         self.kv_full, self.kv_empty = [Bar(1) for _ in range(n)], [Bar(1) for _ in range(n)]
-        self.q_full, self.q_empty = [Bar(1) for _ in range(2)], [Bar(1) for _ in range(2)]
-        self.s_full, self.p_full, self.o_done, self.o_free = (
-            [Bar(1) for _ in range(2)] for _ in range(4))
+        self.q_full, self.q_empty = [Bar(1) for _ in range(2)], [Bar(2) for _ in range(2)]
+        self.s_full, self.p_full, self.o_staged, self.o_done, self.o_free = (
+            [Bar(1) for _ in range(2)] for _ in range(5))
         self.kv, self.q = [None] * n, [None] * 2       # what the buffers hold
-        self.readers, self.q_readers = [0] * n, [0] * 2    # MMAs issued on a buffer, not yet run
+        self.readers = [0] * n                         # MMAs issued on a slot, not yet run
         self.loads, self.pipe = [], []                 # in flight
         self.released, self.stored, self.ran = [], [], set()
 
@@ -62,7 +62,6 @@ class Model:
             self.kv[i] = tile
             self.kv_full[i].arrive()
         else:
-            assert self.q_readers[i] == 0, "a load into a Q buffer that an MMA still reads"
             self.q[i] = tile
             self.q_full[i].arrive()
 
@@ -73,15 +72,12 @@ class Model:
         else:
             _, slot, kv_tile, i, q_tile = op
             assert self.kv[slot] == kv_tile, (self.kv[slot], kv_tile)
-            if q_tile is not None:
-                assert self.q[i] == q_tile
-                self.q_readers[i] -= 1
+            assert q_tile is None or self.q[i] == q_tile
             self.readers[slot] -= 1
             self.ran.add(kv_tile)
 
     def mma(self, slot, kv_tile, i=0, q_tile=None):
         self.readers[slot] += 1
-        self.q_readers[i] += q_tile is not None
         self.pipe.append(("mma", slot, kv_tile, i, q_tile))
 
     def commit(self, bar):
@@ -187,7 +183,7 @@ class Model:
 
     def softmax(self, i):
         s_par = o_par = 0
-        for t, (nt, nblk) in enumerate(self.tasks):
+        for nt, nblk in self.tasks:
             if i >= nt:
                 continue
             for _ in range(nblk):
@@ -197,11 +193,22 @@ class Model:
             yield self.o_done[i], o_par
             o_par ^= 1
             self.o_free[i].arrive()
-            self.stored.append((t, i))
+            self.q[i] = "staged O"
+            self.o_staged[i].arrive()
+
+    def store(self):
+        par = [0, 0]
+        for t, (nt, _) in enumerate(self.tasks):
+            for i in range(nt):
+                yield self.o_staged[i], par[i]
+                par[i] ^= 1
+                assert self.q[i] == "staged O"
+                self.stored.append((t, i))
+                self.q_empty[i].arrive()
 
     # -------------------------------------------------------------- any interleaving
     def run(self):
-        roles = [self.producer(), self.issuer(), self.softmax(0), self.softmax(1)]
+        roles = [self.producer(), self.issuer(), self.softmax(0), self.softmax(1), self.store()]
         waits = {}
         for r in roles:
             waits[r] = next(r, None)
@@ -216,7 +223,7 @@ class Model:
             else:
                 pick()
         assert all(w is None for w in waits.values()), "the pipeline stopped"
-        assert sorted(self.stored) == [(t, i) for t, (nt, _) in enumerate(self.tasks) for i in range(nt)]
+        assert self.stored == [(t, i) for t, (nt, _) in enumerate(self.tasks) for i in range(nt)]
         tiles = [(t, jj, which, h) for t, (nt, nblk) in enumerate(self.tasks) for jj in range(nblk)
                  for which in (0, 1) for h in (range(nt) if self.sep else [None])]
         assert sorted(self.released, key=str) == sorted(tiles, key=str)      # each slot, once
