@@ -377,12 +377,14 @@ int ma_upload_meta(const ma_stage_tasks_args* args, uint64_t meta_dev, void* str
  * arrays, num_batch and num_row_tiles are filled in by the call.  cu_q, cu_k: host, num_batch + 1
  * words from 0 (cu_k NULL: the same as cu_q).
  * With page_table set (device, i32 [num_batch][table_pitch], table_width columns of it) the key
- * lengths are cache_seqlens's (device, i32 [num_batch]): a kernel copies both to the plan's own
- * (page_table_out with a pitch of table_pitch_out, cache_seqlens_out) and brings the lengths and the
- * range of the page numbers to host_words (pinned, i32 [num_batch + 2 * MA_STEP_BLOCKS]), and the
- * call waits for that - the only wait in it.  tot_k is 128 times the number of pages.
+ * lengths are cache_seqlens's (device, i32 [num_batch]): a kernel brings the lengths and the range
+ * of the page numbers to host_words (pinned, i32 [num_batch + 2 * MA_STEP_BLOCKS]), and the call waits
+ * for that - the only wait in it.  Once the batch is accepted the plan's own (page_table_out with a
+ * pitch of table_pitch_out, cache_seqlens_out) are written with the metadata; the caller's page table
+ * is read for that on `stream`, behind the call's return, and has to stay as it is until then.  tot_k
+ * is 128 times the number of pages.
  * A batch that does not fit is refused after the wait, with nothing else queued and the plan's
- * inputs as they were: MA_STEP_NARROW (a sequence needs more than table_width pages), MA_STEP_PAGES
+ * inputs, page table and lengths as they were: MA_STEP_NARROW (a sequence needs more than table_width pages), MA_STEP_PAGES
  * (a page number outside the cache), MA_STEP_LENGTHS (not 0 < q_len <= k_len), MA_STEP_TILES (more
  * than max_row_tiles).  Otherwise an ma_error code.
  */

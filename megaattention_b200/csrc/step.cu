@@ -4,8 +4,9 @@
 // of Python and torch calls, and a paged call had another 100 us between the arrival of the key lengths
 // and its launch.  Here the descriptors are encoded, the batch's metadata staged and the kernels
 // launched without leaving C.  A paged batch's lengths and the range of its page numbers come back by
-// one kernel, which writes them to pinned memory and brings the plan's copies of both up to date; it
-// runs while the descriptors are encoded, and what is left after it is the metadata and two launches.
+// one kernel, which writes them to pinned memory; it runs while the descriptors are encoded, and what is
+// left after it is the metadata and two launches.  Nothing of the plan changes before the checks are
+// over: its copies of lengths and table are written with the metadata.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -22,6 +23,7 @@ namespace ma {
 int plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
                        int64_t tot_q, int64_t tot_k, int64_t w_width);
 void plan_take_inputs(ma_plan* pl, const CUtensorMap* fresh);
+int upload_meta(const ma_stage_tasks_args* a, uint64_t meta_dev, const PagedIn& paged, cudaStream_t stream);
 
 namespace {
 
@@ -29,22 +31,16 @@ constexpr int kCollectThreads = 256;
 
 // host: num_batch lengths, then {smallest, largest} page number of every block's share of the table.
 __global__ void __launch_bounds__(kCollectThreads) collect_kernel(
-    const int32_t* lens, const int32_t* table, int32_t num_batch, int32_t width, int64_t pitch, int32_t* lens_out,
-    int32_t* table_out, int32_t pitch_out, int32_t* host) {
+    const int32_t* lens, const int32_t* table, int32_t num_batch, int32_t width, int64_t pitch, int32_t* host) {
   __shared__ int32_t lo_s[kCollectThreads / 32], hi_s[kCollectThreads / 32];
   wait_for_previous();
   const int first = blockIdx.x * kCollectThreads + threadIdx.x, step = gridDim.x * kCollectThreads;
-  for (int b = first; b < num_batch; b += step) {
-    const int32_t n = lens[b];
-    lens_out[b] = n;
-    host[b] = n;
-  }
+  for (int b = first; b < num_batch; b += step) host[b] = lens[b];
   int32_t lo = 0x7fffffff, hi = -0x7fffffff - 1;
   const int64_t total = static_cast<int64_t>(num_batch) * width;
   for (int64_t i = first; i < total; i += step) {
     const int b = static_cast<int>(i / width), j = static_cast<int>(i % width);
     const int32_t page = table[b * pitch + j];
-    table_out[static_cast<int64_t>(b) * pitch_out + j] = page;
     lo = min(lo, page);
     hi = max(hi, page);
   }
@@ -77,8 +73,6 @@ extern "C" int ma_step(ma_plan* plan, const ma_step_args* a, void* stream_) {
     if (ma::launch_behind(ma::collect_kernel, blocks, ma::kCollectThreads, 0, stream,
                           reinterpret_cast<const int32_t*>(a->cache_seqlens),
                           reinterpret_cast<const int32_t*>(a->page_table), B, a->table_width, a->table_pitch,
-                          reinterpret_cast<int32_t*>(a->cache_seqlens_out),
-                          reinterpret_cast<int32_t*>(a->page_table_out), a->table_pitch_out,
                           a->host_words) != cudaSuccess)
       return MA_ERR_CUDA;
   }
@@ -121,7 +115,11 @@ extern "C" int ma_step(ma_plan* plan, const ma_step_args* a, void* stream_) {
     s.meta.num_batch = B; s.meta.num_row_tiles = R;
     s.meta.prime = std::min(s.meta.prime, R);
     ma::plan_take_inputs(plan, fresh);
-    rc = ma_upload_meta(&s, a->meta_dev, stream_);
+    ma::PagedIn in{};
+    if (paged)
+      in = {reinterpret_cast<const int*>(a->page_table), a->host_words, reinterpret_cast<int*>(a->page_table_out),
+            reinterpret_cast<int*>(a->cache_seqlens_out), a->table_pitch, a->table_pitch_out, a->table_width, B};
+    rc = ma::upload_meta(&s, a->meta_dev, in, stream);
     if (rc != MA_OK) return rc;
     rc = ma_launch(plan, &a->launch, stream_);
     return rc == MA_OK ? R : rc;

@@ -470,7 +470,7 @@ class FusedFaOprojArWorkspace:
         if rc < 0:
             assert rc not in _cabi.STEP_REFUSED, _cabi.STEP_REFUSED[rc]
             _cabi.check(rc, "ma_step")
-        self._bound = (Q, K, V, W_o)          # keep them alive
+        self._bound = (Q, K, V, W_o, page_table)      # keep them alive
         self._auto_flags = 0
         self._meta = StepMeta(cu_q, self._host_words[:nb] if self.paged else None, cu_k, rc)
         return self._meta

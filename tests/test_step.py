@@ -113,14 +113,9 @@ def test_a_step_is_what_the_calls_it_stands_for_are(paged):
             assert isinstance(layer.meta, StepMeta) == native and torch.equal(layer.output(), outs[0][0])
 
 
-@pytest.mark.gpu
-def test_refusals_leave_the_last_step_in_place():
-    ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", True)
-    layer(*args, **kwargs)
-    ws.check_status()
-    ref = layer.output().clone()
+def _refused(args, kwargs, pages):
+    """Page tables and key lengths that a step has to refuse."""
     table, lens = kwargs["page_table"], kwargs["cache_seqlens"]
-    ws.csym.zero_()
     bad = []
     for page in (-1, pages):
         for at in ((0, 0), (-1, -1)):
@@ -131,9 +126,22 @@ def test_refusals_leave_the_last_step_in_place():
         x = lens.clone()
         x[0] = n
         bad.append((table, x))
-    for t, x in bad:
+    return bad
+
+
+@pytest.mark.gpu
+def test_refusals_leave_the_last_step_in_place():
+    ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", True)
+    layer(*args, **kwargs)
+    ws.check_status()
+    ref = layer.output().clone()
+    ws.csym.zero_()
+    own = (ws.page_table, ws.cache_seqlens, ws.meta_dev)
+    before = [t.clone() for t in own]
+    for t, x in _refused(args, kwargs, pages):
         with pytest.raises(AssertionError):
             layer(*args, page_table=t, cache_seqlens=x)
+        assert all(torch.equal(a, b) for a, b in zip(own, before))
     q = args[0]
     for other in ([q[:-1], *args[1:]], [q.float(), *args[1:]], [q, args[1].cpu(), *args[2:]],
                   [q, args[1][:, :, :, :64], *args[2:]]):
@@ -141,14 +149,34 @@ def test_refusals_leave_the_last_step_in_place():
             layer(*other, **kwargs)
     torch.cuda.synchronize()
     assert not bool(ws.csym.any())                       # nothing was launched
-    ws.page_table[:table.shape[0], :table.shape[1]].copy_(table)
-    ws.cache_seqlens[:lens.shape[0]].copy_(lens)
-    ws.launch()                                          # the plan still has the first step's inputs
+    assert all(torch.equal(a, b) for a, b in zip(own, before))
+    ws.launch()                                          # the plan still has all of the first step
     ws.check_status()
     assert torch.equal(ws.output(), ref)
     layer(*args, **kwargs)
     ws.check_status()
     assert torch.equal(layer.output(), ref)
+
+
+@pytest.mark.gpu
+def test_a_captured_launch_after_refusals():
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", True)
+        layer(*args, **kwargs)
+        ws.check_status()
+        ref = layer.output().clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            ws.launch()
+        for t, x in _refused(args, kwargs, pages):
+            assert ws.can_step(t, x)
+            with pytest.raises(AssertionError):
+                layer(*args, page_table=t, cache_seqlens=x)
+            ws.csym.zero_()
+            graph.replay()
+            ws.check_status()
+            assert torch.equal(ws.output(), ref)
 
 
 @pytest.mark.gpu
