@@ -386,7 +386,8 @@ int ma_upload_meta(const ma_stage_tasks_args* args, uint64_t meta_dev, void* str
  * A batch that does not fit is refused after the wait, with nothing else queued and the plan's
  * inputs, page table and lengths as they were: MA_STEP_NARROW (a sequence needs more than table_width pages), MA_STEP_PAGES
  * (a page number outside the cache), MA_STEP_LENGTHS (not 0 < q_len <= k_len), MA_STEP_TILES (more
- * than max_row_tiles).  Otherwise an ma_error code.
+ * than max_row_tiles).  Otherwise an ma_error code, with the plan's inputs as they were; launch
+ * arguments that ma_launch refuses are refused before anything but that kernel is queued.
  */
 #define MA_STEP_BLOCKS 32
 #define MA_STEP_NARROW (-101)

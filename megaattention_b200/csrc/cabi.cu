@@ -21,6 +21,8 @@ int encode_path_maps(CUtensorMap* maps, uint64_t Q, uint64_t K, uint64_t V, uint
 int plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
                        int64_t tot_q, int64_t tot_k, int64_t w_width);
 void plan_take_inputs(ma_plan* pl, const CUtensorMap* fresh);
+void plan_inputs(const ma_plan* pl, CUtensorMap* maps);
+int plan_check_launch(const ma_plan* pl, const ma_launch_args* a);
 }  // namespace ma
 
 struct ma_plan {
@@ -144,6 +146,29 @@ int ma::plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, ui
 void ma::plan_take_inputs(ma_plan* pl, const CUtensorMap* fresh) {
   pl->maps[0] = fresh[0]; pl->maps[1] = fresh[1]; pl->maps[2] = fresh[2]; pl->maps[4] = fresh[4];
   pl->maps[6] = fresh[6];
+}
+
+void ma::plan_inputs(const ma_plan* pl, CUtensorMap* maps) {
+  for (int i : {0, 1, 2, 4, 6}) maps[i] = pl->maps[i];
+}
+
+// Launch arguments that would send the kernel down a path its buffers do not back are refused
+// here, before anything is launched.
+int ma::plan_check_launch(const ma_plan* pl, const ma_launch_args* a) {
+  const ma::KParams& kp = pl->kp;
+  const uint32_t flags = a->flags;
+  const uint32_t stage = flags & (MA_FLAG_FA_ONLY | MA_FLAG_AR_ONLY | MA_FLAG_NO_AR | MA_FLAG_OPROJ_ONLY);
+  if (stage & (stage - 1u)) return MA_ERR_INVALID;              // at most one stage selector
+  if ((flags & MA_FLAG_AR_ONLY) && (kp.tp < 2 || kp.csym_mc == 0)) return MA_ERR_INVALID;
+  if ((flags & MA_FLAG_OPROJ_ONLY) && kp.tp != 1) return MA_ERR_INVALID;
+  if ((flags & MA_FLAG_AR_P2P) && (kp.tp != 2 || !pl->desc.peer_csym[0] || !pl->desc.peer_csym[1]))
+    return MA_ERR_INVALID;
+  if (flags & ~(MA_FLAG_FA_ONLY | MA_FLAG_DRAIN_FIRST | MA_FLAG_TILE_ORDER | MA_FLAG_AR_ONLY |
+                MA_FLAG_NO_AR | MA_FLAG_OPROJ_ONLY | MA_FLAG_AR_P2P))
+    return MA_ERR_INVALID;
+  const int w_ar = kp.tp > 1 ? a->w_ar : 0;
+  if (a->w_fa < 0 || a->w_oproj < 0 || w_ar < 0 || a->w_fa + a->w_oproj + w_ar < 1) return MA_ERR_INVALID;
+  return MA_OK;
 }
 
 extern "C" {
@@ -286,25 +311,12 @@ int ma_plan_create(const ma_plan_desc* d, ma_plan** out) {
 
 int ma_launch(ma_plan* pl, const ma_launch_args* a, void* stream) {
   if (!pl || !a) return MA_ERR_INVALID;
+  const int rc = ma::plan_check_launch(pl, a);
+  if (rc != MA_OK) return rc;
   ma::KParams kp = pl->kp;
   kp.w_fa = a->w_fa; kp.w_oproj = a->w_oproj;
   kp.w_ar = (kp.tp > 1) ? a->w_ar : 0;          // one rank: no AllReduce role
   kp.flags = a->flags;
-  // Flag combinations that would send the kernel down a path its buffers do not back are
-  // refused here, before anything is launched.
-  const uint32_t stage = kp.flags & (MA_FLAG_FA_ONLY | MA_FLAG_AR_ONLY | MA_FLAG_NO_AR |
-                                     MA_FLAG_OPROJ_ONLY);
-  if (stage & (stage - 1u)) return MA_ERR_INVALID;              // at most one stage selector
-  if ((kp.flags & MA_FLAG_AR_ONLY) && (kp.tp < 2 || kp.csym_mc == 0)) return MA_ERR_INVALID;
-  if ((kp.flags & MA_FLAG_OPROJ_ONLY) && kp.tp != 1) return MA_ERR_INVALID;
-  if ((kp.flags & MA_FLAG_AR_P2P) &&
-      (kp.tp != 2 || !pl->desc.peer_csym[0] || !pl->desc.peer_csym[1]))
-    return MA_ERR_INVALID;
-  if (kp.flags & ~(MA_FLAG_FA_ONLY | MA_FLAG_DRAIN_FIRST | MA_FLAG_TILE_ORDER | MA_FLAG_AR_ONLY |
-                   MA_FLAG_NO_AR | MA_FLAG_OPROJ_ONLY | MA_FLAG_AR_P2P))
-    return MA_ERR_INVALID;
-  if (kp.w_fa < 0 || kp.w_oproj < 0 || kp.w_ar < 0 || kp.w_fa + kp.w_oproj + kp.w_ar < 1)
-    return MA_ERR_INVALID;
   const bool alone = (kp.flags & MA_FLAG_OPROJ_ONLY) != 0;
   kp.op_two_from = alone ? ma::kOpTwoFromAlone : ma::kOpTwoFrom;
   kp.op_cols2_from = alone ? ma::kOpCols2FromAlone : ma::kOpCols2From;

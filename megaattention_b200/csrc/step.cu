@@ -23,6 +23,8 @@ namespace ma {
 int plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
                        int64_t tot_q, int64_t tot_k, int64_t w_width);
 void plan_take_inputs(ma_plan* pl, const CUtensorMap* fresh);
+void plan_inputs(const ma_plan* pl, CUtensorMap* maps);
+int plan_check_launch(const ma_plan* pl, const ma_launch_args* a);
 int upload_meta(const ma_stage_tasks_args* a, uint64_t meta_dev, const PagedIn& paged, cudaStream_t stream);
 
 namespace {
@@ -114,14 +116,20 @@ extern "C" int ma_step(ma_plan* plan, const ma_step_args* a, void* stream_) {
     s.meta.cu_q = cu_q32; s.meta.cu_k = cu_k32; s.meta.batch_idx = batch_idx; s.meta.m_block = m_block;
     s.meta.num_batch = B; s.meta.num_row_tiles = R;
     s.meta.prime = std::min(s.meta.prime, R);
-    ma::plan_take_inputs(plan, fresh);
+    rc = ma::plan_check_launch(plan, &a->launch);
+    if (rc != MA_OK) return rc;
     ma::PagedIn in{};
     if (paged)
       in = {reinterpret_cast<const int*>(a->page_table), a->host_words, reinterpret_cast<int*>(a->page_table_out),
             reinterpret_cast<int*>(a->cache_seqlens_out), a->table_pitch, a->table_pitch_out, a->table_width, B};
     rc = ma::upload_meta(&s, a->meta_dev, in, stream);
     if (rc != MA_OK) return rc;
+    // (a launch that fails leaves the plan with the inputs that its owner knows of)
+    CUtensorMap before[7];
+    ma::plan_inputs(plan, before);
+    ma::plan_take_inputs(plan, fresh);
     rc = ma_launch(plan, &a->launch, stream_);
+    if (rc != MA_OK) ma::plan_take_inputs(plan, before);
     return rc == MA_OK ? R : rc;
   } catch (const std::bad_alloc&) {
     return MA_ERR_CAPACITY;

@@ -159,6 +159,36 @@ def test_refusals_leave_the_last_step_in_place():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("paged", [False, True])
+def test_launch_flags_that_are_refused_leave_the_plans_inputs(paged):
+    """A workspace on its own buffers keeps them, and one that reads a caller's keeps those."""
+    ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", paged)
+    kv = dict(page_table=kwargs["page_table"], cache_seqlens=kwargs["cache_seqlens"]) if paged else {}
+    ws.set_layer(want, *args[:3], layer.W_o, **kv)
+    ws.launch()
+    ws.check_status()
+    ref, before = ws.output().clone(), ws.meta_dev.clone()
+    others = [torch.zeros_like(t) for t in args[:3]] + args[3:]
+    for first in (lambda: None, lambda: layer(*args, **kwargs)):
+        first()
+        bound = getattr(ws, "_bound", None)
+        for flags in (_cabi.MA_FLAG_AR_ONLY, 1 << 20, _cabi.MA_FLAG_FA_ONLY | _cabi.MA_FLAG_OPROJ_ONLY):
+            assert ws.can_step()
+            with pytest.raises(RuntimeError):
+                layer(*others, **kwargs, flags=flags)
+        assert getattr(ws, "_bound", None) is bound and torch.equal(ws.meta_dev, before)
+        ws.csym.zero_()
+        ws.launch()
+        ws.check_status()
+        assert torch.equal(ws.output(), ref)
+        ws.csym.zero_()
+        ws.set_layer(want, *args[:3], layer.W_o, **kv)
+        ws.launch()
+        ws.check_status()
+        assert torch.equal(ws.output(), ref)
+
+
+@pytest.mark.gpu
 def test_a_captured_launch_after_refusals():
     s = torch.cuda.Stream()
     with torch.cuda.stream(s):
