@@ -82,7 +82,7 @@ constexpr int kPartFloats = kPartSum + 128;                      // reference ma
 constexpr int kMaxParts = 16;
 
 // A paged step's page table (device) and key lengths (host, as they were checked) and where the plan
-// has its own copies of them (table null: none).
+// has its own copies of them (lens null: no paged step; table null: lengths only).
 struct PagedIn {
   const int* table;
   const int* lens;

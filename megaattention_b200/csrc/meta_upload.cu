@@ -23,45 +23,60 @@
 namespace ma {
 namespace {
 
-constexpr int kParts = 8;           // the last: key lengths, to the plan's own
+constexpr int kParts = 7, kPagedParts = 8;     // (a paged step's key lengths: to the plan's own)
 constexpr int kUpThreads = 512;
 constexpr int kMaxBlocks = 32;
 
-template <int N>
+template <int N, int P>
 struct Words {
-  int part_end[kParts];     // parts lie one after another in w: where each ends,
-  int part_to[kParts];      // and what is added to a word's place to get where it goes
+  int part_end[P];          // parts lie one after another in w: where each ends,
+  int part_to[P];           // and what is added to a word's place to get where it goes
   int32_t w[N];
 };
 
-template <int N>
-__global__ void __launch_bounds__(kUpThreads)
-upload_kernel(int32_t* dst, const __grid_constant__ Words<N> s, const __grid_constant__ PagedIn paged) {
-  let_next_start();
-  wait_for_previous();       // (it may be reading the arrays)
-  if (paged.table) {
-    const int first = blockIdx.x * kUpThreads + threadIdx.x, step = gridDim.x * kUpThreads;
-    const long long total = static_cast<long long>(paged.num_batch) * paged.width;
-    for (long long i = first; i < total; i += step) {
-      const int b = static_cast<int>(i / paged.width), j = static_cast<int>(i % paged.width);
-      paged.table_out[static_cast<long long>(b) * paged.pitch_out + j] = paged.table[b * paged.pitch + j];
-    }
-  }
-  if (blockIdx.x != 0) return;
-  for (int i = threadIdx.x; i < s.part_end[kParts - 1]; i += kUpThreads) {
+// One block's job; the page table's copy has as many as its size asks for.
+template <int N, int P>
+__device__ __forceinline__ void put_words(int32_t* dst, int32_t* lens_out, const Words<N, P>& s) {
+  for (int i = threadIdx.x; i < s.part_end[P - 1]; i += kUpThreads) {
     int k = 0;
 #pragma unroll
-    for (int j = 0; j + 1 < kParts; ++j) k += i >= s.part_end[j];
-    (k == kParts - 1 ? paged.lens_out : dst)[i + s.part_to[k]] = s.w[i];
+    for (int j = 0; j + 1 < P; ++j) k += i >= s.part_end[j];
+    (P == kPagedParts && k == P - 1 ? lens_out : dst)[i + s.part_to[k]] = s.w[i];
   }
 }
 
+// (Packed steps have a kernel of their own: with the paged one's parameters in it three short prompts
+// took 30.4 us for 29.9.)
 template <int N>
-cudaError_t upload(int32_t* dst, const int32_t* const (&src)[kParts], const int (&off)[kParts],
-                   const int (&len)[kParts], int from, int to, const PagedIn& paged, cudaStream_t stream) {
-  Words<N> s;
+__global__ void __launch_bounds__(kUpThreads)
+upload_kernel(int32_t* dst, const __grid_constant__ Words<N, kParts> s) {
+  let_next_start();
+  wait_for_previous();       // (it may be reading the arrays)
+  put_words(dst, dst, s);
+}
+
+template <int N>
+__global__ void __launch_bounds__(kUpThreads)
+upload_paged_kernel(int32_t* dst, const __grid_constant__ PagedIn in, const __grid_constant__ Words<N, kPagedParts> s) {
+  let_next_start();
+  wait_for_previous();
+  if (in.table) {
+    const int first = blockIdx.x * kUpThreads + threadIdx.x, step = gridDim.x * kUpThreads;
+    const long long total = static_cast<long long>(in.num_batch) * in.width;
+    for (long long i = first; i < total; i += step) {
+      const int b = static_cast<int>(i / in.width), j = static_cast<int>(i % in.width);
+      in.table_out[static_cast<long long>(b) * in.pitch_out + j] = in.table[b * in.pitch + j];
+    }
+  }
+  if (blockIdx.x == 0) put_words(dst, in.lens_out, s);
+}
+
+// Words [from, to) of the parts laid end to end.
+template <int N, int P>
+void pack(Words<N, P>& s, const int32_t* const (&src)[kPagedParts], const int (&off)[kPagedParts],
+          const int (&len)[kPagedParts], int from, int to) {
   int at = 0, seen = 0;
-  for (int k = 0; k < kParts; ++k) {              // words [from, to) of the parts laid end to end
+  for (int k = 0; k < P; ++k) {
     const int lo = std::max(from - seen, 0), hi = std::min(to - seen, len[k]);
     if (hi > lo) memcpy(s.w + at, src[k] + lo, sizeof(int32_t) * (hi - lo));
     s.part_to[k] = off[k] + lo - at;
@@ -69,9 +84,21 @@ cudaError_t upload(int32_t* dst, const int32_t* const (&src)[kParts], const int 
     s.part_end[k] = at;
     seen += len[k];
   }
-  const long long entries = paged.table ? static_cast<long long>(paged.num_batch) * paged.width : 0;
+}
+
+template <int N>
+cudaError_t upload(int32_t* dst, const int32_t* const (&src)[kPagedParts], const int (&off)[kPagedParts],
+                   const int (&len)[kPagedParts], int from, int to, const PagedIn& in, cudaStream_t stream) {
+  if (!in.lens) {
+    Words<N, kParts> s;
+    pack(s, src, off, len, from, to);
+    return launch_behind(upload_kernel<N>, 1, kUpThreads, 0, stream, dst, s);
+  }
+  Words<N, kPagedParts> s;
+  pack(s, src, off, len, from, to);
+  const long long entries = in.table ? static_cast<long long>(in.num_batch) * in.width : 0;
   const int blocks = static_cast<int>(std::min<long long>(1 + entries / 2048, kMaxBlocks));
-  return launch_behind(upload_kernel<N>, blocks, kUpThreads, 0, stream, dst, s, paged);
+  return launch_behind(upload_paged_kernel<N>, blocks, kUpThreads, 0, stream, dst, in, s);
 }
 
 }  // namespace
@@ -82,12 +109,13 @@ int upload_meta(const ma_stage_tasks_args* a, uint64_t meta_dev, const PagedIn& 
   if (rc < 0) return rc;
   const ma_stage_meta_args& m = a->meta;
   const int R = m.num_row_tiles, B = m.num_batch;
-  const int off[kParts] = {m.off_cu_q, m.off_cu_k, m.off_batch_idx, m.off_m_block, m.off_order, m.off_actv,
+  const int off[kPagedParts] = {m.off_cu_q, m.off_cu_k, m.off_batch_idx, m.off_m_block, m.off_order, m.off_actv,
                            a->off_tasks, 0};
-  const int len[kParts] = {B + 1, B + 1, R, R, R, MA_NUM_ACTV, 4 + kTaskWords * m.staging[a->off_tasks],
-                           paged.table ? B : 0};
-  const int32_t* src[kParts];
-  for (int k = 0; k < kParts; ++k) src[k] = k == kParts - 1 ? paged.lens : m.staging + off[k];
+  const int len[kPagedParts] = {B + 1, B + 1, R, R, R, MA_NUM_ACTV, 4 + kTaskWords * m.staging[a->off_tasks],
+                           paged.lens ? B : 0};
+  const int32_t* src[kPagedParts];
+  for (int k = 0; k < kParts; ++k) src[k] = m.staging + off[k];
+  src[kParts] = paged.lens;
   int total = 0;
   for (int n : len) total += n;
   int32_t* dst = reinterpret_cast<int32_t*>(meta_dev);
