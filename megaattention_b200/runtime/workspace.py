@@ -430,6 +430,7 @@ class FusedFaOprojArWorkspace:
         assert W_o.shape[0] == self.K_local and W_o.shape[1] >= self.hidden and W_o.shape[1] % 64 == 0
         want = (128, self.H_kv, self.D) if self.paged else (self.H_kv, self.D)
         assert K.shape[1:] == want == V.shape[1:]
+        assert V.shape[0] >= K.shape[0], "V has fewer rows (pages) than K"    # read by K's count
 
     def can_step(self, *tables):
         """Whether ``step`` takes a call made here and now: one rank, on the stream and device that

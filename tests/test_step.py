@@ -159,6 +159,26 @@ def test_refusals_leave_the_last_step_in_place():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("paged", [False, True])
+def test_values_with_fewer_rows_than_keys_are_refused(paged, native):
+    """K's count is what both are read by; more values than keys are left alone as before."""
+    ws, layer, args, kwargs, want, pages = _layer("chunk_multiseq", paged)
+    if not native:
+        ws.can_step = lambda *t: False
+    layer(*args, **kwargs)
+    ws.check_status()
+    ref = layer.output().clone()
+    q, k, v, cu = args
+    with pytest.raises(AssertionError):
+        layer(q, k, v[:-1].clone(), cu, **kwargs)
+    more = torch.cat((v, torch.full_like(v[:1], 7.0)))
+    layer(q, k, more, cu, **kwargs)
+    ws.check_status()
+    assert torch.equal(layer.output(), ref)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("paged", [False, True])
 def test_launch_flags_that_are_refused_leave_the_plans_inputs(paged):
     """A workspace on its own buffers keeps them, and one that reads a caller's keeps those."""
