@@ -117,6 +117,20 @@ __device__ __forceinline__ bool wait_bar(const Env& e, uint32_t bar, uint32_t pa
   return true;
 }
 
+// A compute warp's look at the next task.  An abort does not end it, the scheduler's end does (all of
+// whose waits have limits): the four warps of a warpgroup look one by one, their epilogues have
+// barriers that wait for all of them without a limit, and a task that is posted after the abort has to
+// be found by all of them or by none.
+__device__ __noinline__ bool wait_task_or_end(uint32_t bar, uint32_t parity, const volatile int* posted_all) {
+  while (!mbar_try_wait_for(bar, parity, kWaitSleepNs)) {
+    if (*posted_all) {
+      __threadfence_block();               // (the flag was set behind the last post)
+      return mbar_test_wait(bar, parity);
+    }
+  }
+  return true;
+}
+
 // ---------------------------------------------------------------- scheduler (thread 0)
 // One rank, or partial sums only: what a task leaves is read by nobody in this launch.
 __device__ __forceinline__ bool without_ar(const KParams& p) { return p.tp == 1 || (p.flags & 16u); }
@@ -644,6 +658,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
   __shared__ __align__(128) int s_abort_line[32];
   __shared__ __align__(128) int s_desc[2][T_WORDS];
   int& s_abort = s_abort_line[0];
+  int& s_posted_all = s_abort_line[1];       // the scheduler has left: no task will follow
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -652,7 +667,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
   Env env{&p, &s_abort};
 
   if (tid == 0) {
-    s_abort = 0;
+    s_abort = s_posted_all = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars.task_full[i]), 1);
       mbar_init(smem_u32(&bars.task_empty[i]), 11);
@@ -729,6 +744,12 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 // times, and what follows has instructions that wait for all of them.
 #define MA_NEXT_TASK_WARP(desc_ptr, mode_var) \
   MA_NEXT_TASK_IF(__all_sync(0xffffffffu, MA_TASK_FULL), desc_ptr, mode_var)
+// A compute warpgroup finds the task with all of its warps or with none (wait_task_or_end).
+#define MA_TASK_FULL_OR_END                                                                \
+  (mbar_test_wait(smem_u32(&bars.task_full[slot_k]), (tf_par >> slot_k) & 1u) ||          \
+   wait_task_or_end(smem_u32(&bars.task_full[slot_k]), (tf_par >> slot_k) & 1u, &s_posted_all))
+#define MA_NEXT_TASK_WARPGROUP(desc_ptr, mode_var) \
+  MA_NEXT_TASK_IF(__all_sync(0xffffffffu, MA_TASK_FULL_OR_END), desc_ptr, mode_var)
 #define MA_DRAIN_IF_SWITCH(mode_var)                                                       \
   if (is_tile_mode(mode_var) && is_tile_mode(prev_mode) && mode_var != prev_mode)          \
     wait_bar(env, smem_u32(&bars.task_empty[prev_k]), ((arrived >> prev_k) & 1u) ^ 1u, 0x110 + warp);
@@ -820,7 +841,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
       };
       while (true) {
         if (occupied[k]) {
-          wait_bar(env, smem_u32(&bars.task_empty[k]), te_par[k], 0x120 + k);
+          // (who gives up here posts nothing more: the slot may still be looked at)
+          if (!wait_bar(env, smem_u32(&bars.task_empty[k]), te_par[k], 0x120 + k)) break;
           te_par[k] ^= 1u;
           occupied[k] = false;
           publish(k);
@@ -954,6 +976,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
         ld_skip[k] = !ld_pending[k];
         k ^= 1;
       }
+      __threadfence_block();
+      *const_cast<volatile int*>(&s_posted_all) = 1;
     } else if (warp == 0 && lane == 0) {
       // ==================================================================== TMA producer
       uint32_t kv_slot = 0, kv_ph = 0, op_st = 0, op_ph = 0, q_uses = 0;
@@ -1231,7 +1255,7 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     uint32_t s_par = 0, o_par = 0, acc_par = 0;
     while (true) {
-      MA_NEXT_TASK_WARP(d, mode)
+      MA_NEXT_TASK_WARPGROUP(d, mode)
       if (mode == MODE_FA && wg < d[TF_NT]) {
         // -------------------------------------------- softmax + epilogue of tile `wg`
         const int valid_m = d[TF_VALID];
@@ -1507,6 +1531,8 @@ fused_prefill_kernel(const __grid_constant__ CUtensorMap tmQ,
 #undef MA_NEXT_TASK_IF
 #undef MA_NEXT_TASK
 #undef MA_NEXT_TASK_WARP
+#undef MA_NEXT_TASK_WARPGROUP
+#undef MA_TASK_FULL_OR_END
 #undef MA_DRAIN_IF_SWITCH
 #undef MA_TASK_DONE
 
