@@ -2,6 +2,7 @@
 // metadata/row_desc.py), the attention claim order (runtime/workspace.py: claim_order) and the
 // active counts, written where the caller wants them.  In numpy these took 95 us of a step's
 // host time - more than the whole launch of a small layer; here a few.
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -55,21 +56,31 @@ void arrange(const int32_t* sorted, int n, int prime, int32_t* order) {
 // heads 243 / 152 / 122 / 106 / 93 / 89; 100 and 300 behind 1500 and 2500 81 / 77 / 75 / 69 / 73 / 75;
 // 2000 behind 15871 270 / 179 / 212 / 185; 12 short turns on up to 5217 keys 122 / 95 / 89 / 89 / 97 / 101.
 constexpr int kMinPart = 5;
-constexpr double kTaskCost = 2.0, kPartCost = 1.0, kJoinCost = 0.5, kOprojCost = 0.2, kWorthIt = 0.9;
+constexpr int kTaskCost = 2, kPartCost = 1;
+constexpr double kJoinCost = 0.5, kOprojCost = 0.2, kWorthIt = 0.9;
 
 struct Unit { int32_t tile, split, len; };    // split: as in the task table
+struct Group { int32_t at, n; };              // n tasks of one cost, or n row tiles of one length
 
-// What the launch's attention takes, claimed longest first by `lanes` groups of CTAs (one CTA of
-// a group per task of a row tile).
-double makespan(std::vector<double>& costs, int lanes, std::vector<double>& busy) {
-  std::sort(costs.begin(), costs.end(), std::greater<double>());
-  busy.assign(static_cast<size_t>(lanes), 0.0);     // a heap, the first free lane at its top
-  double most = 0.0;
-  for (double c : costs) {
-    std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
-    busy.back() += c;
-    most = std::max(most, busy.back());
-    std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+// What the launch's attention takes, claimed longest first (costs come in that order) by `lanes`
+// groups of CTAs (one CTA of a group per task of a row tile), or something above `limit` where it takes
+// longer than that.  free_at: lanes by the time they are free at.
+int32_t makespan(const std::vector<Group>& costs, int lanes, double limit, std::vector<int32_t>& free_at) {
+  int64_t sum = 0;
+  for (const Group& c : costs) sum += static_cast<int64_t>(c.at) * c.n;
+  free_at.assign(static_cast<size_t>(sum / lanes) + costs.front().at + 2, 0);
+  free_at[0] = lanes;
+  int32_t now = 0, most = 0;
+  for (const Group& c : costs) {
+    for (int32_t left = c.n; left > 0;) {
+      while (free_at[now] == 0) ++now;
+      const int32_t n = std::min(left, free_at[now]);
+      left -= n;
+      free_at[now] -= n;
+      free_at[now + c.at] += n;
+      most = std::max(most, now + c.at);
+    }
+    if (most > limit) return most;
   }
   return most;
 }
@@ -78,6 +89,10 @@ double makespan(std::vector<double>& costs, int lanes, std::vector<double>& busy
 // parts of that length; false: none is worth it.  A launch ends with its attention, or once all of
 // its work is done, O_proj's too (CTAs without attention have that to do: 4500 tokens of one prompt,
 // 4096 columns, attention alone would be shorter in two parts, the launch is 118 us and 119).
+// The host does this in every call, a paged call's behind its wait (one head, prefixed batches: 31 us when
+// every split was simulated task by task, now 4; 8 heads 8 and 3).  So the splits are taken in the
+// order of what their longest part and their work come to at least, up to the one that cannot be
+// better any more, and row tiles of one length are one thing.
 bool choose_parts(const std::vector<int32_t>& nblk, int H, int num_out, int ctas, int slots,
                   std::vector<int32_t>& parts) {
   const int R = static_cast<int>(nblk.size()), per_tile = (H + 1) / 2;
@@ -86,28 +101,64 @@ bool choose_parts(const std::vector<int32_t>& nblk, int H, int num_out, int ctas
   // (three tasks per CTA fill each other's gaps)
   if (slots < 2 || most < 2 * kMinPart || static_cast<int64_t>(R) * per_tile > 3 * ctas) return false;
   const double oproj = kOprojCost * R * num_out * H / ctas;
-  std::vector<double> costs(R), busy;
-  double sum = 0.0;
-  for (int t = 0; t < R; ++t) sum += costs[t] = nblk[t] + kTaskCost;
-  if (most + kTaskCost <= sum / lanes + oproj) return false;
-  double best = kWorthIt * std::max(makespan(costs, lanes, busy), sum / lanes + oproj);
-  int32_t best_len = 0;
+  int64_t whole = 0;
+  for (int32_t n : nblk) whole += n + kTaskCost;
+  if (most + kTaskCost <= static_cast<double>(whole) / lanes + oproj) return false;
+
+  std::vector<int32_t> sorted(nblk);
+  std::sort(sorted.begin(), sorted.end(), std::greater<int32_t>());
+  std::vector<Group> tiles, costs;              // tiles: longest first
+  std::vector<int32_t> free_at;
+  for (int32_t n : sorted) {
+    if (n == 0) break;                          // (nothing to see: no part at all)
+    if (tiles.empty() || tiles.back().at != n) tiles.push_back({n, 0});
+    ++tiles.back().n;
+  }
+  costs = tiles;
+  for (Group& c : costs) c.at += kTaskCost;
+  const int empty = static_cast<int>(std::count(sorted.begin(), sorted.end(), 0));
+  if (empty) costs.push_back({kTaskCost, empty});
+  const double all = static_cast<double>(whole) / lanes + oproj;
+  double best = kWorthIt * std::max<double>(makespan(costs, lanes, HUGE_VAL, free_at), all);
+
+  whole -= static_cast<int64_t>(kTaskCost) * empty;
+  struct Split { double least, mean; int k; int32_t len; } splits[ma::kMaxParts];
+  int num = 0, best_k = 0;
   for (int k = 2; k <= ma::kMaxParts && most >= k * kMinPart; ++k) {
     const int32_t len = (most + k - 1) / k;
-    costs.clear();
-    int used = 0;
-    sum = 0.0;
-    for (int32_t n : nblk) {
-      const int m = (n + len - 1) / len;
-      if (m > 1) used += m;
-      for (int i = 0; i < m; ++i) {
-        costs.push_back(n * (i + 1) / m - n * i / m + kTaskCost + (m > 1 ? kPartCost : 0.0));
-        sum += costs.back();
+    int64_t used = 0, sum = whole;
+    int32_t longest = 0;
+    for (const Group& t : tiles) {
+      if (t.at <= len) {                        // (this one and the shorter ones stay whole)
+        longest = std::max(longest, t.at + kTaskCost);
+        break;
       }
+      const int32_t m = (t.at + len - 1) / len;
+      used += static_cast<int64_t>(m) * t.n;
+      sum += static_cast<int64_t>((m - 1) * kTaskCost + m * kPartCost) * t.n;
+      longest = std::max(longest, (t.at + m - 1) / m + kTaskCost + kPartCost);
     }
     if (used > slots) break;
-    const double t = std::max(makespan(costs, lanes, busy), sum / lanes + oproj) + k * kJoinCost;
-    if (t < best) { best = t; best_len = len; }
+    const double mean = static_cast<double>(sum) / lanes + oproj;
+    splits[num++] = {std::max<double>(longest, mean) + k * kJoinCost, mean, k, len};
+  }
+  std::sort(splits, splits + num, [](const Split& x, const Split& y) {
+    return x.least < y.least || (x.least == y.least && x.k < y.k);
+  });
+  int32_t best_len = 0;
+  for (int i = 0; i < num && splits[i].least <= best; ++i) {
+    const Split& sp = splits[i];
+    costs.clear();
+    for (const Group& t : tiles) {
+      const int32_t m = (t.at + sp.len - 1) / sp.len, cost = t.at / m + kTaskCost + (m > 1 ? kPartCost : 0);
+      const int32_t longer = t.at % m;
+      if (longer) costs.push_back({cost + 1, longer * t.n});
+      costs.push_back({cost, (m - longer) * t.n});
+    }
+    std::sort(costs.begin(), costs.end(), [](const Group& x, const Group& y) { return x.at > y.at; });
+    const double join = sp.k * kJoinCost;
+    const double t = std::max<double>(makespan(costs, lanes, best - join, free_at), sp.mean) + join;
+    if (t < best || (t == best && best_k && sp.k < best_k)) { best = t; best_k = sp.k; best_len = sp.len; }
   }
   if (best_len == 0) return false;
   for (int t = 0; t < R; ++t) parts[t] = std::max(1, (nblk[t] + best_len - 1) / best_len);

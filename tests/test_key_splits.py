@@ -1,6 +1,8 @@
 """Row tiles whose keys are split into parts (ma_stage_tasks, ma_plan_set_split): what the task table
 says of them, and on the GPU the result against the oracle and against whole tasks."""
 import ctypes as C
+import heapq
+import time
 
 import numpy as np
 import pytest
@@ -12,7 +14,7 @@ from megaattention_b200.runtime import FusedFaOprojArWorkspace
 from oracle.chain_oracle import err_beyond_rounding, full_chain_oracle
 
 
-def _table(q, k, heads, ctas=148, slots=80, room=None, prime=0):
+def _staged(q, k, heads, ctas, slots, room, prime):
     meta = build_row_desc(q, seqlens_k=k)
     R, nb = meta.num_row_tiles, meta.num_batch
     offs = [int(x) for x in np.cumsum([0, nb + 1, nb + 1, R, R, R])]
@@ -23,6 +25,12 @@ def _table(q, k, heads, ctas=148, slots=80, room=None, prime=0):
         meta.cu_seqlens_q.ctypes.data, meta.cu_seqlens_k.ctypes.data, meta.batch_idx.ctypes.data,
         meta.m_block.ctypes.data, buf.ctypes.data, nb, R, 4096, heads, 8, 1, 0, 0, prime, *offs, 0),
         off, room, slots, ctas)
+    return a, buf, meta
+
+
+def _table(q, k, heads, ctas=148, slots=80, room=None, prime=0):
+    a, buf, meta = _staged(q, k, heads, ctas, slots, room, prime)
+    off = a.off_tasks
     assert _cabi.lib.ma_stage_tasks(C.byref(a)) == _cabi.MA_OK and buf[-1] == -9
     n = int(buf[off])
     rows = buf[off + 4:off + 4 + _cabi.TASK_WORDS * n].reshape(n, -1)
@@ -91,6 +99,75 @@ def test_drawn_batches(seed):
     slots = 640 // heads
     rows, nblk = _table(q, k, heads, ctas=int(rng.choice([1, 5, 148])), slots=slots)
     _check(rows, nblk, slots)
+
+
+def _parts(nblk, heads, hidden, ctas, slots):
+    """The model that csrc/meta.cpp chooses by, candidate by candidate and task by task."""
+    lanes, most = max(1, ctas // ((heads + 1) // 2)), max(nblk)
+    whole = [1] * len(nblk)
+    if slots < 2 or most < 10 or len(nblk) * ((heads + 1) // 2) > 3 * ctas:
+        return whole
+    oproj = 0.2 * len(nblk) * -(-hidden // 128) * heads / ctas
+
+    def takes(costs):
+        busy = [0] * lanes
+        for c in sorted(costs, reverse=True):
+            heapq.heapreplace(busy, busy[0] + c)
+        return max(max(busy), sum(costs) / lanes + oproj)
+
+    if most + 2 <= sum(n + 2 for n in nblk) / lanes + oproj:
+        return whole
+    best, parts = 0.9 * takes([n + 2 for n in nblk]), whole
+    for k in range(2, min(16, most // 5) + 1):
+        split = [-(-n // -(-most // k)) for n in nblk]
+        if sum(m for m in split if m > 1) > slots:
+            break
+        t = takes([n * (i + 1) // m - n * i // m + 2 + (m > 1)
+                   for n, m in zip(nblk, split) for i in range(m)]) + 0.5 * k
+        if t < best:
+            best, parts = t, split
+    return parts
+
+
+def _prefixed(seed, most_keys=12000):
+    rng = np.random.RandomState(seed)
+    n = int(np.exp(rng.uniform(0, np.log(24))))
+    q = [int(x) for x in np.exp(rng.uniform(0, np.log(3000), n)).astype(int) + 1]
+    return q, [a + int(rng.uniform(0, most_keys)) for a in q], rng
+
+
+@pytest.mark.parametrize("heads", [1, 2, 3, 8, 16, 64])
+def test_the_parts_are_the_models(heads):
+    split = 0
+    for seed in range(40):
+        q, k, rng = _prefixed(seed, 60000 if seed % 4 == 0 else 12000)
+        ctas, slots = int(rng.choice([1, 7, 148, 148])), int(rng.choice([640 // heads, 640 // heads, 9]))
+        rows, nblk = _table(q, k, heads, ctas=ctas, slots=slots)
+        got = np.bincount(rows[:, 0], minlength=len(nblk)).tolist()
+        assert got == _parts(nblk, heads, 4096, ctas, slots), (seed, q, k, ctas, slots)
+        split += max(got) > 1
+    assert split >= 3
+
+
+def test_the_choice_is_a_small_part_of_a_steps_host_time():
+    """It runs in every call, a paged call's while the GPU waits: with few heads there are many tasks and
+    many lanes to look at.  (One candidate after the other, each with all of its tasks sorted and
+    simulated: 30 times the rest of ma_stage_tasks; now 4.)"""
+    args = []
+    for seed in range(24):
+        q, k, _ = _prefixed(seed)
+        args.append((_staged(q, k, 1, 148, 640, None, 0), _staged(q, k, 1, 148, 0, None, 0)))
+
+    def spent(a):
+        t = []
+        for _ in range(9):
+            t0 = time.perf_counter()
+            _cabi.lib.ma_stage_tasks(C.byref(a))
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    with_parts, without = (sum(spent(a[i][0]) for a in args) for i in (0, 1))
+    assert with_parts < 12 * without, (with_parts, without)
 
 
 def _inputs(q, k, heads, kv, hidden):
