@@ -146,7 +146,9 @@ class FusedFaOprojArWorkspace:
                tp_size=1, rank=0, N_TILE=128, super_group_n_tiles=4, q_per_kv=1,
                max_num_batch=None, max_tot_k=None, dtype=torch.bfloat16, device=None,
                paged=False, page_size=128, max_num_pages=None,
-               max_num_pages_per_seq=None):
+               max_num_pages_per_seq=None, key_splits=True):
+        """``key_splits=False`` leaves out the room for parts of long attention tasks (up to 42 MB,
+        ``parts``): batches of few long sequences then run their row tiles whole."""
         assert dtype == torch.bfloat16 and D == 128 and N_TILE == 128
         assert H_local % q_per_kv == 0
         assert 1 <= super_group_n_tiles <= 4, "a super-group is at most 512 TMEM columns"
@@ -213,7 +215,7 @@ class FusedFaOprojArWorkspace:
         # Slots for parts of row tiles' keys: up to SPLIT_HEADS heads' parts (fp32, 65 KB each),
         # and no more than a row tile can have
         slots = min(SPLIT_HEADS // H_local, MAX_PARTS * max_num_row_tiles)
-        slots = slots if slots >= 2 else 0
+        slots = slots if key_splits and slots >= 2 else 0
         max_tasks = max_num_row_tiles + slots
         sizes = (max_num_batch + 1, max_num_batch + 1, max_num_row_tiles, max_num_row_tiles,
                  max_num_row_tiles, 8, 4 + _cabi.TASK_WORDS * max_tasks)

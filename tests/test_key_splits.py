@@ -234,3 +234,22 @@ def test_paged_lengths_on_the_device_decide(lens):
     assert int(ws.tasks[0]) > meta.num_row_tiles and not ws.part_count.any()
     _, Yp, _ = full_chain_oracle(Q, K, V, W, q, lens)
     assert err_beyond_rounding(ws.output().cpu(), Yp) <= 8e-3
+
+
+@pytest.mark.gpu
+def test_a_workspace_without_room_for_parts():
+    q, k, heads, hidden = [130, 1, 40], [4000, 2049, 300], 8, 384
+    meta = build_row_desc(q, seqlens_k=k)
+    Q, K, V, W = _inputs(q, k, heads, 1, hidden)
+    out = []
+    for room in (True, False):
+        ws = FusedFaOprojArWorkspace.create(None, meta.num_row_tiles, hidden, heads, 128, q_per_kv=heads,
+                                            max_num_batch=len(q), max_tot_k=sum(k), device=torch.device("cuda:0"),
+                                            key_splits=room).compile()
+        ws.set_layer(meta, Q, K, V, W)
+        ws.launch()
+        ws.check_status()
+        assert (int(ws.tasks[0]) > meta.num_row_tiles) == room and bool(ws.parts.numel()) == room
+        out.append(ws.output().cpu())
+    _, Yp, _ = full_chain_oracle(Q, K, V, W, q, k)
+    assert all(err_beyond_rounding(o, Yp) <= 8e-3 for o in out)
