@@ -465,7 +465,8 @@ class FusedFaOprojArWorkspace:
         a.Q, a.K, a.V, a.W_o = Q.data_ptr(), K.data_ptr(), V.data_ptr(), W_o.data_ptr()
         a.tot_q, a.w_width = Q.shape[0], W_o.shape[1]
         prime = self.fa_prime_tiles
-        a.stage.meta.auto_prime, a.stage.meta.prime = int(prime is None), 0 if prime is None else max(-1, int(prime))
+        a.stage.meta.auto_prime = int(prime is None)
+        a.stage.meta.prime = 0 if prime is None else max(-1, min(int(prime), self.max_num_row_tiles))
         if flags is None:
             flags = self.default_flags or 0      # (launch_flags_b200 is 0 on one rank)
         a.launch.flags = int(flags)

@@ -12,7 +12,7 @@ from cases import CASES, make_inputs
 from megaattention_b200 import _cabi
 from megaattention_b200.metadata import build_row_desc
 from megaattention_b200.runtime import FusedFaOprojArWorkspace, FusedPrefillLayer
-from megaattention_b200.runtime.workspace import StepMeta
+from megaattention_b200.runtime.workspace import StepMeta, claim_order
 from oracle.chain_oracle import make_paged_kv
 
 HEADER = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include", "megaattn_b200.h")
@@ -176,6 +176,17 @@ def test_values_with_fewer_rows_than_keys_are_refused(paged, native):
     layer(q, k, more, cu, **kwargs)
     ws.check_status()
     assert torch.equal(layer.output(), ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prime", [-(2 ** 40), -1, 0, 2, 2 ** 31, 2 ** 40])
+def test_a_pinned_claim_order_of_any_size(prime):
+    ws, layer, args, kwargs, want, _ = _layer("chunk_multiseq", False)
+    ws.fa_prime_tiles = prime
+    layer(*args, **kwargs)
+    ws.check_status()
+    assert isinstance(layer.meta, StepMeta)
+    assert ws.fa_order[:want.num_row_tiles].tolist() == claim_order(want, prime).tolist()
 
 
 @pytest.mark.gpu
