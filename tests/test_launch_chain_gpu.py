@@ -4,14 +4,21 @@ import numpy as np
 import pytest
 import torch
 
+from megaattention_b200 import _cabi
 from megaattention_b200.metadata import build_row_desc
 from megaattention_b200.runtime import FusedFaOprojArWorkspace, FusedPrefillLayer, residual_rmsnorm, rope_qk_
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("q", [[64, 200], [128 * 40], [1] * 90])      # the last: several upload launches
-def test_a_chain_of_blocks(q):
+def _upload_launches(ws, meta):
+    """Of the metadata upload: up to 7680 words travel with each (csrc/meta_upload.cu)."""
+    words = 2 * (meta.num_batch + 1) + 3 * meta.num_row_tiles + 6 + 4 + _cabi.TASK_WORDS * int(ws.tasks[0])
+    return -(-words // 7680)
+
+
+@pytest.mark.parametrize("q,uploads", [([64, 200], 1), ([128 * 40], 1), ([1] * 90, 1), ([1] * 700, 2)])
+def test_a_chain_of_blocks(q, uploads):
     H, Hkv, hidden, n = 8, 2, 512, sum(q)
     dev = torch.device("cuda:0")
     g = torch.Generator(device=dev).manual_seed(7)
@@ -46,10 +53,12 @@ def test_a_chain_of_blocks(q):
         got = chain(lambda: None)
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     ws.check_status()
+    assert _upload_launches(ws, meta) == uploads
 
 
-def test_launches_in_a_graph():
-    dev, q = torch.device("cuda:0"), [300, 40]
+@pytest.mark.parametrize("q,uploads", [([300, 40], 1), ([1] * 1300, 3)])
+def test_launches_in_a_graph(q, uploads):
+    dev = torch.device("cuda:0")
     meta = build_row_desc(q)
     s = torch.cuda.Stream()
     with torch.cuda.stream(s):
@@ -72,3 +81,4 @@ def test_launches_in_a_graph():
             s.synchronize()
             assert torch.equal(got, want) and torch.equal(again, want)
         ws.check_status()
+        assert _upload_launches(ws, meta) == uploads
