@@ -6,7 +6,8 @@ namespace ma {
 
 // Control-word indices: same numbering as the reference kernel
 // (src/mega_attention/kernels/sm90/fused_fa_oproj_ar.py:47-67), which host code reads.  (The ready
-// queue's entries are published one by one here, so C_OP_PUBLISH stays 0 and its wait is gone.)
+// queue's entries are published one by one here, so C_OP_PUBLISH stays 0; the done counts decide
+// only where an AllReduce follows.)
 enum : int {
   C_FA_COUNTER = 0, C_FA_DONE = 1, C_OP_RESERVE = 2, C_OP_PUBLISH = 3,
   C_OP_CONSUME = 4, C_OP_DONE = 5, C_AR_DONE = 6, C_AR_CURSOR = 7
@@ -16,8 +17,7 @@ enum : int { MODE_IDLE = 0, MODE_FA = 1, MODE_OPROJ = 2, MODE_AR = 3, MODE_DONE 
 
 // status[0] codes
 enum : uint32_t {
-  ST_OK = 0, ST_TIMEOUT_MBAR = 1, ST_TIMEOUT_PUBLISH = 2, ST_TIMEOUT_GRID = 3,
-  ST_TIMEOUT_NVL = 4, ST_BAD_DESC = 5, ST_TIMEOUT_IDLE = 6
+  ST_OK = 0, ST_TIMEOUT_MBAR = 1, ST_TIMEOUT_NVL = 4, ST_TIMEOUT_IDLE = 6
 };
 
 constexpr int kMaxTp = 8;

@@ -341,12 +341,6 @@ __device__ __forceinline__ uint32_t atom_add_release_gpu(uint32_t* p, uint32_t v
                : "memory");
   return o;
 }
-__device__ __forceinline__ uint32_t atom_add_acqrel_gpu(uint32_t* p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v)
-               : "memory");
-  return o;
-}
 __device__ __forceinline__ int atom_add_release_sys_s32(int* p, int v) {
   int o;
   asm volatile("atom.release.sys.global.add.s32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v)

@@ -221,7 +221,7 @@ void cta_main(World& w, int rank, int cta) {
       const int owner = arg % c.tp, idx = arg / c.tp;
       if (c.tp > 1 && !(rank == c.drop_rank && arg == c.drop_slot))   // injected lost arrival
         w.ranks[owner]->ready_count[idx >> 2].fetch_add(1u << ((idx & 3) * 8), std::memory_order_release);
-      r.ctrl[C_OP_DONE].fetch_add(1, std::memory_order_release);
+      if (c.tp > 1) r.ctrl[C_OP_DONE].fetch_add(1, std::memory_order_release);
     } else {
       r.ar_runs[arg / c.tp].fetch_add(1);
       r.ctrl[C_AR_DONE].fetch_add(1, std::memory_order_release);
