@@ -18,7 +18,8 @@ ships no code for it.  The contract built here:
   descriptors (a few KB) are uploaded;
 * the two KV layouts are two workspaces (``create(paged=...)``); a layer object is tied to
   one of them and refuses the other's arguments, a page size other than 128, a page table
-  that is too narrow for the longest sequence, or a wrong dtype, before anything is queued;
+  that is too narrow for the longest sequence, or a wrong dtype, with the workspace and its plan
+  as they were (a paged call has queued no more than the kernel that reports the lengths);
 * many layers share one workspace (the kernel's exit path leaves the control state clean,
   so there is no host reset between layers);
 * the launch flags and the attention claim order are chosen per step from the batch at hand
