@@ -15,7 +15,7 @@ LIB = os.path.join(HERE, "libmegaattn_b200.so")
 LIB_AUDIT = os.path.join(HERE, "libmegaattn_b200_audit.so")
 SOURCES = ["fused_prefill.cu", "cabi.cu", "noalloc.cu", "residual_rmsnorm.cu", "rope.cu",
            "detile.cu", "meta_upload.cu", "step.cu", "meta.cpp"]
-HEADERS = ["ptx.cuh", "kparams.h", "launch.cuh", os.path.join("..", "..", "include", "megaattn_b200.h")]
+HEADERS = ["ptx.cuh", "kparams.h", "launch.cuh", "paged.cuh", os.path.join("..", "..", "include", "megaattn_b200.h")]
 
 
 def _stale(lib: str = None) -> bool:

@@ -81,17 +81,6 @@ constexpr int kPartMax = 128 * 128, kPartSum = kPartMax + 128;   // a part's O, 
 constexpr int kPartFloats = kPartSum + 128;                      // reference maxima and sums
 constexpr int kMaxParts = 16;
 
-// A paged step's page table (device) and key lengths (host, as they were checked) and where the plan
-// has its own copies of them (lens null: no paged step; table null: lengths only).
-struct PagedIn {
-  const int* table;
-  const int* lens;
-  int* table_out;
-  int* lens_out;
-  long long pitch;
-  int pitch_out, width, num_batch;
-};
-
 constexpr int kThreads = 384;
 constexpr int kSmemDynamic = 65536 + 5 * 32768 + 1024;   // Q x2, K/V ring x5, align slack
 

@@ -19,6 +19,7 @@
 #include "../../include/megaattn_b200.h"
 #include "kparams.h"
 #include "launch.cuh"
+#include "paged.cuh"
 
 namespace ma {
 namespace {
@@ -61,12 +62,10 @@ upload_paged_kernel(int32_t* dst, const __grid_constant__ PagedIn in, const __gr
   let_next_start();
   wait_for_previous();
   if (in.table) {
-    const int first = blockIdx.x * kUpThreads + threadIdx.x, step = gridDim.x * kUpThreads;
-    const long long total = static_cast<long long>(in.num_batch) * in.width;
-    for (long long i = first; i < total; i += step) {
-      const int b = static_cast<int>(i / in.width), j = static_cast<int>(i % in.width);
-      in.table_out[static_cast<long long>(b) * in.pitch_out + j] = in.table[b * in.pitch + j];
-    }
+    for_each_entry(in.num_batch, in.width, blockIdx.x * kUpThreads + threadIdx.x, gridDim.x * kUpThreads,
+                   [&](int b, int j) {
+                     in.table_out[static_cast<long long>(b) * in.pitch_out + j] = in.table[b * in.pitch + j];
+                   });
   }
   if (blockIdx.x == 0) put_words(dst, in.lens_out, s);
 }

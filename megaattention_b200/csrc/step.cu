@@ -18,6 +18,7 @@
 #include "../../include/megaattn_b200.h"
 #include "kparams.h"
 #include "launch.cuh"
+#include "paged.cuh"
 
 namespace ma {
 int plan_encode_inputs(const ma_plan* pl, CUtensorMap* fresh, uint64_t Q, uint64_t K, uint64_t V, uint64_t W_o,
@@ -39,13 +40,11 @@ __global__ void __launch_bounds__(kCollectThreads) collect_kernel(
   const int first = blockIdx.x * kCollectThreads + threadIdx.x, step = gridDim.x * kCollectThreads;
   for (int b = first; b < num_batch; b += step) host[b] = lens[b];
   int32_t lo = 0x7fffffff, hi = -0x7fffffff - 1;
-  const int64_t total = static_cast<int64_t>(num_batch) * width;
-  for (int64_t i = first; i < total; i += step) {
-    const int b = static_cast<int>(i / width), j = static_cast<int>(i % width);
+  for_each_entry(num_batch, width, first, step, [&](int b, int j) {
     const int32_t page = table[b * pitch + j];
     lo = min(lo, page);
     hi = max(hi, page);
-  }
+  });
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
   if ((threadIdx.x & 31) == 0) { lo_s[threadIdx.x >> 5] = lo; hi_s[threadIdx.x >> 5] = hi; }

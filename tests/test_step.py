@@ -44,6 +44,28 @@ def test_the_struct_is_the_headers(tmp_path):
                                      + [C.sizeof(_cabi.StepArgs), _cabi.STEP_BLOCKS])
 
 
+@pytest.mark.parametrize("rows,width,first,step", [
+    (1, 1, 0, 512), (1, 1, 1, 512), (12, 41, 7, 512), (3, 2001, 100, 8192), (1, 40000, 16383, 16384),
+    (3, 1 << 29, 5, (1 << 24) + 1), (2, (1 << 31) - 1, 77, 1 << 25), (5, (1 << 28) + 3, (1 << 25) - 1, 1 << 25)])
+def test_every_entry_of_a_table_is_somebodys(tmp_path, rows, width, first, step):
+    """csrc/paged.cuh on the host: a thread's entries are every step-th of a group of rows, and the groups
+    (of 2^30 entries or a row) cover the table."""
+    (tmp_path / "cuda_runtime.h").write_text(
+        "#include <algorithm>\nusing std::min; using std::max;\n#define __device__\n#define __forceinline__ inline\n")
+    src = tmp_path / "t.cpp"
+    src.write_text('#include <stdio.h>\n#include "%s"\nint main() { ma::for_each_entry(%d, %d, %du, %du, '
+                   '[](int b, int j) { printf("%%d %%d\\n", b, j); }); }\n'
+                   % (os.path.join(os.path.dirname(HEADER), "..", "megaattention_b200", "csrc", "paged.cuh"),
+                      rows, width, first, step))
+    subprocess.run(["g++", "-std=c++17", "-I", str(tmp_path), "-o", str(tmp_path / "t"), str(src)], check=True)
+    got = [tuple(map(int, x.split())) for x in subprocess.run(
+        [str(tmp_path / "t")], check=True, capture_output=True, text=True).stdout.splitlines()]
+    group = max(1, (1 << 30) // width)
+    want = [(b0 + i // width, i % width) for b0 in range(0, rows, group)
+            for i in range(first, min(group, rows - b0) * width, step)]
+    assert got == want
+
+
 @pytest.mark.parametrize("q,k", [([3, 200, 128], [3, 900, 128]), ([1], [1])])
 def test_the_schedule_is_made_when_looked_at(q, k):
     want = build_row_desc(q, seqlens_k=k)
