@@ -175,7 +175,8 @@ int ma_plan_set_tasks(ma_plan* plan, uint64_t tasks);
 
 /* Gives the plan room for parts of an attention task's keys (device addresses; 0, 0: none, and a
  * row tile that the task table splits is then one task all the same): parts, 16-byte aligned,
- * float[slots * H_local * MA_PART_FLOATS], and counts u32[slots * H_local], zero at first.  slots as
+ * float[slots * H_local * MA_PART_FLOATS], and counts u32[slots * H_local], zero at first (and, like the
+ * control buffers, again after a launch that gave up).  slots as
  * in ma_stage_tasks_args; the plan's launches must not overlap with others that use the same room. */
 #define MA_PART_FLOATS (128 * 128 + 2 * 128)
 int ma_plan_set_split(ma_plan* plan, uint64_t parts, uint64_t counts);
